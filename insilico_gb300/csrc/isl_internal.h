@@ -103,6 +103,30 @@ struct CGScal {
     int bad;
     int fault;   // persistent CG: a grid barrier timed out
     unsigned int ticket1, ticket2;
+    // two-level solve: its reliable updates are decided on the device
+    double rzloc;             // r.z without the coarse term
+    double rr_true, rr_last;  // FP64 residuals of the last two reliable updates
+    double rr_best;           // the smallest so far
+    double drop;
+    int max_iter;
+    int stall;   // reliable updates in a row without progress
+    int fin;     // 1 converged, 2 iteration limit, 3 breakdown or stagnation
+    int rst;     // a restart from the FP64 residual is due
+    int fresh;   // ... with new directions
+};
+
+// two-level preconditioner (isl_coarse.cu): aggregates of the current pattern
+// and their matrices for the current assembly
+struct CzPlan {
+    bool ok = false;
+    int64_t serial = -1, num_serial = -1, nrow = 0;
+    int nc = 0, m = 0;        // components per row (3: node blocks), modes per aggregate
+    int nagg = 0, nd = 0, ndp = 0;
+    DBuf<float4> lnode, yrow;
+    DBuf<int32_t> sofs;
+    DBuf<int> amax;
+    DBuf<unsigned long long> acc;
+    DBuf<float> dsub, dagg, scale, rc, a, ainv, panel;
 };
 
 }  // namespace isl
@@ -291,6 +315,11 @@ struct isl_ctx {
     isl::DBuf<isl::CGScal> dscal;
     isl::CGScal* hscal = nullptr;  // pinned host mirror
     int spmv_lpr64 = 0, spmv_lpr32 = 0;  // autotuned lanes per row (FP32: 100 + U = sliced-ELL, U slots in flight)
+    isl::CzPlan cz;              // two-level preconditioner of the mixed solve
+    bool use_coarse = true;      // ISL_OPT_TWO_LEVEL
+    cudaGraphExec_t cz_exec = nullptr;   // captured iterations of the two-level solve
+    std::vector<uint64_t> cz_key;        // what the capture depends on
+    cudaEvent_t cz_ev[2] = {nullptr, nullptr};
     int spmv32_forced = 0;               // FP32 SpMV kind set through ISL_OPT_SPMV32_KIND (0: autotune)
 
     // timing

@@ -30,6 +30,7 @@
 
 #include <cooperative_groups.h>
 
+#include "isl_coarse.h"
 #include "isl_internal.h"
 #include "isl_device.cuh"
 
@@ -1654,6 +1655,85 @@ __global__ void __launch_bounds__(BS, MINB) k_bspmv_dir(int nbr, int nslice, con
     }
 }
 
+// The folded product for few slices: one CTA per slice, its eight warps take
+// the slots in turn (at most four each for 27 blocks a row, all their loads
+// in flight at once), and the warps' partial rows are added in warp order
+// through shared memory.  A warp per slice leaves most SMs idle below a few
+// hundred slices and walks its slots one batch after the other.  Bound by
+// latency: at 9,261 nodes the iteration took 30.1 us with a warp per slice,
+// 25.8 us with this product.
+template <typename TC>
+__global__ void __launch_bounds__(BS) k_bspmv_dir_split(int nbr, int nslice, const int* __restrict__ soff,
+                                                        const int* __restrict__ swid, const TC* __restrict__ scol,
+                                                        const float* __restrict__ sv, const float* __restrict__ z,
+                                                        float* pa, float* pb, float* __restrict__ q, CGScal* S,
+                                                        double* part) {
+    if (S->done) return;
+    constexpr int U = 4, NWP = BS / 32;
+    __shared__ double sh[32];
+    __shared__ float acc[NWP][3][32];
+    const bool odd = S->iters & 1;
+    const float beta = (float)S->beta;
+    const float* __restrict__ pold = odd ? pb : pa;
+    float* __restrict__ pnew = odd ? pa : pb;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float loc = 0.f;
+    for (int s = blockIdx.x; s < nslice; s += gridDim.x) {
+        const int i = s * 32 + lane;
+        const int o = soff[s], wid = swid[s];
+        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+        for (int k = w; k < wid; k += U * NWP) {
+            int j[U];
+            float v[U][9];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int kk = k + u * NWP;
+                if (kk < wid) {
+                    j[u] = __ldg(scol + o + kk * 32 + lane) + (sizeof(TC) == 2 ? i : 0);
+                    const float* vp = sv + (size_t)((o >> 5) + kk) * 288 + lane;
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) v[u][e] = __ldg(vp + 32 * e);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (k + u * NWP < wid) {
+                    const size_t b = 3 * (size_t)j[u];
+                    const float x0 = fmaf(beta, __ldg(pold + b), __ldg(z + b));
+                    const float x1 = fmaf(beta, __ldg(pold + b + 1), __ldg(z + b + 1));
+                    const float x2 = fmaf(beta, __ldg(pold + b + 2), __ldg(z + b + 2));
+                    a0 += v[u][0] * x0 + v[u][1] * x1 + v[u][2] * x2;
+                    a1 += v[u][3] * x0 + v[u][4] * x1 + v[u][5] * x2;
+                    a2 += v[u][6] * x0 + v[u][7] * x1 + v[u][8] * x2;
+                }
+            }
+        }
+        acc[w][0][lane] = a0; acc[w][1][lane] = a1; acc[w][2][lane] = a2;
+        __syncthreads();
+        if (w < 3 && i < nbr) {  // warp c: component c of the slice's rows
+            float t = 0.f;
+#pragma unroll
+            for (int k = 0; k < NWP; ++k) t += acc[k][w][lane];
+            const size_t b = 3 * (size_t)i + w;
+            const float p = fmaf(beta, __ldg(pold + b), __ldg(z + b));
+            pnew[b] = p;
+            q[b] = t;
+            loc += p * t;
+        }
+        __syncthreads();
+    }
+    const double bsum = block_sum_f(loc, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = bsum;
+    if (last_block(&S->ticket1)) {
+        const double tot = reduce_parts_blk<BS>(part, gridDim.x, 1, 0, sh);
+        if (threadIdx.x == 0) {
+            S->pAp = tot;
+            S->alpha = S->absNew / tot;
+            S->ticket1 = 0;
+        }
+    }
+}
+
 // q = A p on the block-row CSR copy: LPB lanes per block row
 template <int LPB>
 __global__ void __launch_bounds__(BS, 8) k_brow_spmv(int nbr, const int* __restrict__ bptr, const int* __restrict__ bcol,
@@ -2080,6 +2160,10 @@ static void launch_bspmv_dir_t(int kind, cudaStream_t st, isl_ctx* c, const TC* 
                                float* pb, float* q, CGScal* S, double* part) {
     const int nbr = (int)c->nbr, ns = (int)c->nslice;
     const unsigned g = sell_grid(c);
+    if (kind == 9) {
+        k_bspmv_dir_split<TC><<<(unsigned)std::min<long long>(c->nslice, 4LL * c->sm_count), BS, 0, st>>>(nbr, ns, c->dsoff.p, c->dswid.p, scol, c->dsval.p, z, pa, pb, q, S, part);
+        return;
+    }
     switch (kind) {
         case 5: k_bspmv_dir<2, 4, TC><<<std::min(g, 4u * c->sm_count), BS, 0, st>>>(nbr, ns, c->dsoff.p, c->dswid.p, scol, c->dsval.p, z, pa, pb, q, S, part); break;
         case 6: k_bspmv_dir<4, 3, TC><<<std::min(g, 3u * c->sm_count), BS, 0, st>>>(nbr, ns, c->dsoff.p, c->dswid.p, scol, c->dsval.p, z, pa, pb, q, S, part); break;
@@ -2688,6 +2772,232 @@ int time_bspmv(isl_ctx* c, int nrep, double* ms) {
     return ISL_OK;
 }
 
+// ===========================================================================
+// Two-level solve: the mixed CG with the preconditioner of isl_coarse.cu, for
+// node blocks and for scalar systems.  An iteration is the update with the
+// local part of the preconditioner, the coarse correction, and the product
+// (with the direction update folded in for node blocks, in its own launch
+// otherwise).  The reliable updates are decided on the device: every CZ_CHUNK
+// iterations the captured graph holds one update's kernels, which return at
+// once unless the iteration has stopped for one.  The host only watches for
+// the end, one graph launch behind the device.  Eight iterations per update
+// slot: a shorter chunk runs the (mostly idle) update kernels more often, a
+// longer one idles for longer after a stop.
+constexpr int CZ_CHUNK = 8;
+
+__global__ void __launch_bounds__(BS) k_rl_fold(int n, const int* __restrict__ aeq, float* __restrict__ x32,
+                                                double* __restrict__ x64, const CGScal* S) {
+    if (!S->done || S->fin) return;
+    for (int a = blockIdx.x * BS + threadIdx.x; a < n; a += gridDim.x * BS) {
+        const int e = aeq ? aeq[a] : a;
+        if (e >= 0) x64[e] += (double)x32[a];
+        x32[a] = 0.0f;
+    }
+}
+
+// r64 = b - A64 x64; the last block decides: converged, iteration limit,
+// breakdown, or a restart (with new directions when the true residual has not
+// dropped since the previous reliable update)
+template <int LPR>
+__global__ void __launch_bounds__(BS) k_rl_residual(int n, const int* __restrict__ rowptr, const int* __restrict__ colind,
+                                                    const double* __restrict__ val, const double* __restrict__ x,
+                                                    const double* __restrict__ b, double* __restrict__ r, CGScal* S,
+                                                    double* part) {
+    if (!S->done || S->fin) return;
+    __shared__ double sh[32];
+    const int lane = threadIdx.x % LPR;
+    const int grp = (blockIdx.x * BS + threadIdx.x) / LPR, ngrp = gridDim.x * BS / LPR;
+    const int wgrp = grp - grp % (32 / LPR);
+    double loc = 0.0;
+    for (int base = wgrp; base < n; base += ngrp) {
+        const int row = base + (grp - wgrp);
+        const bool act = row < n;
+        const double ax = row_dot<double, double, LPR>(row, act, rowptr, colind, val, x, lane);
+        if (act && lane == 0) {
+            const double ri = b[row] - ax;
+            r[row] = ri;
+            loc += ri * ri;
+        }
+    }
+    const double bs = block_sum(loc, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = bs;
+    if (!last_block(&S->ticket1)) return;
+    const double tot = reduce_parts_blk<BS>(part, gridDim.x, 1, 0, sh);
+    if (threadIdx.x != 0) return;
+    S->ticket1 = 0;
+    if (S->bad || !(tot == tot)) { S->bad = 1; S->fin = 3; return; }
+    S->rr_true = tot;
+    if (tot <= S->threshold) { S->fin = 1; return; }
+    if (S->iters >= S->max_iter) { S->fin = 2; return; }
+    // four updates in a row that did not halve the best residual: near the
+    // accuracy FP64 residuals can reach, the one-level iteration may still
+    // get below a tolerance that this one circles
+    S->stall = tot > 0.25 * S->rr_best ? S->stall + 1 : 0;
+    S->rr_best = fmin(S->rr_best, tot);
+    if (S->stall >= 4) { S->fin = 3; return; }
+    S->fresh = S->rr_last > 0.0 && tot >= S->rr_last;
+    S->rr_last = tot;
+    S->rrtrig = S->drop * tot;
+    S->rst = 1;
+}
+
+// without the FP64 matrix the iterated residual decides
+__global__ void k_rl_iterated(CGScal* S) {
+    if (!S->done || S->fin) return;
+    S->rr_true = S->rr;
+    S->fin = S->bad ? 3 : (S->done == 1 ? 1 : 2);
+}
+
+static void launch_rl_residual(isl_ctx* c, unsigned grid, cudaStream_t st, const double* x, double* r, CGScal* S) {
+    const int n = (int)c->neq;
+    const int *rp = c->drowptr.p, *ci = c->dcolind.p;
+    const double *v = c->dval64.p, *b = c->drhs.p;
+    double* part = c->dpart.p;
+    switch (c->spmv_lpr64) {
+        case 2: k_rl_residual<2><<<grid, BS, 0, st>>>(n, rp, ci, v, x, b, r, S, part); break;
+        case 4: k_rl_residual<4><<<grid, BS, 0, st>>>(n, rp, ci, v, x, b, r, S, part); break;
+        case 8: k_rl_residual<8><<<grid, BS, 0, st>>>(n, rp, ci, v, x, b, r, S, part); break;
+        case 16: k_rl_residual<16><<<grid, BS, 0, st>>>(n, rp, ci, v, x, b, r, S, part); break;
+        default: k_rl_residual<32><<<grid, BS, 0, st>>>(n, rp, ci, v, x, b, r, S, part); break;
+    }
+}
+
+// *ran = false: no usable coarse space, or the iteration broke down or
+// stagnated; the caller solves one-level
+static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* notconv,
+                           bool* ran) {
+    *ran = false;
+    cudaStream_t st = c->stream;
+    const size_t n = (size_t)c->neq;
+    const int64_t rows = nc == 3 ? c->nbr : c->neq;
+    const size_t na = (size_t)nc * rows;
+    int rc = coarse_plan(c, nc, rows);
+    if (rc != ISL_OK || !c->cz.ok) return rc;
+    rc = nc == 3 ? ensure_bsr(c) : ensure_ssell(c);
+    if (rc != ISL_OK) return rc;
+    const bool exact64 = c->have64;
+    CGScal* S = c->dscal.p;
+    double* W = c->w64.p;
+    double *x64 = W, *r64 = W + n;
+    float* V = c->w32.p;
+    float *x32 = V, *r32 = V + na, *p32 = V + 2 * na, *q32 = V + 3 * na;
+    float *z32 = nc == 3 ? V + 4 * na : V + 5 * na, *p32b = nc == 3 ? V + 5 * na : nullptr;
+    float* d32 = nc == 3 ? c->dbinv.p : V + 4 * na;
+    const unsigned grid = vec_grid(c);
+    int kind;
+    if (nc == 3) {
+        if (!c->bspmv_lpb && c->nslot <= c->nblk + c->nblk / 10) {
+            c->bspmv_lpb = 7;  // little padding: the batched sliced-ELL product, the autotune's first choice, without timing it
+        } else if (!c->bspmv_lpb) {
+            ISL_CHECK_CUDA(c, cudaMemsetAsync(p32, 0, na * 4, st));
+            c->bspmv_lpb = autotune_lpb(c, p32, q32, S, c->dpart.p);
+        }
+        kind = c->nbr < 8000 ? 7 : c->bspmv_lpb;
+        // below about a thousand slices the split product is the faster one
+        // (solve at 9,261 nodes 3.48 ms against 4.06, at 31,744 4.45 against
+        // 5.21; at 270,400 nodes 21.4 against 18.5)
+        if (c->fuse_dir && c->nslice <= 1024) kind = 9;
+    } else {
+        if (!c->spmv_lpr32) {
+            ISL_CHECK_CUDA(c, cudaMemsetAsync(p32, 0, na * 4, st));
+            c->spmv_lpr32 = autotune_spmv32(c, p32, q32, S, c->dpart.p);
+        }
+        kind = c->spmv_lpr32;
+        k_dinv<float, float><<<grid, BS, 0, st>>>((int)n, c->ddiag.p, c->dval32.p, d32);
+        c->launches += 1;
+    }
+    if (exact64 && !c->spmv_lpr64)
+        c->spmv_lpr64 = autotune_lpr<double, double>(c, c->dval64.p, c->drhs.p, W + 3 * n, S, c->dpart.p);
+    CzMat A = {c->dsoff.p, c->dswid.p, c->drowptr.p, nc == 3 ? c->dscol.p : c->dcolind.p, nc == 3 ? c->dsval.p : c->dval32.p};
+    rc = coarse_numeric(c, A);
+    if (rc != ISL_OK) return rc;
+    const bool fused = nc == 3 && c->fuse_dir && (kind == 9 || bspmv_dir_kind(kind));
+    CzIter a = {};
+    coarse_args(c, a);
+    a.x = x32; a.r = r32; a.z = z32;
+    a.p1 = p32; a.p2 = fused ? p32b : nullptr; a.pz = p32;
+    a.q = q32; a.dinv = d32;
+    a.b64 = c->drhs.p;
+    a.aeq = nc == 3 && c->bpad ? c->dbaeq.p : nullptr;
+    a.S = S; a.part = c->dpart.p;
+    a.tol = tol; a.drop = exact64 ? c->ru_drop2 : 0.0;
+    a.max_iter = (int)std::min<int64_t>(max_iter, INT32_MAX - 1);
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(S, 0, 2 * sizeof(CGScal), st));
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(x64, 0, n * 8, st));
+    launch_coarse(c, st, a, CZ_INIT);
+    ISL_CHECK_CUDA(c, cudaGetLastError());
+    c->launches += 2;
+    const int per_chunk = CZ_CHUNK * (fused ? 3 : 4) + (exact64 ? 4 : 2);
+    // the captured iterations are kept while every argument stays the same
+    // (the tolerance and the limits travel in the scalar record)
+    a.b64 = r64;
+    a.tol = a.drop = 0.0;
+    a.max_iter = 0;
+    auto u = [](const void* p) { return (uint64_t)(uintptr_t)p; };
+    std::vector<uint64_t> key = {(uint64_t)nc, (uint64_t)kind, (uint64_t)fused, (uint64_t)exact64, (uint64_t)rows, (uint64_t)n,
+                                 (uint64_t)c->cz.nagg, (uint64_t)c->cz.ndp, (uint64_t)c->spmv_lpr64,
+                                 (uint64_t)(c->use_scol16 && (nc == 3 ? c->scol16 : c->ss16)), (uint64_t)c->pattern_serial,
+                                 u(a.lnode), u(a.sofs), u(a.dsub), u(a.ainv), u(a.rc), u(V), u(W), u(a.dinv), u(a.aeq), u(S),
+                                 u(a.part), u(c->dsval.p), u(c->dbval.p), u(c->dss_val.p), u(c->dval32.p), u(c->dval64.p),
+                                 u(c->drhs.p), u(c->drowptr.p), u(c->dcolind.p), u(c->dscol.p), u(c->dscol16.p)};
+    if (!c->cz_exec || key != c->cz_key) {
+        if (c->cz_exec) { cudaGraphExecDestroy(c->cz_exec); c->cz_exec = nullptr; }
+        cudaGraph_t graph;
+        ISL_CHECK_CUDA(c, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        for (int k = 0; k < CZ_CHUNK; ++k) {
+            if (fused) {
+                launch_bspmv_dir(kind, st, c, z32, p32, p32b, q32, S, c->dpart.p);
+            } else {
+                launch_coarse_dir(c, st, (int)na, z32, p32, S);
+                if (nc == 3) launch_bspmv(kind, grid, st, c, p32, q32, S, c->dpart.p);
+                else launch_spmv32(c, kind, grid, st, p32, q32, S, c->dpart.p);
+            }
+            launch_coarse(c, st, a, CZ_UPDATE);
+        }
+        k_rl_fold<<<grid, BS, 0, st>>>((int)na, a.aeq, x32, x64, S);
+        if (exact64) {
+            launch_rl_residual(c, grid, st, x64, r64, S);
+            launch_coarse(c, st, a, CZ_RESTART);
+        } else {
+            k_rl_iterated<<<1, 1, 0, st>>>(S);
+        }
+        ISL_CHECK_CUDA(c, cudaStreamEndCapture(st, &graph));
+        cudaError_t e = cudaGraphInstantiate(&c->cz_exec, graph, 0);
+        cudaGraphDestroy(graph);
+        if (e != cudaSuccess) c->cz_exec = nullptr;
+        ISL_CHECK_CUDA(c, e);
+        c->cz_key = key;
+    }
+    for (auto& ev : c->cz_ev)
+        if (!ev) ISL_CHECK_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    // one graph in flight beyond the one whose record is being read
+    const int64_t max_replays = (int64_t)std::min<int64_t>(max_iter, INT32_MAX - 1) + 64;
+    int64_t k = 0;
+    for (;; ++k) {
+        if (k > max_replays) ISL_FAIL(c, ISL_ERR_TIMEOUT, "mixed CG made no progress");
+        ISL_CHECK_CUDA(c, cudaGraphLaunch(c->cz_exec, st));
+        ISL_CHECK_CUDA(c, cudaMemcpyAsync(c->hscal + (k & 1), S, sizeof(CGScal), cudaMemcpyDeviceToHost, st));
+        ISL_CHECK_CUDA(c, cudaEventRecord(c->cz_ev[k & 1], st));
+        c->launches += per_chunk;
+        if (k == 0) continue;
+        ISL_CHECK_CUDA(c, cudaEventSynchronize(c->cz_ev[(k - 1) & 1]));
+        if (c->hscal[(k - 1) & 1].fin) break;
+    }
+    const CGScal h = c->hscal[(k - 1) & 1];
+    if (h.fin == 3) return ISL_OK;  // *ran stays false
+    *ran = true;
+    *iters = h.iters;
+    *rel = h.rhsNorm2 > 0 ? std::sqrt(h.rr_true / h.rhsNorm2) : 0.0;
+    *notconv = h.fin == 2;
+    k_copy64<<<grid, BS, 0, st>>>((int)n, x64, c->dsol.p);
+    c->launches += 1;
+    return ISL_OK;
+}
+
+// Sizes from which the two-level solve takes over from the one-launch kernels
+// of small systems, whose iterations cost less than three launches.
+constexpr int64_t CZ_MIN_NODES = 1280, CZ_MIN_EQ = 2048;
+
 int solve_device(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t* iters, double* relres) {
     int rc = ensure_work(c);
     if (rc != ISL_OK) return rc;
@@ -2709,8 +3019,14 @@ int solve_device(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t* 
         if (rc == ISL_ERR_NOT_CONVERGED) rc = ISL_OK;
     } else if (method == ISL_SOLVE_BICGSTAB) rc = solve_bicgstab(c, tol, max_iter, &it, &rel, &nc);
     else if (method == ISL_SOLVE_CG_FP64) rc = solve_fp64(c, tol, max_iter, &it, &rel, &nc);
-    else if (c->blocked && c->use_block && (c->have64 || c->have32)) rc = solve_mixed_b3(c, tol, max_iter, &it, &rel, &nc);
-    else rc = solve_mixed(c, tol, max_iter, &it, &rel, &nc);
+    else {
+        const bool b3 = c->blocked && c->use_block && (c->have64 || c->have32);
+        bool ran = false;
+        if (c->use_coarse && c->use_persist != 2 && (b3 ? c->nbr >= CZ_MIN_NODES : (int64_t)c->neq >= CZ_MIN_EQ))
+            rc = solve_two_level(c, b3 ? 3 : 1, tol, max_iter, &it, &rel, &nc, &ran);
+        if (rc == ISL_OK && !ran)
+            rc = b3 ? solve_mixed_b3(c, tol, max_iter, &it, &rel, &nc) : solve_mixed(c, tol, max_iter, &it, &rel, &nc);
+    }
     if (rc != ISL_OK) return rc;
     ISL_CHECK_CUDA(c, cudaGetLastError());
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
