@@ -333,8 +333,10 @@ int isl_timings(isl_ctx* ctx, double* ms /* [ISL_NTIMERS] */, int64_t* counts /*
  * kernels), 1 (default) for small systems, where launch latency dominates:
  * a scalar system of at most 65,536 equations is solved whole, FP64 reliable
  * updates included, by one thread-block cluster; a node-blocked system of at
- * most 32,768 nodes runs its iterations in a persistent cooperative kernel.
- * 2: the persistent block kernel at every size.  ISL_OPT_BARRIER_TEST (test
+ * most 32,768 nodes runs its iterations in a persistent cooperative kernel;
+ * with the two-level preconditioner (ISL_OPT_TWO_LEVEL) the smallest of these
+ * run in one cluster and the others in one cooperative launch over every SM.
+ * 2: the persistent one-level block kernel at every size.  ISL_OPT_BARRIER_TEST (test
  * hook, write-only, one-shot): the next persistent launch starts with its grid
  * barrier armed so that it cannot complete; its bounded wait runs out and the
  * solve returns ISL_ERR_TIMEOUT with the context still usable.
@@ -359,13 +361,16 @@ enum { ISL_OPT_BLOCK_SOLVER = 0, ISL_OPT_BLOCKED = 1, ISL_OPT_NBLOCKS = 2, ISL_O
        ISL_OPT_BICGSTAB_KIND = 9, ISL_OPT_BATCHED_SOLVE = 10, ISL_OPT_DIRECT_BLOCKS = 11, ISL_OPT_TUNE_RUNS = 12,
        ISL_OPT_ELEM_VARIANT = 13, ISL_OPT_FOLD_DIRECTION = 14, ISL_OPT_BLOCK_UPDATE = 15,
        ISL_OPT_SHORT_COLUMNS = 16, ISL_OPT_RELIABLE_DROP = 17, ISL_OPT_SHARED_GEOMETRY = 18, ISL_OPT_TWO_LEVEL = 19 };
-/* ISL_OPT_TWO_LEVEL (default 1): the mixed CG of one system (at least 1,280
- * node blocks, or 2,048 equations where it is not node-blocked) is
- * preconditioned by (block) Jacobi plus a coarse space of aggregates (their
- * rigid-body or linear modes, the dense inverse of the Galerkin matrix), which
- * takes far fewer iterations to the same tolerance; 0 keeps (block) Jacobi
- * alone.  A system without usable support points, or one on which the
- * two-level iteration breaks down, is solved with (block) Jacobi. */
+/* ISL_OPT_TWO_LEVEL (default 1): the mixed CG of one system (at least 64 node
+ * blocks, or 1,280 with ISL_OPT_PERSISTENT 0; at least 2,048 equations where it
+ * is not node-blocked) is preconditioned by (block) Jacobi plus a coarse space
+ * of aggregates (their rigid-body or linear modes, the dense inverse of the
+ * Galerkin matrix), which takes far fewer iterations to the same tolerance; 0
+ * keeps (block) Jacobi alone.  A system without usable support points, or one
+ * that the two-level iteration does not bring to the tolerance, is solved with
+ * (block) Jacobi.  A scalar system is multiplied in the order of its
+ * aggregates: ISL_OPT_SPMV32_KIND then chooses the slots in flight (102, 104,
+ * 108); its CSR kinds apply to the one-level solve. */
 /* ISL_OPT_SHARED_GEOMETRY (default 1): the direct block assembly
  * (ISL_OPT_DIRECT_BLOCKS) of a mesh whose hexahedra are all translates of the
  * first (edge vectors equal within 1e-13) forms the 64 local pairs' Lame
@@ -506,7 +511,8 @@ typedef struct {
                                  its first request's (requests of other sizes wait for a batch of their own);
                                  <= 1: any size */
     int persistent;           /* ISL_OPT_PERSISTENT of single-request batches' contexts: 0 (default) CUDA graphs
-                                 of separate kernels, which overlap with the other batches' launches; 1 the
+                                 of separate kernels, or one thread-block cluster where the two-level solve of a
+                                 small system fits, which overlap with the other batches' launches; 1 the
                                  library default (small systems solved in one launch: a cooperative grid over
                                  every SM, or one thread-block cluster) */
     int order;                /* 0 (default): batches start from the oldest queued request; 1: from the

@@ -32,8 +32,10 @@
 // add to, are summed in 64-bit fixed point.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include "isl_coarse.h"
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
         S->absOld = S->absNew;
         if (!(trr == trr) || !(trz == trz)) { S->bad = 1; S->done = 1; }
         else if (trr < S->threshold) S->done = 1;
-        else if (trr < S->rrtrig || trr > 1e8 * S->rr_true) S->done = 3;  // dropped enough, or diverging
+        else if (trr < S->rrtrig || (S->drop > 0.0 && trr > 1e8 * S->rr_true)) S->done = 3;  // dropped enough, or diverging
         else if (S->iters >= S->max_iter) S->done = 2;
     } else if (MODE == CZ_INIT) {
         S->rhsNorm2 = trr;
@@ -241,6 +243,7 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
         S->rr_last = 0.0;
         S->rr_best = trr;
         S->stall = 0;
+        S->careful = 0;
         S->threshold = a.tol * a.tol * trr;
         S->rrtrig = a.drop * trr;
         S->drop = a.drop;
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_coarse(CzIter a) {
     S->ticket2 = 0;
     const double rzn = S->rzloc + tot;
     S->absNew = rzn;
-    if (MODE == CZ_UPDATE) S->beta = rzn / S->absOld;
+    if (MODE == CZ_UPDATE) S->beta = (float)rzn / (float)S->absOld;
     else if (MODE == CZ_INIT) { S->absOld = rzn; S->beta = 0.0; }
     else {
         S->beta = S->fresh ? 0.0 : rzn / S->absOld;
@@ -326,6 +329,532 @@ __global__ void __launch_bounds__(256) k_cz_dir(int n, const float* __restrict__
     if (S->done) return;
     const float beta = (float)S->beta;
     for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) p[i] = fmaf(beta, p[i], z[i]);
+}
+
+// ---------------------------------------------------------------------------
+// Small systems: the whole two-level solve in one thread-block cluster.  Every
+// CTA owns whole aggregates (list order), with their vectors, inverse blocks
+// and row lists in shared memory, and, with MS, its rows of the matrix too.
+// An iteration has three cluster barriers: after the update (r.r, r.z, P^T r),
+// after the coarse correction (its term of r.z; w = z + P z_c visible), and
+// after the product with the folded direction p = w + beta p (p.q).  The sums
+// travel as double-float pairs through distributed shared memory, each CTA
+// storing its pair into every peer before the barrier, so that no CTA reads
+// remotely after it.  The FP64 reliable updates run in the same launch.
+// One iteration takes about a third of the three launches of the graph path,
+// whose latency does not shrink with the system, and uses 16 SMs, so that
+// concurrent solves run side by side.
+namespace cgrp = cooperative_groups;
+
+struct CzClu {
+    const float4* lnode;
+    const int *sofs, *cta, *perm;
+    const float *dsub, *ainv;
+    int ndp;
+    const int *rp, *ci;      // (block) CSR in list order
+    const float* val;        // [NC * NC][nent]
+    int nent;
+    const float* dinv;       // node blocks: by natural row; scalar: in list order
+    float *rc, *w, *pa, *pb; // P^T r (two buffers of ndp), w and the direction buffers, list order
+    const int* aeq;          // equation of every component of a natural row (null: NC row + c)
+    const double* b;
+    double* x64;
+    const int *rowptr, *colind;  // FP64 CSR by equation
+    const double* val64;
+    CGScal* S;
+    double tol, drop;
+    int max_iter, exact64;
+    int max_rows, max_aggs, max_ent;
+    float2* part;            // grid form: the CTAs' sums, four slots
+    unsigned* bar;
+    int inv_smem;            // the CTA's rows of the inverse are held in shared memory
+    unsigned armed;          // test hook: added to the arrivals a grid barrier waits for
+};
+
+
+template <int NC, int M, int NW>
+size_t clu_smem(int rows, int aggs, int ndp, int ent, bool ms, bool as) {
+    size_t f = (size_t)rows * (5 * NC + NC * NC + 4 + 1) + (size_t)aggs * (NW * M + M) + ndp + 8;
+    f += (size_t)aggs * NW * M * M;             // sub-aggregate blocks
+    if (as) f += (size_t)aggs * M * ndp;        // rows of the inverse
+    if (ms) f += (size_t)ent * (NC * NC + 1) + rows + 1;
+    return 4 * f + 64;
+}
+
+template <int NC, int M, int NW, int LPR, bool MS, bool GRID, int CLT>
+__global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
+    cgrp::cluster_group cl = cgrp::this_cluster();
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float2 red[4][16];
+    __shared__ int sc_ok;
+    __shared__ float bs[2][32];
+    __shared__ double shd[32];
+    __shared__ float sc_alpha, sc_beta;
+    __shared__ int sc_ctl;
+    const int rank = GRID ? (int)blockIdx.x : (int)cl.block_rank(), ncta = GRID ? (int)gridDim.x : (int)cl.num_blocks();
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int ag0 = a.cta[rank], ag1 = a.cta[rank + 1], na = ag1 - ag0;
+    const int t0 = a.sofs[ag0 * NW], nr = a.sofs[ag1 * NW] - t0;
+    const int R = a.max_rows;
+    float4* ln = reinterpret_cast<float4*>(smem);     // positions; w: aggregate (local), mask above
+    float* rcs = smem + 4 * (size_t)R;                // [ndp], 16-byte aligned as ln
+    float* ais = rcs + a.ndp;                         // [agg M][ndp]
+    float* xs = ais + (a.inv_smem ? (size_t)a.max_aggs * M * a.ndp : 0);
+    float* rs = xs + (size_t)NC * R;
+    float* qs = rs + (size_t)NC * R;
+    float* zs = qs + (size_t)NC * R;
+    float* ps = zs + (size_t)NC * R;
+    float* ds = ps + (size_t)NC * R;                  // [NC * NC][row]
+    float* src = ds + (size_t)(NC * NC) * R;          // [sub][M]
+    float* zcs = src + (size_t)a.max_aggs * NW * M;   // [agg][M]
+    float* dss = zcs + (size_t)a.max_aggs * M;        // [sub][M * M]
+    int* nat = reinterpret_cast<int*>(dss + (size_t)a.max_aggs * NW * M * M);  // natural row
+    int* rps = nat + R;                               // MS: rows, columns, values
+    int* cis = rps + R + 1;
+    float* vs = reinterpret_cast<float*>(cis + a.max_ent);
+    for (int u = w; u < na * NW; u += CLT / 32) {
+        const int s0 = a.sofs[ag0 * NW + u], s1 = a.sofs[ag0 * NW + u + 1];
+        for (int t = s0 + lane; t < s1; t += 32) {
+            float4 L = a.lnode[t];
+            L.w = __int_as_float((u / NW) | (NC == 3 ? lmask(L) << ROW_BITS : 0));
+            ln[t - t0] = L;
+        }
+    }
+    for (int k = tid; a.inv_smem && k < na * M * (a.ndp / 4); k += CLT)
+        reinterpret_cast<float4*>(ais)[k] = reinterpret_cast<const float4*>(a.ainv + (size_t)(ag0 * M) * a.ndp)[k];
+    for (int k = tid; k < na * NW * M * M; k += CLT) dss[k] = a.dsub[(size_t)(ag0 * NW) * (M * M) + k];
+    const int e0 = a.rp[t0];
+    for (int i = tid; i < nr; i += CLT) {
+        const int row = a.perm[t0 + i];
+        nat[i] = row;
+#pragma unroll
+        for (int k = 0; k < NC * NC; ++k) ds[k * R + i] = NC == 1 ? a.dinv[t0 + i] : a.dinv[(size_t)9 * row + k];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            xs[NC * i + c] = 0.f;
+            ps[NC * i + c] = 0.f;
+            qs[NC * i + c] = 0.f;
+            a.pa[(size_t)NC * (t0 + i) + c] = 0.f;
+        }
+    }
+    if (MS) {
+        const int ne = a.rp[t0 + nr] - e0;
+        for (int i = tid; i <= nr; i += CLT) rps[i] = a.rp[t0 + i] - e0;
+        for (int k = tid; k < ne; k += CLT) {
+            cis[k] = a.ci[e0 + k];
+#pragma unroll
+            for (int e = 0; e < NC * NC; ++e) vs[(size_t)e * a.max_ent + k] = a.val[(size_t)e * a.nent + e0 + k];
+        }
+    }
+    int slot = 0;
+    bool alive = true;  // grid form: false in every thread once a barrier has timed out
+    unsigned goal = a.armed;  // grid form: arrivals that complete the next barrier
+    auto sync_all = [&]() {
+        if constexpr (GRID) {
+            // one counter that only grows: arrive with a release add, poll it
+            // with acquire loads (bounded; a fault makes every CTA leave)
+            goal += gridDim.x;
+            __syncthreads();
+            if (tid == 0) {
+                unsigned v;
+                int ok = 1;
+                asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(a.bar) : "memory");
+                for (unsigned it = 0;; ++it) {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+                    if (v >= goal) break;
+                    if (it > GRID_SYNC_LIMIT || ((it & 255) == 255 && *(volatile int*)&a.S->fault)) {
+                        ok = 0;
+                        atomicExch(&a.S->fault, 1);
+                        break;
+                    }
+                }
+                sc_ok = ok;
+            }
+            __syncthreads();
+            alive = sc_ok != 0;
+        } else {
+            cl.sync();
+        }
+    };
+    // sums over all CTAs of u, and of v if TWO: valid in thread 0 of every CTA.
+    // FP32 inside a CTA (at most a few thousand rows), double-float across.
+    auto cl_sum = [&](auto two, float u, float v, double& ou, double& ov) {
+        constexpr bool TWO = decltype(two)::value;
+        for (int o = 16; o > 0; o >>= 1) {
+            u += __shfl_xor_sync(0xffffffffu, u, o);
+            if (TWO) v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
+        if (lane == 0) { bs[0][w] = u; if (TWO) bs[1][w] = v; }
+        __syncthreads();
+        if (w == 0) {
+            u = lane < CLT / 32 ? bs[0][lane] : 0.f;
+            v = TWO && lane < CLT / 32 ? bs[1][lane] : 0.f;
+            for (int o = 16; o > 0; o >>= 1) {
+                u += __shfl_xor_sync(0xffffffffu, u, o);
+                if (TWO) v += __shfl_xor_sync(0xffffffffu, v, o);
+            }
+            if constexpr (GRID) {
+                if (lane == 0) __stcg(a.part + slot * ncta + rank, make_float2(u, v));
+            } else {
+                if (lane < ncta) *cl.map_shared_rank(&red[slot][rank], lane) = make_float2(u, v);
+            }
+        }
+        sync_all();
+        ou = ov = 0.0;
+        if (w == 0) {
+            df du = {0.f, 0.f}, dv = {0.f, 0.f};
+            if constexpr (GRID) {
+                for (int base = 0; base < ncta; base += 160) {
+                    float2 r[5];
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) {
+                        const int i = base + 32 * k + lane;
+                        r[k] = i < ncta ? __ldcg(a.part + slot * ncta + i) : make_float2(0.f, 0.f);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) {
+                        du = df_add_acc(du, df{r[k].x, 0.f});
+                        if (TWO) dv = df_add_acc(dv, df{r[k].y, 0.f});
+                    }
+                }
+            } else if (lane < ncta) {
+                du.hi = red[slot][lane].x;
+                dv.hi = red[slot][lane].y;
+            }
+            ou = df_value(warp_sum_df(du));
+            if (TWO) ov = df_value(warp_sum_df(dv));
+        }
+        slot = (slot + 1) & 3;
+    };
+    auto cl_sum_d = [&](double u, double& o) {  // one FP64 value (rare)
+        const double t = block_sum(u, shd);
+        if (w == 0) {
+            const double tt = __shfl_sync(0xffffffffu, t, 0);
+            if constexpr (GRID) {
+                if (lane == 0) __stcg(reinterpret_cast<double*>(a.part + slot * ncta + rank), tt);
+            } else {
+                if (lane < ncta) *reinterpret_cast<double*>(cl.map_shared_rank(&red[slot][rank], lane)) = tt;
+            }
+        }
+        sync_all();
+        o = 0.0;
+        if (w == 0) {
+            double r = 0.0;
+            if constexpr (GRID) {
+                for (int i = lane; i < ncta; i += 32) r += __ldcg(reinterpret_cast<const double*>(a.part + slot * ncta + i));
+            } else if (lane < ncta) {
+                r = *reinterpret_cast<const double*>(&red[slot][lane]);
+            }
+            for (int k = 16; k > 0; k >>= 1) r += __shfl_xor_sync(0xffffffffu, r, k);
+            o = r;
+        }
+        slot = (slot + 1) & 3;
+    };
+    // scalars, held by thread 0 of every CTA (the same values everywhere)
+    double rz = 0.0, rz_old = 0.0, rzl = 0.0, rr = 0.0, thr = 0.0, trig = 0.0, rr_true = 0.0, rr_last = 0.0, rr_best = 0.0, bn = 0.0;
+    int iters = 0, stall = 0, careful = 0;
+    enum { GO = 0, FIN1 = 1, FIN2 = 2, FIN3 = 3, STOP = 4 };
+
+    // z = D0^-1 r + P_s D_s^-1 P_s^T r from rs, with rr and rz of this thread; rc written
+    int par = 0;
+    auto local_part = [&](float alpha, bool update, float& frr, float& frz) {
+        for (int u = w; u < na * NW; u += CLT / 32) {
+            const int sub = ag0 * NW + u;
+            const int i0 = a.sofs[sub] - t0, i1 = a.sofs[sub + 1] - t0;
+            float rc[M];
+#pragma unroll
+            for (int m = 0; m < M; ++m) rc[m] = 0.f;
+            for (int i = i0 + lane; i < i1; i += 32) {
+                float rv[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    rv[c] = rs[NC * i + c];
+                    if (update) {
+                        xs[NC * i + c] += alpha * ps[NC * i + c];
+                        rv[c] -= alpha * qs[NC * i + c];
+                        rs[NC * i + c] = rv[c];
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    float z = 0.f;
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) z += ds[(NC * c + k) * R + i] * rv[k];
+                    zs[NC * i + c] = z;
+                    frr += rv[c] * rv[c];
+                    frz += rv[c] * z;
+                }
+                restrict_add<NC, M>(rc, rv, ln[i]);
+            }
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) rc[m] += __shfl_xor_sync(0xffffffffu, rc[m], o);
+            float z1[M], rz1 = 0.f;
+            const float* D = dss + (size_t)u * (M * M);
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                z1[m] = 0.f;
+#pragma unroll
+                for (int k = 0; k < M; ++k) z1[m] += D[M * m + k] * rc[k];
+                rz1 += rc[m] * z1[m];
+            }
+            if (lane == 0) {
+                frz += rz1;
+#pragma unroll
+                for (int m = 0; m < M; ++m) src[u * M + m] = rc[m];
+            }
+            for (int i = i0 + lane; i < i1; i += 32) {
+                float o[NC];
+                const float4 L = ln[i];
+                prolong<NC, M>(z1, L, o);
+                const int mk = NC == 3 ? lmask(L) : 0;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (!((mk >> c) & 1)) zs[NC * i + c] += o[c];
+            }
+        }
+        __syncthreads();
+        float* rcg = a.rc + (size_t)par * a.ndp;
+        for (int k = tid; k < na * M; k += CLT) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < NW; ++j) s += src[((k / M) * NW + j) * M + k % M];
+            rcg[ag0 * M + k] = s;
+        }
+    };
+    // after the barrier that made P^T r visible: w = z + P A_c^-1 P^T r (own rows);
+    // this CTA's part of the coarse term of r.z in thread 0's return value
+    auto coarse_part = [&]() -> float {
+        const float* rcg = a.rc + (size_t)par * a.ndp;
+        for (int k = tid; k < a.ndp; k += CLT) rcs[k] = rcg[k];
+        par ^= 1;
+        __syncthreads();
+        const int n4 = a.ndp / 4;
+        const float4* rc4 = reinterpret_cast<const float4*>(rcs);
+        float part = 0.f;
+        for (int k = w; k < na * M; k += CLT / 32) {
+            const float4* row = reinterpret_cast<const float4*>(a.inv_smem ? ais + (size_t)k * a.ndp : a.ainv + (size_t)(ag0 * M + k) * a.ndp);
+            float s = 0.f;
+#pragma unroll 4
+            for (int j = lane; j < n4; j += 32) {
+                const float4 v = row[j], u = rc4[j];
+                s += v.x * u.x + v.y * u.y + v.z * u.z + v.w * u.w;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) {
+                zcs[k] = s;
+                part += s * rcs[ag0 * M + k];
+            }
+        }
+        __syncthreads();
+        for (int i = tid; i < nr; i += CLT) {
+            const float4 L = ln[i];
+            float c6[M], o[NC];
+            const int ag = lrow(L);
+#pragma unroll
+            for (int m = 0; m < M; ++m) c6[m] = zcs[ag * M + m];
+            prolong<NC, M>(c6, L, o);
+            const int mk = NC == 3 ? lmask(L) : 0;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const float z = zs[NC * i + c] + ((mk >> c) & 1 ? 0.f : o[c]);
+                a.w[(size_t)NC * (t0 + i) + c] = z;
+                zs[NC * i + c] = z;
+            }
+        }
+        return part;
+    };
+
+    sync_all();  // every CTA runs: its shared memory may be written
+    if (!alive) return;
+    // start: r = b
+    {
+        double bb = 0.0;
+        for (int i = tid; i < nr; i += CLT)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const int e = a.aeq ? a.aeq[NC * nat[i] + c] : NC * nat[i] + c;
+                const double v = e >= 0 ? a.b[e] : 0.0;
+                rs[NC * i + c] = (float)v;
+                bb += v * v;
+                if (e >= 0) a.x64[e] = 0.0;
+            }
+        __syncthreads();
+        double t;
+        cl_sum_d(bb, t);
+        if (!alive) return;
+        if (tid == 0) {
+            bn = rr_true = rr_best = rr = t;
+            thr = a.tol * a.tol * t;
+            trig = a.drop * t;
+            sc_ctl = !(t == t) ? FIN3 : (t == 0.0 ? FIN1 : GO);
+        }
+        __syncthreads();
+    }
+    int ctl = sc_ctl;
+    bool restart = true, fresh = true;  // the first pass starts like a restart with beta = 0
+    const int lr = tid % LPR, grp = tid / LPR;
+    constexpr int NG = CLT / LPR;
+    float alpha = 0.f;
+    while (ctl == GO) {
+        double s0, s1;
+        float frr = 0.f, frz = 0.f;
+        local_part(alpha, !restart, frr, frz);
+        cl_sum(std::true_type{}, frr, frz, s0, s1);
+        if (!alive) return;
+        if (tid == 0) {
+            int k = GO;
+            rzl = s1;
+            if (!restart) {
+                rr = s0;
+                iters += 1;
+                rz_old = rz;
+                if (!(s0 == s0) || !(s1 == s1)) k = FIN3;
+                else if (s0 < thr || s0 < trig || (a.exact64 && s0 > 1e8 * rr_true) || iters >= a.max_iter) k = STOP;
+            }
+            sc_ctl = k;
+        }
+        __syncthreads();
+        ctl = sc_ctl;
+        if (ctl == FIN3) break;
+        if (ctl == STOP) {
+            // fold the increment, then the FP64 residual
+            for (int i = tid; i < nr; i += CLT)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const int e = a.aeq ? a.aeq[NC * nat[i] + c] : NC * nat[i] + c;
+                    if (e >= 0) a.x64[e] += (double)xs[NC * i + c];
+                    xs[NC * i + c] = 0.f;
+                }
+            if (!a.exact64) {
+                __syncthreads();  // every thread has read the code that thread 0 replaces
+                if (tid == 0) { sc_ctl = rr < thr ? FIN1 : FIN2; rr_true = rr; }
+                __syncthreads();
+                ctl = sc_ctl;
+                break;
+            }
+            sync_all();
+            if (!alive) return;
+            double loc = 0.0;
+            for (int base = grp - grp % (32 / LPR); base < nr * NC; base += NG) {  // warp-uniform
+                const int k = base + grp % (32 / LPR);
+                const bool act = k < nr * NC;
+                int e = -1;
+                if (act) e = a.aeq ? a.aeq[NC * nat[k / NC] + k % NC] : NC * nat[k / NC] + k % NC;
+                double acc = 0.0;
+                if (e >= 0)
+                    for (int j = a.rowptr[e] + lr; j < a.rowptr[e + 1]; j += LPR) acc += __ldg(a.val64 + j) * a.x64[__ldg(a.colind + j)];
+#pragma unroll
+                for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, LPR);
+                if (act && lr == 0) {
+                    const double ri = e >= 0 ? a.b[e] - acc : 0.0;
+                    rs[k] = (float)ri;
+                    loc += ri * ri;
+                }
+            }
+            double t;
+            cl_sum_d(loc, t);
+            if (!alive) return;
+            if (tid == 0) {
+                int k = GO;
+                if (!(t == t)) k = FIN3;
+                else {
+                    const double rec = rr;
+                    rr_true = t;
+                    if (t <= thr) k = FIN1;
+                    else if (iters >= a.max_iter) k = FIN2;
+                    else {
+                        stall = t > 0.81 * rr_best ? stall + 1 : 0;
+                        rr_best = fmin(rr_best, t);
+                        if (stall >= 6) k = FIN3;
+                        fresh = rr_last > 0.0 && t >= rr_last;
+                        rr_last = t;
+                        if (t > 2.0 * rec) careful = 1;
+                        trig = (!careful && t < 1.003 * rec ? a.drop * a.drop : a.drop) * t;
+                    }
+                }
+                sc_ctl = k;
+            }
+            __syncthreads();
+            ctl = sc_ctl;
+            restart = true;
+            continue;
+        }
+        const float cp = coarse_part();
+        cl_sum(std::false_type{}, cp, 0.f, s0, s1);
+        if (!alive) return;
+        if (tid == 0) {
+            rz = rzl + s0;
+            const bool first = rz_old == 0.0;
+            sc_beta = (restart && (fresh || first)) ? 0.f : (float)rz / (float)rz_old;  // FP64 division: 0.3 us
+            sc_ctl = rz > 0.0 ? GO : FIN3;  // also when it is not a number
+            fresh = false;
+        }
+        __syncthreads();
+        ctl = sc_ctl;
+        if (ctl != GO) break;
+        restart = false;
+        // p = w + beta p, q = A p
+        const float beta = sc_beta;
+        const float* pold = a.pa;
+        float* pnew = a.pb;
+        float loc = 0.f;
+        for (int base = grp - grp % (32 / LPR); base < nr; base += NG) {
+            const int i = base + grp % (32 / LPR);
+            const bool act = i < nr;
+            float acc[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) acc[c] = 0.f;
+            int k = 0, k1 = 0;
+            if (act) {
+                k = (MS ? rps[i] : a.rp[t0 + i]) + lr;
+                k1 = MS ? rps[i + 1] : a.rp[t0 + i + 1];
+            }
+#pragma unroll 2
+            for (; k < k1; k += LPR) {
+                const size_t j = (size_t)NC * (MS ? cis[k] : __ldg(a.ci + k));
+                float x[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) x[c] = fmaf(beta, pold[j + c], a.w[j + c]);
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int e = 0; e < NC; ++e)
+                        acc[c] += (MS ? vs[(size_t)(NC * c + e) * a.max_ent + k] : __ldg(a.val + (size_t)(NC * c + e) * a.nent + k)) * x[e];
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int o = LPR / 2; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o, LPR);
+            if (act && lr == 0) {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float p = fmaf(beta, ps[NC * i + c], zs[NC * i + c]);  // the bits the gathers form
+                    ps[NC * i + c] = p;
+                    pnew[(size_t)NC * (t0 + i) + c] = p;
+                    qs[NC * i + c] = acc[c];
+                    loc += p * acc[c];
+                }
+            }
+        }
+        { float* sw = a.pa; a.pa = a.pb; a.pb = sw; }  // the buffer just written is read next time
+        cl_sum(std::false_type{}, loc, 0.f, s0, s1);
+        if (!alive) return;
+        if (tid == 0) sc_alpha = (float)rz / (float)s0;
+        __syncthreads();
+        alpha = sc_alpha;
+    }
+    if (rank == 0 && tid == 0) {
+        CGScal* S = a.S;
+        S->fin = ctl;
+        S->iters = iters;
+        S->rr_true = rr_true;
+        S->rhsNorm2 = bn;
+        S->rr = rr;
+    }
+    if constexpr (!GRID) cl.sync();  // no CTA leaves while a peer can still store into it
 }
 
 // ---------------------------------------------------------------------------
@@ -403,7 +932,7 @@ __global__ void __launch_bounds__(NW * 32) k_cz_galerkin(CzMat A, const float4* 
                 for (int m = 0; m < M; ++m) Tc[c][m] = 0.f;
         };
         int k0, k1, step;
-        if (NC == 3) {
+        if (NC == 3 || A.soff) {
             const int s = i >> 5;
             k0 = A.soff[s] + (i & 31);
             k1 = k0 + 32 * A.swid[s];
@@ -550,101 +1079,72 @@ __global__ void k_cz_form(int nd, int ndp, const unsigned long long* __restrict_
 
 // Dense inversion of the coarse matrix (symmetric positive definite, unit
 // diagonal) by block sweeps without pivoting, TB rows per step.  Sweeping
-// block k takes A_kk to -D^-1, A_Ik to A_Ik D^-1 and A_IJ to A_IJ - A_Ik D^-1
-// A_kJ, keeps the matrix symmetric, and leaves -A^-1 after the last block; only
-// the tiles on and below the diagonal are stored and updated.
+// block k takes A_kk to -D^-1, A_Ik to G_I = A_Ik D^-1 and A_IJ to
+// A_IJ - G_I A_Jk^T, keeps the matrix symmetric, and leaves -A^-1 after the
+// last block; only the tiles on and below the diagonal are stored.
 //
-// Two launches per step: the panel kernel forms G_I = A_Ik D^-1 for every tile
-// row I and saves the old panel P_I = A_Ik; the update kernel subtracts
-// G_I P_J^T from the other tiles.  The inverse of the next diagonal tile is
-// computed by the CTA that updates it, beside the other tiles' updates: a warp
-// inverts 32 x 32 in registers (a lane per row), and the tile is two of those
-// around a Schur complement.  1.5 ms of setup at 64^3 (1,764 rows) with the
-// Galerkin blocks; pivoting a whole tile with one block barrier per row took
-// 78 us a step, 3.3 ms in all.
+// One launch per step, one CTA per tile.  Every CTA reads the panel (the tiles
+// A_Ik) from a copy that the step before wrote, forms its own G_I, and the
+// CTAs of the next panel's tiles write the next copy.  The next diagonal tile
+// is also inverted by the CTA that updates it, beside the other tiles'
+// updates: that chain, TB pivots with one block barrier each, is what a step
+// waits for.  Measured at 64^3 (1,764 rows, 28 steps): see numeric().
 
-// inverse of the 32 x 32 matrix in X (leading dimension TB + 1) by one warp
-__device__ __forceinline__ void warp_inv32(float* X) {
-    const int l = threadIdx.x & 31;
-    float a[32];
+// inverse of the TB x TB matrix in X by 256 threads, Gauss-Jordan: thread
+// (ty, tx) holds rows ty + 16 r and columns tx + 16 c; pivot 16 a + b belongs to
+// r = c = a, so that the registers are indexed by unrolled loops only
+__device__ __forceinline__ void tile_inv(float (*X)[TB + 1], float (*buf)[2 * TB]) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    float d[4][4];
 #pragma unroll
-    for (int c = 0; c < 32; ++c) a[c] = X[l * (TB + 1) + c];
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int p = 0; p < 32; ++p) {
-        const float ip = 1.f / fmaxf(__shfl_sync(0xffffffffu, a[p], p), 0.1f * REG);
-        const float f = l == p ? 1.f - ip : a[p] * ip;  // row l minus f times the pivot row; the pivot row scales by ip
+        for (int c = 0; c < 4; ++c) d[r][c] = X[ty + 16 * r][tx + 16 * c];
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-            if (c != p) a[c] -= f * __shfl_sync(0xffffffffu, a[c], p);
-        a[p] = l == p ? ip : -f;
-    }
+    for (int a = 0; a < 4; ++a)
+        for (int b = 0; b < 16; ++b) {
+            float* row = buf[b & 1];
+            float* col = row + TB;
+            if (ty == b) {
 #pragma unroll
-    for (int c = 0; c < 32; ++c) X[l * (TB + 1) + c] = a[c];
-    __syncwarp();
-}
-
-// inverse of the symmetric TB x TB matrix D in shared memory by 256 threads;
-// T: scratch of the same size
-__device__ __forceinline__ void tile_inv(float (*D)[TB + 1], float (*T)[TB + 1]) {
-    const int r = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 4;  // 32 rows, 4 columns per thread
-    if (threadIdx.x < 32) warp_inv32(&D[0][0]);                  // A <- A^-1
+                for (int c = 0; c < 4; ++c) row[tx + 16 * c] = d[a][c];
+            }
+            if (tx == b) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) col[ty + 16 * r] = d[r][a];
+            }
+            __syncthreads();
+            const float ip = __fdividef(1.f, fmaxf(row[16 * a + b], 0.1f * REG));
+            float pr[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) pr[c] = row[tx + 16 * c];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float f = col[ty + 16 * r] * ip;
+                const bool prow = r == a && ty == b;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const bool pcol = c == a && tx == b;
+                    const float v = pcol ? -f : d[r][c] - f * pr[c];
+                    d[r][c] = prow ? (pcol ? ip : pr[c] * ip) : v;
+                }
+            }
+        }
     __syncthreads();
-    {   // T_01 = A^-1 B
-        float o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int m = 0; m < 32; ++m)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) o[c] += D[r][m] * D[m][32 + c0 + c];
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) T[r][32 + c0 + c] = o[c];
-    }
-    __syncthreads();
-    {   // C <- C - B^T A^-1 B
-        float o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int m = 0; m < 32; ++m)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) o[c] += D[m][32 + r] * T[m][32 + c0 + c];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) D[32 + r][32 + c0 + c] -= o[c];
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) warp_inv32(&D[32][32]);  // C <- S^-1
-    __syncthreads();
-    {   // T_10^T = A^-1 B S^-1
-        float o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int m = 0; m < 32; ++m)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) o[c] += T[r][32 + m] * D[32 + m][32 + c0 + c];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { D[r][32 + c0 + c] = -o[c]; D[32 + c0 + c][r] = -o[c]; }
-    }
-    __syncthreads();
-    {   // A^-1 + (A^-1 B) S^-1 (A^-1 B)^T
-        float o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int m = 0; m < 32; ++m)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) o[c] -= D[r][32 + m] * T[c0 + c][32 + m];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) D[r][c0 + c] += o[c];
-    }
+        for (int c = 0; c < 4; ++c) X[ty + 16 * r][tx + 16 * c] = d[r][c];
     __syncthreads();
 }
 
-// the inverse of the first diagonal tile
-__global__ void __launch_bounds__(256) k_gj_first(const float* __restrict__ A, int n, float* __restrict__ Dinv) {
-    __shared__ float D[TB][TB + 1], T[TB][TB + 1];
-    for (int e = threadIdx.x; e < TB * TB; e += 256) D[e / TB][e % TB] = A[(size_t)(e / TB) * n + e % TB];
-    __syncthreads();
-    tile_inv(D, T);
-    for (int e = threadIdx.x; e < TB * TB; e += 256) Dinv[e] = D[e / TB][e % TB];
-}
-
-// C[4 ty + r][tx + 16 c] += sum_m X[4 ty + r][m] Y[tx + 16 c][m]
+// o[r][c] = sum_m X[4 ty + r][m] Y[tx + 16 c][m]
 __device__ __forceinline__ void tile_mul(const float (*X)[TB + 1], const float (*Y)[TB + 1], float (&o)[4][4]) {
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[r][c] = 0.f;
 #pragma unroll 8
     for (int m = 0; m < TB; ++m) {
         float u[4], v[4];
@@ -657,32 +1157,40 @@ __device__ __forceinline__ void tile_mul(const float (*X)[TB + 1], const float (
     }
 }
 
-// G_I = A_Ik D^-1, P_I = A_Ik (A_Ik = A_kI^T above the diagonal)
-__global__ void __launch_bounds__(256) k_gj_panel(const float* __restrict__ A, int n, int k, const float* __restrict__ Dinv,
-                                                  float* __restrict__ G, float* __restrict__ P) {
-    __shared__ float X[TB][TB + 1], D[TB][TB + 1];
-    const int I = blockIdx.x, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    if (I == k) return;
-    for (int e = threadIdx.x; e < TB * TB; e += 256) {
-        const int r = e / TB, c = e % TB;
-        if (I > k) X[r][c] = A[(size_t)(I * TB + r) * n + k * TB + c];
-        else X[c][r] = A[(size_t)(k * TB + r) * n + I * TB + c];
-        D[r][c] = Dinv[e];
+// a TB x TB tile (row stride ld) into shared memory
+__device__ __forceinline__ void tile_load(const float* g, int ld, float (*X)[TB + 1]) {
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int e = threadIdx.x + 256 * k;
+        v[k] = *reinterpret_cast<const float4*>(g + (size_t)(e / 16) * ld + 4 * (e % 16));
     }
-    __syncthreads();
-    float o[4][4] = {};
-    tile_mul(X, D, o);  // D^-1 is symmetric
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) G[(size_t)(I * TB + 4 * ty + r) * TB + tx + 16 * c] = o[r][c];
-    for (int e = threadIdx.x; e < TB * TB; e += 256) P[(size_t)I * TB * TB + e] = X[e / TB][e % TB];
+    for (int k = 0; k < 4; ++k) {
+        const int e = threadIdx.x + 256 * k, r = e / 16, c = 4 * (e % 16);
+        X[r][c] = v[k].x; X[r][c + 1] = v[k].y; X[r][c + 2] = v[k].z; X[r][c + 3] = v[k].w;
+    }
 }
 
-__global__ void __launch_bounds__(256) k_gj_update(float* __restrict__ A, int n, int k, float* __restrict__ Dinv,
-                                                   float* __restrict__ Dnext, const float* __restrict__ G,
-                                                   const float* __restrict__ P) {
-    __shared__ float X[TB][TB + 1], Y[TB][TB + 1];
+// the first panel and the inverse of the first diagonal tile
+__global__ void __launch_bounds__(256) k_gj_first(const float* __restrict__ A, int n, float* __restrict__ P, float* __restrict__ Dinv) {
+    __shared__ float X[TB][TB + 1];
+    __shared__ float buf[2][2 * TB];
+    const int I = blockIdx.x;
+    tile_load(A + (size_t)(I * TB) * n, n, X);
+    __syncthreads();
+    for (int e = threadIdx.x; e < TB * TB; e += 256) P[(size_t)I * TB * TB + e] = X[e / TB][e % TB];
+    if (I) return;
+    tile_inv(X, buf);
+    for (int e = threadIdx.x; e < TB * TB; e += 256) Dinv[e] = X[e / TB][e % TB];
+}
+
+__global__ void __launch_bounds__(256) k_gj_step(float* __restrict__ A, int n, int k, const float* __restrict__ Dinv,
+                                                 float* __restrict__ Dnext, const float* __restrict__ P, float* __restrict__ Pnext) {
+    extern __shared__ __align__(16) float gj_smem[];
+    typedef float (*Tile)[TB + 1];
+    Tile X = reinterpret_cast<Tile>(gj_smem), Y = X + TB, Z = Y + TB;
+    __shared__ float buf[2][2 * TB];
     // tile (I, J), J <= I, of the linear index; the next diagonal tile comes first
     int t = blockIdx.x;
     const int nt = n / TB, first = k + 1 < nt ? (k + 1) * (k + 2) / 2 + k + 1 : -1;
@@ -692,44 +1200,84 @@ __global__ void __launch_bounds__(256) k_gj_update(float* __restrict__ A, int n,
     while (I * (I + 1) / 2 > t) --I;
     const int J = t - I * (I + 1) / 2, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     float* g = A + (size_t)(I * TB) * n + J * TB;
-    if (I == k || J == k) {
-        for (int e = threadIdx.x; e < TB * TB; e += 256) {
-            const int r = e / TB, c = e % TB;
-            if (I == J) g[(size_t)r * n + c] = -Dinv[e];
-            else if (J == k) g[(size_t)r * n + c] = G[(size_t)(I * TB + r) * TB + c];
-            else g[(size_t)r * n + c] = G[(size_t)(J * TB + c) * TB + r];
+    float v[4][4];  // the tile's new entries, rows 4 ty + r, columns tx + 16 c
+    if (I == k && J == k) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[r][c] = -Dinv[(4 * ty + r) * TB + tx + 16 * c];
+    } else {
+        // I == k: the tile is G_J^T
+        const int R = I == k ? J : I;
+        tile_load(P + (size_t)R * TB * TB, TB, X);
+        tile_load(Dinv, TB, Y);
+        float a[4][4];
+        if (I != k && J != k) {
+            tile_load(P + (size_t)J * TB * TB, TB, Z);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) a[r][c] = g[(size_t)(4 * ty + r) * n + tx + 16 * c];
         }
-        return;
+        __syncthreads();
+        float o[4][4];
+        tile_mul(X, Y, o);  // G_R: D^-1 is symmetric
+        __syncthreads();
+        if (I == k) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) X[tx + 16 * c][4 * ty + r] = o[r][c];
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[r][c] = X[4 * ty + r][tx + 16 * c];
+        } else if (J == k) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[r][c] = o[r][c];
+        } else {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) X[4 * ty + r][tx + 16 * c] = o[r][c];
+            __syncthreads();
+            tile_mul(X, Z, o);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[r][c] = a[r][c] - o[r][c];
+        }
     }
-    for (int e = threadIdx.x; e < TB * TB; e += 256) {
-        X[e / TB][e % TB] = G[(size_t)I * TB * TB + e];
-        Y[e / TB][e % TB] = P[(size_t)J * TB * TB + e];
-    }
-    float a[4][4];
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) a[r][c] = g[(size_t)(4 * ty + r) * n + tx + 16 * c];
-    __syncthreads();
-    float o[4][4] = {};
-    tile_mul(X, Y, o);
+        for (int c = 0; c < 4; ++c) g[(size_t)(4 * ty + r) * n + tx + 16 * c] = v[r][c];
+    // the next panel, column k + 1: tiles (I, k + 1), and (k + 1, J) transposed
+    if (J == k + 1) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            a[r][c] -= o[r][c];
-            g[(size_t)(4 * ty + r) * n + tx + 16 * c] = a[r][c];
-        }
+            for (int c = 0; c < 4; ++c) Pnext[(size_t)I * TB * TB + (4 * ty + r) * TB + tx + 16 * c] = v[r][c];
+    } else if (I == k + 1) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) Pnext[(size_t)J * TB * TB + (tx + 16 * c) * TB + 4 * ty + r] = v[r][c];
+    }
     if (I != J || I != k + 1) return;
     __syncthreads();  // the next diagonal tile: its inverse
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) X[4 * ty + r][tx + 16 * c] = a[r][c];
+        for (int c = 0; c < 4; ++c) X[4 * ty + r][tx + 16 * c] = v[r][c];
     __syncthreads();
-    tile_inv(X, Y);
+    tile_inv(X, buf);
     for (int e = threadIdx.x; e < TB * TB; e += 256) Dnext[e] = X[e / TB][e % TB];
 }
+constexpr int GJ_SMEM = 3 * TB * (TB + 1) * 4;
 
 // undo the sign and the scaling, and fill the upper triangle from the lower
 __global__ void k_cz_unscale(int nd, int ndp, const float* __restrict__ A, const float* __restrict__ s, float* __restrict__ out) {
@@ -869,11 +1417,18 @@ __global__ void k_cz_key(int n, Box3 b, const unsigned short* __restrict__ cut, 
     }
 }
 
-template <int NW>
-__global__ void k_cz_rekey(int n, const int* __restrict__ map, int* __restrict__ key, int* __restrict__ row) {
+// sort key of every row: sub-aggregate, then (scalar rows) the length, falling
+// and rising in turn, so that the slices of the aggregate-ordered copy need
+// little padding inside a sub-aggregate and across two
+constexpr int LEN_BITS = 10;
+template <int NC, int NW>
+__global__ void k_cz_rekey(int n, const int* __restrict__ map, const int* __restrict__ rowptr, int* __restrict__ key,
+                           int* __restrict__ row) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int k = key[i];
-        key[i] = map[k / NW] * NW + k % NW;
+        const int k = key[i], top = (1 << LEN_BITS) - 1;
+        const int sub = map[k / NW] * NW + k % NW;
+        const int len = NC == 1 ? min(top, rowptr[i + 1] - rowptr[i]) : 0;
+        key[i] = sub << LEN_BITS | (sub & 1 ? len : top - len);
         row[i] = i;
     }
 }
@@ -882,7 +1437,8 @@ __global__ void k_cz_rekey(int n, const int* __restrict__ map, int* __restrict__
 template <int NC, int NW>
 __global__ void __launch_bounds__(NW * 32) k_cz_nodes(const int* __restrict__ sofs, const int* __restrict__ list,
                                                       const int* __restrict__ key, const float4* __restrict__ xr,
-                                                      float4* __restrict__ lnode, float4* __restrict__ yrow) {
+                                                      float4* __restrict__ lnode, float4* __restrict__ yrow,
+                                                      int* __restrict__ pos) {
     __shared__ double sh[32];
     __shared__ double cen[3], irad;
     const int t0 = sofs[blockIdx.x * NW], t1 = sofs[(blockIdx.x + 1) * NW];
@@ -909,10 +1465,11 @@ __global__ void __launch_bounds__(NW * 32) k_cz_nodes(const int* __restrict__ so
         const int row = list[t];
         const float4 v = xr[row];
         float4 y = make_float4((float)((v.x - cen[0]) * irad), (float)((v.y - cen[1]) * irad), (float)((v.z - cen[2]) * irad), 0.f);
-        y.w = __int_as_float(row | (NC == 3 ? __float_as_int(v.w) << ROW_BITS : 0));
+        y.w = __int_as_float(NC == 3 ? row | __float_as_int(v.w) << ROW_BITS : t);
         lnode[t] = y;
-        y.w = __int_as_float(key[t]);
-        yrow[row] = y;
+        y.w = __int_as_float(key[t] >> LEN_BITS);
+        yrow[NC == 3 ? row : t] = y;
+        pos[row] = t;
     }
 }
 
@@ -923,7 +1480,7 @@ __global__ void __launch_bounds__(NW * 32) k_cz_nodes(const int* __restrict__ so
 // 5.50 with 150, 5.70 with 300; 270,400 rows 21.9 with 150, 20.0 with 300,
 // 21.3 with 400.
 int target_aggs(int64_t n) {
-    return (int)std::clamp<int64_t>(n / 60, 8, std::clamp<int64_t>(n / 900, 150, 300));
+    return (int)std::clamp<int64_t>(n / 60, 16, std::clamp<int64_t>(n / 900, 150, 300));
 }
 
 unsigned grid_for(const isl_ctx* c, int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 8LL * c->sm_count)); }
@@ -934,7 +1491,7 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     const int D = c->dim, n = (int)z.nrow;
     DBuf<float> P;
     DBuf<float4> xr;
-    DBuf<int32_t> eqrow, hist, key, key2, row, list, cnt, map;
+    DBuf<int32_t> eqrow, hist, key, key2, row, cnt, map;
     DBuf<unsigned> mm;
     DBuf<unsigned short> dcut;
     DBuf<char> tmp;
@@ -973,23 +1530,37 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     std::vector<int32_t> hh(3 * NBIN);
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(hh.data(), hist.p, hh.size() * 4, cudaMemcpyDeviceToHost, st));
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
-    // near-cubic boxes: the edge h that gives the target number of them
+    // near-cubic boxes: the edge h that gives the target number of them over
+    // the directions that are at least one edge long
     const int comps = NC == 1 ? c->ncomp : 1;
     const int target = std::max(1, target_aggs(z.nrow) / comps);
-    double vol = 1.0;
-    int nd = 0;
-    for (int d = 0; d < D; ++d)
-        if (L[d] > 1e-3 * Lmax) { vol *= L[d]; ++nd; }
-    double h = std::pow(vol / target, 1.0 / nd);
-    for (;;) {
-        int64_t tot = 1;
-        for (int d = 0; d < 3; ++d) {
-            b.m[d] = d < D ? std::max(1, (int)std::lround(L[d] / h)) : 1;
-            tot *= b.m[d];
-        }
-        if (tot <= std::max(target, 1)) break;
-        h *= 1.02;
+    bool use[3] = {L[0] > 0.0, L[1] > 0.0, L[2] > 0.0};
+    double h = Lmax;
+    for (bool again = true; again;) {
+        double vol = 1.0;
+        int nd = 0;
+        for (int d = 0; d < D; ++d)
+            if (use[d]) { vol *= L[d]; ++nd; }
+        h = std::pow(vol / target, 1.0 / nd);
+        again = false;
+        for (int d = 0; d < D; ++d)
+            if (use[d] && nd > 1 && L[d] < h) { use[d] = false; again = true; break; }
     }
+    // the largest product of rounded-down or rounded-up counts within the target
+    int64_t best = 0;
+    for (int pick = 0; pick < 1 << D; ++pick) {
+        int64_t tot = 1;
+        int m[3] = {1, 1, 1};
+        for (int d = 0; d < D; ++d) {
+            m[d] = use[d] ? std::max(1, (int)std::min(L[d] / h, (double)target) + ((pick >> d) & 1)) : 1;
+            tot *= m[d];
+        }
+        if (tot <= target && tot > best) {
+            best = tot;
+            for (int d = 0; d < 3; ++d) b.m[d] = m[d];
+        }
+    }
+    if (!best) { b.m[0] = b.m[1] = b.m[2] = 1; }
     const int nbox = b.m[0] * b.m[1] * b.m[2] * comps;
     // cuts at the quantiles of the rows, two half-boxes per box
     std::vector<unsigned short> cut(3 * NBIN, 0);
@@ -1006,7 +1577,8 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     ISL_CHECK_CUDA(c, key.alloc(n));
     ISL_CHECK_CUDA(c, key2.alloc(n));
     ISL_CHECK_CUDA(c, row.alloc(n));
-    ISL_CHECK_CUDA(c, list.alloc(n));
+    ISL_CHECK_CUDA(c, z.perm.alloc(n));
+    ISL_CHECK_CUDA(c, z.pos.alloc(n));
     ISL_CHECK_CUDA(c, cnt.alloc((size_t)nbox * NW));
     ISL_CHECK_CUDA(c, map.alloc(nbox));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(dcut.p, cut.data(), cut.size() * 2, cudaMemcpyHostToDevice, st));
@@ -1032,28 +1604,187 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     ISL_CHECK_CUDA(c, z.yrow.alloc(n));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.sofs.p, so.data(), so.size() * 4, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(map.p, hmap.data(), hmap.size() * 4, cudaMemcpyHostToDevice, st));
-    k_cz_rekey<NW><<<g, 256, 0, st>>>(n, map.p, key.p, row.p);
+    k_cz_rekey<NC, NW><<<g, 256, 0, st>>>(n, map.p, c->drowptr.p, key.p, row.p);
     int bits = 1;
     while ((1 << bits) < na * NW) ++bits;
+    bits += LEN_BITS;
     size_t tb = 0;
-    ISL_CHECK_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key2.p, row.p, list.p, n, 0, bits, st));
+    ISL_CHECK_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key2.p, row.p, z.perm.p, n, 0, bits, st));
     ISL_CHECK_CUDA(c, tmp.alloc(std::max<size_t>(tb, 1)));
-    ISL_CHECK_CUDA(c, cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key2.p, row.p, list.p, n, 0, bits, st));
-    k_cz_nodes<NC, NW><<<na, NW * 32, 0, st>>>(z.sofs.p, list.p, key2.p, xr.p, z.lnode.p, z.yrow.p);
+    ISL_CHECK_CUDA(c, cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key2.p, row.p, z.perm.p, n, 0, bits, st));
+    k_cz_nodes<NC, NW><<<na, NW * 32, 0, st>>>(z.sofs.p, z.perm.p, key2.p, xr.p, z.lnode.p, z.yrow.p, z.pos.p);
     ISL_CHECK_CUDA(c, cudaGetLastError());
     ISL_CHECK_CUDA(c, z.dsub.alloc((size_t)na * NW * M * M));
     ISL_CHECK_CUDA(c, z.dagg.alloc((size_t)na * M * M));
     ISL_CHECK_CUDA(c, z.scale.alloc(z.ndp));
-    ISL_CHECK_CUDA(c, z.rc.alloc(z.ndp));
+    ISL_CHECK_CUDA(c, z.rc.alloc((size_t)2 * z.ndp));
     ISL_CHECK_CUDA(c, z.acc.alloc((size_t)z.ndp * z.ndp));
     ISL_CHECK_CUDA(c, z.a.alloc((size_t)z.ndp * z.ndp));
     ISL_CHECK_CUDA(c, z.ainv.alloc((size_t)z.ndp * z.ndp));
     ISL_CHECK_CUDA(c, z.panel.alloc((size_t)2 * TB * z.ndp + 2 * TB * TB));
     ISL_CHECK_CUDA(c, z.amax.alloc(1));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.rc.p, 0, (size_t)z.ndp * 4, st));  // the padding stays zero
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.rc.p, 0, (size_t)2 * z.ndp * 4, st));  // the padding stays zero
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));  // the scratch buffers above go out of scope
     c->launches += 10;
+    z.hsofs = std::move(so);
     z.ok = true;
+    return ISL_OK;
+}
+
+// Aggregate-ordered copies of the matrix (t-space: the order of the row list).
+// The update and coarse kernels then read their vectors contiguously, and the
+// rows of a slice gather from a few neighbouring boxes.
+
+// scalar rows: row lengths of a slice
+__global__ void k_pz_width(int n, int nslice, const int* __restrict__ perm, const int* __restrict__ rowptr, int* __restrict__ wid) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nslice) return;
+    int w = 0;
+    for (int t = s * 32; t < min(n, s * 32 + 32); ++t) w = max(w, rowptr[perm[t] + 1] - rowptr[perm[t]]);
+    wid[s] = w;
+}
+__global__ void k_pz_cols(int n, int nslice, const int* __restrict__ perm, const int* __restrict__ pos, const int* __restrict__ rowptr,
+                          const int* __restrict__ colind, const int* __restrict__ soff, const int* __restrict__ swid,
+                          int* __restrict__ col, short* __restrict__ col16, int* __restrict__ srow, int* __restrict__ far) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nslice * 32) return;
+    const int row = t < n ? perm[t] : -1, base = t < n ? t : 0;
+    const int lo = row >= 0 ? rowptr[row] : 0, len = row >= 0 ? rowptr[row + 1] - lo : 0;
+    const int o = soff[t >> 5] + (t & 31), w = swid[t >> 5];
+    srow[t] = t < n ? t : -1;
+    for (int k = 0; k < w; ++k) {
+        const int j = k < len ? pos[colind[lo + k]] : base, d = j - base;
+        col[o + 32 * k] = j;
+        if (d < -32767 || d > 32767) atomicOr(far, 1);
+        col16[o + 32 * k] = (short)d;
+    }
+}
+// values: the loads of a lane run along its CSR row
+__global__ void k_pz_values(int n, const int* __restrict__ perm, const int* __restrict__ rowptr, const float* __restrict__ val,
+                            const int* __restrict__ soff, float* __restrict__ sv) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int lo = rowptr[perm[t]], hi = rowptr[perm[t] + 1], o = soff[t >> 5] + (t & 31);
+        for (int k = lo; k < hi; ++k) sv[o + 32 * (k - lo)] = val[k];
+    }
+}
+__global__ void k_pz_dinv(int n, const int* __restrict__ perm, const int* __restrict__ diag, const float* __restrict__ val,
+                          float* __restrict__ dinv) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const float d = val[diag[perm[t]]];
+        dinv[t] = d != 0.f ? 1.f / d : 1.f;
+    }
+}
+
+// row lists for the one-cluster solve: (block) CSR in t-space
+__global__ void k_pz_len(int n, const int* __restrict__ perm, const int* __restrict__ ptr, int* __restrict__ len) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t <= n) len[t] = t < n ? ptr[perm[t] + 1] - ptr[perm[t]] : 0;
+}
+__global__ void k_pz_csr_cols(int n, const int* __restrict__ perm, const int* __restrict__ pos, const int* __restrict__ ptr,
+                              const int* __restrict__ colind, const int* __restrict__ rp, int* __restrict__ col) {
+    for (int t = blockIdx.x * 8 + (threadIdx.x >> 5); t < n; t += gridDim.x * 8) {
+        const int lo = ptr[perm[t]], len = rp[t + 1] - rp[t];
+        for (int k = threadIdx.x & 31; k < len; k += 32) col[rp[t] + k] = pos[colind[lo + k]];
+    }
+}
+template <int NC>
+__global__ void k_pz_csr_values(int n, const int* __restrict__ perm, const int* __restrict__ ptr, const int* __restrict__ sdst,
+                                const float* __restrict__ src, const int* __restrict__ rp, int nblk, float* __restrict__ val) {
+    for (int t = blockIdx.x * 8 + (threadIdx.x >> 5); t < n; t += gridDim.x * 8) {
+        const int lo = ptr[perm[t]], len = rp[t + 1] - rp[t];
+        for (int k = threadIdx.x & 31; k < len; k += 32) {
+            if (NC == 1) {
+                val[rp[t] + k] = src[lo + k];
+            } else {
+                const int slot = sdst[lo + k];
+                const float* g = src + (size_t)(slot >> 5) * 288 + (slot & 31);
+#pragma unroll
+                for (int e = 0; e < 9; ++e) val[(size_t)e * nblk + rp[t] + k] = g[32 * e];
+            }
+        }
+    }
+}
+
+// columns of the aggregate-ordered sliced-ELL copy (scalar systems), once per pattern
+int build_sell(isl_ctx* c, CzPlan& z) {
+    if (z.sell_built) return ISL_OK;
+    cudaStream_t st = c->stream;
+    const int n = (int)z.nrow, ns = (n + 31) / 32;
+    ISL_CHECK_CUDA(c, z.swid.alloc(ns));
+    ISL_CHECK_CUDA(c, z.soff.alloc(ns + 1));
+    k_pz_width<<<(ns + 127) / 128, 128, 0, st>>>(n, ns, z.perm.p, c->drowptr.p, z.swid.p);
+    std::vector<int32_t> wid(ns), off(ns + 1);
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(wid.data(), z.swid.p, (size_t)ns * 4, cudaMemcpyDeviceToHost, st));
+    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+    int64_t tot = 0;
+    for (int s = 0; s < ns; ++s) {
+        off[s] = (int32_t)tot;
+        tot += 32LL * wid[s];
+        if (tot >= INT32_MAX) { z.ok = false; return ISL_OK; }
+    }
+    off[ns] = (int32_t)tot;
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.soff.p, off.data(), (size_t)(ns + 1) * 4, cudaMemcpyHostToDevice, st));
+    ISL_CHECK_CUDA(c, z.srow.alloc((size_t)ns * 32));
+    ISL_CHECK_CUDA(c, z.col.alloc(tot));
+    ISL_CHECK_CUDA(c, z.col16.alloc(tot));
+    ISL_CHECK_CUDA(c, z.val.alloc(tot));
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.val.p, 0, (size_t)tot * 4, st));
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(c->dflags.p + 1, 0, sizeof(int), st));
+    k_pz_cols<<<(ns * 32 + 255) / 256, 256, 0, st>>>(n, ns, z.perm.p, z.pos.p, c->drowptr.p, c->dcolind.p, z.soff.p, z.swid.p,
+                                                      z.col.p, z.col16.p, z.srow.p, c->dflags.p + 1);
+    int far = 0;
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(&far, c->dflags.p + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+    z.short_cols = far == 0;
+    if (far) z.col16.release();
+    z.nslice = ns;
+    c->launches += 2;
+    z.sell_built = true;
+    return ISL_OK;
+}
+
+// (block) CSR in t-space for the one-cluster solve, once per pattern
+int build_csr(isl_ctx* c, CzPlan& z) {
+    if (z.csr_built) return ISL_OK;
+    cudaStream_t st = c->stream;
+    const int n = (int)z.nrow;
+    const int* ptr = z.nc == 3 ? c->dbptr.p : c->drowptr.p;
+    z.nent = z.nc == 3 ? c->nblk : c->nnz;
+    DBuf<int32_t> len;
+    DBuf<char> tmp;
+    ISL_CHECK_CUDA(c, len.alloc(n + 1));
+    ISL_CHECK_CUDA(c, z.rp.alloc(n + 1));
+    ISL_CHECK_CUDA(c, z.ci.alloc(z.nent));
+    ISL_CHECK_CUDA(c, z.cv.alloc((size_t)z.nc * z.nc * z.nent));
+    k_pz_len<<<n / 256 + 1, 256, 0, st>>>(n, z.perm.p, ptr, len.p);
+    size_t tb = 0;
+    ISL_CHECK_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, tb, len.p, z.rp.p, n + 1, st));
+    ISL_CHECK_CUDA(c, tmp.alloc(std::max<size_t>(tb, 1)));
+    ISL_CHECK_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp.p, tb, len.p, z.rp.p, n + 1, st));
+    k_pz_csr_cols<<<(n + 7) / 8, 256, 0, st>>>(n, z.perm.p, z.pos.p, ptr, z.nc == 3 ? c->dbcol.p : c->dcolind.p, z.rp.p, z.ci.p);
+    std::vector<int32_t> rp(n + 1);
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(rp.data(), z.rp.p, (size_t)(n + 1) * 4, cudaMemcpyDeviceToHost, st));
+    ISL_CHECK_CUDA(c, cudaGetLastError());
+    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+    // aggregates per CTA: contiguous, balanced by rows and stored entries
+    const int nw = z.m == 3 ? 4 : 8;
+    z.hcta.assign(z.ncta + 1, 0);
+    z.max_rows = z.max_aggs = 0;
+    z.max_ent = 0;
+    for (int k = 0, ag = 0; k < z.ncta; ++k) {
+        const int64_t goal = z.nent * (k + 1) / z.ncta;
+        while (ag < z.nagg && (k == z.ncta - 1 || (int64_t)rp[z.hsofs[(size_t)ag * nw]] + rp[z.hsofs[(size_t)(ag + 1) * nw]] < 2 * goal)) ++ag;
+        z.hcta[k + 1] = ag;
+        const int t0 = z.hsofs[(size_t)z.hcta[k] * nw], t1 = z.hsofs[(size_t)ag * nw];
+        z.max_rows = std::max(z.max_rows, t1 - t0);
+        z.max_aggs = std::max(z.max_aggs, ag - z.hcta[k]);
+        z.max_ent = std::max(z.max_ent, rp[t1] - rp[t0]);
+    }
+    ISL_CHECK_CUDA(c, z.cta.alloc(z.ncta + 1));
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.cta.p, z.hcta.data(), (size_t)(z.ncta + 1) * 4, cudaMemcpyHostToDevice, st));
+    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+    c->launches += 3;
+    z.csr_built = true;
     return ISL_OK;
 }
 
@@ -1072,15 +1803,16 @@ int numeric(isl_ctx* c, CzPlan& z, const CzMat& A) {
     k_cz_scale<M><<<(z.nagg + 127) / 128, 128, 0, st>>>(z.nagg, z.dagg.p, z.scale.p);
     const dim3 g32(ndp / 32, ndp / 32);
     k_cz_form<M><<<g32, 256, 0, st>>>(z.nd, ndp, z.acc.p, z.dagg.p, z.scale.p, z.amax.p, z.a.p);
-    float *G = z.panel.p, *P = G + (size_t)TB * ndp, *D[2] = {P + (size_t)TB * ndp, P + (size_t)TB * ndp + TB * TB};
-    k_gj_first<<<1, 256, 0, st>>>(z.a.p, ndp, D[0]);
-    for (int k = 0; k < nt; ++k) {
-        if (nt > 1) k_gj_panel<<<nt, 256, 0, st>>>(z.a.p, ndp, k, D[k & 1], G, P);
-        k_gj_update<<<nt * (nt + 1) / 2, 256, 0, st>>>(z.a.p, ndp, k, D[k & 1], D[(k + 1) & 1], G, P);
-    }
+    // inverse: 28 steps at 64^3
+    float *P[2] = {z.panel.p, z.panel.p + (size_t)TB * ndp};
+    float *Di[2] = {z.panel.p + (size_t)2 * TB * ndp, z.panel.p + (size_t)2 * TB * ndp + TB * TB};
+    ISL_CHECK_CUDA(c, cudaFuncSetAttribute(k_gj_step, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SMEM));
+    k_gj_first<<<nt, 256, 0, st>>>(z.a.p, ndp, P[0], Di[0]);
+    for (int k = 0; k < nt; ++k)
+        k_gj_step<<<nt * (nt + 1) / 2, 256, GJ_SMEM, st>>>(z.a.p, ndp, k, Di[k & 1], Di[(k + 1) & 1], P[k & 1], P[(k + 1) & 1]);
     k_cz_unscale<<<g32, 256, 0, st>>>(z.nd, ndp, z.a.p, z.scale.p, z.ainv.p);
     ISL_CHECK_CUDA(c, cudaGetLastError());
-    c->launches += 7 + 2 * nt;
+    c->launches += 7 + nt;
     return ISL_OK;
 }
 
@@ -1112,25 +1844,133 @@ void launch_iter(const CzPlan& z, cudaStream_t st, const CzIter& a, int mode) {
     ((z).nc == 3 ? F<3, 6, 8>(__VA_ARGS__)                     \
                  : (z).m == 4 ? F<1, 4, 8>(__VA_ARGS__) : F<1, 3, 4>(__VA_ARGS__))
 
-int coarse_plan(isl_ctx* c, int nc, int64_t nrow) {
+int coarse_plan(isl_ctx* c, int nc, int64_t nrow, int ncta) {
     CzPlan& z = c->cz;
-    if (z.serial == c->pattern_serial && z.nc == nc) return ISL_OK;
-    z.ok = false;
-    z.num_serial = -1;
-    z.nc = nc;
-    z.m = nc == 3 ? 6 : 1 + c->dim;
-    z.nrow = nrow;
-    z.serial = c->pattern_serial;
-    if (nrow >= (1 << ROW_BITS) || c->fedeg > 2 || (c->fedeg == 2 && c->shape == ISL_HEX) || c->ninst != 1) return ISL_OK;
-    return CZ_DISPATCH(z, build_plan, c, z);
+    if (z.serial != c->pattern_serial || z.nc != nc) {
+        z.ok = z.sell_built = z.csr_built = false;
+        z.num_serial = z.sell_serial = z.csr_serial = -1;
+        z.nc = nc;
+        z.m = nc == 3 ? 6 : 1 + c->dim;
+        z.nrow = nrow;
+        z.serial = c->pattern_serial;
+        if (nrow >= (1 << ROW_BITS) || c->fedeg > 2 || (c->fedeg == 2 && c->shape == ISL_HEX) || c->ninst != 1) return ISL_OK;
+        const int rc = CZ_DISPATCH(z, build_plan, c, z);
+        if (rc != ISL_OK) return rc;
+    }
+    if (!z.ok) return ISL_OK;
+    if (ncta > 0) {
+        if (ncta != z.ncta) z.csr_built = false;
+        z.ncta = ncta;
+        return build_csr(c, z);
+    }
+    return nc == 1 ? build_sell(c, z) : ISL_OK;
 }
 
-int coarse_numeric(isl_ctx* c, const CzMat& A) {
+int coarse_numeric(isl_ctx* c, bool csr, float* dinv) {
     CzPlan& z = c->cz;
+    cudaStream_t st = c->stream;
+    const int n = (int)z.nrow;
+    CzMat A = {c->dsoff.p, c->dswid.p, nullptr, c->dscol.p, c->dsval.p};
+    if (csr && z.csr_serial != c->asm_serial) {
+        const unsigned g = (unsigned)std::min<int64_t>((n + 7) / 8, 32LL * c->sm_count);
+        if (z.nc == 3) k_pz_csr_values<3><<<g, 256, 0, st>>>(n, z.perm.p, c->dbptr.p, c->dsdst.p, c->dsval.p, z.rp.p, (int)z.nent, z.cv.p);
+        else k_pz_csr_values<1><<<g, 256, 0, st>>>(n, z.perm.p, c->drowptr.p, nullptr, c->dval32.p, z.rp.p, (int)z.nent, z.cv.p);
+        c->launches += 1;
+        z.csr_serial = c->asm_serial;
+    }
+    if (z.nc == 1) {
+        if (!csr && z.sell_serial != c->asm_serial) {
+            k_pz_values<<<grid_for(c, n), 256, 0, st>>>(n, z.perm.p, c->drowptr.p, c->dval32.p, z.soff.p, z.val.p);
+            c->launches += 1;
+            z.sell_serial = c->asm_serial;
+        }
+        k_pz_dinv<<<grid_for(c, n), 256, 0, st>>>(n, z.perm.p, c->ddiag.p, c->dval32.p, dinv);
+        c->launches += 1;
+        if (csr) A = {nullptr, nullptr, z.rp.p, z.ci.p, z.cv.p};
+        else A = {z.soff.p, z.swid.p, nullptr, z.col.p, z.val.p};
+    }
+    ISL_CHECK_CUDA(c, cudaGetLastError());
     if (z.num_serial == c->asm_serial) return ISL_OK;
     const int rc = CZ_DISPATCH(z, numeric, c, z, A);
     if (rc == ISL_OK) z.num_serial = c->asm_serial;
     return rc;
+}
+
+// shared memory of the one-launch solve; *ms, *as: the matrix and the rows of
+// the inverse fit too (in that order)
+constexpr size_t CLU_SMEM_MAX = 224 * 1024;
+static size_t cluster_smem(const CzPlan& z, bool* ms, bool* as) {
+    auto need = [&](bool m, bool s) {
+        return z.nc == 3 ? clu_smem<3, 6, 8>(z.max_rows, z.max_aggs, z.ndp, z.max_ent, m, s)
+               : z.m == 4 ? clu_smem<1, 4, 8>(z.max_rows, z.max_aggs, z.ndp, z.max_ent, m, s)
+                          : clu_smem<1, 3, 4>(z.max_rows, z.max_aggs, z.ndp, z.max_ent, m, s);
+    };
+    *ms = need(true, false) <= CLU_SMEM_MAX;
+    *as = need(*ms, true) <= CLU_SMEM_MAX;
+    return need(*ms, *as);
+}
+
+// 2: with its matrix on chip, 1: without, 0: not at all
+int coarse_cluster_fits(const isl_ctx* c, bool grid) {
+    bool ms = false, as = false;
+    int coop = 0;
+    if (grid && (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !coop)) return 0;
+    if (!c->cz.ok || !c->cz.csr_built || cluster_smem(c->cz, &ms, &as) > CLU_SMEM_MAX) return 0;
+    return ms ? 2 : 1;
+}
+
+// (the shared-memory limit of a kernel is the process's: always the same value,
+// as other threads may be launching it too)
+template <int NC, int M, int NW, int LPR, bool MS>
+static cudaError_t launch_clu(const CzPlan& z, bool grid, size_t smem, cudaStream_t st, CzClu a) {
+    if (grid) {
+        const bool wide = z.max_rows * LPR > 1024;  // more than two rounds of 512 threads in a product
+        const void* k = wide ? (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 1024>
+                             : (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 512>;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX);
+        if (e == cudaSuccess) e = cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), st);
+        void* args[] = {&a};
+        return e == cudaSuccess ? cudaLaunchCooperativeKernel(k, dim3(z.ncta), dim3(wide ? 1024 : 512), args, smem, st) : e;
+    }
+    auto k = k_cz_cluster<NC, M, NW, LPR, MS, false, 1024>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(z.ncta);
+    cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = z.ncta;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, k, &cfg);
+    if (e != cudaSuccess) return e;
+    if (n < 1) return cudaErrorInvalidConfiguration;
+    return cudaLaunchKernelEx(&cfg, k, a);
+}
+
+cudaError_t launch_coarse_cluster(isl_ctx* c, bool grid, bool arm, float* work, const float* dinv, double* x64, double tol, double drop,
+                                  int max_iter) {
+    CzPlan& z = c->cz;
+    bool ms, as;
+    const size_t smem = cluster_smem(z, &ms, &as);
+    const size_t na = (size_t)z.nc * z.nrow;
+    CzClu a = {z.lnode.p, z.sofs.p, z.cta.p, z.perm.p, z.dsub.p, z.ainv.p, z.ndp, z.rp.p, z.ci.p, z.cv.p, (int)z.nent, dinv,
+               z.rc.p, work, work + na, work + 2 * na, z.nc == 3 && c->bpad ? c->dbaeq.p : nullptr, c->drhs.p, x64,
+               c->drowptr.p, c->dcolind.p, c->dval64.p, c->dscal.p, tol, drop, max_iter, c->have64 ? 1 : 0,
+               z.max_rows, z.max_aggs, z.max_ent, reinterpret_cast<float2*>(c->dpart.p), c->dbar.p, as ? 1 : 0, arm ? 0x40000000u : 0u};
+    const double avg = (double)z.nent / (double)z.nrow;
+    cudaStream_t st = c->stream;
+    if (z.nc == 3) return ms ? launch_clu<3, 6, 8, 8, true>(z, grid, smem, st, a) : launch_clu<3, 6, 8, 8, false>(z, grid, smem, st, a);
+    if (z.m == 4) return ms ? launch_clu<1, 4, 8, 8, true>(z, grid, smem, st, a) : launch_clu<1, 4, 8, 8, false>(z, grid, smem, st, a);
+    if (avg > 12) return ms ? launch_clu<1, 3, 4, 8, true>(z, grid, smem, st, a) : launch_clu<1, 3, 4, 8, false>(z, grid, smem, st, a);
+    return ms ? launch_clu<1, 3, 4, 4, true>(z, grid, smem, st, a) : launch_clu<1, 3, 4, 4, false>(z, grid, smem, st, a);
 }
 
 void coarse_args(const isl_ctx* c, CzIter& a) {

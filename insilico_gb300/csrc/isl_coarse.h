@@ -28,20 +28,30 @@ struct CzIter {
     int max_iter;
 };
 
-// the FP32 matrix: sliced-ELL 3x3 blocks, or scalar CSR
+// the FP32 matrix: sliced-ELL 3x3 blocks, scalar sliced ELL, or scalar CSR
 struct CzMat {
     const int *soff, *swid, *rowptr, *col;
     const float* val;
 };
 
 // support points, boxes and row lists for the current pattern; c->cz.ok says
-// whether the two-level solve is available
-int coarse_plan(isl_ctx* c, int nc, int64_t nrow);
-// Galerkin blocks and the dense inverse for the current assembly
-int coarse_numeric(isl_ctx* c, const CzMat& A);
+// whether the two-level solve is available.  Scalar systems get their
+// aggregate-ordered sliced-ELL copy, or, with ncta > 0, the (block) CSR copy
+// of the one-cluster solve and its distribution over ncta CTAs.
+int coarse_plan(isl_ctx* c, int nc, int64_t nrow, int ncta);
+// for the current assembly: values of the aggregate-ordered copy, inverse
+// diagonal of scalar rows (in that order), Galerkin blocks, dense inverse
+int coarse_numeric(isl_ctx* c, bool csr, float* dinv);
 void coarse_args(const isl_ctx* c, CzIter& a);
 // update (or start, or restart) and coarse correction: two launches
 void launch_coarse(const isl_ctx* c, cudaStream_t st, const CzIter& a, int mode);
+// the whole solve in one launch, a thread-block cluster or a cooperative grid
+// of z.ncta CTAs (after coarse_plan with ncta > 0 and coarse_numeric): work
+// holds 3 vectors, the FP64 iterate goes to x64 and the record's fin, iters
+// and residuals to c->dscal.  arm: test hook, the grid barrier cannot complete
+int coarse_cluster_fits(const isl_ctx* c, bool grid);
+cudaError_t launch_coarse_cluster(isl_ctx* c, bool grid, bool arm, float* work, const float* dinv, double* x64, double tol,
+                                  double drop, int max_iter);
 void launch_coarse_dir(const isl_ctx* c, cudaStream_t st, int n, const float* z, float* p, const CGScal* S);
 
 }  // namespace isl

@@ -110,6 +110,7 @@ struct CGScal {
     double drop;
     int max_iter;
     int stall;   // reliable updates in a row without progress
+    int careful; // the iterated residual has drifted from the true one
     int fin;     // 1 converged, 2 iteration limit, 3 breakdown or stagnation
     int rst;     // a restart from the FP64 residual is due
     int fresh;   // ... with new directions
@@ -127,6 +128,22 @@ struct CzPlan {
     DBuf<int> amax;
     DBuf<unsigned long long> acc;
     DBuf<float> dsub, dagg, scale, rc, a, ainv, panel;
+    DBuf<int32_t> perm, pos;  // list order: row of every entry, entry of every row
+    std::vector<int32_t> hsofs;
+    // scalar systems: sliced-ELL copy in list order
+    bool sell_built = false, short_cols = false;
+    int64_t sell_serial = -1;
+    int nslice = 0;
+    DBuf<int32_t> soff, swid, srow, col;
+    DBuf<int16_t> col16;
+    DBuf<float> val;
+    // one-cluster solve: (block) CSR in list order, aggregates of every CTA
+    bool csr_built = false;
+    int64_t csr_serial = -1, nent = 0;
+    int ncta = 0, max_rows = 0, max_aggs = 0, max_ent = 0;
+    DBuf<int32_t> rp, ci, cta;
+    DBuf<float> cv;
+    std::vector<int32_t> hcta;
 };
 
 }  // namespace isl
@@ -317,6 +334,7 @@ struct isl_ctx {
     int spmv_lpr64 = 0, spmv_lpr32 = 0;  // autotuned lanes per row (FP32: 100 + U = sliced-ELL, U slots in flight)
     isl::CzPlan cz;              // two-level preconditioner of the mixed solve
     bool use_coarse = true;      // ISL_OPT_TWO_LEVEL
+    bool side_by_side = false;   // shares the GPU with other contexts: no launch over every SM
     cudaGraphExec_t cz_exec = nullptr;   // captured iterations of the two-level solve
     std::vector<uint64_t> cz_key;        // what the capture depends on
     cudaEvent_t cz_ev[2] = {nullptr, nullptr};

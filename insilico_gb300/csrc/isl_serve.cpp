@@ -263,6 +263,7 @@ void run_batch(isl_server* s, Batch& b) {
         // a one-launch solve of a small system holds every SM (cooperative
         // grid) and would serialise the batches that run at the same time
         SV_CHECK(isl_set_option(c, ISL_OPT_PERSISTENT, s->cfg.persistent == 1 ? 1 : 0));
+        c->side_by_side = s->cfg.persistent != 1;
     }
     std::vector<int64_t> eq_off(n + 1), dof_off(n + 1);
     int64_t ninst = 0;

@@ -2784,6 +2784,12 @@ int time_bspmv(isl_ctx* c, int nrep, double* ms) {
 // slot: a shorter chunk runs the (mostly idle) update kernels more often, a
 // longer one idles for longer after a stop.
 constexpr int CZ_CHUNK = 8;
+// Sizes from which the two-level solve is used: node blocks in one launch, node
+// blocks on the graph path (below, the one-level iteration of two launches and
+// a few hundred iterations ends as early), equations of scalar systems (below,
+// the one-level cluster solve: 7.9 us an iteration).
+constexpr int64_t CZ_MIN_NODES_ONE = 64, CZ_MIN_NODES = 1280, CZ_MIN_EQ = 2048;
+constexpr int64_t CZ_CLUSTER_ENTRIES = 160000;
 
 __global__ void __launch_bounds__(BS) k_rl_fold(int n, const int* __restrict__ aeq, float* __restrict__ x32,
                                                 double* __restrict__ x64, const CGScal* S) {
@@ -2829,15 +2835,18 @@ __global__ void __launch_bounds__(BS) k_rl_residual(int n, const int* __restrict
     S->rr_true = tot;
     if (tot <= S->threshold) { S->fin = 1; return; }
     if (S->iters >= S->max_iter) { S->fin = 2; return; }
-    // four updates in a row that did not halve the best residual: near the
-    // accuracy FP64 residuals can reach, the one-level iteration may still
-    // get below a tolerance that this one circles
-    S->stall = tot > 0.25 * S->rr_best ? S->stall + 1 : 0;
+    // six updates in a row that did not bring the best residual down by a
+    // tenth: near the accuracy FP64 residuals can reach, the one-level
+    // iteration may still get below a tolerance that this one circles
+    S->stall = tot > 0.81 * S->rr_best ? S->stall + 1 : 0;
     S->rr_best = fmin(S->rr_best, tot);
-    if (S->stall >= 4) { S->fin = 3; return; }
+    if (S->stall >= 6) { S->fin = 3; return; }
     S->fresh = S->rr_last > 0.0 && tot >= S->rr_last;
     S->rr_last = tot;
-    S->rrtrig = S->drop * tot;
+    // a recursion that agrees with the true residual may run twice as far (in
+    // digits) before the next update, unless it has ever been far from it
+    if (tot > 2.0 * S->rr) S->careful = 1;
+    S->rrtrig = (!S->careful && tot < 1.003 * S->rr ? S->drop * S->drop : S->drop) * tot;
     S->rst = 1;
 }
 
@@ -2862,19 +2871,113 @@ static void launch_rl_residual(isl_ctx* c, unsigned grid, cudaStream_t st, const
     }
 }
 
-// *ran = false: no usable coarse space, or the iteration broke down or
-// stagnated; the caller solves one-level
-static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* notconv,
-                           bool* ran) {
+// scalar product on the aggregate-ordered copy (t-space): the sliced-ELL
+// kernels of the one-level solve with U = 2, 4 or 8 slots in flight
+static void launch_pz_spmv(isl_ctx* c, int kind, cudaStream_t st, const float* p, float* q, CGScal* S) {
+    const CzPlan& z = c->cz;
+    const unsigned need = (unsigned)std::max(1, (z.nslice + BS / 32 - 1) / (BS / 32));
+    const bool s16 = z.short_cols && c->use_scol16;
+    auto run = [&](auto k16, auto k32, unsigned per_sm) {
+        const unsigned g = std::min(need, per_sm * (unsigned)c->sm_count);
+        if (s16) k16<<<g, BS, 0, st>>>(z.nslice, z.soff.p, z.swid.p, z.srow.p, z.col16.p, z.val.p, p, q, S, c->dpart.p);
+        else k32<<<g, BS, 0, st>>>(z.nslice, z.soff.p, z.swid.p, z.srow.p, z.col.p, z.val.p, p, q, S, c->dpart.p);
+    };
+    if (kind == 102) run(k_sspmv_batch<2, 8, short>, k_sspmv_batch<2, 8, int>, 8);
+    else if (kind == 108) run(k_sspmv_batch<8, 6, short>, k_sspmv_batch<8, 6, int>, 6);
+    else run(k_sspmv_batch<4, 8, short>, k_sspmv_batch<4, 8, int>, 8);
+}
+
+// slots in flight of that product: as set, from the tuning cache, or timed
+// (the first within 2 % of the fastest in a fixed order)
+static int pz_kind(isl_ctx* c, const float* p, float* q, CGScal* S) {
+    if (c->spmv32_forced) return c->spmv32_forced;
+    if (c->neq < 20000) return 104;
+    const int cand[3] = {104, 102, 108};
+    int cached = 0, best = 104;
+    if (tune_lookup(c, "spmv32", &cached) && std::find(cand, cand + 3, cached) != cand + 3) return cached;
+    float ms_of[3], bestms = 1e30f;
+    cudaMemsetAsync(S, 0, sizeof(CGScal), c->stream);
+    c->launches += 33;
+    for (int k = 0; k < 3; ++k) {
+        launch_pz_spmv(c, cand[k], c->stream, p, q, S);
+        cudaEventRecord(c->ev[2], c->stream);
+        for (int r = 0; r < 10; ++r) launch_pz_spmv(c, cand[k], c->stream, p, q, S);
+        cudaEventRecord(c->ev[3], c->stream);
+        cudaEventSynchronize(c->ev[3]);
+        cudaEventElapsedTime(&ms_of[k], c->ev[2], c->ev[3]);
+        bestms = std::min(bestms, ms_of[k]);
+    }
+    for (int k = 2; k >= 0; --k)
+        if (ms_of[k] <= 1.02f * bestms) best = cand[k];
+    tune_store(c, "spmv32", best);
+    return best;
+}
+
+// the one-launch form for small systems
+static int solve_two_level_cluster(isl_ctx* c, int nc, bool grid, double tol, int64_t max_iter, int64_t* iters,
+                                   double* rel, bool* ran) {
+    cudaStream_t st = c->stream;
+    const size_t n = (size_t)c->neq, na = (size_t)nc * c->cz.nrow;
+    double* x64 = c->w64.p;
+    float *V = c->w32.p, *d32 = nc == 3 ? c->dbinv.p : V + 3 * na;
+    int rc = coarse_numeric(c, true, d32);
+    if (rc != ISL_OK) return rc;
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(c->dscal.p, 0, sizeof(CGScal), st));
+    const bool arm = grid && c->barrier_test;
+    if (arm) c->barrier_test = false;
+    ISL_CHECK_CUDA(c, launch_coarse_cluster(c, grid, arm, V, d32, x64, tol, c->have64 ? c->ru_drop2 : 0.0,
+                                            (int)std::min<int64_t>(max_iter, INT32_MAX - 1)));
+    c->launches += 1;
+    rc = read_scal(c);
+    if (rc != ISL_OK) return rc;
+    const CGScal& h = *c->hscal;
+    if (h.fault) ISL_FAIL(c, ISL_ERR_TIMEOUT, "two-level CG: a grid barrier timed out");
+    if (h.fin != 1) return ISL_OK;
+    *ran = true;
+    *iters = h.iters;
+    *rel = h.rhsNorm2 > 0 ? std::sqrt(h.rr_true / h.rhsNorm2) : 0.0;
+    k_copy64<<<vec_grid(c), BS, 0, st>>>((int)n, x64, c->dsol.p);
+    c->launches += 1;
+    return ISL_OK;
+}
+
+// *ran = false: no usable coarse space, or the iteration broke down, stagnated
+// or met its limit; the caller solves one-level, so that a solve that does not
+// converge here ends as it does there
+static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* ran) {
     *ran = false;
     cudaStream_t st = c->stream;
     const size_t n = (size_t)c->neq;
     const int64_t rows = nc == 3 ? c->nbr : c->neq;
     const size_t na = (size_t)nc * rows;
-    int rc = coarse_plan(c, nc, rows);
+    int rc = ISL_OK;
+    if (nc == 3) {
+        rc = ensure_bsr(c);
+        if (rc != ISL_OK) return rc;
+    }
+    // One launch for the whole solve: a 16-CTA cluster for the smallest
+    // systems (a cluster barrier costs less than a grid barrier), a
+    // cooperative grid with one CTA per SM above (its shared memory holds
+    // matrices of up to about 30 MB), up to the sizes where the one-level solve
+    // leaves its one-launch kernels.  us per iteration, cluster / grid / three
+    // graph launches: 35k entries 9.5 / 11.3 / 28.7, 150k 9.7 / 12.4 / -,
+    // 190k 15.1 / 12.7 / 33, 1.9M - / 13.3 / 25, 6.9M - / 26.3 / 34.  A context that shares the GPU
+    // with others (side_by_side) takes the cluster, 16 SMs, or the graph.
+    const int64_t ent = nc == 3 ? 9 * c->nblk : c->nnz;
+    const bool one = c->use_persist == 1;
+    if ((one || c->side_by_side) && rows <= (nc == 3 ? PERSIST_MAX_NBR : CLUSTER_MAX_N)) {
+        for (int grid = one && ent > CZ_CLUSTER_ENTRIES; grid < (one ? 2 : 1); ++grid) {
+            const int ncta = grid ? c->sm_count : cluster_ctas(c);
+            if (ncta <= 0) continue;
+            rc = coarse_plan(c, nc, rows, ncta);
+            if (rc != ISL_OK || !c->cz.ok) return rc;
+            const int fit = coarse_cluster_fits(c, grid != 0);
+            if (grid ? fit > 0 : fit == 2) return solve_two_level_cluster(c, nc, grid != 0, tol, max_iter, iters, rel, ran);
+        }
+    }
+    if (rows < (nc == 3 ? CZ_MIN_NODES : CZ_MIN_EQ)) return ISL_OK;
+    rc = coarse_plan(c, nc, rows, 0);
     if (rc != ISL_OK || !c->cz.ok) return rc;
-    rc = nc == 3 ? ensure_bsr(c) : ensure_ssell(c);
-    if (rc != ISL_OK) return rc;
     const bool exact64 = c->have64;
     CGScal* S = c->dscal.p;
     double* W = c->w64.p;
@@ -2898,19 +3001,19 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
         // 5.21; at 270,400 nodes 21.4 against 18.5)
         if (c->fuse_dir && c->nslice <= 1024) kind = 9;
     } else {
-        if (!c->spmv_lpr32) {
-            ISL_CHECK_CUDA(c, cudaMemsetAsync(p32, 0, na * 4, st));
-            c->spmv_lpr32 = autotune_spmv32(c, p32, q32, S, c->dpart.p);
-        }
-        kind = c->spmv_lpr32;
-        k_dinv<float, float><<<grid, BS, 0, st>>>((int)n, c->ddiag.p, c->dval32.p, d32);
-        c->launches += 1;
+        kind = 104;
     }
     if (exact64 && !c->spmv_lpr64)
         c->spmv_lpr64 = autotune_lpr<double, double>(c, c->dval64.p, c->drhs.p, W + 3 * n, S, c->dpart.p);
-    CzMat A = {c->dsoff.p, c->dswid.p, c->drowptr.p, nc == 3 ? c->dscol.p : c->dcolind.p, nc == 3 ? c->dsval.p : c->dval32.p};
-    rc = coarse_numeric(c, A);
+    rc = coarse_numeric(c, false, d32);
     if (rc != ISL_OK) return rc;
+    if (nc == 1) {
+        if (!c->spmv_lpr32) {
+            ISL_CHECK_CUDA(c, cudaMemsetAsync(p32, 0, na * 4, st));
+            c->spmv_lpr32 = pz_kind(c, p32, q32, S);
+        }
+        kind = c->spmv_lpr32 >= 100 ? c->spmv_lpr32 : 104;  // CSR kinds: the one-level solve's
+    }
     const bool fused = nc == 3 && c->fuse_dir && (kind == 9 || bspmv_dir_kind(kind));
     CzIter a = {};
     coarse_args(c, a);
@@ -2918,7 +3021,7 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
     a.p1 = p32; a.p2 = fused ? p32b : nullptr; a.pz = p32;
     a.q = q32; a.dinv = d32;
     a.b64 = c->drhs.p;
-    a.aeq = nc == 3 && c->bpad ? c->dbaeq.p : nullptr;
+    a.aeq = nc == 1 ? c->cz.perm.p : c->bpad ? c->dbaeq.p : nullptr;
     a.S = S; a.part = c->dpart.p;
     a.tol = tol; a.drop = exact64 ? c->ru_drop2 : 0.0;
     a.max_iter = (int)std::min<int64_t>(max_iter, INT32_MAX - 1);
@@ -2936,9 +3039,9 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
     auto u = [](const void* p) { return (uint64_t)(uintptr_t)p; };
     std::vector<uint64_t> key = {(uint64_t)nc, (uint64_t)kind, (uint64_t)fused, (uint64_t)exact64, (uint64_t)rows, (uint64_t)n,
                                  (uint64_t)c->cz.nagg, (uint64_t)c->cz.ndp, (uint64_t)c->spmv_lpr64,
-                                 (uint64_t)(c->use_scol16 && (nc == 3 ? c->scol16 : c->ss16)), (uint64_t)c->pattern_serial,
+                                 (uint64_t)(c->use_scol16 && (nc == 3 ? c->scol16 : c->cz.short_cols)), (uint64_t)c->pattern_serial,
                                  u(a.lnode), u(a.sofs), u(a.dsub), u(a.ainv), u(a.rc), u(V), u(W), u(a.dinv), u(a.aeq), u(S),
-                                 u(a.part), u(c->dsval.p), u(c->dbval.p), u(c->dss_val.p), u(c->dval32.p), u(c->dval64.p),
+                                 u(a.part), u(c->dsval.p), u(c->dbval.p), u(c->cz.val.p), u(c->dval32.p), u(c->dval64.p),
                                  u(c->drhs.p), u(c->drowptr.p), u(c->dcolind.p), u(c->dscol.p), u(c->dscol16.p)};
     if (!c->cz_exec || key != c->cz_key) {
         if (c->cz_exec) { cudaGraphExecDestroy(c->cz_exec); c->cz_exec = nullptr; }
@@ -2950,7 +3053,7 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
             } else {
                 launch_coarse_dir(c, st, (int)na, z32, p32, S);
                 if (nc == 3) launch_bspmv(kind, grid, st, c, p32, q32, S, c->dpart.p);
-                else launch_spmv32(c, kind, grid, st, p32, q32, S, c->dpart.p);
+                else launch_pz_spmv(c, kind, st, p32, q32, S);
             }
             launch_coarse(c, st, a, CZ_UPDATE);
         }
@@ -2984,19 +3087,14 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
         if (c->hscal[(k - 1) & 1].fin) break;
     }
     const CGScal h = c->hscal[(k - 1) & 1];
-    if (h.fin == 3) return ISL_OK;  // *ran stays false
+    if (h.fin != 1) return ISL_OK;  // *ran stays false
     *ran = true;
     *iters = h.iters;
     *rel = h.rhsNorm2 > 0 ? std::sqrt(h.rr_true / h.rhsNorm2) : 0.0;
-    *notconv = h.fin == 2;
     k_copy64<<<grid, BS, 0, st>>>((int)n, x64, c->dsol.p);
     c->launches += 1;
     return ISL_OK;
 }
-
-// Sizes from which the two-level solve takes over from the one-launch kernels
-// of small systems, whose iterations cost less than three launches.
-constexpr int64_t CZ_MIN_NODES = 1280, CZ_MIN_EQ = 2048;
 
 int solve_device(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t* iters, double* relres) {
     int rc = ensure_work(c);
@@ -3022,8 +3120,11 @@ int solve_device(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t* 
     else {
         const bool b3 = c->blocked && c->use_block && (c->have64 || c->have32);
         bool ran = false;
-        if (c->use_coarse && c->use_persist != 2 && (b3 ? c->nbr >= CZ_MIN_NODES : (int64_t)c->neq >= CZ_MIN_EQ))
-            rc = solve_two_level(c, b3 ? 3 : 1, tol, max_iter, &it, &rel, &nc, &ran);
+        if (c->use_coarse && c->use_persist != 2 && (b3 ? c->nbr >= CZ_MIN_NODES_ONE : (int64_t)c->neq >= CZ_MIN_EQ)) {
+            // a healthy two-level solve takes far fewer iterations than this
+            const int64_t limit = std::min(max_iter, std::max<int64_t>(1000, (int64_t)c->neq / 4));
+            rc = solve_two_level(c, b3 ? 3 : 1, tol, limit, &it, &rel, &ran);
+        }
         if (rc == ISL_OK && !ran)
             rc = b3 ? solve_mixed_b3(c, tol, max_iter, &it, &rel, &nc) : solve_mixed(c, tol, max_iter, &it, &rel, &nc);
     }
