@@ -336,7 +336,9 @@ int isl_timings(isl_ctx* ctx, double* ms /* [ISL_NTIMERS] */, int64_t* counts /*
  * most 32,768 nodes runs its iterations in a persistent cooperative kernel;
  * with the two-level preconditioner (ISL_OPT_TWO_LEVEL) the smallest of these
  * run in one cluster and the others in one cooperative launch over every SM.
- * 2: the persistent one-level block kernel at every size.  ISL_OPT_BARRIER_TEST (test
+ * 2: the persistent one-level block kernel at every size.  With 1, the FP64
+ * CG and BiCGSTAB of at most 65,536 equations run in one cooperative launch too
+ * (the same recurrences; ISL_OPT_BICGSTAB_KIND then reads 8).  ISL_OPT_BARRIER_TEST (test
  * hook, write-only, one-shot): the next persistent launch starts with its grid
  * barrier armed so that it cannot complete; its bounded wait runs out and the
  * solve returns ISL_ERR_TIMEOUT with the context still usable.

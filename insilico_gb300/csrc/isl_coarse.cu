@@ -386,7 +386,6 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     cgrp::cluster_group cl = cgrp::this_cluster();
     extern __shared__ __align__(16) float smem[];
     __shared__ float2 red[4][16];
-    __shared__ int sc_ok;
     __shared__ float bs[2][32];
     __shared__ double shd[32];
     __shared__ float sc_alpha, sc_beta;
@@ -448,33 +447,10 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     }
     int slot = 0;
     bool alive = true;  // grid form: false in every thread once a barrier has timed out
-    unsigned goal = a.armed;  // grid form: arrivals that complete the next barrier
+    GridBarrier gb(a.bar, &a.S->fault, a.armed);
     auto sync_all = [&]() {
-        if constexpr (GRID) {
-            // one counter that only grows: arrive with a release add, poll it
-            // with acquire loads (bounded; a fault makes every CTA leave)
-            goal += gridDim.x;
-            __syncthreads();
-            if (tid == 0) {
-                unsigned v;
-                int ok = 1;
-                asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(a.bar) : "memory");
-                for (unsigned it = 0;; ++it) {
-                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-                    if (v >= goal) break;
-                    if (it > GRID_SYNC_LIMIT || ((it & 255) == 255 && *(volatile int*)&a.S->fault)) {
-                        ok = 0;
-                        atomicExch(&a.S->fault, 1);
-                        break;
-                    }
-                }
-                sc_ok = ok;
-            }
-            __syncthreads();
-            alive = sc_ok != 0;
-        } else {
-            cl.sync();
-        }
+        if constexpr (GRID) alive = gb.sync();
+        else cl.sync();
     };
     // sums over all CTAs of u, and of v if TWO: valid in thread 0 of every CTA.
     // FP32 inside a CTA (at most a few thousand rows), double-float across.

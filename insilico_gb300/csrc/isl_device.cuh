@@ -82,6 +82,39 @@ __device__ inline bool grid_sync(unsigned* bar, int* fault) {
     return gs_ok != 0;
 }
 
+// Grid barrier on one counter that only grows (zeroed before the launch): every
+// CTA arrives with a release add and polls for the arrivals that complete the
+// barrier, without the second word of grid_sync.  Bounded; on expiry, or when
+// another CTA has set *fault, it reports false in every thread of the CTA.
+struct GridBarrier {
+    unsigned* bar;
+    int* fault;
+    unsigned goal;
+    __device__ GridBarrier(unsigned* b, int* f, unsigned start = 0) : bar(b), fault(f), goal(start) {}
+    __device__ bool sync() {
+        __shared__ int gb_ok;
+        goal += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned v;
+            int ok = 1;
+            asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(bar) : "memory");
+            for (unsigned it = 0;; ++it) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+                if (v >= goal) break;
+                if (it > GRID_SYNC_LIMIT || ((it & 255) == 255 && *(volatile int*)fault)) {
+                    ok = 0;
+                    atomicExch(fault, 1);
+                    break;
+                }
+            }
+            gb_ok = ok;
+        }
+        __syncthreads();
+        return gb_ok != 0;
+    }
+};
+
 // fixed-order block reduction of a double (deterministic); result in thread 0
 __device__ inline double block_sum(double v, double* sh) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

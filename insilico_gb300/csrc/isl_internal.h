@@ -116,6 +116,12 @@ struct CGScal {
     int fresh;   // ... with new directions
 };
 
+// result of a one-launch FP64 solve (isl_onelaunch.cu)
+struct OlScal {
+    double rr, rhs2;
+    int fin, iters, fault, over;
+};
+
 // two-level preconditioner (isl_coarse.cu): aggregates of the current pattern
 // and their matrices for the current assembly
 struct CzPlan {
@@ -332,6 +338,8 @@ struct isl_ctx {
     isl::DBuf<isl::CGScal> dscal;
     isl::CGScal* hscal = nullptr;  // pinned host mirror
     int spmv_lpr64 = 0, spmv_lpr32 = 0;  // autotuned lanes per row (FP32: 100 + U = sliced-ELL, U slots in flight)
+    isl::DBuf<int32_t> ol_row0;  // one-launch FP64 solves: row ranges of the CTAs, result
+    isl::DBuf<isl::OlScal> ol_scal;
     isl::CzPlan cz;              // two-level preconditioner of the mixed solve
     bool use_coarse = true;      // ISL_OPT_TWO_LEVEL
     bool side_by_side = false;   // shares the GPU with other contexts: no launch over every SM
@@ -439,6 +447,7 @@ int ensure_val32(isl_ctx* c);
 int affine_lift(isl_ctx* c, int incremental);
 int inst_norms_device(isl_ctx* c, double* out);
 int distribute_masked(isl_ctx* c, int add);
+int solve_onelaunch(isl_ctx* c, bool bicg, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* nc, bool* ran);
 int solve_bicgstab(isl_ctx* c, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* nc);
 bool bicgstab_kind_valid(const isl_ctx* c, int kind);
 }  // namespace isl

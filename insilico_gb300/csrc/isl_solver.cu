@@ -3115,8 +3115,14 @@ int solve_device(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t* 
         rc = solve_batched(c, method, tol, max_iter, &it, &rel);
         nc = (rc == ISL_ERR_NOT_CONVERGED);
         if (rc == ISL_ERR_NOT_CONVERGED) rc = ISL_OK;
-    } else if (method == ISL_SOLVE_BICGSTAB) rc = solve_bicgstab(c, tol, max_iter, &it, &rel, &nc);
-    else if (method == ISL_SOLVE_CG_FP64) rc = solve_fp64(c, tol, max_iter, &it, &rel, &nc);
+    } else if (method == ISL_SOLVE_BICGSTAB || method == ISL_SOLVE_CG_FP64) {
+        const bool bicg = method == ISL_SOLVE_BICGSTAB;
+        bool ran = false;
+        if (!bicg || !c->bicg_forced) rc = solve_onelaunch(c, bicg, tol, max_iter, &it, &rel, &nc, &ran);
+        if (rc == ISL_OK && ran && bicg && !c->bicg_lpr) c->bicg_lpr = 8;  // lanes per row of its product
+        if (rc == ISL_OK && !ran)
+            rc = bicg ? solve_bicgstab(c, tol, max_iter, &it, &rel, &nc) : solve_fp64(c, tol, max_iter, &it, &rel, &nc);
+    }
     else {
         const bool b3 = c->blocked && c->use_block && (c->have64 || c->have32);
         bool ran = false;
