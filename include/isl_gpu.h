@@ -349,7 +349,8 @@ int isl_timings(isl_ctx* ctx, double* ms /* [ISL_NTIMERS] */, int64_t* counts /*
  * its copy at its first mixed solve); read back, the kind in use (0 before
  * the first mixed solve).  ISL_OPT_SCALAR_SLOTS (read-only): slots
  * of the scalar sliced-ELL copy, padding included; 0 when there is none
- * (node-blocked, batched, or fewer than 20,000 equations).
+ * (node-blocked, batched, or fewer than 20,000 equations); on a batch, the
+ * stored entries of the copy that its last mixed solve read.
  * ISL_OPT_HOST_SETUP (default 0): with a device, isl_field_create numbers the
  * DOF objects of fields of degree > 1 and isl_boundary_faces /
  * isl_boundary_points find the boundary on the GPU (sorts and scans, the
@@ -370,7 +371,10 @@ enum { ISL_OPT_BLOCK_SOLVER = 0, ISL_OPT_BLOCKED = 1, ISL_OPT_NBLOCKS = 2, ISL_O
  * Galerkin matrix), which takes far fewer iterations to the same tolerance; 0
  * keeps (block) Jacobi alone.  A system without usable support points, or one
  * that the two-level iteration does not bring to the tolerance, is solved with
- * (block) Jacobi.  A scalar system is multiplied in the order of its
+ * (block) Jacobi.  Every instance of a batch is solved so, in launches that
+ * hold as many instances at once as the GPU takes (unless
+ * ISL_OPT_SPMV32_KIND sets a product of the one-level batched solve, or
+ * ISL_OPT_PERSISTENT is not 1).  A scalar system is multiplied in the order of its
  * aggregates: ISL_OPT_SPMV32_KIND then chooses the slots in flight (102, 104,
  * 108); its CSR kinds apply to the one-level solve. */
 /* ISL_OPT_SHARED_GEOMETRY (default 1): the direct block assembly

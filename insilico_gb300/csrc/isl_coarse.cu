@@ -350,7 +350,11 @@ struct CzClu {
     const float4* lnode;
     const int *sofs, *cta, *perm;
     const float *dsub, *ainv;
-    int ndp;
+    const CzInst* inst;
+    const int* order;        // batch: the instance of every cluster
+    int inst_id;             // the instance, where order is null
+    OlScal* res;             // batch: results (null: S)
+    int max_ndp;
     const int *rp, *ci;      // (block) CSR in list order
     const float* val;        // [NC * NC][nent]
     int nent;
@@ -391,14 +395,20 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     __shared__ float sc_alpha, sc_beta;
     __shared__ int sc_ctl;
     const int rank = GRID ? (int)blockIdx.x : (int)cl.block_rank(), ncta = GRID ? (int)gridDim.x : (int)cl.num_blocks();
+    const int inst = !GRID && a.order ? a.order[blockIdx.x / ncta] : a.inst_id;
+    const CzInst in = a.inst[inst];
+    const int ndp = in.ndp;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const int ag0 = a.cta[rank], ag1 = a.cta[rank + 1], na = ag1 - ag0;
+    const int* cta = a.cta + (!GRID && a.order ? (size_t)inst * (ncta + 1) : 0);
+    const int ag0 = cta[rank], ag1 = cta[rank + 1], na = ag1 - ag0;
+    const int c0 = (ag0 - in.agg0) * M;                // first coarse unknown of this CTA
+    const float* ainv = a.ainv + in.a0 + (size_t)c0 * ndp;
     const int t0 = a.sofs[ag0 * NW], nr = a.sofs[ag1 * NW] - t0;
     const int R = a.max_rows;
     float4* ln = reinterpret_cast<float4*>(smem);     // positions; w: aggregate (local), mask above
     float* rcs = smem + 4 * (size_t)R;                // [ndp], 16-byte aligned as ln
-    float* ais = rcs + a.ndp;                         // [agg M][ndp]
-    float* xs = ais + (a.inv_smem ? (size_t)a.max_aggs * M * a.ndp : 0);
+    float* ais = rcs + a.max_ndp;                     // [agg M][ndp]
+    float* xs = ais + (a.inv_smem ? (size_t)a.max_aggs * M * a.max_ndp : 0);
     float* rs = xs + (size_t)NC * R;
     float* qs = rs + (size_t)NC * R;
     float* zs = qs + (size_t)NC * R;
@@ -419,8 +429,8 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
             ln[t - t0] = L;
         }
     }
-    for (int k = tid; a.inv_smem && k < na * M * (a.ndp / 4); k += CLT)
-        reinterpret_cast<float4*>(ais)[k] = reinterpret_cast<const float4*>(a.ainv + (size_t)(ag0 * M) * a.ndp)[k];
+    for (int k = tid; a.inv_smem && k < na * M * (ndp / 4); k += CLT)
+        reinterpret_cast<float4*>(ais)[k] = reinterpret_cast<const float4*>(ainv)[k];
     for (int k = tid; k < na * NW * M * M; k += CLT) dss[k] = a.dsub[(size_t)(ag0 * NW) * (M * M) + k];
     const int e0 = a.rp[t0];
     for (int i = tid; i < nr; i += CLT) {
@@ -591,26 +601,26 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
             }
         }
         __syncthreads();
-        float* rcg = a.rc + (size_t)par * a.ndp;
+        float* rcg = a.rc + in.rc0 + (size_t)par * ndp;
         for (int k = tid; k < na * M; k += CLT) {
             float s = 0.f;
 #pragma unroll
             for (int j = 0; j < NW; ++j) s += src[((k / M) * NW + j) * M + k % M];
-            rcg[ag0 * M + k] = s;
+            rcg[c0 + k] = s;
         }
     };
     // after the barrier that made P^T r visible: w = z + P A_c^-1 P^T r (own rows);
     // this CTA's part of the coarse term of r.z in thread 0's return value
     auto coarse_part = [&]() -> float {
-        const float* rcg = a.rc + (size_t)par * a.ndp;
-        for (int k = tid; k < a.ndp; k += CLT) rcs[k] = rcg[k];
+        const float* rcg = a.rc + in.rc0 + (size_t)par * ndp;
+        for (int k = tid; k < ndp; k += CLT) rcs[k] = rcg[k];
         par ^= 1;
         __syncthreads();
-        const int n4 = a.ndp / 4;
+        const int n4 = ndp / 4;
         const float4* rc4 = reinterpret_cast<const float4*>(rcs);
         float part = 0.f;
         for (int k = w; k < na * M; k += CLT / 32) {
-            const float4* row = reinterpret_cast<const float4*>(a.inv_smem ? ais + (size_t)k * a.ndp : a.ainv + (size_t)(ag0 * M + k) * a.ndp);
+            const float4* row = reinterpret_cast<const float4*>((a.inv_smem ? ais : ainv) + (size_t)k * ndp);
             float s = 0.f;
 #pragma unroll 4
             for (int j = lane; j < n4; j += 32) {
@@ -621,7 +631,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             if (lane == 0) {
                 zcs[k] = s;
-                part += s * rcs[ag0 * M + k];
+                part += s * rcs[c0 + k];
             }
         }
         __syncthreads();
@@ -822,7 +832,13 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
         __syncthreads();
         alpha = sc_alpha;
     }
-    if (rank == 0 && tid == 0) {
+    if (rank == 0 && tid == 0 && a.res) {
+        OlScal* S = a.res + inst;
+        S->fin = ctl;
+        S->iters = iters;
+        S->rr = rr_true;
+        S->rhs2 = bn;
+    } else if (rank == 0 && tid == 0) {
         CGScal* S = a.S;
         S->fin = ctl;
         S->iters = iters;
@@ -836,14 +852,33 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
 // ---------------------------------------------------------------------------
 // Numeric setup, once per assembly
 
-// largest diagonal entry (its bits order as integers)
+// instance of a row
+__device__ inline int inst_of(const CzInst* __restrict__ inst, int ninst, int row) {
+    int lo = 0, hi = ninst;  // the last one that starts at or before the row (empty ones start where the next does)
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (inst[mid].row0 <= row) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// largest diagonal entry of every instance (its bits order as integers)
 template <typename T>
-__global__ void k_cz_amax(int n, const int* __restrict__ diag, const T* __restrict__ val, int* __restrict__ out) {
+__global__ void k_cz_amax(int n, int ninst, const CzInst* __restrict__ inst, const int* __restrict__ diag, const T* __restrict__ val,
+                          int* __restrict__ out) {
     float m = 0.f;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float v = fabsf((float)val[diag[i]]);
-        if (v < INFINITY) m = fmaxf(m, v);
+        if (!(v < INFINITY)) continue;
+        if (ninst > 1) {
+            int* o = out + inst_of(inst, ninst, i);
+            if (__float_as_int(v) > *(volatile int*)o) atomicMax(o, __float_as_int(v));
+        } else {
+            m = fmaxf(m, v);
+        }
     }
+    if (ninst > 1) return;
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_int(m));
 }
@@ -860,13 +895,16 @@ __device__ inline float fix_scale(int amax_bits) {  // 2^(FIX_BITS - e), amax < 
 // entries towards earlier ones follow by symmetry).
 template <int NC, int M, int NW>
 __global__ void __launch_bounds__(NW * 32) k_cz_galerkin(CzMat A, const float4* __restrict__ lnode, const float4* __restrict__ yrow,
-                                                         const int* __restrict__ sofs, int ndp, const int* __restrict__ amax,
+                                                         const int* __restrict__ sofs, const CzInst* __restrict__ inst,
+                                                         const int* __restrict__ agg_inst, const int* __restrict__ amax,
                                                          unsigned long long* __restrict__ acc, float* __restrict__ dsub,
                                                          float* __restrict__ dagg) {
     __shared__ float own[NW][M * M];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int I = blockIdx.x, sub = I * NW + w;
-    const float scale = fix_scale(*amax);
+    const int ik = agg_inst[I], ndp = inst[ik].ndp, agg0 = inst[ik].agg0;
+    acc += inst[ik].a0;
+    const float scale = fix_scale(amax[ik]);
     float a1[M * M], a2[M * M];
 #pragma unroll
     for (int k = 0; k < M * M; ++k) a1[k] = a2[k] = 0.f;
@@ -896,7 +934,7 @@ __global__ void __launch_bounds__(NW * 32) k_cz_galerkin(CzMat A, const float4* 
         auto flush = [&]() {
             float o[M * M];
             outer(Tc, L, o, false);
-            unsigned long long* dst = acc + (size_t)(I * M) * ndp + (size_t)J * M;
+            unsigned long long* dst = acc + (size_t)((I - agg0) * M) * ndp + (size_t)(J - agg0) * M;
 #pragma unroll
             for (int m = 0; m < M; ++m)
 #pragma unroll
@@ -1034,13 +1072,20 @@ __global__ void k_cz_scale(int nagg, const float* __restrict__ dagg, float* __re
     }
 }
 
-// the scaled coarse matrix, padded with the identity to whole tiles
+// the scaled coarse matrix of every instance, padded with the identity to whole tiles
 template <int M>
-__global__ void k_cz_form(int nd, int ndp, const unsigned long long* __restrict__ acc, const float* __restrict__ dagg,
+__global__ void k_cz_form(const CzInst* __restrict__ inst, const unsigned long long* __restrict__ acc, const float* __restrict__ dagg,
                           const float* __restrict__ s, const int* __restrict__ amax, float* __restrict__ A) {
-    const float inv = 1.f / fix_scale(*amax);
+    const CzInst in = inst[blockIdx.z];
+    const int nd = in.nd, ndp = in.ndp;
+    if ((int)blockIdx.x * 32 >= ndp || (int)blockIdx.y * 32 >= ndp) return;
+    acc += in.a0;
+    A += in.a0;
+    dagg += (size_t)in.agg0 * (M * M);
+    s += in.agg0 * M;
+    const float inv = 1.f / fix_scale(amax[blockIdx.z]);
     const int j = blockIdx.x * 32 + (threadIdx.x & 31);
-    for (int i = blockIdx.y * 32 + (threadIdx.x >> 5); i < blockIdx.y * 32 + 32; i += 8) {
+    for (int i = blockIdx.y * 32 + (threadIdx.x >> 5); i < (int)blockIdx.y * 32 + 32; i += 8) {
         float v = 0.f;
         if (i == j) v = 1.f + REG;
         else if (i < nd && j < nd) {
@@ -1149,10 +1194,14 @@ __device__ __forceinline__ void tile_load(const float* g, int ld, float (*X)[TB 
 }
 
 // the first panel and the inverse of the first diagonal tile
-__global__ void __launch_bounds__(256) k_gj_first(const float* __restrict__ A, int n, float* __restrict__ P, float* __restrict__ Dinv) {
+__global__ void __launch_bounds__(256) k_gj_first(const CzInst* __restrict__ inst, const float* __restrict__ A, float* __restrict__ panel) {
     __shared__ float X[TB][TB + 1];
     __shared__ float buf[2][2 * TB];
-    const int I = blockIdx.x;
+    const CzInst in = inst[blockIdx.y];
+    const int n = in.ndp, I = blockIdx.x;
+    if (I * TB >= n) return;
+    A += in.a0;
+    float *P = panel + in.p0, *Dinv = P + (size_t)2 * TB * n;
     tile_load(A + (size_t)(I * TB) * n, n, X);
     __syncthreads();
     for (int e = threadIdx.x; e < TB * TB; e += 256) P[(size_t)I * TB * TB + e] = X[e / TB][e % TB];
@@ -1161,15 +1210,23 @@ __global__ void __launch_bounds__(256) k_gj_first(const float* __restrict__ A, i
     for (int e = threadIdx.x; e < TB * TB; e += 256) Dinv[e] = X[e / TB][e % TB];
 }
 
-__global__ void __launch_bounds__(256) k_gj_step(float* __restrict__ A, int n, int k, const float* __restrict__ Dinv,
-                                                 float* __restrict__ Dnext, const float* __restrict__ P, float* __restrict__ Pnext) {
+__global__ void __launch_bounds__(256) k_gj_step(const CzInst* __restrict__ inst, int k, float* __restrict__ A, float* __restrict__ panel) {
     extern __shared__ __align__(16) float gj_smem[];
     typedef float (*Tile)[TB + 1];
     Tile X = reinterpret_cast<Tile>(gj_smem), Y = X + TB, Z = Y + TB;
     __shared__ float buf[2][2 * TB];
+    const CzInst in = inst[blockIdx.y];
+    const int n = in.ndp, nt = n / TB;
+    if (k >= nt || (int)blockIdx.x >= nt * (nt + 1) / 2) return;
+    A += in.a0;
+    panel += in.p0;
+    const float* P = panel + (size_t)(k & 1) * TB * n;
+    float* Pnext = panel + (size_t)((k + 1) & 1) * TB * n;
+    const float* Dinv = panel + (size_t)2 * TB * n + (k & 1) * TB * TB;
+    float* Dnext = panel + (size_t)2 * TB * n + ((k + 1) & 1) * TB * TB;
     // tile (I, J), J <= I, of the linear index; the next diagonal tile comes first
     int t = blockIdx.x;
-    const int nt = n / TB, first = k + 1 < nt ? (k + 1) * (k + 2) / 2 + k + 1 : -1;
+    const int first = k + 1 < nt ? (k + 1) * (k + 2) / 2 + k + 1 : -1;
     if (first >= 0) t = t == 0 ? first : (t <= first ? t - 1 : t);
     int I = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
     while ((I + 1) * (I + 2) / 2 <= t) ++I;
@@ -1256,8 +1313,16 @@ __global__ void __launch_bounds__(256) k_gj_step(float* __restrict__ A, int n, i
 constexpr int GJ_SMEM = 3 * TB * (TB + 1) * 4;
 
 // undo the sign and the scaling, and fill the upper triangle from the lower
-__global__ void k_cz_unscale(int nd, int ndp, const float* __restrict__ A, const float* __restrict__ s, float* __restrict__ out) {
+template <int M>
+__global__ void k_cz_unscale(const CzInst* __restrict__ inst, const float* __restrict__ A, const float* __restrict__ s,
+                             float* __restrict__ out) {
     __shared__ float T[32][33];
+    const CzInst in = inst[blockIdx.z];
+    const int nd = in.nd, ndp = in.ndp;
+    if ((int)blockIdx.x * 32 >= ndp || (int)blockIdx.y * 32 >= ndp) return;
+    A += in.a0;
+    out += in.a0;
+    s += in.agg0 * M;
     const int bi = blockIdx.y, bj = blockIdx.x, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const bool low = bj <= bi;
     for (int r = ty; r < 32; r += 8)
@@ -1340,13 +1405,23 @@ inline float f_unorder(unsigned u) {
     return c.f;
 }
 
-__global__ void k_cz_bounds(int n, const float4* __restrict__ xr, unsigned* __restrict__ mm) {
+__global__ void k_cz_bounds(int n, int ninst, const CzInst* __restrict__ inst, const float4* __restrict__ xr, unsigned* __restrict__ mm) {
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float v[3] = {xr[i].x, xr[i].y, xr[i].z};
+        if (ninst > 1) {
+            unsigned* o = mm + 6 * inst_of(inst, ninst, i);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const unsigned u = f_order(v[d]);
+                if (u < *(volatile unsigned*)(o + d)) atomicMin(o + d, u);
+                if (u > *(volatile unsigned*)(o + 3 + d)) atomicMax(o + 3 + d, u);
+            }
+        }
 #pragma unroll
         for (int d = 0; d < 3; ++d) { lo[d] = fminf(lo[d], v[d]); hi[d] = fmaxf(hi[d], v[d]); }
     }
+    if (ninst > 1) return;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -1357,14 +1432,27 @@ __global__ void k_cz_bounds(int n, const float4* __restrict__ xr, unsigned* __re
     }
 }
 
-struct Box3 { float lo[3], inv[3]; int m[3]; };  // m: boxes per direction
+struct Box3 { float lo[3], inv[3]; int m[3], base; };  // m: boxes per direction, base: the instance's first box
 
 __device__ inline int bin_of(const Box3& b, int d, float x) {
     return min(NBIN - 1, max(0, (int)((x - b.lo[d]) * b.inv[d])));
 }
 
-__global__ void k_cz_hist(int n, Box3 b, const float4* __restrict__ xr, int* __restrict__ hist) {
+// rows per bin, axis and instance
+__global__ void k_cz_hist(int n, int ninst, const CzInst* __restrict__ inst, const Box3* __restrict__ box,
+                          const float4* __restrict__ xr, int* __restrict__ hist) {
     __shared__ int h[3 * NBIN];
+    if (ninst > 1) {
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            const int k = inst_of(inst, ninst, i);
+            const Box3 b = box[k];
+            const float v[3] = {xr[i].x, xr[i].y, xr[i].z};
+#pragma unroll
+            for (int d = 0; d < 3; ++d) atomicAdd(&hist[((size_t)k * 3 + d) * NBIN + bin_of(b, d, v[d])], 1);
+        }
+        return;
+    }
+    const Box3 b = box[0];
     for (int k = threadIdx.x; k < 3 * NBIN; k += blockDim.x) h[k] = 0;
     __syncthreads();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1377,16 +1465,21 @@ __global__ void k_cz_hist(int n, Box3 b, const float4* __restrict__ xr, int* __r
         if (h[k]) atomicAdd(&hist[k], h[k]);
 }
 
-// raw key of every row: (box, component) and sub-box; cut[d][bin] is the
-// half-box index along d
+// raw key of every row: (box, component) and sub-box; cut[instance][d][bin] is
+// the half-box index along d
 template <int NC, int NW>
-__global__ void k_cz_key(int n, Box3 b, const unsigned short* __restrict__ cut, int ncomp, const float4* __restrict__ xr,
-                         int* __restrict__ key, int* __restrict__ cnt) {
+__global__ void k_cz_key(int n, int ninst, const CzInst* __restrict__ inst, const Box3* __restrict__ box,
+                         const unsigned short* __restrict__ cut, int ncomp, const float4* __restrict__ xr, int* __restrict__ key,
+                         int* __restrict__ cnt) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int k = ninst > 1 ? inst_of(inst, ninst, i) : 0;
+        const Box3 b = box[k];
+        const unsigned short* q = cut + (size_t)k * 3 * NBIN;
         const float4 v = xr[i];
-        const int h0 = cut[bin_of(b, 0, v.x)], h1 = cut[NBIN + bin_of(b, 1, v.y)], h2 = cut[2 * NBIN + bin_of(b, 2, v.z)];
+        const int h0 = q[bin_of(b, 0, v.x)], h1 = q[NBIN + bin_of(b, 1, v.y)], h2 = q[2 * NBIN + bin_of(b, 2, v.z)];
         int g = ((h2 >> 1) * b.m[1] + (h1 >> 1)) * b.m[0] + (h0 >> 1);
         if (NC == 1) g = g * ncomp + __float_as_int(v.w);
+        g += b.base;
         const int s = (h0 & 1) | (h1 & 1) << 1 | (NW == 8 ? (h2 & 1) << 2 : 0);
         key[i] = g * NW + s;
         atomicAdd(&cnt[g * NW + s], 1);
@@ -1461,56 +1554,14 @@ int target_aggs(int64_t n) {
 
 unsigned grid_for(const isl_ctx* c, int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 8LL * c->sm_count)); }
 
-template <int NC, int M, int NW>
-int build_plan(isl_ctx* c, CzPlan& z) {
-    cudaStream_t st = c->stream;
-    const int D = c->dim, n = (int)z.nrow;
-    DBuf<float> P;
-    DBuf<float4> xr;
-    DBuf<int32_t> eqrow, hist, key, key2, row, cnt, map;
-    DBuf<unsigned> mm;
-    DBuf<unsigned short> dcut;
-    DBuf<char> tmp;
-    ISL_CHECK_CUDA(c, P.alloc((size_t)c->ndofobj * D));
-    ISL_CHECK_CUDA(c, xr.alloc(n));
-    ISL_CHECK_CUDA(c, mm.alloc(6));
-    ISL_CHECK_CUDA(c, hist.alloc(3 * NBIN));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(mm.p, 0xff, 3 * 4, st));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(mm.p + 3, 0, 3 * 4, st));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(hist.p, 0, 3 * NBIN * 4, st));
-    k_cz_points<<<(unsigned)((c->nelem + 255) / 256), 256, 0, st>>>(c->shape, c->ngeom, c->nfun, c->nelem, c->dconn.p,
-                                                                     c->dedof.p, c->dX.p, D, P.p);
-    if (NC == 3 && c->bpad) {
-        ISL_CHECK_CUDA(c, eqrow.alloc((size_t)c->neq));
-        k_cz_eqrow<<<(3 * n + 255) / 256, 256, 0, st>>>(3 * n, c->dbaeq.p, eqrow.p);
-        c->launches += 1;
-    }
-    k_cz_rowpts<NC><<<(unsigned)((c->ndofobj + 255) / 256), 256, 0, st>>>(c->ndofobj, c->ncomp, c->deq.p, eqrow.p, D, P.p, xr.p);
-    const unsigned g = grid_for(c, n);
-    k_cz_bounds<<<g, 256, 0, st>>>(n, xr.p, mm.p);
-    unsigned hmm[6];
-    ISL_CHECK_CUDA(c, cudaMemcpyAsync(hmm, mm.p, sizeof(hmm), cudaMemcpyDeviceToHost, st));
-    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
-    Box3 b;
-    double L[3] = {0, 0, 0}, Lmax = 0;
-    for (int d = 0; d < 3; ++d) {
-        const float lo = f_unorder(hmm[d]), hi = f_unorder(hmm[3 + d]);
-        L[d] = d < D ? (double)hi - lo : 0.0;
-        if (!(L[d] >= 0.0) || !std::isfinite(L[d])) return ISL_OK;  // no usable coordinates: one-level
-        Lmax = std::max(Lmax, L[d]);
-        b.lo[d] = lo;
-        b.inv[d] = L[d] > 0.0 ? (float)(NBIN / L[d]) : 0.f;
-    }
-    if (!(Lmax > 0.0)) return ISL_OK;
-    k_cz_hist<<<std::min(g, (unsigned)c->sm_count), 256, 0, st>>>(n, b, xr.p, hist.p);
-    std::vector<int32_t> hh(3 * NBIN);
-    ISL_CHECK_CUDA(c, cudaMemcpyAsync(hh.data(), hist.p, hh.size() * 4, cudaMemcpyDeviceToHost, st));
-    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
-    // near-cubic boxes: the edge h that gives the target number of them over
-    // the directions that are at least one edge long
-    const int comps = NC == 1 ? c->ncomp : 1;
-    const int target = std::max(1, target_aggs(z.nrow) / comps);
+// Boxes per direction of one instance: near-cubic boxes of edge h, which gives
+// the target number of them over the directions that are at least one edge
+// long; then the largest product of rounded-down or rounded-up counts within it.
+void choose_boxes(int D, const double* L, int target, int* mbox) {
+    const double Lmax = std::max(L[0], std::max(L[1], L[2]));
     bool use[3] = {L[0] > 0.0, L[1] > 0.0, L[2] > 0.0};
+    mbox[0] = mbox[1] = mbox[2] = 1;
+    if (!(Lmax > 0.0)) return;
     double h = Lmax;
     for (bool again = true; again;) {
         double vol = 1.0;
@@ -1522,7 +1573,6 @@ int build_plan(isl_ctx* c, CzPlan& z) {
         for (int d = 0; d < D; ++d)
             if (use[d] && nd > 1 && L[d] < h) { use[d] = false; again = true; break; }
     }
-    // the largest product of rounded-down or rounded-up counts within the target
     int64_t best = 0;
     for (int pick = 0; pick < 1 << D; ++pick) {
         int64_t tot = 1;
@@ -1533,23 +1583,88 @@ int build_plan(isl_ctx* c, CzPlan& z) {
         }
         if (tot <= target && tot > best) {
             best = tot;
-            for (int d = 0; d < 3; ++d) b.m[d] = m[d];
+            for (int d = 0; d < 3; ++d) mbox[d] = m[d];
         }
     }
-    if (!best) { b.m[0] = b.m[1] = b.m[2] = 1; }
-    const int nbox = b.m[0] * b.m[1] * b.m[2] * comps;
+}
+
+template <int NC, int M, int NW>
+int build_plan(isl_ctx* c, CzPlan& z) {
+    cudaStream_t st = c->stream;
+    const int D = c->dim, n = (int)z.nrow, ni = (int)c->ninst;
+    z.ninst = ni;
+    z.hinst.assign((size_t)ni, CzInst{});
+    for (int k = 0; k < ni; ++k) {
+        z.hinst[k].row0 = ni > 1 ? (int)c->inst_eq_off[k] : 0;
+        z.hinst[k].nrow = ni > 1 ? (int)(c->inst_eq_off[k + 1] - c->inst_eq_off[k]) : n;
+    }
+    DBuf<float> P;
+    DBuf<float4> xr;
+    DBuf<int32_t> eqrow, hist, key, key2, row, cnt, map;
+    DBuf<unsigned> mm;
+    DBuf<unsigned short> dcut;
+    DBuf<Box3> dbox;
+    DBuf<char> tmp;
+    std::vector<unsigned> hmm((size_t)6 * ni, 0u);
+    for (int k = 0; k < ni; ++k)
+        for (int d = 0; d < 3; ++d) hmm[6 * k + d] = 0xffffffffu;
+    ISL_CHECK_CUDA(c, P.alloc((size_t)c->ndofobj * D));
+    ISL_CHECK_CUDA(c, xr.alloc(n));
+    ISL_CHECK_CUDA(c, mm.alloc(hmm.size()));
+    ISL_CHECK_CUDA(c, hist.alloc((size_t)3 * NBIN * ni));
+    ISL_CHECK_CUDA(c, z.inst.alloc(ni));
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(mm.p, hmm.data(), hmm.size() * 4, cudaMemcpyHostToDevice, st));
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.inst.p, z.hinst.data(), (size_t)ni * sizeof(CzInst), cudaMemcpyHostToDevice, st));
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(hist.p, 0, (size_t)3 * NBIN * ni * 4, st));
+    k_cz_points<<<(unsigned)((c->nelem + 255) / 256), 256, 0, st>>>(c->shape, c->ngeom, c->nfun, c->nelem, c->dconn.p,
+                                                                     c->dedof.p, c->dX.p, D, P.p);
+    if (NC == 3 && c->bpad) {
+        ISL_CHECK_CUDA(c, eqrow.alloc((size_t)c->neq));
+        k_cz_eqrow<<<(3 * n + 255) / 256, 256, 0, st>>>(3 * n, c->dbaeq.p, eqrow.p);
+        c->launches += 1;
+    }
+    k_cz_rowpts<NC><<<(unsigned)((c->ndofobj + 255) / 256), 256, 0, st>>>(c->ndofobj, c->ncomp, c->deq.p, eqrow.p, D, P.p, xr.p);
+    const unsigned g = grid_for(c, n);
+    k_cz_bounds<<<g, 256, 0, st>>>(n, ni, z.inst.p, xr.p, mm.p);
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(hmm.data(), mm.p, hmm.size() * 4, cudaMemcpyDeviceToHost, st));
+    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+    const int comps = NC == 1 ? c->ncomp : 1;
+    std::vector<Box3> box((size_t)ni);
+    int64_t nbox = 0;
+    for (int k = 0; k < ni; ++k) {
+        Box3& b = box[k];
+        double L[3] = {0, 0, 0};
+        for (int d = 0; d < 3; ++d) {
+            const float lo = f_unorder(hmm[6 * k + d]), hi = f_unorder(hmm[6 * k + 3 + d]);
+            L[d] = d < D && z.hinst[k].nrow ? (double)hi - lo : 0.0;
+            if (!(L[d] >= 0.0) || !std::isfinite(L[d])) return ISL_OK;  // no usable coordinates: one-level
+            b.lo[d] = z.hinst[k].nrow ? lo : 0.f;
+            b.inv[d] = L[d] > 0.0 ? (float)(NBIN / L[d]) : 0.f;
+        }
+        choose_boxes(D, L, std::max(1, target_aggs(z.hinst[k].nrow) / comps), b.m);
+        b.base = (int)nbox;
+        nbox += (int64_t)b.m[0] * b.m[1] * b.m[2] * comps;
+    }
+    if (nbox * NW >= (int64_t)1 << (31 - LEN_BITS) || ni > 65535) return ISL_OK;  // sort keys, launch grids
+    ISL_CHECK_CUDA(c, dbox.alloc(ni));
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(dbox.p, box.data(), (size_t)ni * sizeof(Box3), cudaMemcpyHostToDevice, st));
+    k_cz_hist<<<ni > 1 ? g : std::min(g, (unsigned)c->sm_count), 256, 0, st>>>(n, ni, z.inst.p, dbox.p, xr.p, hist.p);
+    std::vector<int32_t> hh((size_t)3 * NBIN * ni);
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(hh.data(), hist.p, hh.size() * 4, cudaMemcpyDeviceToHost, st));
+    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
     // cuts at the quantiles of the rows, two half-boxes per box
-    std::vector<unsigned short> cut(3 * NBIN, 0);
-    for (int d = 0; d < D; ++d) {
-        const int64_t parts = 2 * b.m[d];
-        int64_t run = 0;
-        for (int k = 0; k < NBIN; ++k) {
-            const int64_t mid = run + hh[d * NBIN + k] / 2;
-            cut[d * NBIN + k] = (unsigned short)std::min<int64_t>(parts - 1, mid * parts / std::max(n, 1));
-            run += hh[d * NBIN + k];
+    std::vector<unsigned short> cut((size_t)3 * NBIN * ni, 0);
+    for (int k = 0; k < ni; ++k)
+        for (int d = 0; d < D; ++d) {
+            const int64_t parts = 2 * box[k].m[d];
+            int64_t run = 0;
+            for (int b = 0; b < NBIN; ++b) {
+                const size_t i = ((size_t)k * 3 + d) * NBIN + b;
+                cut[i] = (unsigned short)std::min<int64_t>(parts - 1, (run + hh[i] / 2) * parts / std::max(z.hinst[k].nrow, 1));
+                run += hh[i];
+            }
         }
-    }
-    ISL_CHECK_CUDA(c, dcut.alloc(3 * NBIN));
+    ISL_CHECK_CUDA(c, dcut.alloc(cut.size()));
     ISL_CHECK_CUDA(c, key.alloc(n));
     ISL_CHECK_CUDA(c, key2.alloc(n));
     ISL_CHECK_CUDA(c, row.alloc(n));
@@ -1559,26 +1674,50 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     ISL_CHECK_CUDA(c, map.alloc(nbox));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(dcut.p, cut.data(), cut.size() * 2, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemsetAsync(cnt.p, 0, (size_t)nbox * NW * 4, st));
-    k_cz_key<NC, NW><<<g, 256, 0, st>>>(n, b, dcut.p, c->ncomp, xr.p, key.p, cnt.p);
-    std::vector<int32_t> hc((size_t)nbox * NW), hmap(nbox, -1), so;
+    k_cz_key<NC, NW><<<g, 256, 0, st>>>(n, ni, z.inst.p, dbox.p, dcut.p, c->ncomp, xr.p, key.p, cnt.p);
+    std::vector<int32_t> hc((size_t)nbox * NW), hmap((size_t)nbox, -1), so, ai;
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(hc.data(), cnt.p, hc.size() * 4, cudaMemcpyDeviceToHost, st));
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+    // the boxes that hold rows, per instance
     int32_t run = 0, na = 0;
-    for (int k = 0; k < nbox; ++k) {
-        int32_t tot = 0;
-        for (int s = 0; s < NW; ++s) tot += hc[(size_t)k * NW + s];
-        if (!tot) continue;
-        hmap[k] = na++;
-        for (int s = 0; s < NW; ++s) { so.push_back(run); run += hc[(size_t)k * NW + s]; }
+    long long a0 = 0, p0 = 0;
+    int rc0 = 0;
+    z.max_ndp = 0;
+    for (int k = 0; k < ni; ++k) {
+        CzInst& in = z.hinst[k];
+        in.agg0 = na;
+        const int64_t end = k + 1 < ni ? box[k + 1].base : nbox;
+        for (int64_t b = box[k].base; b < end; ++b) {
+            int32_t tot = 0;
+            for (int s = 0; s < NW; ++s) tot += hc[(size_t)b * NW + s];
+            if (!tot) continue;
+            hmap[(size_t)b] = na++;
+            ai.push_back(k);
+            for (int s = 0; s < NW; ++s) { so.push_back(run); run += hc[(size_t)b * NW + s]; }
+        }
+        in.nagg = na - in.agg0;
+        in.nd = in.nagg * M;
+        in.ndp = std::max(1, (in.nd + TB - 1) / TB) * TB;
+        in.a0 = a0;
+        in.p0 = p0;
+        in.rc0 = rc0;
+        a0 += (long long)in.ndp * in.ndp;
+        p0 += 2LL * TB * in.ndp + 2 * TB * TB;
+        rc0 += 2 * in.ndp;
+        z.max_ndp = std::max(z.max_ndp, in.ndp);
     }
     so.push_back(run);
     z.nagg = na;
-    z.nd = na * M;
-    z.ndp = (z.nd + TB - 1) / TB * TB;
+    z.nd = z.hinst[0].nd;
+    z.ndp = z.hinst[0].ndp;
+    if (na == 0) return ISL_OK;
     ISL_CHECK_CUDA(c, z.sofs.alloc(so.size()));
+    ISL_CHECK_CUDA(c, z.agg_inst.alloc(ai.size()));
     ISL_CHECK_CUDA(c, z.lnode.alloc(n));
     ISL_CHECK_CUDA(c, z.yrow.alloc(n));
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.inst.p, z.hinst.data(), (size_t)ni * sizeof(CzInst), cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.sofs.p, so.data(), so.size() * 4, cudaMemcpyHostToDevice, st));
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.agg_inst.p, ai.data(), ai.size() * 4, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(map.p, hmap.data(), hmap.size() * 4, cudaMemcpyHostToDevice, st));
     k_cz_rekey<NC, NW><<<g, 256, 0, st>>>(n, map.p, c->drowptr.p, key.p, row.p);
     int bits = 1;
@@ -1592,14 +1731,14 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     ISL_CHECK_CUDA(c, cudaGetLastError());
     ISL_CHECK_CUDA(c, z.dsub.alloc((size_t)na * NW * M * M));
     ISL_CHECK_CUDA(c, z.dagg.alloc((size_t)na * M * M));
-    ISL_CHECK_CUDA(c, z.scale.alloc(z.ndp));
-    ISL_CHECK_CUDA(c, z.rc.alloc((size_t)2 * z.ndp));
-    ISL_CHECK_CUDA(c, z.acc.alloc((size_t)z.ndp * z.ndp));
-    ISL_CHECK_CUDA(c, z.a.alloc((size_t)z.ndp * z.ndp));
-    ISL_CHECK_CUDA(c, z.ainv.alloc((size_t)z.ndp * z.ndp));
-    ISL_CHECK_CUDA(c, z.panel.alloc((size_t)2 * TB * z.ndp + 2 * TB * TB));
-    ISL_CHECK_CUDA(c, z.amax.alloc(1));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.rc.p, 0, (size_t)2 * z.ndp * 4, st));  // the padding stays zero
+    ISL_CHECK_CUDA(c, z.scale.alloc((size_t)na * M));
+    ISL_CHECK_CUDA(c, z.rc.alloc(rc0));
+    ISL_CHECK_CUDA(c, z.acc.alloc((size_t)a0));
+    ISL_CHECK_CUDA(c, z.a.alloc((size_t)a0));
+    ISL_CHECK_CUDA(c, z.ainv.alloc((size_t)a0));
+    ISL_CHECK_CUDA(c, z.panel.alloc((size_t)p0));
+    ISL_CHECK_CUDA(c, z.amax.alloc(ni));
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.rc.p, 0, (size_t)rc0 * 4, st));  // the padding stays zero
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));  // the scratch buffers above go out of scope
     c->launches += 10;
     z.hsofs = std::move(so);
@@ -1681,6 +1820,23 @@ __global__ void k_pz_csr_values(int n, const int* __restrict__ perm, const int* 
     }
 }
 
+// shared memory of the one-launch solve; *ms, *as: the matrix and the rows of
+// the inverse fit too (in that order)
+constexpr size_t CLU_SMEM_MAX = 224 * 1024;
+size_t cluster_need(const CzPlan& z, int rows, int aggs, int ndp, int ent, bool m, bool s) {
+    return z.nc == 3 ? clu_smem<3, 6, 8>(rows, aggs, ndp, ent, m, s)
+           : z.m == 4 ? clu_smem<1, 4, 8>(rows, aggs, ndp, ent, m, s) : clu_smem<1, 3, 4>(rows, aggs, ndp, ent, m, s);
+}
+size_t cluster_smem(const CzPlan& z, bool* ms, bool* as, bool big = false) {
+    auto need = [&](bool m, bool s) {
+        return big ? cluster_need(z, z.big_rows, z.big_aggs, z.big_ndp, z.big_ent, m, s)
+                   : cluster_need(z, z.max_rows, z.max_aggs, z.max_ndp, z.max_ent, m, s);
+    };
+    *ms = need(true, false) <= CLU_SMEM_MAX;
+    *as = need(*ms, true) <= CLU_SMEM_MAX;
+    return need(*ms, *as);
+}
+
 // columns of the aggregate-ordered sliced-ELL copy (scalar systems), once per pattern
 int build_sell(isl_ctx* c, CzPlan& z) {
     if (z.sell_built) return ISL_OK;
@@ -1742,22 +1898,71 @@ int build_csr(isl_ctx* c, CzPlan& z) {
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(rp.data(), z.rp.p, (size_t)(n + 1) * 4, cudaMemcpyDeviceToHost, st));
     ISL_CHECK_CUDA(c, cudaGetLastError());
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
-    // aggregates per CTA: contiguous, balanced by rows and stored entries
+    // per instance: contiguous aggregates per CTA, balanced by stored entries; in
+    // a batch, the instances whose share of a CTA fits its shared memory
     const int nw = z.m == 3 ? 4 : 8;
-    z.hcta.assign(z.ncta + 1, 0);
-    z.max_rows = z.max_aggs = 0;
-    z.max_ent = 0;
-    for (int k = 0, ag = 0; k < z.ncta; ++k) {
-        const int64_t goal = z.nent * (k + 1) / z.ncta;
-        while (ag < z.nagg && (k == z.ncta - 1 || (int64_t)rp[z.hsofs[(size_t)ag * nw]] + rp[z.hsofs[(size_t)(ag + 1) * nw]] < 2 * goal)) ++ag;
-        z.hcta[k + 1] = ag;
-        const int t0 = z.hsofs[(size_t)z.hcta[k] * nw], t1 = z.hsofs[(size_t)ag * nw];
-        z.max_rows = std::max(z.max_rows, t1 - t0);
-        z.max_aggs = std::max(z.max_aggs, ag - z.hcta[k]);
-        z.max_ent = std::max(z.max_ent, rp[t1] - rp[t0]);
+    const size_t nc1 = (size_t)z.ncta + 1;
+    z.hcta.assign(nc1 * z.ninst, 0);
+    z.max_rows = z.max_aggs = z.max_ent = 0;
+    int max_ndp = 0;
+    std::vector<int32_t> order, big_cta;
+    struct Share { int rows = 0, aggs = 0, ent = 0; };
+    auto split = [&](const CzInst& in, int ncta, int32_t* cta) {
+        Share sh;
+        const int64_t e0 = rp[in.row0], ent = rp[in.row0 + in.nrow] - e0;
+        int ag = in.agg0;
+        cta[0] = ag;
+        for (int k = 0; k < ncta; ++k) {
+            const int from = ag, end = in.agg0 + in.nagg;
+            const int64_t goal = 2 * (e0 + ent * (k + 1) / ncta);
+            while (ag < end && (k == ncta - 1 ||
+                                (int64_t)rp[z.hsofs[(size_t)ag * nw]] + rp[z.hsofs[(size_t)(ag + 1) * nw]] < goal)) ++ag;
+            cta[k + 1] = ag;
+            const int t0 = z.hsofs[(size_t)from * nw], t1 = z.hsofs[(size_t)ag * nw];
+            sh.rows = std::max(sh.rows, t1 - t0);
+            sh.aggs = std::max(sh.aggs, ag - from);
+            sh.ent = std::max(sh.ent, rp[t1] - rp[t0]);
+        }
+        return sh;
+    };
+    z.big.clear();
+    z.big_ncta = c->sm_count;
+    z.big_rows = z.big_aggs = z.big_ent = z.big_ndp = 0;
+    for (int i = 0; i < z.ninst; ++i) {
+        const CzInst& in = z.hinst[i];
+        const Share sh = split(in, z.ncta, &z.hcta[nc1 * i]);
+        if (z.ninst > 1 && cluster_need(z, sh.rows, sh.aggs, in.ndp, sh.ent, false, false) > CLU_SMEM_MAX) {
+            std::vector<int32_t> cb((size_t)z.big_ncta + 1);
+            const Share b = split(in, z.big_ncta, cb.data());
+            if (cluster_need(z, b.rows, b.aggs, in.ndp, b.ent, false, false) > CLU_SMEM_MAX) continue;  // one-level
+            z.big.push_back(i);
+            big_cta.insert(big_cta.end(), cb.begin(), cb.end());
+            z.big_rows = std::max(z.big_rows, b.rows);
+            z.big_aggs = std::max(z.big_aggs, b.aggs);
+            z.big_ent = std::max(z.big_ent, b.ent);
+            z.big_ndp = std::max(z.big_ndp, in.ndp);
+            continue;
+        }
+        order.push_back(i);
+        z.max_rows = std::max(z.max_rows, sh.rows);
+        z.max_aggs = std::max(z.max_aggs, sh.aggs);
+        z.max_ent = std::max(z.max_ent, sh.ent);
+        max_ndp = std::max(max_ndp, in.ndp);
     }
-    ISL_CHECK_CUDA(c, z.cta.alloc(z.ncta + 1));
-    ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.cta.p, z.hcta.data(), (size_t)(z.ncta + 1) * 4, cudaMemcpyHostToDevice, st));
+    if (!z.big.empty()) {
+        ISL_CHECK_CUDA(c, z.cta_big.alloc(big_cta.size()));
+        ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.cta_big.p, big_cta.data(), big_cta.size() * 4, cudaMemcpyHostToDevice, st));
+        ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+    }
+    z.max_ndp = max_ndp;
+    z.norder = (int)order.size();
+    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return z.hinst[a].nrow > z.hinst[b].nrow; });
+    if (z.ninst > 1 && z.norder) {
+        ISL_CHECK_CUDA(c, z.order.alloc(order.size()));
+        ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.order.p, order.data(), order.size() * 4, cudaMemcpyHostToDevice, st));
+    }
+    ISL_CHECK_CUDA(c, z.cta.alloc(z.hcta.size()));
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.cta.p, z.hcta.data(), z.hcta.size() * 4, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
     c->launches += 3;
     z.csr_built = true;
@@ -1767,26 +1972,24 @@ int build_csr(isl_ctx* c, CzPlan& z) {
 template <int NC, int M, int NW>
 int numeric(isl_ctx* c, CzPlan& z, const CzMat& A) {
     cudaStream_t st = c->stream;
-    const int ndp = z.ndp, nt = ndp / TB;
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.acc.p, 0, (size_t)ndp * ndp * 8, st));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.amax.p, 0, 4, st));
+    int ndp = 0;
+    for (const CzInst& in : z.hinst) ndp = std::max(ndp, in.ndp);
+    const int nt = ndp / TB, ni = z.ninst;
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.acc.p, 0, z.acc.n * 8, st));
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.amax.p, 0, (size_t)ni * 4, st));
     const unsigned g = grid_for(c, c->neq);
-    if (c->have64) k_cz_amax<double><<<g, 256, 0, st>>>((int)c->neq, c->ddiag.p, c->dval64.p, z.amax.p);
-    else k_cz_amax<float><<<g, 256, 0, st>>>((int)c->neq, c->ddiag.p, c->dval32.p, z.amax.p);
-    k_cz_galerkin<NC, M, NW><<<z.nagg, NW * 32, 0, st>>>(A, z.lnode.p, z.yrow.p, z.sofs.p, ndp, z.amax.p, z.acc.p, z.dsub.p,
-                                                         z.dagg.p);
+    if (c->have64) k_cz_amax<double><<<g, 256, 0, st>>>((int)c->neq, ni, z.inst.p, c->ddiag.p, c->dval64.p, z.amax.p);
+    else k_cz_amax<float><<<g, 256, 0, st>>>((int)c->neq, ni, z.inst.p, c->ddiag.p, c->dval32.p, z.amax.p);
+    k_cz_galerkin<NC, M, NW><<<z.nagg, NW * 32, 0, st>>>(A, z.lnode.p, z.yrow.p, z.sofs.p, z.inst.p, z.agg_inst.p, z.amax.p,
+                                                         z.acc.p, z.dsub.p, z.dagg.p);
     k_cz_sub_inv<M><<<(z.nagg * NW + 63) / 64, 64, 0, st>>>(z.nagg * NW, z.dsub.p);
     k_cz_scale<M><<<(z.nagg + 127) / 128, 128, 0, st>>>(z.nagg, z.dagg.p, z.scale.p);
-    const dim3 g32(ndp / 32, ndp / 32);
-    k_cz_form<M><<<g32, 256, 0, st>>>(z.nd, ndp, z.acc.p, z.dagg.p, z.scale.p, z.amax.p, z.a.p);
-    // inverse: 28 steps at 64^3
-    float *P[2] = {z.panel.p, z.panel.p + (size_t)TB * ndp};
-    float *Di[2] = {z.panel.p + (size_t)2 * TB * ndp, z.panel.p + (size_t)2 * TB * ndp + TB * TB};
+    const dim3 g32(ndp / 32, ndp / 32, ni);
+    k_cz_form<M><<<g32, 256, 0, st>>>(z.inst.p, z.acc.p, z.dagg.p, z.scale.p, z.amax.p, z.a.p);
     ISL_CHECK_CUDA(c, cudaFuncSetAttribute(k_gj_step, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SMEM));
-    k_gj_first<<<nt, 256, 0, st>>>(z.a.p, ndp, P[0], Di[0]);
-    for (int k = 0; k < nt; ++k)
-        k_gj_step<<<nt * (nt + 1) / 2, 256, GJ_SMEM, st>>>(z.a.p, ndp, k, Di[k & 1], Di[(k + 1) & 1], P[k & 1], P[(k + 1) & 1]);
-    k_cz_unscale<<<g32, 256, 0, st>>>(z.nd, ndp, z.a.p, z.scale.p, z.ainv.p);
+    k_gj_first<<<dim3(nt, ni), 256, 0, st>>>(z.inst.p, z.a.p, z.panel.p);
+    for (int k = 0; k < nt; ++k) k_gj_step<<<dim3(nt * (nt + 1) / 2, ni), 256, GJ_SMEM, st>>>(z.inst.p, k, z.a.p, z.panel.p);
+    k_cz_unscale<M><<<g32, 256, 0, st>>>(z.inst.p, z.a.p, z.scale.p, z.ainv.p);
     ISL_CHECK_CUDA(c, cudaGetLastError());
     c->launches += 7 + nt;
     return ISL_OK;
@@ -1829,7 +2032,7 @@ int coarse_plan(isl_ctx* c, int nc, int64_t nrow, int ncta) {
         z.m = nc == 3 ? 6 : 1 + c->dim;
         z.nrow = nrow;
         z.serial = c->pattern_serial;
-        if (nrow >= (1 << ROW_BITS) || c->fedeg > 2 || (c->fedeg == 2 && c->shape == ISL_HEX) || c->ninst != 1) return ISL_OK;
+        if (nrow >= (1 << ROW_BITS) || c->fedeg > 2 || (c->fedeg == 2 && c->shape == ISL_HEX) || (c->ninst != 1 && nc != 1)) return ISL_OK;
         const int rc = CZ_DISPATCH(z, build_plan, c, z);
         if (rc != ISL_OK) return rc;
     }
@@ -1872,20 +2075,6 @@ int coarse_numeric(isl_ctx* c, bool csr, float* dinv) {
     return rc;
 }
 
-// shared memory of the one-launch solve; *ms, *as: the matrix and the rows of
-// the inverse fit too (in that order)
-constexpr size_t CLU_SMEM_MAX = 224 * 1024;
-static size_t cluster_smem(const CzPlan& z, bool* ms, bool* as) {
-    auto need = [&](bool m, bool s) {
-        return z.nc == 3 ? clu_smem<3, 6, 8>(z.max_rows, z.max_aggs, z.ndp, z.max_ent, m, s)
-               : z.m == 4 ? clu_smem<1, 4, 8>(z.max_rows, z.max_aggs, z.ndp, z.max_ent, m, s)
-                          : clu_smem<1, 3, 4>(z.max_rows, z.max_aggs, z.ndp, z.max_ent, m, s);
-    };
-    *ms = need(true, false) <= CLU_SMEM_MAX;
-    *as = need(*ms, true) <= CLU_SMEM_MAX;
-    return need(*ms, *as);
-}
-
 // 2: with its matrix on chip, 1: without, 0: not at all
 int coarse_cluster_fits(const isl_ctx* c, bool grid) {
     bool ms = false, as = false;
@@ -1898,22 +2087,23 @@ int coarse_cluster_fits(const isl_ctx* c, bool grid) {
 // (the shared-memory limit of a kernel is the process's: always the same value,
 // as other threads may be launching it too)
 template <int NC, int M, int NW, int LPR, bool MS>
-static cudaError_t launch_clu(const CzPlan& z, bool grid, size_t smem, cudaStream_t st, CzClu a) {
+static cudaError_t launch_clu(const CzPlan& z, int grid, size_t smem, cudaStream_t st, CzClu a) {
+    const int ncl = a.order ? z.norder : 1;  // clusters
     if (grid) {
-        const bool wide = z.max_rows * LPR > 1024;  // more than two rounds of 512 threads in a product
+        const bool wide = a.max_rows * LPR > 1024;  // more than two rounds of 512 threads in a product
         const void* k = wide ? (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 1024>
                              : (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 512>;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX);
         if (e == cudaSuccess) e = cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), st);
         void* args[] = {&a};
-        return e == cudaSuccess ? cudaLaunchCooperativeKernel(k, dim3(z.ncta), dim3(wide ? 1024 : 512), args, smem, st) : e;
+        return e == cudaSuccess ? cudaLaunchCooperativeKernel(k, dim3(grid), dim3(wide ? 1024 : 512), args, smem, st) : e;
     }
     auto k = k_cz_cluster<NC, M, NW, LPR, MS, false, 1024>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(z.ncta);
+    cfg.gridDim = dim3(z.ncta * ncl);
     cfg.blockDim = dim3(1024);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -1931,21 +2121,43 @@ static cudaError_t launch_clu(const CzPlan& z, bool grid, size_t smem, cudaStrea
     return cudaLaunchKernelEx(&cfg, k, a);
 }
 
-cudaError_t launch_coarse_cluster(isl_ctx* c, bool grid, bool arm, float* work, const float* dinv, double* x64, double tol, double drop,
-                                  int max_iter) {
+cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, bool arm, float* work, const float* dinv, double* x64, double tol,
+                                  double drop, int max_iter, int big) {
     CzPlan& z = c->cz;
     bool ms, as;
-    const size_t smem = cluster_smem(z, &ms, &as);
+    const size_t smem = cluster_smem(z, &ms, &as, big >= 0);
+    const int grid = big >= 0 ? z.big_ncta : use_grid ? z.ncta : 0;  // CTAs of the cooperative form
     const size_t na = (size_t)z.nc * z.nrow;
-    CzClu a = {z.lnode.p, z.sofs.p, z.cta.p, z.perm.p, z.dsub.p, z.ainv.p, z.ndp, z.rp.p, z.ci.p, z.cv.p, (int)z.nent, dinv,
-               z.rc.p, work, work + na, work + 2 * na, z.nc == 3 && c->bpad ? c->dbaeq.p : nullptr, c->drhs.p, x64,
-               c->drowptr.p, c->dcolind.p, c->dval64.p, c->dscal.p, tol, drop, max_iter, c->have64 ? 1 : 0,
-               z.max_rows, z.max_aggs, z.max_ent, reinterpret_cast<float2*>(c->dpart.p), c->dbar.p, as ? 1 : 0, arm ? 0x40000000u : 0u};
-    const double avg = (double)z.nent / (double)z.nrow;
+    const bool batch = c->ninst > 1 || c->force_batched;
+    CzClu a = {};
+    a.lnode = z.lnode.p; a.sofs = z.sofs.p; a.cta = z.cta.p; a.perm = z.perm.p;
+    a.dsub = z.dsub.p; a.ainv = z.ainv.p; a.inst = z.inst.p;
+    a.order = z.ninst > 1 && big < 0 ? z.order.p : nullptr;
+    a.inst_id = big >= 0 ? z.big[big] : 0;
+    if (big >= 0) a.cta = z.cta_big.p + (size_t)big * (z.big_ncta + 1);
+    a.res = batch ? z.res.p : nullptr;
+    a.max_ndp = big >= 0 ? z.big_ndp : z.max_ndp;
+    a.rp = z.rp.p; a.ci = z.ci.p; a.val = z.cv.p; a.nent = (int)z.nent;
+    a.dinv = dinv;
+    a.rc = z.rc.p; a.w = work; a.pa = work + na; a.pb = work + 2 * na;
+    a.aeq = z.nc == 1 ? nullptr : c->bpad ? c->dbaeq.p : nullptr;
+    a.b = c->drhs.p; a.x64 = x64;
+    a.rowptr = c->drowptr.p; a.colind = c->dcolind.p; a.val64 = c->dval64.p;
+    a.S = c->dscal.p;
+    a.tol = tol; a.drop = drop; a.max_iter = max_iter; a.exact64 = c->have64 ? 1 : 0;
+    a.max_rows = big >= 0 ? z.big_rows : z.max_rows;
+    a.max_aggs = big >= 0 ? z.big_aggs : z.max_aggs;
+    a.max_ent = big >= 0 ? z.big_ent : z.max_ent;
+    a.part = reinterpret_cast<float2*>(c->dpart.p); a.bar = c->dbar.p;
+    a.inv_smem = as ? 1 : 0;
+    a.armed = arm ? 0x40000000u : 0u;
+    // lanes per row: by the mean row length; in a batch by the element alone, so
+    // that an instance's sums do not depend on the others
+    const bool wide = batch ? !(c->dim == 2 && c->fedeg == 1) : (double)z.nent > 12.0 * (double)z.nrow;
     cudaStream_t st = c->stream;
     if (z.nc == 3) return ms ? launch_clu<3, 6, 8, 8, true>(z, grid, smem, st, a) : launch_clu<3, 6, 8, 8, false>(z, grid, smem, st, a);
     if (z.m == 4) return ms ? launch_clu<1, 4, 8, 8, true>(z, grid, smem, st, a) : launch_clu<1, 4, 8, 8, false>(z, grid, smem, st, a);
-    if (avg > 12) return ms ? launch_clu<1, 3, 4, 8, true>(z, grid, smem, st, a) : launch_clu<1, 3, 4, 8, false>(z, grid, smem, st, a);
+    if (wide) return ms ? launch_clu<1, 3, 4, 8, true>(z, grid, smem, st, a) : launch_clu<1, 3, 4, 8, false>(z, grid, smem, st, a);
     return ms ? launch_clu<1, 3, 4, 4, true>(z, grid, smem, st, a) : launch_clu<1, 3, 4, 4, false>(z, grid, smem, st, a);
 }
 

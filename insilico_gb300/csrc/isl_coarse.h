@@ -48,10 +48,11 @@ void launch_coarse(const isl_ctx* c, cudaStream_t st, const CzIter& a, int mode)
 // the whole solve in one launch, a thread-block cluster or a cooperative grid
 // of z.ncta CTAs (after coarse_plan with ncta > 0 and coarse_numeric): work
 // holds 3 vectors, the FP64 iterate goes to x64 and the record's fin, iters
-// and residuals to c->dscal.  arm: test hook, the grid barrier cannot complete
+// and residuals to c->dscal; on a batch, every instance of z.order in a cluster
+// of its own, or the instance z.big[big] in a grid, results in z.res.  arm: test hook, the grid barrier cannot complete
 int coarse_cluster_fits(const isl_ctx* c, bool grid);
 cudaError_t launch_coarse_cluster(isl_ctx* c, bool grid, bool arm, float* work, const float* dinv, double* x64, double tol,
-                                  double drop, int max_iter);
+                                  double drop, int max_iter, int big = -1);
 void launch_coarse_dir(const isl_ctx* c, cudaStream_t st, int n, const float* z, float* p, const CGScal* S);
 
 }  // namespace isl

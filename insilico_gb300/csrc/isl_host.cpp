@@ -1547,7 +1547,10 @@ int isl_get_option(isl_ctx* c, int key, int64_t* value) {
     if (key == ISL_OPT_SPMV32_KIND) { *value = c->spmv_lpr32; return ISL_OK; }
     if (key == ISL_OPT_HOST_SETUP) { *value = c->host_setup; return ISL_OK; }
     if (key == ISL_OPT_BICGSTAB_KIND) { *value = c->bicg_lpr; return ISL_OK; }
-    if (key == ISL_OPT_SCALAR_SLOTS) { *value = c->ss_nslot; return ISL_OK; }
+    if (key == ISL_OPT_SCALAR_SLOTS) {
+        *value = c->ss_nslot ? c->ss_nslot : (c->ninst > 1 && c->cz.csr_built ? c->cz.nent : 0);
+        return ISL_OK;
+    }
     ISL_FAIL(c, ISL_ERR_ARG, "unknown option");
     ISL_CATCH(c)
 }

@@ -124,7 +124,23 @@ struct OlScal {
 
 // two-level preconditioner (isl_coarse.cu): aggregates of the current pattern
 // and their matrices for the current assembly
+struct CzInst {               // one instance (a single system: the only one)
+    int row0, nrow;           // its rows (list order and natural order)
+    int agg0, nagg, nd, ndp;  // its aggregates, coarse unknowns, padded to whole tiles
+    int rc0, pad;             // first coarse vector entry (two vectors of ndp)
+    long long a0, p0;         // first entry of its coarse matrices, of its inversion scratch
+};
 struct CzPlan {
+    int ninst = 0, max_ndp = 0;
+    std::vector<CzInst> hinst;
+    DBuf<CzInst> inst;
+    DBuf<int32_t> agg_inst;   // instance of every aggregate
+    DBuf<int32_t> order;      // batch: instances solved in clusters, largest first
+    int norder = 0;
+    std::vector<int32_t> big; // batch: instances too large for a cluster, one cooperative grid each
+    DBuf<int32_t> cta_big;    // ... and the aggregates of its CTAs
+    int big_ncta = 0, big_rows = 0, big_aggs = 0, big_ent = 0, big_ndp = 0;
+    DBuf<OlScal> res;         // batch: result per instance
     bool ok = false;
     int64_t serial = -1, num_serial = -1, nrow = 0;
     int nc = 0, m = 0;        // components per row (3: node blocks), modes per aggregate
@@ -447,6 +463,7 @@ int ensure_val32(isl_ctx* c);
 int affine_lift(isl_ctx* c, int incremental);
 int inst_norms_device(isl_ctx* c, double* out);
 int distribute_masked(isl_ctx* c, int add);
+int cluster_ctas(isl_ctx* c);  // CTAs of the largest cluster that can be launched (0: none)
 int solve_onelaunch(isl_ctx* c, bool bicg, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* nc, bool* ran);
 int solve_bicgstab(isl_ctx* c, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* nc);
 bool bicgstab_kind_valid(const isl_ctx* c, int kind);

@@ -1035,7 +1035,7 @@ static int probe_cluster(isl_ctx* c) {
     return 0;
 }
 
-static int cluster_ctas(isl_ctx* c) {
+int cluster_ctas(isl_ctx* c) {
     if (c->cluster_size < 0) {
         // every LPR variant shares the size limits; probe all so that each can be launched
         int a = probe_cluster<2>(c), b = probe_cluster<4>(c), d = probe_cluster<8>(c), e = probe_cluster<16>(c),
