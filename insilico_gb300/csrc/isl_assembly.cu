@@ -396,12 +396,22 @@ __global__ void __launch_bounds__(128) k_heat_static(const ElemArgs A, const Tab
 // solid::HyperElastic on trilinear hexahedra, 2x2x2 quadrature.
 // 8 threads per element: in phase 1 thread q evaluates quadrature point q
 // (geometry, deformation, stress, effective elasticity), in phase 2 thread M
-// accumulates row-node M's 3x3 blocks K_MN (N >= M) over the quadrature points.
+// accumulates four or five 3x3 blocks K_MN of row node M over the quadrature points.
 //   K[Md+i, Nd+k] += sum_JL phi_M,J (d_ik S_JL + F_iA C_AJBL F_kB) phi_N,L detJ w
 //                                           solid/HyperElastic.hpp:110-179,282-310
 //   F[Md+i] -= sum_J (F S)_iJ phi_M,J detJ w  solid/HyperElastic.hpp:209-257 (x -1)
 // Materials: StVenant mat/hypel/StVenant.hpp:77-114,
 //            NeoHookeanCompressible mat/hypel/NeoHookeanCompressible.hpp:77-172.
+// NeoHookeanCompressible: with H = F^-T and b_M = H g_M, its tangent moduli
+// C_ABCD = lam Ci_AB Ci_CD + (mu - lam ln J) (Ci_AC Ci_BD + Ci_AD Ci_BC) and
+// S = (lam ln J - mu) Ci + mu I contract in closed form, because F Ci F^T = I:
+//   K_MN = c (mu (g_M.g_N) I + lam b_M b_N^T + (mu - lam ln J) b_N b_M^T)
+//   F S = mu F - (mu - lam ln J) H
+// which takes about 11k FP64 operations per element where forming the moduli
+// and their product with F took some 30k, and needs no 81 entries per point in
+// shared memory.  FP64 runs at about 1.2 FMAs per clock and SM here, and bounds
+// the kernel: 2,964 elements, FP64 tangent 371 -> 118 us; 8,000 elements, FP32
+// tangent 280 -> 94 us.
 // At u == 0 (F = I, S = 0) both reduce to isotropic linear elasticity and the
 // kernel uses  K_MN = c (lam g_M g_N^T + mu g_N g_M^T + mu (g_M.g_N) I).
 // TI compiles in the time-integration terms of a vector field (the plain
@@ -422,7 +432,10 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
     double* sfq = su + 8 * 3 * EPB;                 // [8 q][8 node][3][EPB] residual contributions
     R* sg = (R*)(sfq + (A.general ? 8 * 8 * 3 * EPB : 0));  // [8 q][8 node][3][EPB]
     R* sc = sg + 8 * 8 * 3 * EPB;                   // [8][EPB]
-    R* sA = sc + 8 * EPB;                           // [8 q][81][EPB] (general only)
+    R* sA = sc + 8 * EPB;                           // [8 q][81][EPB] (general StVenant)
+    R* sb = sc + 8 * EPB;                           // [8 q][8 node][3][EPB] H g (general NeoHooke), then [8 q][EPB]
+    R* sf2 = sb + 8 * 8 * 3 * EPB;                  // c (mu - lam ln J)
+    const bool neo = A.general && A.material == ISL_MAT_NEOHOOKE;
 
     const int el = threadIdx.x % EPB, role = threadIdx.x / EPB;
     const int E = A.nelem;
@@ -512,13 +525,40 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
 #pragma unroll
                     for (int J = 0; J < 3; ++J) F[i][J] += g[f][J] * uf;
                 }
-            double S[3][3], C[6][6];
-            material_eval(A.material, lam, mu, F, S, C);
             bool nan = false;
+            double P[3][3], S[3][3], C[6][6];
+            if (neo) {
+                double H[3][3];  // cofactors, then F^-T
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int J = 0; J < 3; ++J) {
+                        const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, J1 = (J + 1) % 3, J2 = (J + 2) % 3;
+                        H[i][J] = F[i1][J1] * F[i2][J2] - F[i1][J2] * F[i2][J1];
+                    }
+                const double detF = F[0][0] * H[0][0] + F[0][1] * H[0][1] + F[0][2] * H[0][2], iJ = 1.0 / detF;
+                const double f2 = mu - lam * log(detF);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int J = 0; J < 3; ++J) {
+                        H[i][J] *= iJ;
+                        P[i][J] = mu * F[i][J] - f2 * H[i][J];
+                    }
+                sf2[q * EPB + el] = R(c * f2);
+#pragma unroll
+                for (int M = 0; M < 8; ++M)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+                        sb[((q * 8 + M) * 3 + i) * EPB + el] = R(H[i][0] * g[M][0] + H[i][1] * g[M][1] + H[i][2] * g[M][2]);
+            } else {
+                material_eval(A.material, lam, mu, F, S, C);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int J = 0; J < 3; ++J) P[i][J] = F[i][0] * S[0][J] + F[i][1] * S[1][J] + F[i][2] * S[2][J];
+            }
             // residual contribution of this quadrature point: c (F S)_iJ g_N,J
-            double P[3][3];
-            for (int i = 0; i < 3; ++i)
-                for (int J = 0; J < 3; ++J) P[i][J] = F[i][0] * S[0][J] + F[i][1] * S[1][J] + F[i][2] * S[2][J];
 #pragma unroll
             for (int N = 0; N < 8; ++N)
 #pragma unroll
@@ -553,29 +593,44 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
             }
             if (valid && nan) atomicOr(A.flags, 2);
             // effective elasticity A[iJ][kL] = d_ik S_JL + F_iA C_V(A,J)V(B,L) F_kB
-            for (int i = 0; i < 3; ++i)
-                for (int J = 0; J < 3; ++J)
-                    for (int k = 0; k < 3; ++k)
-                        for (int L = 0; L < 3; ++L) {
-                            double s = (i == k) ? S[J][L] : 0.0;
-                            for (int Aa = 0; Aa < 3; ++Aa) {
-                                const int v1 = voigt(Aa, J);
-                                double t = 0.0;
-                                for (int B = 0; B < 3; ++B) t += C[v1][voigt(B, L)] * F[k][B];
-                                s += F[i][Aa] * t;
-                            }
-                            sA[((q * 81) + ((i * 3 + J) * 9 + k * 3 + L)) * EPB + el] = R(s);
+            if (!neo) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+#pragma unroll
+                    for (int L = 0; L < 3; ++L) {
+                        double Y[6];  // C_v,V(B,L) F_kB
+#pragma unroll
+                        for (int v = 0; v < 6; ++v) {
+                            double t = 0.0;
+#pragma unroll
+                            for (int B = 0; B < 3; ++B) t += C[v][voigt(B, L)] * F[k][B];
+                            Y[v] = t;
                         }
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+#pragma unroll
+                            for (int J = 0; J < 3; ++J) {
+                                double s = (i == k) ? S[J][L] : 0.0;
+#pragma unroll
+                                for (int Aa = 0; Aa < 3; ++Aa) s += F[i][Aa] * Y[voigt(Aa, J)];
+                                sA[((q * 81) + ((i * 3 + J) * 9 + k * 3 + L)) * EPB + el] = R(s);
+                            }
+                    }
+            }
         }
     }
     __syncthreads();
-    // ---- phase 2: row node M = role
+    // ---- phase 2: row node M = role, blocks (M, N) for N = M + d mod 8, d = 0 .. 4
+    // (d = 4: M < 4), so that every row node forms four or five of the 36 blocks
+    // (rows M <= N would give node 0 eight and node 7 one, and the longest row
+    // is what the block waits for); N < M is the transpose of block (N, M)
     const int M = role;
-    R acc[8][9];
+    constexpr int ND = 5;
+    R acc[ND][9];
 #pragma unroll
-    for (int N = 0; N < 8; ++N)
+    for (int d = 0; d < ND; ++d)
 #pragma unroll
-        for (int t = 0; t < 9; ++t) acc[N][t] = R(0);
+        for (int t = 0; t < 9; ++t) acc[d][t] = R(0);
 #pragma unroll 1
     for (int q = 0; q < 8; ++q) {
         const R c = sc[q * EPB + el];
@@ -588,8 +643,9 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
 #pragma unroll
             for (int i = 0; i < 3; ++i) { a_[i] = cl * gM[i]; b_[i] = cm * gM[i]; }
 #pragma unroll
-            for (int N = 0; N < 8; ++N) {
-                if (N < M) continue;
+            for (int d = 0; d < ND; ++d) {
+                if (d == 4 && M >= 4) continue;
+                const int N = (M + d) & 7;
                 R gN[3];
 #pragma unroll
                 for (int a = 0; a < 3; ++a) gN[a] = sg[((q * 8 + N) * 3 + a) * EPB + el];
@@ -597,7 +653,33 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
 #pragma unroll
-                    for (int k = 0; k < 3; ++k) acc[N][i * 3 + k] += a_[i] * gN[k] + b_[k] * gN[i] + (i == k ? db : R(0));
+                    for (int k = 0; k < 3; ++k) acc[d][i * 3 + k] += a_[i] * gN[k] + b_[k] * gN[i] + (i == k ? db : R(0));
+            }
+        } else if (neo) {
+            const R cl = c * R(lam), cm = c * R(mu), cf = sf2[q * EPB + el];
+            R bM[3], a_[3], d_[3], e_[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                bM[i] = sb[((q * 8 + M) * 3 + i) * EPB + el];
+                a_[i] = cl * bM[i];
+                d_[i] = cf * bM[i];
+                e_[i] = cm * gM[i];
+            }
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                if (d == 4 && M >= 4) continue;
+                const int N = (M + d) & 7;
+                R gN[3], bN[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    gN[a] = sg[((q * 8 + N) * 3 + a) * EPB + el];
+                    bN[a] = sb[((q * 8 + N) * 3 + a) * EPB + el];
+                }
+                const R db = e_[0] * gN[0] + e_[1] * gN[1] + e_[2] * gN[2];
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) acc[d][i * 3 + k] += a_[i] * bN[k] + d_[k] * bN[i] + (i == k ? db : R(0));
             }
         } else {
             // h[i][k][L] = c sum_J gM_J A[iJ][kL]
@@ -614,40 +696,43 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
                         h[i][k][L] = s * c;
                     }
 #pragma unroll
-            for (int N = 0; N < 8; ++N) {
-                if (N < M) continue;
+            for (int d = 0; d < ND; ++d) {
+                if (d == 4 && M >= 4) continue;
+                const int N = (M + d) & 7;
                 R gN[3];
 #pragma unroll
                 for (int a = 0; a < 3; ++a) gN[a] = sg[((q * 8 + N) * 3 + a) * EPB + el];
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
 #pragma unroll
-                    for (int k = 0; k < 3; ++k) acc[N][i * 3 + k] += h[i][k][0] * gN[0] + h[i][k][1] * gN[1] + h[i][k][2] * gN[2];
+                    for (int k = 0; k < 3; ++k) acc[d][i * 3 + k] += h[i][k][0] * gN[0] + h[i][k][1] * gN[1] + h[i][k][2] * gN[2];
             }
         }
         if (TI && A.rho) {  // mass per component: the diagonal of each 3x3 block
             const R mM = R(A.mass_w * A.rho[ec] * T.phi[q][M]) * c;
 #pragma unroll
-            for (int N = 0; N < 8; ++N) {
-                if (N < M) continue;
-                const R v = mM * R(T.phi[q][N]);
-                acc[N][0] += v;
-                acc[N][4] += v;
-                acc[N][8] += v;
+            for (int d = 0; d < ND; ++d) {
+                if (d == 4 && M >= 4) continue;
+                const R v = mM * R(T.phi[q][(M + d) & 7]);
+                acc[d][0] += v;
+                acc[d][4] += v;
+                acc[d][8] += v;
             }
         }
     }
     if (!valid) return;
     R* SK = (R*)A.stageK;
 #pragma unroll
-    for (int N = 0; N < 8; ++N) {
-        if (N < M) continue;
+    for (int d = 0; d < ND; ++d) {
+        if (d == 4 && M >= 4) continue;
+        const int N = (M + d) & 7;
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const int a = 3 * M + i, b = 3 * N + k;
-                if (a <= b) SK[(size_t)e * (NLOC * (NLOC + 1) / 2) + upidx(a, b, NLOC)] = acc[N][i * 3 + k];
+                if (a <= b) SK[(size_t)e * (NLOC * (NLOC + 1) / 2) + upidx(a, b, NLOC)] = acc[d][i * 3 + k];
+                else if (d > 0) SK[(size_t)e * (NLOC * (NLOC + 1) / 2) + upidx(b, a, NLOC)] = acc[d][i * 3 + k];
             }
     }
     // forces of row node M: -(internal) + body
@@ -1289,32 +1374,37 @@ static int dispatch_hyper(isl_ctx* c, const ElemArgs& A) {
     auto smem_of = [&](int epb) {
         return (size_t)8 * 3 * epb * 8 * 2 + (A.general ? (size_t)8 * 8 * 3 * epb * 8 : 0) +
                (size_t)8 * 8 * 3 * epb * sizeof(R) + (size_t)8 * epb * sizeof(R) +
-               (A.general ? (size_t)8 * 81 * epb * sizeof(R) : 0);
+               (!A.general ? 0 : A.material == ISL_MAT_NEOHOOKE ? (size_t)8 * 25 * epb * sizeof(R) : (size_t)8 * 81 * epb * sizeof(R));
     };
-    auto launch = [&](int epb) {
-        const size_t smem = smem_of(epb);
-        if (epb == 32) {
-            auto kern = ti ? k_hyper_hex8<R, 32, true> : k_hyper_hex8<R, 32, false>;
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<nblk(c->nelem, 32), 32 * 8, smem, c->stream>>>(A, T);
-        } else if (epb == 16) {
-            auto kern = ti ? k_hyper_hex8<R, 16, true> : k_hyper_hex8<R, 16, false>;
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<nblk(c->nelem, 16), 16 * 8, smem, c->stream>>>(A, T);
-        } else {
-            auto kern = ti ? k_hyper_hex8<R, 8, true> : k_hyper_hex8<R, 8, false>;
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<nblk(c->nelem, 8), 8 * 8, smem, c->stream>>>(A, T);
-        }
+    // (the limit is the process's: the same value whatever this call needs, as
+    // other threads may be launching the kernel for another material)
+    const int smem_max = 220 * 1024;
+    auto launch = [&](auto kern, int epb) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+        kern<<<nblk(c->nelem, epb), epb * 8, smem_of(epb), c->stream>>>(A, T);
     };
-    // elements per block: the candidates whose shared memory fits
-    int cand[3], ncand = 0;
-    for (int epb : {32, 16, 8})
-        if (smem_of(epb) <= 200 * 1024) cand[ncand++] = epb;
-    char tuner[48];
-    std::snprintf(tuner, sizeof tuner, "elem_hex8_r%d_g%d_t%d", (int)sizeof(R), A.general ? 1 : 0, ti ? 1 : 0);
-    const int epb = tune_elem(c, tuner, cand, ncand, launch);
-    launch(epb);
+    // Elements per block.  The kernel is bound by FP64 (FP32 tangents: in phase
+    // 1), so what counts is the work of the SM with the most blocks, and fewer
+    // elements a block spread them more evenly.  FP64 operations per element
+    // (thousands), phase 1 and phase 2, from the loops above: 3.4 and 7.5, or
+    // 8.3 where all eight row nodes share a warp (phase 2 costs next to nothing
+    // in FP32).  2,964 elements: 166 us with 32 (93 blocks on 152 SMs), 118 us
+    // with 4; 512 elements: 163 us with 32, 105 us with 4; 8,000 elements, FP32
+    // tangent: 101 us with 32, 94 us with 8.
+    int epb = 0;
+    double best = 0.0;
+    const int cand[4] = {32, 16, 8, 4};
+    const double phase2[4] = {7.5, 7.5, 7.5, 8.3};
+    for (int k = 0; k < 4; ++k) {
+        if (smem_of(cand[k]) > 200 * 1024) continue;
+        const int64_t blocks = (c->nelem + cand[k] - 1) / cand[k], rounds = (blocks + c->sm_count - 1) / c->sm_count;
+        const double t = (double)(rounds * cand[k]) * (3.4 + phase2[k] * (sizeof(R) == 8 ? 1.0 : 0.05));
+        if (!epb || t < best) { epb = cand[k]; best = t; }
+    }
+    if (epb == 32) ti ? launch(k_hyper_hex8<R, 32, true>, 32) : launch(k_hyper_hex8<R, 32, false>, 32);
+    else if (epb == 16) ti ? launch(k_hyper_hex8<R, 16, true>, 16) : launch(k_hyper_hex8<R, 16, false>, 16);
+    else if (epb == 8) ti ? launch(k_hyper_hex8<R, 8, true>, 8) : launch(k_hyper_hex8<R, 8, false>, 8);
+    else ti ? launch(k_hyper_hex8<R, 4, true>, 4) : launch(k_hyper_hex8<R, 4, false>, 4);
     c->elem_variant = epb;
     ISL_CHECK_CUDA(c, cudaGetLastError());
     c->launches += 1;
