@@ -867,20 +867,28 @@ __device__ inline int inst_of(const CzInst* __restrict__ inst, int ninst, int ro
 template <typename T>
 __global__ void k_cz_amax(int n, int ninst, const CzInst* __restrict__ inst, const int* __restrict__ diag, const T* __restrict__ val,
                           int* __restrict__ out) {
+    // a warp takes 32 consecutive rows, mostly of one instance
+    const int lane = threadIdx.x & 31;
+    int cur = -1;
     float m = 0.f;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float v = fabsf((float)val[diag[i]]);
-        if (!(v < INFINITY)) continue;
-        if (ninst > 1) {
-            int* o = out + inst_of(inst, ninst, i);
-            if (__float_as_int(v) > *(volatile int*)o) atomicMax(o, __float_as_int(v));
-        } else {
-            m = fmaxf(m, v);
+    auto flush = [&](int k, float v) {
+        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane == 0 && k >= 0) atomicMax(out + k, __float_as_int(v));
+    };
+    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) - lane; base < n; base += gridDim.x * blockDim.x) {
+        const int i = base + lane;
+        float v = i < n ? fabsf((float)val[diag[i]]) : 0.f;
+        if (!(v < INFINITY)) v = 0.f;
+        const int first = ninst > 1 ? inst_of(inst, ninst, base) : 0, last = ninst > 1 ? inst_of(inst, ninst, min(base + 31, n - 1)) : 0;
+        if (first != cur) {
+            flush(cur, m);
+            m = 0.f;
+            cur = first;
         }
+        if (first == last) m = fmaxf(m, v);
+        else if (i < n) atomicMax(out + inst_of(inst, ninst, i), __float_as_int(v));
     }
-    if (ninst > 1) return;
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_int(m));
+    flush(cur, m);
 }
 
 __device__ inline float fix_scale(int amax_bits) {  // 2^(FIX_BITS - e), amax < 2^e
