@@ -375,8 +375,8 @@ enum { ISL_OPT_BLOCK_SOLVER = 0, ISL_OPT_BLOCKED = 1, ISL_OPT_NBLOCKS = 2, ISL_O
  * hold as many instances at once as the GPU takes (unless
  * ISL_OPT_SPMV32_KIND sets a product of the one-level batched solve, or
  * ISL_OPT_PERSISTENT is not 1).  A scalar system is multiplied in the order of its
- * aggregates: ISL_OPT_SPMV32_KIND then chooses the slots in flight (102, 104,
- * 108); its CSR kinds apply to the one-level solve. */
+ * aggregates: ISL_OPT_SPMV32_KIND then chooses the slots in flight (102: 4,
+ * 104: 8, 108: 12); its CSR kinds apply to the one-level solve. */
 /* ISL_OPT_SHARED_GEOMETRY (default 1): the direct block assembly
  * (ISL_OPT_DIRECT_BLOCKS) of a mesh whose hexahedra are all translates of the
  * first (edge vectors equal within 1e-13) forms the 64 local pairs' Lame

@@ -49,6 +49,7 @@ constexpr int TB = 64;            // tile of the dense inversion
 constexpr int NBIN = 1024;        // bins per axis of the quantile cuts
 constexpr int ROW_BITS = 29;      // lnode.w: row, and the constrained components of a padded node block above
 constexpr float REG = 1e-5f;      // added to the unit diagonal of the scaled coarse matrices
+constexpr int CZ_KEEP = 2;        // rows of a thread that k_cz_update and k_cz_coarse hold in registers
 constexpr int FIX_BITS = 32;      // fixed point of the coarse entries: the largest diagonal entry is 2^32
 
 __device__ inline int lrow(float4 l) { return __float_as_int(l.w) & ((1 << ROW_BITS) - 1); }
@@ -116,7 +117,6 @@ __device__ __forceinline__ void reduce_parts2_df_warp(const float4* part, int n,
 // the sums r.r and r.z (without the coarse term, which k_cz_coarse adds).
 template <int NC, int M, int NW, int WPS, int MODE>
 __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
-    constexpr int NT = NW * WPS * 32;
     CGScal* S = a.S;
     if (MODE == CZ_UPDATE && S->done) return;
     if (MODE == CZ_RESTART && !S->rst) return;
@@ -132,41 +132,66 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
     for (int m = 0; m < M; ++m) rc[m] = 0.f;
     float rr = 0.f, rz = 0.f;
     double bb = 0.0;
-#pragma unroll 2
-    for (int t = t0; t < t1; t += 32 * WPS) {
-        const float4 L = __ldg(a.lnode + t);
-        const int row = lrow(L);
-        const size_t d = (size_t)NC * row;
-        float rv[NC], zv[NC], bi[NC * NC];
-#pragma unroll
-        for (int k = 0; k < NC * NC; ++k) bi[k] = __ldg(a.dinv + (size_t)(NC * NC) * row + k);
+    // loads of a row, then (in row_step) its stores: the rows held in registers load together
+    struct Row {
+        float4 L;
+        float x[NC], r[NC];
+    };
+    auto row_load = [&](int t, Row& R) {
+        R.L = __ldg(a.lnode + t);
+        const size_t d = (size_t)NC * lrow(R.L);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             if (MODE == CZ_UPDATE) {
-                a.x[d + c] += alpha * __ldg(p + d + c);
-                rv[c] = a.r[d + c] - alpha * __ldg(a.q + d + c);
+                R.x[c] = a.x[d + c] + alpha * __ldg(p + d + c);
+                R.r[c] = a.r[d + c] - alpha * __ldg(a.q + d + c);
             } else {
                 const int e = a.aeq ? a.aeq[d + c] : (int)(d + c);
                 const double v = e >= 0 ? a.b64[e] : 0.0;
-                rv[c] = (float)v;
-                if (MODE == CZ_INIT) {
-                    bb += v * v;
-                    a.x[d + c] = 0.f;
-                    a.pz[d + c] = 0.f;
-                }
+                R.r[c] = (float)v;
+                if (MODE == CZ_INIT) bb += v * v;
             }
         }
+    };
+    auto row_step = [&](int t, const Row& R, float (&zv)[NC]) {
+        const size_t d = (size_t)NC * lrow(R.L);
+        float bi[NC * NC];
+#pragma unroll
+        for (int k = 0; k < NC * NC; ++k) bi[k] = __ldg(a.dinv + (size_t)k * a.nrow + t);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            a.r[d + c] = rv[c];
+            if (MODE == CZ_UPDATE) a.x[d + c] = R.x[c];
+            if (MODE == CZ_INIT) a.x[d + c] = a.pz[d + c] = 0.f;
+            a.r[d + c] = R.r[c];
             zv[c] = 0.f;
 #pragma unroll
-            for (int k = 0; k < NC; ++k) zv[c] += bi[NC * c + k] * rv[k];
-            a.z[d + c] = zv[c];
-            rr += rv[c] * rv[c];
-            rz += rv[c] * zv[c];
+            for (int k = 0; k < NC; ++k) zv[c] += bi[NC * c + k] * R.r[k];
+            rr += R.r[c] * R.r[c];
+            rz += R.r[c] * zv[c];
         }
-        restrict_add<NC, M>(rc, rv, L);
+        restrict_add<NC, M>(rc, R.r, R.L);
+    };
+    // the first rows of a thread stay in registers with their part of z
+    Row Rk[CZ_KEEP];
+    float zk[CZ_KEEP][NC];
+#pragma unroll
+    for (int k = 0; k < CZ_KEEP; ++k)
+        if (t0 + 32 * WPS * k < t1) row_load(t0 + 32 * WPS * k, Rk[k]);
+    // row m of the sub-aggregate's inverse block, in lane m
+    float Dm[M];
+#pragma unroll
+    for (int k = 0; k < M; ++k) Dm[k] = lane < M ? __ldg(a.dsub + (size_t)sub * (M * M) + M * lane + k) : 0.f;
+#pragma unroll
+    for (int k = 0; k < CZ_KEEP; ++k)
+        if (t0 + 32 * WPS * k < t1) row_step(t0 + 32 * WPS * k, Rk[k], zk[k]);
+#pragma unroll 1
+    for (int t = t0 + 32 * WPS * CZ_KEEP; t < t1; t += 32 * WPS) {
+        Row R;
+        float zv[NC];
+        row_load(t, R);
+        row_step(t, R, zv);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) a.z[(size_t)NC * lrow(R.L) + c] = zv[c];
     }
 #pragma unroll
     for (int m = 0; m < M; ++m)
@@ -185,26 +210,33 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
             for (int k = 0; k < WPS; ++k) rc[m] += src[sl * WPS + k][m];
         }
     }
-    float z1[M];
-    const float* __restrict__ D = a.dsub + (size_t)sub * (M * M);
-    float rz1 = 0.f;
+    float z1[M], zm = 0.f, rz1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < M; ++k) zm += Dm[k] * rc[k];
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-        z1[m] = 0.f;
-#pragma unroll
-        for (int k = 0; k < M; ++k) z1[m] += __ldg(D + M * m + k) * rc[k];
+        z1[m] = __shfl_sync(0xffffffffu, zm, m);
         rz1 += rc[m] * z1[m];
     }
     if (w % WPS == 0 && lane == 0) rz += rz1;
-    for (int t = t0; t < t1; t += 32 * WPS) {  // each thread adds to the entries of z it wrote
-        const float4 L = __ldg(a.lnode + t);
+    auto add_sub = [&](const float4& L, const float (&zv)[NC]) {
         const size_t d = (size_t)NC * lrow(L);
         float o[NC];
         prolong<NC, M>(z1, L, o);
         const int mk = NC == 3 ? lmask(L) : 0;
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
-            if (!((mk >> c) & 1)) a.z[d + c] += o[c];
+        for (int c = 0; c < NC; ++c) a.z[d + c] = (mk >> c) & 1 ? zv[c] : zv[c] + o[c];
+    };
+#pragma unroll
+    for (int k = 0; k < CZ_KEEP; ++k)
+        if (t0 + 32 * WPS * k < t1) add_sub(Rk[k].L, zk[k]);
+#pragma unroll 1
+    for (int t = t0 + 32 * WPS * CZ_KEEP; t < t1; t += 32 * WPS) {  // each thread adds to the entries of z it wrote
+        const float4 L = __ldg(a.lnode + t);
+        float zv[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) zv[c] = a.z[(size_t)NC * lrow(L) + c];
+        add_sub(L, zv);
     }
     if (threadIdx.x < M) {
         float s = 0.f;
@@ -273,6 +305,17 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_coarse(CzIter a) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n4 = a.ndp / 4;
     const float4* __restrict__ rc4 = reinterpret_cast<const float4*>(a.rc);
+    // z of the first rows of a thread is on its way while the dense rows are multiplied
+    const int t0 = a.sofs[blockIdx.x * NW] + (int)threadIdx.x, t1 = a.sofs[(blockIdx.x + 1) * NW];
+    float4 Lk[CZ_KEEP];
+    float zk[CZ_KEEP][NC];
+#pragma unroll
+    for (int k = 0; k < CZ_KEEP; ++k)
+        if (t0 + TW * 32 * k < t1) {
+            Lk[k] = __ldg(a.lnode + t0 + TW * 32 * k);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) zk[k][c] = a.z[(size_t)NC * lrow(Lk[k]) + c];
+        }
     for (int j = w; j < M * PR; j += TW) {
         const int m = j % M;
         const float4* __restrict__ row = reinterpret_cast<const float4*>(a.ainv + (size_t)(blockIdx.x * M + m) * a.ndp);
@@ -295,16 +338,24 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_coarse(CzIter a) {
         for (int k = 0; k < PR; ++k) zc[m] += zs[k][m];
         rz += zc[m] * __ldg(a.rc + (size_t)blockIdx.x * M + m);
     }
-    const int t1 = a.sofs[(blockIdx.x + 1) * NW];
-    for (int t = a.sofs[blockIdx.x * NW] + (int)threadIdx.x; t < t1; t += TW * 32) {
-        const float4 L = __ldg(a.lnode + t);
+    auto add_coarse = [&](const float4& L, const float (&zv)[NC]) {
         const size_t d = (size_t)NC * lrow(L);
         float o[NC];
         prolong<NC, M>(zc, L, o);
         const int mk = NC == 3 ? lmask(L) : 0;
 #pragma unroll
         for (int c = 0; c < NC; ++c)
-            if (!((mk >> c) & 1)) a.z[d + c] += o[c];
+            if (!((mk >> c) & 1)) a.z[d + c] = zv[c] + o[c];
+    };
+#pragma unroll
+    for (int k = 0; k < CZ_KEEP; ++k)
+        if (t0 + TW * 32 * k < t1) add_coarse(Lk[k], zk[k]);
+    for (int t = t0 + TW * 32 * CZ_KEEP; t < t1; t += TW * 32) {
+        const float4 L = __ldg(a.lnode + t);
+        float zv[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) zv[c] = a.z[(size_t)NC * lrow(L) + c];
+        add_coarse(L, zv);
     }
     if (threadIdx.x == 0) reinterpret_cast<float2*>(a.part)[blockIdx.x] = make_float2(rz, 0.f);
     if (!last_block(&S->ticket2)) return;
@@ -322,6 +373,119 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_coarse(CzIter a) {
     }
     // not positive: the matrix or the inverse is not definite; the host solves one-level
     if (!(rzn > 0.0)) { S->bad = 1; S->done = 1; }
+}
+
+// q = A p and p.q for scalar rows: sliced ELL in aggregate order.
+// The CTAs take contiguous runs of slices with the same number of slots (bnd),
+// and the warps of a CTA contiguous runs of its slots, whatever slices these
+// belong to: a warp that starts inside a slice leaves its sum to be added to
+// the slice's (in warp order).  With one warp per slice the 16,608 slices of a
+// P2 mesh took three rounds of 7,296 warps where 2.3 were work; all gathers of
+// a batch come before its sums, as nothing moves across the tests for a
+// slice's end.  531k rows of P2 tetrahedra: 42.5 -> 32.8 us with 12 slots in
+// flight and 4 CTAs per SM; 41 us with 8 and 6, whose registers spill.
+constexpr int SPMV_PER_SM = 4;
+template <int U, typename TC>
+__global__ void __launch_bounds__(256, SPMV_PER_SM) k_cz_spmv(CzSpmv m, const TC* __restrict__ col) {
+    constexpr int NWP = 8, CAP = 32;
+    CGScal* S = m.S;
+    if (S->done) return;
+    __shared__ double sh[32];
+    __shared__ int so[CAP + 1], hs[NWP];
+    __shared__ float acc[CAP][32], head[NWP][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const float* __restrict__ p = m.p;
+    float loc = 0.f;
+    const int s1 = m.bnd[blockIdx.x + 1];
+    for (int g0 = m.bnd[blockIdx.x]; g0 < s1; g0 += CAP) {
+        const int gn = min(CAP, s1 - g0);
+        if ((int)threadIdx.x <= gn) so[threadIdx.x] = m.soff[g0 + threadIdx.x] >> 5;
+        for (int k = threadIdx.x; k < gn * 32; k += 256) (&acc[0][0])[k] = 0.f;
+        if (lane == 0) hs[w] = -1;
+        __syncthreads();
+        const int T0 = so[0], T = so[gn] - T0;
+        int k = T0 + (int)((long long)T * w / NWP);
+        const int kend = T0 + (int)((long long)T * (w + 1) / NWP);
+        if (k < kend) {
+            int ls = 0;
+            while (so[ls + 1] <= k) ++ls;
+            bool inside = k > so[ls];
+            int next = so[ls + 1];
+            float a = 0.f;
+            auto flush = [&] {
+                if (inside && lane == 0) hs[w] = ls;
+                (inside ? head[w] : acc[ls])[lane] = a;
+                a = 0.f;
+                inside = false;
+            };
+            for (; k < kend; k += U) {
+                int j[U], li = ls, ln = next;
+                float v[U], x[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (k + u < kend) {
+                        j[u] = ld_stream(col + (size_t)(k + u) * 32 + lane);
+                        if (sizeof(TC) == 2) {
+                            while (k + u >= ln) ln = so[++li + 1];
+                            const int i = (g0 + li) * 32 + lane;
+                            j[u] += i < m.nrow ? i : 0;
+                        }
+                        v[u] = ld_stream(m.val + (size_t)(k + u) * 32 + lane);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (k + u < kend) x[u] = __ldg(p + j[u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (k + u < kend) {
+                        while (k + u >= next) {
+                            flush();
+                            next = so[++ls + 1];
+                        }
+                        a += v[u] * x[u];
+                    }
+                }
+            }
+            flush();
+        }
+        __syncthreads();
+        for (int l = w; l < gn; l += NWP) {
+            const int i = (g0 + l) * 32 + lane;
+            if (i >= m.nrow) continue;
+            float t = acc[l][lane];
+#pragma unroll
+            for (int h = 0; h < NWP; ++h)
+                if (hs[h] == l) t += head[h][lane];
+            m.q[i] = t;
+            loc += __ldg(p + i) * t;
+        }
+        __syncthreads();
+    }
+    const df bsum = block_sum_df(loc, reinterpret_cast<float*>(sh));
+    if (threadIdx.x == 0) reinterpret_cast<float2*>(m.part)[blockIdx.x] = make_float2(bsum.hi, bsum.lo);
+    if (last_block(&S->ticket1)) {
+        const double tot = reduce_parts_df_blk<256>(reinterpret_cast<const float2*>(m.part), gridDim.x, sh);
+        if (threadIdx.x == 0) {
+            S->pAp = tot;
+            S->alpha = S->absNew / tot;
+            S->ticket1 = 0;
+        }
+    }
+}
+
+// first slice of every CTA of k_cz_spmv
+__global__ void k_cz_bnd(int ncta, int nslice, const int* __restrict__ soff, int* __restrict__ bnd) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b > ncta) return;
+    const int64_t goal = (int64_t)soff[nslice] * b / ncta;
+    int lo = 0, hi = nslice;
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (soff[mid] < goal) lo = mid + 1;
+        else hi = mid;
+    }
+    bnd[b] = lo;
 }
 
 // p = z + beta p (where the product does not fold the direction update)
@@ -1768,13 +1932,12 @@ __global__ void k_pz_width(int n, int nslice, const int* __restrict__ perm, cons
 }
 __global__ void k_pz_cols(int n, int nslice, const int* __restrict__ perm, const int* __restrict__ pos, const int* __restrict__ rowptr,
                           const int* __restrict__ colind, const int* __restrict__ soff, const int* __restrict__ swid,
-                          int* __restrict__ col, short* __restrict__ col16, int* __restrict__ srow, int* __restrict__ far) {
+                          int* __restrict__ col, short* __restrict__ col16, int* __restrict__ far) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nslice * 32) return;
     const int row = t < n ? perm[t] : -1, base = t < n ? t : 0;
     const int lo = row >= 0 ? rowptr[row] : 0, len = row >= 0 ? rowptr[row + 1] - lo : 0;
     const int o = soff[t >> 5] + (t & 31), w = swid[t >> 5];
-    srow[t] = t < n ? t : -1;
     for (int k = 0; k < w; ++k) {
         const int j = k < len ? pos[colind[lo + k]] : base, d = j - base;
         col[o + 32 * k] = j;
@@ -1809,6 +1972,11 @@ __global__ void k_pz_csr_cols(int n, const int* __restrict__ perm, const int* __
         const int lo = ptr[perm[t]], len = rp[t + 1] - rp[t];
         for (int k = threadIdx.x & 31; k < len; k += 32) col[rp[t] + k] = pos[colind[lo + k]];
     }
+}
+// node blocks: inverse diagonal blocks in list order, [9][n]
+__global__ void k_pz_binv(int n, const int* __restrict__ perm, const float* __restrict__ binv, float* __restrict__ dinv) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+        for (int k = 0; k < 9; ++k) dinv[(size_t)k * n + t] = binv[(size_t)9 * perm[t] + k];
 }
 template <int NC>
 __global__ void k_pz_csr_values(int n, const int* __restrict__ perm, const int* __restrict__ ptr, const int* __restrict__ sdst,
@@ -1864,14 +2032,13 @@ int build_sell(isl_ctx* c, CzPlan& z) {
     }
     off[ns] = (int32_t)tot;
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.soff.p, off.data(), (size_t)(ns + 1) * 4, cudaMemcpyHostToDevice, st));
-    ISL_CHECK_CUDA(c, z.srow.alloc((size_t)ns * 32));
     ISL_CHECK_CUDA(c, z.col.alloc(tot));
     ISL_CHECK_CUDA(c, z.col16.alloc(tot));
     ISL_CHECK_CUDA(c, z.val.alloc(tot));
     ISL_CHECK_CUDA(c, cudaMemsetAsync(z.val.p, 0, (size_t)tot * 4, st));
     ISL_CHECK_CUDA(c, cudaMemsetAsync(c->dflags.p + 1, 0, sizeof(int), st));
     k_pz_cols<<<(ns * 32 + 255) / 256, 256, 0, st>>>(n, ns, z.perm.p, z.pos.p, c->drowptr.p, c->dcolind.p, z.soff.p, z.swid.p,
-                                                      z.col.p, z.col16.p, z.srow.p, c->dflags.p + 1);
+                                                      z.col.p, z.col16.p, c->dflags.p + 1);
     int far = 0;
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(&far, c->dflags.p + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
@@ -2035,7 +2202,7 @@ int coarse_plan(isl_ctx* c, int nc, int64_t nrow, int ncta) {
     CzPlan& z = c->cz;
     if (z.serial != c->pattern_serial || z.nc != nc) {
         z.ok = z.sell_built = z.csr_built = false;
-        z.num_serial = z.sell_serial = z.csr_serial = -1;
+        z.num_serial = z.sell_serial = z.csr_serial = z.binv_serial = -1;
         z.nc = nc;
         z.m = nc == 3 ? 6 : 1 + c->dim;
         z.nrow = nrow;
@@ -2075,6 +2242,11 @@ int coarse_numeric(isl_ctx* c, bool csr, float* dinv) {
         c->launches += 1;
         if (csr) A = {nullptr, nullptr, z.rp.p, z.ci.p, z.cv.p};
         else A = {z.soff.p, z.swid.p, nullptr, z.col.p, z.val.p};
+    } else if (!csr && z.binv_serial != c->asm_serial) {
+        ISL_CHECK_CUDA(c, z.binv.alloc((size_t)9 * n));
+        k_pz_binv<<<grid_for(c, n), 256, 0, st>>>(n, z.perm.p, dinv, z.binv.p);
+        c->launches += 1;
+        z.binv_serial = c->asm_serial;
     }
     ISL_CHECK_CUDA(c, cudaGetLastError());
     if (z.num_serial == c->asm_serial) return ISL_OK;
@@ -2184,6 +2356,29 @@ void launch_coarse(const isl_ctx* c, cudaStream_t st, const CzIter& a, int mode)
     CZ_DISPATCH(z, launch_iter, z, st, a, mode);
 }
 
+int coarse_spmv_plan(isl_ctx* c) {
+    CzPlan& z = c->cz;
+    const int g = (int)std::min<int64_t>(z.nslice, (int64_t)SPMV_PER_SM * c->sm_count);
+    if (z.bnd_serial == z.serial && z.spmv_ncta == g) return ISL_OK;
+    ISL_CHECK_CUDA(c, z.bnd.alloc((size_t)g + 1));
+    k_cz_bnd<<<g / 256 + 1, 256, 0, c->stream>>>(g, z.nslice, z.soff.p, z.bnd.p);
+    ISL_CHECK_CUDA(c, cudaGetLastError());
+    c->launches += 1;
+    z.spmv_ncta = g;
+    z.bnd_serial = z.serial;
+    return ISL_OK;
+}
+void launch_coarse_spmv(const isl_ctx* c, int kind, cudaStream_t st, const CzSpmv& m) {
+    const CzPlan& z = c->cz;
+    const bool s16 = z.short_cols && c->use_scol16;
+    auto run = [&](auto k16, auto k32) {
+        if (s16) k16<<<z.spmv_ncta, 256, 0, st>>>(m, z.col16.p);
+        else k32<<<z.spmv_ncta, 256, 0, st>>>(m, z.col.p);
+    };
+    if (kind == 102) run(k_cz_spmv<4, short>, k_cz_spmv<4, int>);
+    else if (kind == 104) run(k_cz_spmv<8, short>, k_cz_spmv<8, int>);
+    else run(k_cz_spmv<12, short>, k_cz_spmv<12, int>);
+}
 void launch_coarse_dir(const isl_ctx* c, cudaStream_t st, int n, const float* z, float* p, const CGScal* S) {
     k_cz_dir<<<(unsigned)std::min<int64_t>(((int64_t)n + 255) / 256, 16LL * c->sm_count), 256, 0, st>>>(n, z, p, S);
 }

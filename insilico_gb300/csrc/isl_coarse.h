@@ -19,7 +19,9 @@ struct CzIter {
     float *x, *r, *z;
     const float *p1, *p2; // direction (p2: the buffer of even iteration counts, null when there is one)
     float* pz;            // direction buffer zeroed at the start
-    const float *q, *dinv;
+    const float *q;
+    const float* dinv;    // inverse diagonal (blocks) in list order, [1 or 9][nrow]
+    int nrow;
     const double* b64;    // right-hand side (init) or FP64 residual (restart), by equation
     const int* aeq;       // padded node blocks: equation of every component, else null
     CGScal* S;
@@ -32,6 +34,16 @@ struct CzIter {
 struct CzMat {
     const int *soff, *swid, *rowptr, *col;
     const float* val;
+};
+
+// arguments of the scalar product q = A p
+struct CzSpmv {
+    const int *bnd, *soff;  // first slice of every CTA; first entry of every slice
+    const float *val, *p;
+    float* q;
+    CGScal* S;
+    double* part;
+    int nrow;
 };
 
 // support points, boxes and row lists for the current pattern; c->cz.ok says
@@ -53,6 +65,9 @@ void launch_coarse(const isl_ctx* c, cudaStream_t st, const CzIter& a, int mode)
 int coarse_cluster_fits(const isl_ctx* c, bool grid);
 cudaError_t launch_coarse_cluster(isl_ctx* c, bool grid, bool arm, float* work, const float* dinv, double* x64, double tol,
                                   double drop, int max_iter, int big = -1);
+// scalar product (kind 102, 104, 108: 4, 8 or 12 slots in flight), and its CTAs' runs of slices (once per pattern)
+int coarse_spmv_plan(isl_ctx* c);
+void launch_coarse_spmv(const isl_ctx* c, int kind, cudaStream_t st, const CzSpmv& m);
 void launch_coarse_dir(const isl_ctx* c, cudaStream_t st, int n, const float* z, float* p, const CGScal* S);
 
 }  // namespace isl

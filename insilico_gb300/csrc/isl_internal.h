@@ -151,14 +151,19 @@ struct CzPlan {
     DBuf<unsigned long long> acc;
     DBuf<float> dsub, dagg, scale, rc, a, ainv, panel;
     DBuf<int32_t> perm, pos;  // list order: row of every entry, entry of every row
+    DBuf<float> binv;         // node blocks: inverse diagonal blocks in list order, [9][nrow]
+    int64_t binv_serial = -1;
     std::vector<int32_t> hsofs;
     // scalar systems: sliced-ELL copy in list order
     bool sell_built = false, short_cols = false;
     int64_t sell_serial = -1;
     int nslice = 0;
-    DBuf<int32_t> soff, swid, srow, col;
+    DBuf<int32_t> soff, swid, col;
     DBuf<int16_t> col16;
     DBuf<float> val;
+    DBuf<int32_t> bnd;        // product: first slice of every CTA
+    int64_t bnd_serial = -1;
+    int spmv_ncta = 0;
     // one-cluster solve: (block) CSR in list order, aggregates of every CTA
     bool csr_built = false;
     int64_t csr_serial = -1, nent = 0;

@@ -2871,37 +2871,21 @@ static void launch_rl_residual(isl_ctx* c, unsigned grid, cudaStream_t st, const
     }
 }
 
-// scalar product on the aggregate-ordered copy (t-space): the sliced-ELL
-// kernels of the one-level solve with U = 2, 4 or 8 slots in flight
-static void launch_pz_spmv(isl_ctx* c, int kind, cudaStream_t st, const float* p, float* q, CGScal* S) {
-    const CzPlan& z = c->cz;
-    const unsigned need = (unsigned)std::max(1, (z.nslice + BS / 32 - 1) / (BS / 32));
-    const bool s16 = z.short_cols && c->use_scol16;
-    auto run = [&](auto k16, auto k32, unsigned per_sm) {
-        const unsigned g = std::min(need, per_sm * (unsigned)c->sm_count);
-        if (s16) k16<<<g, BS, 0, st>>>(z.nslice, z.soff.p, z.swid.p, z.srow.p, z.col16.p, z.val.p, p, q, S, c->dpart.p);
-        else k32<<<g, BS, 0, st>>>(z.nslice, z.soff.p, z.swid.p, z.srow.p, z.col.p, z.val.p, p, q, S, c->dpart.p);
-    };
-    if (kind == 102) run(k_sspmv_batch<2, 8, short>, k_sspmv_batch<2, 8, int>, 8);
-    else if (kind == 108) run(k_sspmv_batch<8, 6, short>, k_sspmv_batch<8, 6, int>, 6);
-    else run(k_sspmv_batch<4, 8, short>, k_sspmv_batch<4, 8, int>, 8);
-}
-
-// slots in flight of that product: as set, from the tuning cache, or timed
-// (the first within 2 % of the fastest in a fixed order)
-static int pz_kind(isl_ctx* c, const float* p, float* q, CGScal* S) {
+// slots in flight of the scalar two-level product: as set, from the tuning
+// cache, or timed (the first within 2 % of the fastest in a fixed order)
+static int pz_kind(isl_ctx* c, const CzSpmv& m) {
     if (c->spmv32_forced) return c->spmv32_forced;
-    if (c->neq < 20000) return 104;
-    const int cand[3] = {104, 102, 108};
-    int cached = 0, best = 104;
+    if (c->neq < 20000) return 108;
+    const int cand[3] = {108, 104, 102};
+    int cached = 0, best = 108;
     if (tune_lookup(c, "spmv32", &cached) && std::find(cand, cand + 3, cached) != cand + 3) return cached;
     float ms_of[3], bestms = 1e30f;
-    cudaMemsetAsync(S, 0, sizeof(CGScal), c->stream);
+    cudaMemsetAsync(m.S, 0, sizeof(CGScal), c->stream);
     c->launches += 33;
     for (int k = 0; k < 3; ++k) {
-        launch_pz_spmv(c, cand[k], c->stream, p, q, S);
+        launch_coarse_spmv(c, cand[k], c->stream, m);
         cudaEventRecord(c->ev[2], c->stream);
-        for (int r = 0; r < 10; ++r) launch_pz_spmv(c, cand[k], c->stream, p, q, S);
+        for (int r = 0; r < 10; ++r) launch_coarse_spmv(c, cand[k], c->stream, m);
         cudaEventRecord(c->ev[3], c->stream);
         cudaEventSynchronize(c->ev[3]);
         cudaEventElapsedTime(&ms_of[k], c->ev[2], c->ev[3]);
@@ -3001,25 +2985,29 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
         // 5.21; at 270,400 nodes 21.4 against 18.5)
         if (c->fuse_dir && c->nslice <= 1024) kind = 9;
     } else {
-        kind = 104;
+        kind = 108;
     }
     if (exact64 && !c->spmv_lpr64)
         c->spmv_lpr64 = autotune_lpr<double, double>(c, c->dval64.p, c->drhs.p, W + 3 * n, S, c->dpart.p);
     rc = coarse_numeric(c, false, d32);
     if (rc != ISL_OK) return rc;
+    CzSpmv m = {};
     if (nc == 1) {
+        rc = coarse_spmv_plan(c);
+        if (rc != ISL_OK) return rc;
+        m = {c->cz.bnd.p, c->cz.soff.p, c->cz.val.p, p32, q32, S, c->dpart.p, (int)rows};
         if (!c->spmv_lpr32) {
             ISL_CHECK_CUDA(c, cudaMemsetAsync(p32, 0, na * 4, st));
-            c->spmv_lpr32 = pz_kind(c, p32, q32, S);
+            c->spmv_lpr32 = pz_kind(c, m);
         }
-        kind = c->spmv_lpr32 >= 100 ? c->spmv_lpr32 : 104;  // CSR kinds: the one-level solve's
+        kind = c->spmv_lpr32 >= 100 ? c->spmv_lpr32 : 108;  // CSR kinds: the one-level solve's
     }
     const bool fused = nc == 3 && c->fuse_dir && (kind == 9 || bspmv_dir_kind(kind));
     CzIter a = {};
     coarse_args(c, a);
     a.x = x32; a.r = r32; a.z = z32;
     a.p1 = p32; a.p2 = fused ? p32b : nullptr; a.pz = p32;
-    a.q = q32; a.dinv = d32;
+    a.q = q32; a.dinv = nc == 3 ? c->cz.binv.p : d32; a.nrow = (int)rows;
     a.b64 = c->drhs.p;
     a.aeq = nc == 1 ? c->cz.perm.p : c->bpad ? c->dbaeq.p : nullptr;
     a.S = S; a.part = c->dpart.p;
@@ -3042,7 +3030,8 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
                                  (uint64_t)(c->use_scol16 && (nc == 3 ? c->scol16 : c->cz.short_cols)), (uint64_t)c->pattern_serial,
                                  u(a.lnode), u(a.sofs), u(a.dsub), u(a.ainv), u(a.rc), u(V), u(W), u(a.dinv), u(a.aeq), u(S),
                                  u(a.part), u(c->dsval.p), u(c->dbval.p), u(c->cz.val.p), u(c->dval32.p), u(c->dval64.p),
-                                 u(c->drhs.p), u(c->drowptr.p), u(c->dcolind.p), u(c->dscol.p), u(c->dscol16.p)};
+                                 u(c->drhs.p), u(c->drowptr.p), u(c->dcolind.p), u(c->dscol.p), u(c->dscol16.p), u(m.bnd), (uint64_t)c->cz.spmv_ncta,
+                                 u(m.soff), u(c->cz.col.p), u(c->cz.col16.p)};
     if (!c->cz_exec || key != c->cz_key) {
         if (c->cz_exec) { cudaGraphExecDestroy(c->cz_exec); c->cz_exec = nullptr; }
         cudaGraph_t graph;
@@ -3053,7 +3042,7 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
             } else {
                 launch_coarse_dir(c, st, (int)na, z32, p32, S);
                 if (nc == 3) launch_bspmv(kind, grid, st, c, p32, q32, S, c->dpart.p);
-                else launch_pz_spmv(c, kind, st, p32, q32, S);
+                else launch_coarse_spmv(c, kind, st, m);
             }
             launch_coarse(c, st, a, CZ_UPDATE);
         }
