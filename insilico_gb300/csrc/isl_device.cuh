@@ -29,6 +29,30 @@ __device__ __forceinline__ int ld_stream(const short* p) {
     return v;
 }
 
+// Programmatic launch chains: a kernel launched with launch_chained may start
+// once every block of the kernel before it has called chain_next (or ended),
+// and waits in chain_wait for the end of that kernel and its writes.  A chained
+// kernel calls both first thing, whatever it does then, so that the wait also
+// covers the kernels further back.  Only data that no kernel of the chain
+// writes may be read before chain_wait, or through the read-only path (__ldg,
+// const __restrict__) at all: that path asks for data constant from the
+// kernel's start.  Without the attribute both do nothing.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_chained(void (*kern)(P...), unsigned grid, unsigned threads, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // Row dot product of a CSR matrix by a group of LPR lanes.  Every lane of the
 // warp must call it the same number of times (the shuffles use the full-warp
 // mask); lanes of a group without a row pass active = false and contribute 0.
