@@ -126,6 +126,7 @@ def l2_flush(device):
 
 
 # sliced-ELL / block-row SpMV variants by autotune kind (isl_solver.cu)
+CZ_SPMV_KERNEL = {102: "k_cz_spmv<4>", 104: "k_cz_spmv<8>", 108: "k_cz_spmv<12>"}  # two-level solve, graph of kernels
 SSPMV_KERNEL = {102: "k_sspmv_batch<2,8>", 104: "k_sspmv_batch<4,8>", 108: "k_sspmv_batch<8,6>"}
 BSPMV_KERNEL = {1: "k_bspmv_pap<1>", 2: "k_bspmv_pap<2>", 3: "k_bspmv_pap<4>", 5: "k_bspmv_batch<2,4>",
                 6: "k_bspmv_batch<4,3>", 7: "k_bspmv_batch<8,2>", 4: "k_brow_spmv<4>", 8: "k_brow_spmv<8>",
@@ -509,7 +510,7 @@ def run_serve(args, rank, world, local, pg):
                        "requests": nreq, "parallelism": "replicas" if world > 1 else "single",
                        "l2": "per-request meshes are set up, assembled and solved from host inputs"},
             "method": (f"native server: one request per batch, {args.slots} at once, each request's FP32 block CG "
-                       f"(padded 3x3 node blocks, block Jacobi) on its own stream" if args.batch == 1 else
+                       f"(padded 3x3 node blocks, two-level) on its own stream" if args.batch == 1 else
                        f"native server: batches of up to {args.batch} requests share every launch of a Newton "
                        f"iteration, {args.slots} batches at once, batching window {win} us") +
                       "; FP32 tangent + FP32 CG to 1e-6, FP64 residual; plain: one request per batch, 8 at once, "
@@ -1022,10 +1023,11 @@ def run_single(args, rank, world, local, pg):
 
     # what the speed-up is made of: the mixed solve with the plain path's
     # point-Jacobi preconditioner and scalar CSR matrix (precision alone),
-    # against the node-block format with block Jacobi
+    # then the node-block format with block Jacobi, then the two-level solve
     split = None
     if S.get_option(A.OPT_BLOCKED):
         S.set_option(A.OPT_BLOCK_SOLVER, 0)
+        S.set_option(A.OPT_TWO_LEVEL, 0)
         S.assemble(A.PREC_MIXED)
         tolq, errq, _ = calibrate(S, A.SOLVE_CG_FP32_IR, x_ref, REF_TOLS)
         step_mixed_point = lambda: (S.assemble(A.PREC_MIXED), S.solve(A.SOLVE_CG_FP32_IR, tol=tolq))[1]  # noqa: E731
@@ -1036,12 +1038,26 @@ def run_single(args, rank, world, local, pg):
         S.mark(5)
         point_ms = S.elapsed_ms(4, 5) / 2
         S.set_option(A.OPT_BLOCK_SOLVER, 1)
+        S.assemble(A.PREC_MIXED)
+        tolb, errb, _ = calibrate(S, A.SOLVE_CG_FP32_IR, x_ref, REF_TOLS)
+        step_mixed_block = lambda: (S.assemble(A.PREC_MIXED), S.solve(A.SOLVE_CG_FP32_IR, tol=tolb))[1]  # noqa: E731
+        step_mixed_block()
+        S.mark(4)
+        for _ in range(2):
+            it_b = step_mixed_block()[0]
+        S.mark(5)
+        block_ms = S.elapsed_ms(4, 5) / 2
+        S.set_option(A.OPT_TWO_LEVEL, 1)
         split = {"mixed_point_jacobi_csr": {"ms_per_step": point_ms, "iters": it_q, "solve_tol": tolq,
                                             "rel_err_vs_fp64": errq},
                  "precision_alone": plain_ms / point_ms,
-                 "block_format_and_block_jacobi": point_ms / ms_step,
+                 "mixed_block_jacobi": {"ms_per_step": block_ms, "iters": it_b, "solve_tol": tolb,
+                                        "rel_err_vs_fp64": errb},
+                 "block_format_and_block_jacobi": point_ms / block_ms,
+                 "two_level": block_ms / ms_step,
                  "note": "plain FP64 (point Jacobi, CSR) -> mixed with the same point Jacobi and CSR (precision "
-                         "alone) -> mixed with 3x3 node blocks and block Jacobi"}
+                         "alone) -> mixed with 3x3 node blocks and block Jacobi -> the same with aggregates "
+                         "(two-level)"}
         # the same block solve with the direction update as its own kernel
         S.assemble(A.PREC_MIXED)
         S.set_option(A.OPT_FOLD_DIRECTION, 0)
@@ -1084,7 +1100,10 @@ def run_single(args, rank, world, local, pg):
         nblk, nslot = 0, S.get_option(A.OPT_SCALAR_SLOTS)
         b32 = spmv_bytes(nnz, neq, 4, 2 if S.get_option(A.OPT_SHORT_COLUMNS) else 4)
         kind = S.get_option(A.OPT_SPMV32_KIND)
-        if kind >= 100:
+        if kind >= 100 and S.get_option(A.OPT_TWO_LEVEL) and neq > 65536:
+            kname = CZ_SPMV_KERNEL.get(kind, "k_cz_spmv") + " (scalar sliced-ELL FP32 in aggregate order, 32-bit " \
+                "columns where 16 bits do not reach, inner CG SpMV of the two-level solve, autotuned)"
+        elif kind >= 100:
             kname = SSPMV_KERNEL.get(kind, "k_sspmv_batch") + \
                 " (scalar sliced-ELL FP32, rows length-sorted in windows of 2048" + \
                 (", 16-bit column offsets" if S.get_option(A.OPT_SHORT_COLUMNS) else "") + ", inner CG SpMV, autotuned)"
@@ -1133,7 +1152,8 @@ def run_single(args, rank, world, local, pg):
         "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64",
         "data": "synthetic (seeded Philox; no dataset)",
         "config": workload_config(args.workload, args.n, neq, nnz, p.nelem, world),
-        "method": "mixed FP32 CG + FP64 reliable updates" + (", 3x3 node blocks + block Jacobi" if blocked else ""),
+        "method": "mixed FP32 CG + FP64 reliable updates" + (", 3x3 node blocks + block Jacobi" if blocked else "") +
+                  (", two-level" if S.get_option(A.OPT_TWO_LEVEL) else ""),
         "assembly_gdofs": neq / (asm_ms * 1e-3) / 1e9, "assembly_ms": asm_ms, "solve_ms": solve_ms_m,
         "solve_tol": tolm, "inner_iters_per_step": int(np.median(its)), "rel_err_vs_fp64": err_m,
         "fp64_reference": ref_kind,

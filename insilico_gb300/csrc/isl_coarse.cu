@@ -19,8 +19,8 @@
 // mesh.
 //
 // Measured (solve with the numeric setup of the assembly, 1e-10): 64^3
-// elasticity 144 -> 19.9 ms (195 iterations instead of 2,257; setup 1.5 ms),
-// 20^3 13.6 -> 3.6 ms, 40^3 P2 tetrahedra 38.9 -> 12.4 ms, Q2 160^2 24.2 -> 5.8 ms.
+// elasticity 144 -> 17.8 ms (194 iterations instead of 2,257; setup 1.3 ms),
+// 20^3 13.6 -> 1.9 ms, 40^3 P2 tetrahedra 38.9 -> 8.9 ms, Q2 160^2 24.2 -> 5.1 ms.
 //
 // Cost per iteration beyond the one-level solve: the update kernel takes one
 // CTA per aggregate and one warp per sub-aggregate, so the restriction and the

@@ -1661,7 +1661,7 @@ __global__ void __launch_bounds__(BS, MINB) k_bspmv_dir(int nbr, int nslice, con
 // through shared memory.  A warp per slice leaves most SMs idle below a few
 // hundred slices and walks its slots one batch after the other.  Bound by
 // latency: at 9,261 nodes the iteration took 30.1 us with a warp per slice,
-// 25.8 us with this product.
+// 25.8 us with this product (22.5 us since the update kernel waits less).
 template <typename TC>
 __global__ void __launch_bounds__(BS) k_bspmv_dir_split(int nbr, int nslice, const int* __restrict__ soff,
                                                         const int* __restrict__ swid, const TC* __restrict__ scol,
@@ -2945,7 +2945,7 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
     // matrices of up to about 30 MB), up to the sizes where the one-level solve
     // leaves its one-launch kernels.  us per iteration, cluster / grid / three
     // graph launches: 35k entries 9.5 / 11.3 / 28.7, 150k 9.7 / 12.4 / -,
-    // 190k 15.1 / 12.7 / 33, 1.9M - / 13.3 / 25, 6.9M - / 26.3 / 34.  A context that shares the GPU
+    // 190k 15.1 / 12.7 / 33, 1.9M - / 13.3 / 22.5, 6.9M - / 26.3 / 29.3.  A context that shares the GPU
     // with others (side_by_side) takes the cluster, 16 SMs, or the graph.
     const int64_t ent = nc == 3 ? 9 * c->nblk : c->nnz;
     const bool one = c->use_persist == 1;
@@ -3178,6 +3178,21 @@ int time_spmv(isl_ctx* c, int precision, int nrep, double* ms) {
         if (rc != ISL_OK) return rc;
         float* V = c->w32.p;
         ISL_CHECK_CUDA(c, cudaMemsetAsync(V + 2 * n, 0, n * 4, st));
+        const CzPlan& z = c->cz;
+        if (c->use_coarse && c->use_persist != 2 && z.ok && z.nc == 1 && z.serial == c->pattern_serial && z.sell_built &&
+            z.sell_serial == c->asm_serial && z.bnd_serial == z.serial) {  // the product of the two-level solve that ran
+            const CzSpmv m = {z.bnd.p, z.soff.p, z.val.p, V + 2 * n, V + 3 * n, S, c->dpart.p, (int)n};
+            if (warm) launch_coarse_spmv(c, c->spmv_lpr32, st, m);
+            cudaEventRecord(c->ev[2], st);
+            for (int r = 0; r < nrep; ++r) launch_coarse_spmv(c, c->spmv_lpr32, st, m);
+            cudaEventRecord(c->ev[3], st);
+            ISL_CHECK_CUDA(c, cudaEventSynchronize(c->ev[3]));
+            float t = 0.f;
+            cudaEventElapsedTime(&t, c->ev[2], c->ev[3]);
+            *ms = (double)t / nrep;
+            c->launches += nrep + (warm ? 1 : 0);
+            return ISL_OK;
+        }
         rc = ensure_ssell(c);
         if (rc != ISL_OK) return rc;
         if (!c->spmv_lpr32) c->spmv_lpr32 = autotune_spmv32(c, V + 2 * n, V + 3 * n, S, c->dpart.p);
