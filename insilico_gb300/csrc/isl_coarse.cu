@@ -395,8 +395,8 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_coarse(CzIter a) {
 // the slice's (in warp order).  With one warp per slice the 16,608 slices of a
 // P2 mesh took three rounds of 7,296 warps where 2.3 were work; all gathers of
 // a batch come before its sums, as nothing moves across the tests for a
-// slice's end.  531k rows of P2 tetrahedra: 42.5 -> 32.8 us with 12 slots in
-// flight and 4 CTAs per SM; 41 us with 8 and 6, whose registers spill.
+// slice's end.  531k rows of P2 tetrahedra: 42.5 -> 32-33 us with 8 or 12 slots
+// in flight and 4 CTAs per SM; 41 us with 8 and 6, whose registers spill.
 constexpr int SPMV_PER_SM = 4;
 template <int U, typename TC>
 __global__ void __launch_bounds__(256, SPMV_PER_SM) k_cz_spmv(CzSpmv m, const TC* __restrict__ col) {

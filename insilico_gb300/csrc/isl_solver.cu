@@ -3179,7 +3179,7 @@ int time_spmv(isl_ctx* c, int precision, int nrep, double* ms) {
         float* V = c->w32.p;
         ISL_CHECK_CUDA(c, cudaMemsetAsync(V + 2 * n, 0, n * 4, st));
         const CzPlan& z = c->cz;
-        if (c->use_coarse && c->use_persist != 2 && z.ok && z.nc == 1 && z.serial == c->pattern_serial && z.sell_built &&
+        if (c->spmv_lpr32 >= 100 && c->use_coarse && c->use_persist != 2 && z.ok && z.nc == 1 && z.serial == c->pattern_serial && z.sell_built &&
             z.sell_serial == c->asm_serial && z.bnd_serial == z.serial) {  // the product of the two-level solve that ran
             const CzSpmv m = {z.bnd.p, z.soff.p, z.val.p, V + 2 * n, V + 3 * n, S, c->dpart.p, (int)n};
             if (warm) launch_coarse_spmv(c, c->spmv_lpr32, st, m);
