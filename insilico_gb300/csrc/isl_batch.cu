@@ -839,7 +839,7 @@ int solve_batched(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t*
                 solved[k] = res[k].fin == 1;
                 left -= solved[k];
             }
-            c->spmv_lpr32 = c->dim == 2 && c->fedeg == 1 ? 4 : 8;  // CSR lanes per row of its product
+            c->spmv32_used = c->dim == 2 && c->fedeg == 1 ? 4 : 8;  // CSR lanes per row of its product
             if (left == 0) {
                 kb_copy<<<vg, BBS, 0, st>>>((int)n, W + 2 * n, c->dsol.p);
                 c->launches += 1;
@@ -946,7 +946,7 @@ int solve_batched(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t*
                 if (ncand > 1) tune_store(c, "bspmv_batch", best);
             }
         }
-        c->spmv_lpr32 = c->bspmv32;
+        c->spmv32_used = c->bspmv32;
         const unsigned g32 = c->bspmv32 >= 100 ? sgrid : lgrid;
         ISL_CHECK_CUDA(c, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         kb_compact<<<1, 1024, 0, st>>>(a, c->dbact.p);

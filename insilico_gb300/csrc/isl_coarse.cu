@@ -2225,6 +2225,7 @@ int coarse_plan(isl_ctx* c, int nc, int64_t nrow, int ncta) {
     if (z.serial != c->pattern_serial || z.nc != nc) {
         z.ok = z.sell_built = z.csr_built = false;
         z.num_serial = z.sell_serial = z.csr_serial = z.binv_serial = -1;
+        z.spmv_kind = 0;
         z.nc = nc;
         z.m = nc == 3 ? 6 : 1 + c->dim;
         z.nrow = nrow;

@@ -759,7 +759,7 @@ int isl_field_create(isl_ctx* c, int fe_degree, int ncomp, int64_t* n_dofobj, in
     // buffers sized by the previous field (a context reused for a new problem)
     c->dcval.release(); c->deq.release(); c->dstatus.release();
     c->inertia = false; c->nhist = 0; c->dhist.release(); c->nforce_w = 0;
-    c->spmv_lpr64 = c->spmv_lpr32 = c->bspmv_lpb = 0;
+    c->spmv_lpr64 = c->spmv_lpr32 = c->spmv32_used = c->bspmv_lpb = 0;
     c->nbblocks = 0;
     c->mask_on = false;
     c->bsell_built = false;
@@ -1005,7 +1005,7 @@ int isl_register_pattern(isl_ctx* c, int64_t* nnz) {
     if (!c || !c->numbered) return ISL_ERR_ARG;
     if (c->device < 0) ISL_FAIL(c, ISL_ERR_ARG, "host-only context: the pattern is built on the device");
     cudaSetDevice(c->device);
-    c->spmv_lpr64 = c->spmv_lpr32 = c->bspmv_lpb = 0;
+    c->spmv_lpr64 = c->spmv_lpr32 = c->spmv32_used = c->bspmv_lpb = 0;
     c->nbblocks = 0;
     c->mask_on = false;
     c->bsell_built = false;
@@ -1516,7 +1516,8 @@ int isl_set_option(isl_ctx* c, int key, int64_t value) {
         if (value < 0 || value > 108 || !isl::spmv32_kind_valid(c, (int)value))
             ISL_FAIL(c, ISL_ERR_ARG, "ISL_OPT_SPMV32_KIND: 0, CSR lanes per row 2..32, or 102/104/108 with a sliced-ELL copy");
         c->spmv32_forced = (int)value;
-        c->spmv_lpr32 = (int)value;
+        c->spmv_lpr32 = c->spmv32_used = (int)value;
+        c->cz.spmv_kind = 0;
         return ISL_OK;
     }
     ISL_FAIL(c, ISL_ERR_ARG, "unknown or read-only option");
@@ -1544,7 +1545,7 @@ int isl_get_option(isl_ctx* c, int key, int64_t* value) {
     if (key == ISL_OPT_BLOCKED) { *value = c->blocked ? (c->bpad ? 2 : 1) : 0; return ISL_OK; }
     if (key == ISL_OPT_NBLOCKS) { *value = c->blocked ? c->nblk : 0; return ISL_OK; }
     if (key == ISL_OPT_NSLOTS) { *value = c->blocked ? c->nslot : 0; return ISL_OK; }
-    if (key == ISL_OPT_SPMV32_KIND) { *value = c->spmv_lpr32; return ISL_OK; }
+    if (key == ISL_OPT_SPMV32_KIND) { *value = c->spmv32_used; return ISL_OK; }
     if (key == ISL_OPT_HOST_SETUP) { *value = c->host_setup; return ISL_OK; }
     if (key == ISL_OPT_BICGSTAB_KIND) { *value = c->bicg_lpr; return ISL_OK; }
     if (key == ISL_OPT_SCALAR_SLOTS) {

@@ -164,6 +164,7 @@ struct CzPlan {
     DBuf<int32_t> bnd;        // product: first slice of every CTA
     int64_t bnd_serial = -1;
     int spmv_ncta = 0;
+    int spmv_kind = 0;        // its slots in flight (102: 4, 104: 8, 108: 12), 0: not chosen yet
     // one-cluster solve: (block) CSR in list order, aggregates of every CTA
     bool csr_built = false;
     int64_t csr_serial = -1, nent = 0;
@@ -358,7 +359,8 @@ struct isl_ctx {
     int64_t bicg_serial = -1, pattern_serial = 0;
     isl::DBuf<isl::CGScal> dscal;
     isl::CGScal* hscal = nullptr;  // pinned host mirror
-    int spmv_lpr64 = 0, spmv_lpr32 = 0;  // autotuned lanes per row (FP32: 100 + U = sliced-ELL, U slots in flight)
+    int spmv_lpr64 = 0, spmv_lpr32 = 0;  // one-level solves: autotuned lanes per row (FP32: 100 + U = sliced-ELL, U slots in flight)
+    int spmv32_used = 0;         // FP32 product kind of the last mixed solve that chose one (ISL_OPT_SPMV32_KIND read back)
     isl::DBuf<int32_t> ol_row0;  // one-launch FP64 solves: row ranges of the CTAs, result
     isl::DBuf<isl::OlScal> ol_scal;
     isl::CzPlan cz;              // two-level preconditioner of the mixed solve

@@ -1131,6 +1131,7 @@ static int solve_mixed(isl_ctx* c, double tol, int64_t max_iter, int64_t* iters,
         ISL_CHECK_CUDA(c, cudaMemsetAsync(p32, 0, n * 4, st));
         c->spmv_lpr32 = autotune_spmv32(c, p32, q32, c->dscal.p, c->dpart.p);
     }
+    c->spmv32_used = c->spmv_lpr32;
     const bool exact64 = c->have64;  // without the FP64 matrix: plain FP32 CG (inexact Newton tangents)
     if (exact64 && !c->spmv_lpr64)
         c->spmv_lpr64 = autotune_lpr<double, double>(c, c->dval64.p, c->drhs.p, W + 3 * n, c->dscal.p, c->dpart.p);
@@ -2871,10 +2872,9 @@ static void launch_rl_residual(isl_ctx* c, unsigned grid, cudaStream_t st, const
     }
 }
 
-// slots in flight of the scalar two-level product: as set, from the tuning
-// cache, or timed (the first within 2 % of the fastest in a fixed order)
+// slots in flight of the scalar two-level product: from the tuning cache, or
+// timed (the first within 2 % of the fastest in a fixed order)
 static int pz_kind(isl_ctx* c, const CzSpmv& m) {
-    if (c->spmv32_forced) return c->spmv32_forced;
     if (c->neq < 20000) return 108;
     const int cand[3] = {108, 104, 102};
     int cached = 0, best = 108;
@@ -2996,11 +2996,15 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
         rc = coarse_spmv_plan(c);
         if (rc != ISL_OK) return rc;
         m = {c->cz.bnd.p, c->cz.soff.p, c->cz.val.p, p32, q32, S, c->dpart.p, (int)rows};
-        if (!c->spmv_lpr32) {
+        // (a CSR kind set through ISL_OPT_SPMV32_KIND is the one-level solve's)
+        if (c->spmv32_forced >= 100) {
+            c->cz.spmv_kind = c->spmv32_forced;
+        } else if (!c->cz.spmv_kind) {
             ISL_CHECK_CUDA(c, cudaMemsetAsync(p32, 0, na * 4, st));
-            c->spmv_lpr32 = pz_kind(c, m);
+            c->cz.spmv_kind = pz_kind(c, m);
         }
-        kind = c->spmv_lpr32 >= 100 ? c->spmv_lpr32 : 108;  // CSR kinds: the one-level solve's
+        kind = c->cz.spmv_kind;
+        c->spmv32_used = c->spmv32_forced ? c->spmv32_forced : kind;
     }
     const bool fused = nc == 3 && c->fuse_dir && (kind == 9 || bspmv_dir_kind(kind));
     CzIter a = {};
@@ -3179,12 +3183,13 @@ int time_spmv(isl_ctx* c, int precision, int nrep, double* ms) {
         float* V = c->w32.p;
         ISL_CHECK_CUDA(c, cudaMemsetAsync(V + 2 * n, 0, n * 4, st));
         const CzPlan& z = c->cz;
-        if (c->spmv_lpr32 >= 100 && c->use_coarse && c->use_persist != 2 && z.ok && z.nc == 1 && z.serial == c->pattern_serial && z.sell_built &&
+        const bool csr = c->spmv32_forced > 0 && c->spmv32_forced < 100;  // (set: the one-level product)
+        if (z.spmv_kind && !csr && c->use_coarse && c->use_persist != 2 && z.ok && z.nc == 1 && z.serial == c->pattern_serial && z.sell_built &&
             z.sell_serial == c->asm_serial && z.bnd_serial == z.serial) {  // the product of the two-level solve that ran
             const CzSpmv m = {z.bnd.p, z.soff.p, z.val.p, V + 2 * n, V + 3 * n, S, c->dpart.p, (int)n};
-            if (warm) launch_coarse_spmv(c, c->spmv_lpr32, st, m);
+            if (warm) launch_coarse_spmv(c, z.spmv_kind, st, m);
             cudaEventRecord(c->ev[2], st);
-            for (int r = 0; r < nrep; ++r) launch_coarse_spmv(c, c->spmv_lpr32, st, m);
+            for (int r = 0; r < nrep; ++r) launch_coarse_spmv(c, z.spmv_kind, st, m);
             cudaEventRecord(c->ev[3], st);
             ISL_CHECK_CUDA(c, cudaEventSynchronize(c->ev[3]));
             float t = 0.f;
@@ -3196,6 +3201,7 @@ int time_spmv(isl_ctx* c, int precision, int nrep, double* ms) {
         rc = ensure_ssell(c);
         if (rc != ISL_OK) return rc;
         if (!c->spmv_lpr32) c->spmv_lpr32 = autotune_spmv32(c, V + 2 * n, V + 3 * n, S, c->dpart.p);
+        c->spmv32_used = c->spmv_lpr32;
         if (warm) launch_spmv32(c, c->spmv_lpr32, vec_grid(c), st, V + 2 * n, V + 3 * n, S, c->dpart.p);
         cudaEventRecord(c->ev[2], st);
         for (int r = 0; r < nrep; ++r) launch_spmv32(c, c->spmv_lpr32, vec_grid(c), st, V + 2 * n, V + 3 * n, S, c->dpart.p);
