@@ -2878,7 +2878,8 @@ static int pz_kind(isl_ctx* c, const CzSpmv& m) {
     if (c->neq < 20000) return 108;
     const int cand[3] = {108, 104, 102};
     int cached = 0, best = 108;
-    if (tune_lookup(c, "spmv32", &cached) && std::find(cand, cand + 3, cached) != cand + 3) return cached;
+    // (a key of its own: the one-level solve's kinds of these numbers are other kernels)
+    if (tune_lookup(c, "spmv32_cz", &cached) && std::find(cand, cand + 3, cached) != cand + 3) return cached;
     float ms_of[3], bestms = 1e30f;
     cudaMemsetAsync(m.S, 0, sizeof(CGScal), c->stream);
     c->launches += 33;
@@ -2893,7 +2894,7 @@ static int pz_kind(isl_ctx* c, const CzSpmv& m) {
     }
     for (int k = 2; k >= 0; --k)
         if (ms_of[k] <= 1.02f * bestms) best = cand[k];
-    tune_store(c, "spmv32", best);
+    tune_store(c, "spmv32_cz", best);
     return best;
 }
 

@@ -48,3 +48,33 @@ def test_iteration_limit_ends_as_one_level(case):
     assert st == A.ISL_ERR_NOT_CONVERGED and it == 5 and np.isfinite(rel) and rel > 1e-12
     assert np.isfinite(S.solution()).all()
     S.close()
+
+
+def test_tuning_one_solve_leaves_the_other_choice_alone(tmp_path):
+    """100,489 equations: both solves time their products; each choice has a line
+    of its own in the tuning file and stays what it was when the other is made"""
+    L = A.load()
+    path = tmp_path / "tune.txt"
+    assert L.isl_tune_cache(str(path).encode()) == A.ISL_OK
+
+    def run(two_level):
+        S = W.setup_system(W.config("c1", n=318))
+        S.set_option(A.OPT_TWO_LEVEL, two_level)
+        S.assemble(A.PREC_MIXED)
+        S.solve(A.SOLVE_CG_FP32_IR, tol=1e-8)
+        out = S.get_option(A.OPT_SPMV32_KIND), S.get_option(A.OPT_TUNE_RUNS)
+        S.close()
+        return out
+    try:
+        two, _ = run(1)
+        one, runs = run(0)
+        assert runs >= 1
+        choice = {}
+        for line in path.read_text().splitlines():
+            if line.startswith("spmv32"):
+                choice.setdefault(line.split()[0], []).append(int(line.split()[-1]))
+        assert len(choice) == 2 and all(len(v) == 1 for v in choice.values())
+        assert sorted(v[0] for v in choice.values()) == sorted([two, one])
+        assert run(1) == (two, 0) and run(0) == (one, 0)
+    finally:
+        L.isl_tune_cache(None)
