@@ -819,13 +819,13 @@ int solve_batched(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t*
             const int limit = (int)std::min<int64_t>(a.max_iter, std::max<int64_t>(1000, rows / 4));
             const double drop = refine ? c->ru_drop2 : 0.0;
             if (z.norder > 0) {
-                ISL_CHECK_CUDA(c, launch_coarse_cluster(c, false, false, V, V + 3 * n, W + 2 * n, tol, drop, limit));
+                ISL_CHECK_CUDA(c, launch_coarse_cluster(c, false, V, V + 3 * n, W + 2 * n, tol, drop, limit));
                 c->launches += 1;
             }
             if (grids) {
                 ISL_CHECK_CUDA(c, cudaMemsetAsync(c->dscal.p, 0, sizeof(CGScal), st));
                 for (int b = 0; b < (int)z.big.size(); ++b)
-                    ISL_CHECK_CUDA(c, launch_coarse_cluster(c, true, false, V, V + 3 * n, W + 2 * n, tol, drop, limit, b));
+                    ISL_CHECK_CUDA(c, launch_coarse_cluster(c, true, V, V + 3 * n, W + 2 * n, tol, drop, limit, b));
                 c->launches += (int64_t)z.big.size();
                 int fault = 0;
                 ISL_CHECK_CUDA(c, cudaMemcpyAsync(&fault, &c->dscal.p->fault, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -553,7 +553,7 @@ struct CzClu {
     float2* part;            // grid form: the CTAs' sums, four slots
     unsigned* bar;
     int inv_smem;            // the CTA's rows of the inverse are held in shared memory
-    unsigned armed;          // test hook: added to the arrivals a grid barrier waits for
+    unsigned bar_start;      // grid form: count at which the barrier starts
 };
 
 
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     }
     int slot = 0;
     bool alive = true;  // grid form: false in every thread once a barrier has timed out
-    GridBarrier gb(a.bar, &a.S->fault, a.armed);
+    GridBarrier gb(a.bar, &a.S->fault, a.bar_start);
     auto sync_all = [&]() {
         if constexpr (GRID) alive = gb.sync();
         else cl.sync();
@@ -2297,7 +2297,6 @@ static cudaError_t launch_clu(const CzPlan& z, int grid, size_t smem, cudaStream
         const void* k = wide ? (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 1024>
                              : (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 512>;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX);
-        if (e == cudaSuccess) e = cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), st);
         void* args[] = {&a};
         return e == cudaSuccess ? cudaLaunchCooperativeKernel(k, dim3(grid), dim3(wide ? 1024 : 512), args, smem, st) : e;
     }
@@ -2324,8 +2323,8 @@ static cudaError_t launch_clu(const CzPlan& z, int grid, size_t smem, cudaStream
     return cudaLaunchKernelEx(&cfg, k, a);
 }
 
-cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, bool arm, float* work, const float* dinv, double* x64, double tol,
-                                  double drop, int max_iter, int big) {
+cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, float* work, const float* dinv, double* x64, double tol, double drop,
+                                  int max_iter, int big) {
     CzPlan& z = c->cz;
     bool ms, as;
     const size_t smem = cluster_smem(z, &ms, &as, big >= 0);
@@ -2353,7 +2352,10 @@ cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, bool arm, float* wo
     a.max_ent = big >= 0 ? z.big_ent : z.max_ent;
     a.part = reinterpret_cast<float2*>(c->dpart.p); a.bar = c->dbar.p;
     a.inv_smem = as ? 1 : 0;
-    a.armed = arm ? 0x40000000u : 0u;
+    if (grid) {
+        const cudaError_t e = grid_barrier_start(c, &a.bar_start);
+        if (e != cudaSuccess) return e;
+    }
     // lanes per row: by the mean row length; in a batch by the element alone, so
     // that an instance's sums do not depend on the others
     const bool wide = batch ? !(c->dim == 2 && c->fedeg == 1) : (double)z.nent > 12.0 * (double)z.nrow;

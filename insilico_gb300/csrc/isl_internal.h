@@ -470,6 +470,8 @@ int ensure_val32(isl_ctx* c);
 int affine_lift(isl_ctx* c, int incremental);
 int inst_norms_device(isl_ctx* c, double* out);
 int distribute_masked(isl_ctx* c, int add);
+// counter of the next GridBarrier launch and the start of its goals (isl_device.cuh); consumes ISL_OPT_BARRIER_TEST
+cudaError_t grid_barrier_start(isl_ctx* c, unsigned* start);
 int cluster_ctas(isl_ctx* c);  // CTAs of the largest cluster that can be launched (0: none)
 int solve_onelaunch(isl_ctx* c, bool bicg, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* nc, bool* ran);
 int solve_bicgstab(isl_ctx* c, double tol, int64_t max_iter, int64_t* iters, double* rel, bool* nc);

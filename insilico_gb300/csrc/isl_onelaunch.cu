@@ -41,6 +41,7 @@ struct OlArgs {
     double *x;
     double* part;                      // [4 slots][2][CTAs]
     unsigned* bar;
+    unsigned bar_start;                // count at which the grid barrier starts
     OlScal* S;
     double tol;
     int max_iter;
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(OT_CG, 1) k_ol_cg(OlArgs a) {
     extern __shared__ __align__(16) unsigned char ol_smem[];
     __shared__ double s[2], sc;
     __shared__ int ctl;
-    GridBarrier gb(a.bar, &a.S->fault);
+    GridBarrier gb(a.bar, &a.S->fault, a.bar_start);
     const OlMem m = ol_mem(a, ol_smem, 6, 1);
     double *xs = m.row, *rs = xs + a.R, *qs = rs + a.R, *ds = qs + a.R, *w1 = ds + a.R, *w2 = w1 + a.R, *ph = m.hal;
     const int tid = threadIdx.x;
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(OT_BI, 1) k_ol_bicgstab(OlArgs a) {
     extern __shared__ __align__(16) unsigned char ol_smem[];
     __shared__ double s[2], sc[2];
     __shared__ int ctl;
-    GridBarrier gb(a.bar, &a.S->fault);
+    GridBarrier gb(a.bar, &a.S->fault, a.bar_start);
     const OlMem m = ol_mem(a, ol_smem, 7, 4);
     double *xs = m.row, *rs = xs + a.R, *r0s = rs + a.R, *vs = r0s + a.R, *ts = vs + a.R, *w1 = ts + a.R, *w2 = w1 + a.R;
     double *ph = m.hal, *dh = ph + a.H, *rh = dh + a.H, *yh = rh + a.H;  // p, D^-1, r, and y or z at the CTA's columns
@@ -461,10 +462,11 @@ int solve_onelaunch(isl_ctx* c, bool bicg, double tol, int64_t max_iter, int64_t
     ISL_CHECK_CUDA(c, c->dsol.alloc(n));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(c->ol_row0.p, row0.data(), row0.size() * 4, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemsetAsync(c->ol_scal.p, 0, sizeof(OlScal), st));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(c->dbar.p, 0, 2 * sizeof(unsigned), st));
+    unsigned bar_start = 0;
+    ISL_CHECK_CUDA(c, grid_barrier_start(c, &bar_start));
     const size_t smem = ol_bytes(n, R, E, (int)H, nd, nh, vals);
     OlArgs a = {n, c->drowptr.p, c->dcolind.p, c->ddiag.p, c->ol_row0.p, c->dval64.p, c->drhs.p, R, E, (int)H, vals ? 1 : 0, c->nnz <= 32 * (int64_t)n ? 2 : 4,
-                c->w64.p, c->w64.p + n, c->w64.p + 2 * (size_t)n, c->dsol.p, c->dpart.p, c->dbar.p, c->ol_scal.p, tol,
+                c->w64.p, c->w64.p + n, c->w64.p + 2 * (size_t)n, c->dsol.p, c->dpart.p, c->dbar.p, bar_start, c->ol_scal.p, tol,
                 (int)std::min<int64_t>(max_iter, INT32_MAX - 1)};
     const void* k = bicg ? (const void*)k_ol_bicgstab : (const void*)k_ol_cg;
     ISL_CHECK_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OL_SMEM_MAX));

@@ -518,6 +518,12 @@ static int capture_chunk(isl_ctx* c, const TV* val, TX* x, TX* r, TX* p, TX* q, 
     return ISL_OK;
 }
 
+cudaError_t grid_barrier_start(isl_ctx* c, unsigned* start) {
+    *start = c->barrier_test ? 0x40000000u : 0u;  // armed: arrivals that never come
+    c->barrier_test = false;
+    return cudaMemsetAsync(c->dbar.p, 0, 2 * sizeof(unsigned), c->stream);
+}
+
 static int read_scal(isl_ctx* c) {
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(c->hscal, c->dscal.p, sizeof(CGScal), cudaMemcpyDeviceToHost, c->stream));
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -2908,9 +2914,7 @@ static int solve_two_level_cluster(isl_ctx* c, int nc, bool grid, double tol, in
     int rc = coarse_numeric(c, true, d32);
     if (rc != ISL_OK) return rc;
     ISL_CHECK_CUDA(c, cudaMemsetAsync(c->dscal.p, 0, sizeof(CGScal), st));
-    const bool arm = grid && c->barrier_test;
-    if (arm) c->barrier_test = false;
-    ISL_CHECK_CUDA(c, launch_coarse_cluster(c, grid, arm, V, d32, x64, tol, c->have64 ? c->ru_drop2 : 0.0,
+    ISL_CHECK_CUDA(c, launch_coarse_cluster(c, grid, V, d32, x64, tol, c->have64 ? c->ru_drop2 : 0.0,
                                             (int)std::min<int64_t>(max_iter, INT32_MAX - 1)));
     c->launches += 1;
     rc = read_scal(c);
@@ -3113,7 +3117,7 @@ int solve_device(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t* 
         const bool bicg = method == ISL_SOLVE_BICGSTAB;
         bool ran = false;
         if (!bicg || !c->bicg_forced) rc = solve_onelaunch(c, bicg, tol, max_iter, &it, &rel, &nc, &ran);
-        if (rc == ISL_OK && ran && bicg && !c->bicg_lpr) c->bicg_lpr = 8;  // lanes per row of its product
+        if (rc == ISL_OK && ran && bicg && !c->bicg_lpr) c->bicg_lpr = 8;  // (reported for the one launch; the graph path still tunes)
         if (rc == ISL_OK && !ran)
             rc = bicg ? solve_bicgstab(c, tol, max_iter, &it, &rel, &nc) : solve_fp64(c, tol, max_iter, &it, &rel, &nc);
     }
