@@ -341,7 +341,8 @@ int isl_timings(isl_ctx* ctx, double* ms /* [ISL_NTIMERS] */, int64_t* counts /*
  * (the same recurrences; ISL_OPT_BICGSTAB_KIND then reads 8).  ISL_OPT_BARRIER_TEST (test
  * hook, write-only, one-shot): the next persistent launch starts with its grid
  * barrier armed so that it cannot complete; its bounded wait runs out and the
- * solve returns ISL_ERR_TIMEOUT with the context still usable.
+ * solve returns ISL_ERR_TIMEOUT with the context still usable (2: the barrier's
+ * counter starts where it wraps at once, and the solve is the usual one).
  * ISL_OPT_SPMV32_KIND: the FP32 SpMV of the scalar mixed solve, 0 (default)
  * autotuned on the matrix, 2, 4, 8, 16 or 32 CSR with that many lanes per
  * row, 102, 104 or 108 the sliced-ELL copy with 2, 4 or 8 slots of loads in

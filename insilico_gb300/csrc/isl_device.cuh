@@ -106,10 +106,13 @@ __device__ inline bool grid_sync(unsigned* bar, int* fault) {
     return gs_ok != 0;
 }
 
-// Grid barrier on one counter that only grows (zeroed before the launch): every
-// CTA arrives with a release add and polls for the arrivals that complete the
-// barrier, without the second word of grid_sync.  Bounded; on expiry, or when
-// another CTA has set *fault, it reports false in every thread of the CTA.
+// Grid barrier on one counter that only grows (set to `start` before the launch):
+// every CTA arrives with a release add and polls for the arrivals that complete
+// the barrier, without the second word of grid_sync.  The counter may wrap (2^32
+// arrivals are 14 million iterations of a CG over 152 CTAs): no CTA is more than
+// one barrier ahead, so the sign of the difference tells before from after.
+// Bounded; on expiry, or when another CTA has set *fault, it reports false in
+// every thread of the CTA.
 struct GridBarrier {
     unsigned* bar;
     int* fault;
@@ -125,7 +128,7 @@ struct GridBarrier {
             asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(bar) : "memory");
             for (unsigned it = 0;; ++it) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-                if (v >= goal) break;
+                if ((int)(v - goal) >= 0) break;
                 if (it > GRID_SYNC_LIMIT || ((it & 255) == 255 && *(volatile int*)fault)) {
                     ok = 0;
                     atomicExch(fault, 1);

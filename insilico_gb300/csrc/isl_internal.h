@@ -272,7 +272,7 @@ struct isl_ctx {
     int use_persist = 1;         // one-launch CG kernels: 0 never, 1 for small systems, 2 always where supported
     int cluster_size = -1;       // CTAs of the small-system cluster solve (-1: not yet probed, 0: unavailable)
     int persist_grid = -1;       // blocks of the persistent kernel (-1: not yet probed, 0: unavailable)
-    bool barrier_test = false;   // test hook: the next persistent launch finds its grid barrier pre-armed (never completes)
+    int barrier_test = 0;        // test hook: the next persistent launch finds its grid barrier pre-armed (1: never completes; 2: its counter wraps)
     isl::DBuf<unsigned int> dbar; // grid barrier of the persistent kernel: arrivals, generation
     int64_t nbr = 0, nblk = 0;
     isl::DBuf<int32_t> dbptr, dbcol, dbrow;

@@ -519,9 +519,13 @@ static int capture_chunk(isl_ctx* c, const TV* val, TX* x, TX* r, TX* p, TX* q, 
 }
 
 cudaError_t grid_barrier_start(isl_ctx* c, unsigned* start) {
-    *start = c->barrier_test ? 0x40000000u : 0u;  // armed: arrivals that never come
-    c->barrier_test = false;
-    return cudaMemsetAsync(c->dbar.p, 0, 2 * sizeof(unsigned), c->stream);
+    // hook: 1: goals that need arrivals that never come; 2: the first barriers wrap
+    const int test = c->barrier_test;
+    c->barrier_test = 0;
+    const unsigned near_wrap = 0xffffffc0u;
+    *start = test == 1 ? 0x40000000u : test == 2 ? near_wrap : 0u;
+    return test == 2 ? cudaMemcpyAsync(c->dbar.p, &near_wrap, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream)
+                     : cudaMemsetAsync(c->dbar.p, 0, sizeof(unsigned), c->stream);
 }
 
 static int read_scal(isl_ctx* c) {
@@ -2690,8 +2694,8 @@ static int solve_mixed_b3(isl_ctx* c, double tol, int64_t max_iter, int64_t* ite
             // mid-count); the test hook arms it with an arrival count that the
             // grid never reaches
             const unsigned armed[2] = {0x40000000u, 0u};
-            const bool arm = c->barrier_test;
-            c->barrier_test = false;
+            const bool arm = c->barrier_test == 1;
+            c->barrier_test = 0;
             if ((arm ? cudaMemcpyAsync(c->dbar.p, armed, sizeof(armed), cudaMemcpyHostToDevice, st)
                      : cudaMemsetAsync(c->dbar.p, 0, 2 * sizeof(unsigned), st)) != cudaSuccess ||
                 cudaLaunchCooperativeKernel((const void*)k_cg_persist_b3, dim3(pgrid), dim3(BS), pargs, 0, st) != cudaSuccess) {

@@ -63,3 +63,15 @@ def test_barrier_timeout_reports_status(name):
     it2, _, st = S.solve(method, tol=1e-10)
     assert st == A.ISL_OK and it2 == it and np.array_equal(S.solution(), x)
     S.close()
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_barrier_counter_wraps(name):
+    """the barrier's 32-bit counter starts 64 arrivals below its wrap"""
+    S, method = CASES[name]()
+    it, _, _ = S.solve(method, tol=1e-10)
+    x = S.solution()
+    S.set_option(A.OPT_BARRIER_TEST, 2)
+    it2, _, st = S.solve(method, tol=1e-10, check=False)
+    assert st == A.ISL_OK and it2 == it and np.array_equal(S.solution(), x)
+    S.close()
