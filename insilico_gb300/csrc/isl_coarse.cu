@@ -535,7 +535,6 @@ struct CzClu {
     const int* order;        // batch: the instance of every cluster
     int inst_id;             // the instance, where order is null
     OlScal* res;             // batch: results (null: S)
-    int max_ndp;
     const int *rp, *ci;      // (block) CSR in list order
     const float* val;        // [NC * NC][nent]
     int nent;
@@ -549,7 +548,6 @@ struct CzClu {
     CGScal* S;
     double tol, drop;
     int max_iter, exact64;
-    int max_rows, max_aggs, max_ent;
     float2* part;            // grid form: the CTAs' sums, four slots
     unsigned* bar;
     int inv_smem;            // the CTA's rows of the inverse are held in shared memory
@@ -585,23 +583,23 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     const int c0 = (ag0 - in.agg0) * M;                // first coarse unknown of this CTA
     const float* ainv = a.ainv + in.a0 + (size_t)c0 * ndp;
     const int t0 = a.sofs[ag0 * NW], nr = a.sofs[ag1 * NW] - t0;
-    const int R = a.max_rows;
+    const int R = in.rows, E = in.ent;
     float4* ln = reinterpret_cast<float4*>(smem);     // positions; w: aggregate (local), mask above
     float* rcs = smem + 4 * (size_t)R;                // [ndp], 16-byte aligned as ln
-    float* ais = rcs + a.max_ndp;                     // [agg M][ndp]
-    float* xs = ais + (a.inv_smem ? (size_t)a.max_aggs * M * a.max_ndp : 0);
+    float* ais = rcs + ndp;                           // [agg M][ndp]
+    float* xs = ais + (a.inv_smem ? (size_t)in.aggs * M * ndp : 0);
     float* rs = xs + (size_t)NC * R;
     float* qs = rs + (size_t)NC * R;
     float* zs = qs + (size_t)NC * R;
     float* ps = zs + (size_t)NC * R;
     float* ds = ps + (size_t)NC * R;                  // [NC * NC][row]
     float* src = ds + (size_t)(NC * NC) * R;          // [sub][M]
-    float* zcs = src + (size_t)a.max_aggs * NW * M;   // [agg][M]
-    float* dss = zcs + (size_t)a.max_aggs * M;        // [sub][M * M]
-    int* nat = reinterpret_cast<int*>(dss + (size_t)a.max_aggs * NW * M * M);  // natural row
+    float* zcs = src + (size_t)in.aggs * NW * M;      // [agg][M]
+    float* dss = zcs + (size_t)in.aggs * M;           // [sub][M * M]
+    int* nat = reinterpret_cast<int*>(dss + (size_t)in.aggs * NW * M * M);  // natural row
     int* rps = nat + R;                               // MS: rows, columns, values
     int* cis = rps + R + 1;
-    float* vs = reinterpret_cast<float*>(cis + a.max_ent);
+    float* vs = reinterpret_cast<float*>(cis + E);
     for (int u = w; u < na * NW; u += CLT / 32) {
         const int s0 = a.sofs[ag0 * NW + u], s1 = a.sofs[ag0 * NW + u + 1];
         for (int t = s0 + lane; t < s1; t += 32) {
@@ -633,7 +631,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
         for (int k = tid; k < ne; k += CLT) {
             cis[k] = a.ci[e0 + k];
 #pragma unroll
-            for (int e = 0; e < NC * NC; ++e) vs[(size_t)e * a.max_ent + k] = a.val[(size_t)e * a.nent + e0 + k];
+            for (int e = 0; e < NC * NC; ++e) vs[(size_t)e * E + k] = a.val[(size_t)e * a.nent + e0 + k];
         }
     }
     int slot = 0;
@@ -989,7 +987,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
                 for (int c = 0; c < NC; ++c)
 #pragma unroll
                     for (int e = 0; e < NC; ++e)
-                        acc[c] += (MS ? vs[(size_t)(NC * c + e) * a.max_ent + k] : __ldg(a.val + (size_t)(NC * c + e) * a.nent + k)) * x[e];
+                        acc[c] += (MS ? vs[(size_t)(NC * c + e) * E + k] : __ldg(a.val + (size_t)(NC * c + e) * a.nent + k)) * x[e];
             }
 #pragma unroll
             for (int c = 0; c < NC; ++c)
@@ -1871,7 +1869,6 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     int32_t run = 0, na = 0;
     long long a0 = 0, p0 = 0;
     int rc0 = 0;
-    z.max_ndp = 0;
     for (int k = 0; k < ni; ++k) {
         CzInst& in = z.hinst[k];
         in.agg0 = na;
@@ -1893,7 +1890,6 @@ int build_plan(isl_ctx* c, CzPlan& z) {
         a0 += (long long)in.ndp * in.ndp;
         p0 += 2LL * TB * in.ndp + 2 * TB * TB;
         rc0 += 2 * in.ndp;
-        z.max_ndp = std::max(z.max_ndp, in.ndp);
     }
     so.push_back(run);
     z.nagg = na;
@@ -2021,13 +2017,10 @@ size_t cluster_need(const CzPlan& z, int rows, int aggs, int ndp, int ent, bool 
            : z.m == 4 ? clu_smem<1, 4, 8>(rows, aggs, ndp, ent, m, s) : clu_smem<1, 3, 4>(rows, aggs, ndp, ent, m, s);
 }
 size_t cluster_smem(const CzPlan& z, bool* ms, bool* as, bool big = false) {
-    auto need = [&](bool m, bool s) {
-        return big ? cluster_need(z, z.big_rows, z.big_aggs, z.big_ndp, z.big_ent, m, s)
-                   : cluster_need(z, z.max_rows, z.max_aggs, z.max_ndp, z.max_ent, m, s);
-    };
-    *ms = need(true, false) <= CLU_SMEM_MAX;
-    *as = need(*ms, true) <= CLU_SMEM_MAX;
-    return need(*ms, *as);
+    const auto& need = z.smem[big];
+    *ms = need[1][0] <= CLU_SMEM_MAX;
+    *as = need[*ms][1] <= CLU_SMEM_MAX;
+    return need[*ms][*as];
 }
 
 // columns of the aggregate-ordered sliced-ELL copy (scalar systems), once per pattern
@@ -2095,12 +2088,10 @@ int build_csr(isl_ctx* c, CzPlan& z) {
     const int nw = z.m == 3 ? 4 : 8;
     const size_t nc1 = (size_t)z.ncta + 1;
     z.hcta.assign(nc1 * z.ninst, 0);
-    z.max_rows = z.max_aggs = z.max_ent = 0;
-    int max_ndp = 0;
+    for (int k = 0; k < 8; ++k) z.smem[k >> 2][(k >> 1) & 1][k & 1] = 0;
     std::vector<int32_t> order, big_cta;
-    struct Share { int rows = 0, aggs = 0, ent = 0; };
-    auto split = [&](const CzInst& in, int ncta, int32_t* cta) {
-        Share sh;
+    auto split = [&](CzInst& in, int ncta, int32_t* cta) {
+        in.rows = in.aggs = in.ent = 0;
         const int64_t e0 = rp[in.row0], ent = rp[in.row0 + in.nrow] - e0;
         int ag = in.agg0;
         cta[0] = ag;
@@ -2111,42 +2102,41 @@ int build_csr(isl_ctx* c, CzPlan& z) {
                                 (int64_t)rp[z.hsofs[(size_t)ag * nw]] + rp[z.hsofs[(size_t)(ag + 1) * nw]] < goal)) ++ag;
             cta[k + 1] = ag;
             const int t0 = z.hsofs[(size_t)from * nw], t1 = z.hsofs[(size_t)ag * nw];
-            sh.rows = std::max(sh.rows, t1 - t0);
-            sh.aggs = std::max(sh.aggs, ag - from);
-            sh.ent = std::max(sh.ent, rp[t1] - rp[t0]);
+            in.rows = std::max(in.rows, t1 - t0);
+            in.aggs = std::max(in.aggs, ag - from);
+            in.ent = std::max(in.ent, rp[t1] - rp[t0]);
         }
-        return sh;
+        return cluster_need(z, in.rows, in.aggs, in.ndp, in.ent, false, false) <= CLU_SMEM_MAX;
+    };
+    // an instance lays its shared memory out for itself: a launch takes what the
+    // largest of its instances needs, and none is sized by the shares of two
+    auto admit = [&](const CzInst& in, int big) {
+        for (int k = 0; k < 4; ++k) {
+            size_t& need = z.smem[big][k >> 1][k & 1];
+            need = std::max(need, cluster_need(z, in.rows, in.aggs, in.ndp, in.ent, k >> 1, k & 1));
+        }
     };
     z.big.clear();
     z.big_ncta = c->sm_count;
-    z.big_rows = z.big_aggs = z.big_ent = z.big_ndp = 0;
     for (int i = 0; i < z.ninst; ++i) {
-        const CzInst& in = z.hinst[i];
-        const Share sh = split(in, z.ncta, &z.hcta[nc1 * i]);
-        if (z.ninst > 1 && cluster_need(z, sh.rows, sh.aggs, in.ndp, sh.ent, false, false) > CLU_SMEM_MAX) {
+        CzInst& in = z.hinst[i];
+        if (!split(in, z.ncta, &z.hcta[nc1 * i]) && z.ninst > 1) {
             std::vector<int32_t> cb((size_t)z.big_ncta + 1);
-            const Share b = split(in, z.big_ncta, cb.data());
-            if (cluster_need(z, b.rows, b.aggs, in.ndp, b.ent, false, false) > CLU_SMEM_MAX) continue;  // one-level
+            if (!split(in, z.big_ncta, cb.data())) continue;  // one-level
             z.big.push_back(i);
             big_cta.insert(big_cta.end(), cb.begin(), cb.end());
-            z.big_rows = std::max(z.big_rows, b.rows);
-            z.big_aggs = std::max(z.big_aggs, b.aggs);
-            z.big_ent = std::max(z.big_ent, b.ent);
-            z.big_ndp = std::max(z.big_ndp, in.ndp);
+            admit(in, 1);
             continue;
         }
         order.push_back(i);
-        z.max_rows = std::max(z.max_rows, sh.rows);
-        z.max_aggs = std::max(z.max_aggs, sh.aggs);
-        z.max_ent = std::max(z.max_ent, sh.ent);
-        max_ndp = std::max(max_ndp, in.ndp);
+        admit(in, 0);
     }
+    ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.inst.p, z.hinst.data(), (size_t)z.ninst * sizeof(CzInst), cudaMemcpyHostToDevice, st));
     if (!z.big.empty()) {
         ISL_CHECK_CUDA(c, z.cta_big.alloc(big_cta.size()));
         ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.cta_big.p, big_cta.data(), big_cta.size() * 4, cudaMemcpyHostToDevice, st));
         ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
     }
-    z.max_ndp = max_ndp;
     z.norder = (int)order.size();
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return z.hinst[a].nrow > z.hinst[b].nrow; });
     if (z.ninst > 1 && z.norder) {
@@ -2291,9 +2281,10 @@ int coarse_cluster_fits(const isl_ctx* c, bool grid) {
 // as other threads may be launching it too)
 template <int NC, int M, int NW, int LPR, bool MS>
 static cudaError_t launch_clu(const CzPlan& z, int grid, size_t smem, cudaStream_t st, CzClu a) {
+    const CzInst& in = z.hinst[a.inst_id];  // grid: the instance
     const int ncl = a.order ? z.norder : 1;  // clusters
     if (grid) {
-        const bool wide = a.max_rows * LPR > 1024;  // more than two rounds of 512 threads in a product
+        const bool wide = z.hinst[a.inst_id].rows * LPR > 1024;  // more than two rounds of 512 threads in a product
         const void* k = wide ? (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 1024>
                              : (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 512>;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX);
@@ -2338,7 +2329,6 @@ cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, float* work, const 
     a.inst_id = big >= 0 ? z.big[big] : 0;
     if (big >= 0) a.cta = z.cta_big.p + (size_t)big * (z.big_ncta + 1);
     a.res = batch ? z.res.p : nullptr;
-    a.max_ndp = big >= 0 ? z.big_ndp : z.max_ndp;
     a.rp = z.rp.p; a.ci = z.ci.p; a.val = z.cv.p; a.nent = (int)z.nent;
     a.dinv = dinv;
     a.rc = z.rc.p; a.w = work; a.pa = work + na; a.pb = work + 2 * na;
@@ -2347,9 +2337,6 @@ cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, float* work, const 
     a.rowptr = c->drowptr.p; a.colind = c->dcolind.p; a.val64 = c->dval64.p;
     a.S = c->dscal.p;
     a.tol = tol; a.drop = drop; a.max_iter = max_iter; a.exact64 = c->have64 ? 1 : 0;
-    a.max_rows = big >= 0 ? z.big_rows : z.max_rows;
-    a.max_aggs = big >= 0 ? z.big_aggs : z.max_aggs;
-    a.max_ent = big >= 0 ? z.big_ent : z.max_ent;
     a.part = reinterpret_cast<float2*>(c->dpart.p); a.bar = c->dbar.p;
     a.inv_smem = as ? 1 : 0;
     if (grid) {

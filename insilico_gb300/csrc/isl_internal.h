@@ -127,11 +127,12 @@ struct OlScal {
 struct CzInst {               // one instance (a single system: the only one)
     int row0, nrow;           // its rows (list order and natural order)
     int agg0, nagg, nd, ndp;  // its aggregates, coarse unknowns, padded to whole tiles
-    int rc0, pad;             // first coarse vector entry (two vectors of ndp)
+    int rc0;                  // first coarse vector entry (two vectors of ndp)
+    int rows, aggs, ent;      // one-launch solve: the largest share of a CTA, in rows, aggregates and stored entries
     long long a0, p0;         // first entry of its coarse matrices, of its inversion scratch
 };
 struct CzPlan {
-    int ninst = 0, max_ndp = 0;
+    int ninst = 0;
     std::vector<CzInst> hinst;
     DBuf<CzInst> inst;
     DBuf<int32_t> agg_inst;   // instance of every aggregate
@@ -139,7 +140,7 @@ struct CzPlan {
     int norder = 0;
     std::vector<int32_t> big; // batch: instances too large for a cluster, one cooperative grid each
     DBuf<int32_t> cta_big;    // ... and the aggregates of its CTAs
-    int big_ncta = 0, big_rows = 0, big_aggs = 0, big_ent = 0, big_ndp = 0;
+    int big_ncta = 0;
     DBuf<OlScal> res;         // batch: result per instance
     bool ok = false;
     int64_t serial = -1, num_serial = -1, nrow = 0;
@@ -168,7 +169,8 @@ struct CzPlan {
     // one-cluster solve: (block) CSR in list order, aggregates of every CTA
     bool csr_built = false;
     int64_t csr_serial = -1, nent = 0;
-    int ncta = 0, max_rows = 0, max_aggs = 0, max_ent = 0;
+    int ncta = 0;
+    size_t smem[2][2][2] = {}; // shared memory of the largest instance: [cluster, grid] [matrix on chip] [rows of the inverse too]
     DBuf<int32_t> rp, ci, cta;
     DBuf<float> cv;
     std::vector<int32_t> hcta;
