@@ -364,7 +364,7 @@ enum { ISL_OPT_BLOCK_SOLVER = 0, ISL_OPT_BLOCKED = 1, ISL_OPT_NBLOCKS = 2, ISL_O
        ISL_OPT_BARRIER_TEST = 5, ISL_OPT_SPMV32_KIND = 6, ISL_OPT_SCALAR_SLOTS = 7, ISL_OPT_HOST_SETUP = 8,
        ISL_OPT_BICGSTAB_KIND = 9, ISL_OPT_BATCHED_SOLVE = 10, ISL_OPT_DIRECT_BLOCKS = 11, ISL_OPT_TUNE_RUNS = 12,
        ISL_OPT_ELEM_VARIANT = 13, ISL_OPT_FOLD_DIRECTION = 14, ISL_OPT_BLOCK_UPDATE = 15,
-       ISL_OPT_SHORT_COLUMNS = 16, ISL_OPT_RELIABLE_DROP = 17, ISL_OPT_SHARED_GEOMETRY = 18, ISL_OPT_TWO_LEVEL = 19 };
+       ISL_OPT_SHORT_COLUMNS = 16, ISL_OPT_RELIABLE_DROP = 17, ISL_OPT_SHARED_GEOMETRY = 18, ISL_OPT_TWO_LEVEL = 19, ISL_OPT_ALLOC_TEST = 20 };
 /* ISL_OPT_TWO_LEVEL (default 1): the mixed CG of one system (at least 64 node
  * blocks, or 1,280 with ISL_OPT_PERSISTENT 0; at least 2,048 equations where it
  * is not node-blocked) is preconditioned by (block) Jacobi plus a coarse space
@@ -372,7 +372,9 @@ enum { ISL_OPT_BLOCK_SOLVER = 0, ISL_OPT_BLOCKED = 1, ISL_OPT_NBLOCKS = 2, ISL_O
  * Galerkin matrix), which takes far fewer iterations to the same tolerance; 0
  * keeps (block) Jacobi alone.  A system without usable support points, or one
  * that the two-level iteration does not bring to the tolerance, is solved with
- * (block) Jacobi.  Every instance of a batch is solved so, in launches that
+ * (block) Jacobi; so is one for whose coarse space the device has no memory left
+ * (ISL_OPT_ALLOC_TEST, test hook, write-only: the n-th allocation for it from
+ * now on fails, 0 none).  Every instance of a batch is solved so, in launches that
  * hold as many instances at once as the GPU takes (unless
  * ISL_OPT_SPMV32_KIND sets a product of the one-level batched solve, or
  * ISL_OPT_PERSISTENT is not 1).  A scalar system is multiplied in the order of its

@@ -801,7 +801,7 @@ int solve_batched(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t*
     std::vector<OlScal> res((size_t)ni);
     int left = ni;
     DBuf<int32_t> dsolved;
-    if (mixed && c->use_coarse && c->use_persist == 1 && !c->spmv32_forced) {
+    auto two_level = [&]() -> int {
         const int ncta = cluster_ctas(c);
         if (ncta > 0) {
             rc = coarse_plan(c, 1, c->neq, ncta);
@@ -810,9 +810,8 @@ int solve_batched(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t*
         CzPlan& z = c->cz;
         const bool grids = ni > 1 && !c->side_by_side && !z.big.empty();
         if (ncta > 0 && z.ok && (ni > 1 ? z.norder > 0 || grids : coarse_cluster_fits(c, false) > 0)) {
-            ISL_CHECK_CUDA(c, z.res.alloc(ni));
-            ISL_CHECK_CUDA(c, cudaMemsetAsync(z.res.p, 0, (size_t)ni * sizeof(OlScal), st));
-            rc = coarse_numeric(c, true, V + 3 * n);
+            rc = coarse_results(c);
+            if (rc == ISL_OK) rc = coarse_numeric(c, true, V + 3 * n);
             if (rc != ISL_OK) return rc;
             int64_t rows = 0;
             for (int64_t k = 0; k < c->ninst; ++k) rows = std::max(rows, c->inst_eq_off[k + 1] - c->inst_eq_off[k]);
@@ -849,6 +848,16 @@ int solve_batched(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t*
                 ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
             }
         }
+        return ISL_OK;
+    };
+    if (mixed && c->use_coarse && c->use_persist == 1 && !c->spmv32_forced) {
+        rc = two_level();
+        if (rc == ISL_ERR_NOMEM) {  // no room for the coarse spaces: one-level
+            coarse_drop(c);
+            left = ni;
+            rc = ISL_OK;
+        }
+        if (rc != ISL_OK) return rc;
     }
     if (left == 0) {
         int64_t itmax = 0;

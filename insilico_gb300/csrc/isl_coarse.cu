@@ -1739,6 +1739,21 @@ int target_aggs(int64_t n) {
     return (int)std::clamp<int64_t>(n / 60, 16, std::clamp<int64_t>(n / 900, 150, 300));
 }
 
+// Allocations of the plan.  One that fails leaves the system to the one-level
+// solve (coarse_drop); the test hook makes the n-th one fail.
+template <typename T>
+cudaError_t cz_alloc(isl_ctx* c, DBuf<T>& b, size_t count) {
+    if (c->alloc_test > 0 && --c->alloc_test == 0) return cudaErrorMemoryAllocation;
+    return b.alloc(count);
+}
+#define CZ_ALLOC(c, b, count) ISL_CHECK_CUDA(c, cz_alloc(c, b, count))
+// declared after the scratch buffers of a function, so that these are given
+// back after the kernels that use them, on every way out
+struct StreamDone {
+    cudaStream_t st;
+    ~StreamDone() { cudaStreamSynchronize(st); }
+};
+
 unsigned grid_for(const isl_ctx* c, int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 8LL * c->sm_count)); }
 
 // Boxes per direction of one instance: near-cubic boxes of edge h, which gives
@@ -1792,21 +1807,22 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     DBuf<unsigned short> dcut;
     DBuf<Box3> dbox;
     DBuf<char> tmp;
+    StreamDone done{st};
     std::vector<unsigned> hmm((size_t)6 * ni, 0u);
     for (int k = 0; k < ni; ++k)
         for (int d = 0; d < 3; ++d) hmm[6 * k + d] = 0xffffffffu;
-    ISL_CHECK_CUDA(c, P.alloc((size_t)c->ndofobj * D));
-    ISL_CHECK_CUDA(c, xr.alloc(n));
-    ISL_CHECK_CUDA(c, mm.alloc(hmm.size()));
-    ISL_CHECK_CUDA(c, hist.alloc((size_t)3 * NBIN * ni));
-    ISL_CHECK_CUDA(c, z.inst.alloc(ni));
+    CZ_ALLOC(c, P, (size_t)c->ndofobj * D);
+    CZ_ALLOC(c, xr, n);
+    CZ_ALLOC(c, mm, hmm.size());
+    CZ_ALLOC(c, hist, (size_t)3 * NBIN * ni);
+    CZ_ALLOC(c, z.inst, ni);
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(mm.p, hmm.data(), hmm.size() * 4, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.inst.p, z.hinst.data(), (size_t)ni * sizeof(CzInst), cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemsetAsync(hist.p, 0, (size_t)3 * NBIN * ni * 4, st));
     k_cz_points<<<(unsigned)((c->nelem + 255) / 256), 256, 0, st>>>(c->shape, c->ngeom, c->nfun, c->nelem, c->dconn.p,
                                                                      c->dedof.p, c->dX.p, D, P.p);
     if (NC == 3 && c->bpad) {
-        ISL_CHECK_CUDA(c, eqrow.alloc((size_t)c->neq));
+        CZ_ALLOC(c, eqrow, (size_t)c->neq);
         k_cz_eqrow<<<(3 * n + 255) / 256, 256, 0, st>>>(3 * n, c->dbaeq.p, eqrow.p);
         c->launches += 1;
     }
@@ -1833,7 +1849,7 @@ int build_plan(isl_ctx* c, CzPlan& z) {
         nbox += (int64_t)b.m[0] * b.m[1] * b.m[2] * comps;
     }
     if (nbox * NW >= (int64_t)1 << (31 - LEN_BITS) || ni > 65535) return ISL_OK;  // sort keys, launch grids
-    ISL_CHECK_CUDA(c, dbox.alloc(ni));
+    CZ_ALLOC(c, dbox, ni);
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(dbox.p, box.data(), (size_t)ni * sizeof(Box3), cudaMemcpyHostToDevice, st));
     k_cz_hist<<<ni > 1 ? g : std::min(g, (unsigned)c->sm_count), 256, 0, st>>>(n, ni, z.inst.p, dbox.p, xr.p, hist.p);
     std::vector<int32_t> hh((size_t)3 * NBIN * ni);
@@ -1851,14 +1867,14 @@ int build_plan(isl_ctx* c, CzPlan& z) {
                 run += hh[i];
             }
         }
-    ISL_CHECK_CUDA(c, dcut.alloc(cut.size()));
-    ISL_CHECK_CUDA(c, key.alloc(n));
-    ISL_CHECK_CUDA(c, key2.alloc(n));
-    ISL_CHECK_CUDA(c, row.alloc(n));
-    ISL_CHECK_CUDA(c, z.perm.alloc(n));
-    ISL_CHECK_CUDA(c, z.pos.alloc(n));
-    ISL_CHECK_CUDA(c, cnt.alloc((size_t)nbox * NW));
-    ISL_CHECK_CUDA(c, map.alloc(nbox));
+    CZ_ALLOC(c, dcut, cut.size());
+    CZ_ALLOC(c, key, n);
+    CZ_ALLOC(c, key2, n);
+    CZ_ALLOC(c, row, n);
+    CZ_ALLOC(c, z.perm, n);
+    CZ_ALLOC(c, z.pos, n);
+    CZ_ALLOC(c, cnt, (size_t)nbox * NW);
+    CZ_ALLOC(c, map, nbox);
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(dcut.p, cut.data(), cut.size() * 2, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemsetAsync(cnt.p, 0, (size_t)nbox * NW * 4, st));
     k_cz_key<NC, NW><<<g, 256, 0, st>>>(n, ni, z.inst.p, dbox.p, dcut.p, c->ncomp, xr.p, key.p, cnt.p);
@@ -1896,10 +1912,10 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     z.nd = z.hinst[0].nd;
     z.ndp = z.hinst[0].ndp;
     if (na == 0) return ISL_OK;
-    ISL_CHECK_CUDA(c, z.sofs.alloc(so.size()));
-    ISL_CHECK_CUDA(c, z.agg_inst.alloc(ai.size()));
-    ISL_CHECK_CUDA(c, z.lnode.alloc(n));
-    ISL_CHECK_CUDA(c, z.yrow.alloc(n));
+    CZ_ALLOC(c, z.sofs, so.size());
+    CZ_ALLOC(c, z.agg_inst, ai.size());
+    CZ_ALLOC(c, z.lnode, n);
+    CZ_ALLOC(c, z.yrow, n);
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.inst.p, z.hinst.data(), (size_t)ni * sizeof(CzInst), cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.sofs.p, so.data(), so.size() * 4, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.agg_inst.p, ai.data(), ai.size() * 4, cudaMemcpyHostToDevice, st));
@@ -1910,21 +1926,20 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     bits += LEN_BITS;
     size_t tb = 0;
     ISL_CHECK_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key2.p, row.p, z.perm.p, n, 0, bits, st));
-    ISL_CHECK_CUDA(c, tmp.alloc(std::max<size_t>(tb, 1)));
+    CZ_ALLOC(c, tmp, std::max<size_t>(tb, 1));
     ISL_CHECK_CUDA(c, cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key2.p, row.p, z.perm.p, n, 0, bits, st));
     k_cz_nodes<NC, NW><<<na, NW * 32, 0, st>>>(z.sofs.p, z.perm.p, key2.p, xr.p, z.lnode.p, z.yrow.p, z.pos.p);
     ISL_CHECK_CUDA(c, cudaGetLastError());
-    ISL_CHECK_CUDA(c, z.dsub.alloc((size_t)na * NW * M * M));
-    ISL_CHECK_CUDA(c, z.dagg.alloc((size_t)na * M * M));
-    ISL_CHECK_CUDA(c, z.scale.alloc((size_t)na * M));
-    ISL_CHECK_CUDA(c, z.rc.alloc(rc0));
-    ISL_CHECK_CUDA(c, z.acc.alloc((size_t)a0));
-    ISL_CHECK_CUDA(c, z.a.alloc((size_t)a0));
-    ISL_CHECK_CUDA(c, z.ainv.alloc((size_t)a0));
-    ISL_CHECK_CUDA(c, z.panel.alloc((size_t)p0));
-    ISL_CHECK_CUDA(c, z.amax.alloc(ni));
+    CZ_ALLOC(c, z.dsub, (size_t)na * NW * M * M);
+    CZ_ALLOC(c, z.dagg, (size_t)na * M * M);
+    CZ_ALLOC(c, z.scale, (size_t)na * M);
+    CZ_ALLOC(c, z.rc, rc0);
+    CZ_ALLOC(c, z.acc, (size_t)a0);
+    CZ_ALLOC(c, z.a, (size_t)a0);
+    CZ_ALLOC(c, z.ainv, (size_t)a0);
+    CZ_ALLOC(c, z.panel, (size_t)p0);
+    CZ_ALLOC(c, z.amax, ni);
     ISL_CHECK_CUDA(c, cudaMemsetAsync(z.rc.p, 0, (size_t)rc0 * 4, st));  // the padding stays zero
-    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));  // the scratch buffers above go out of scope
     c->launches += 10;
     z.hsofs = std::move(so);
     z.ok = true;
@@ -2028,8 +2043,8 @@ int build_sell(isl_ctx* c, CzPlan& z) {
     if (z.sell_built) return ISL_OK;
     cudaStream_t st = c->stream;
     const int n = (int)z.nrow, ns = (n + 31) / 32;
-    ISL_CHECK_CUDA(c, z.swid.alloc(ns));
-    ISL_CHECK_CUDA(c, z.soff.alloc(ns + 1));
+    CZ_ALLOC(c, z.swid, ns);
+    CZ_ALLOC(c, z.soff, ns + 1);
     k_pz_width<<<(ns + 127) / 128, 128, 0, st>>>(n, ns, z.perm.p, c->drowptr.p, z.swid.p);
     std::vector<int32_t> wid(ns), off(ns + 1);
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(wid.data(), z.swid.p, (size_t)ns * 4, cudaMemcpyDeviceToHost, st));
@@ -2042,9 +2057,9 @@ int build_sell(isl_ctx* c, CzPlan& z) {
     }
     off[ns] = (int32_t)tot;
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.soff.p, off.data(), (size_t)(ns + 1) * 4, cudaMemcpyHostToDevice, st));
-    ISL_CHECK_CUDA(c, z.col.alloc(tot));
-    ISL_CHECK_CUDA(c, z.col16.alloc(tot));
-    ISL_CHECK_CUDA(c, z.val.alloc(tot));
+    CZ_ALLOC(c, z.col, tot);
+    CZ_ALLOC(c, z.col16, tot);
+    CZ_ALLOC(c, z.val, tot);
     ISL_CHECK_CUDA(c, cudaMemsetAsync(z.val.p, 0, (size_t)tot * 4, st));
     ISL_CHECK_CUDA(c, cudaMemsetAsync(c->dflags.p + 1, 0, sizeof(int), st));
     k_pz_cols<<<(ns * 32 + 255) / 256, 256, 0, st>>>(n, ns, z.perm.p, z.pos.p, c->drowptr.p, c->dcolind.p, z.soff.p, z.swid.p,
@@ -2069,14 +2084,15 @@ int build_csr(isl_ctx* c, CzPlan& z) {
     z.nent = z.nc == 3 ? c->nblk : c->nnz;
     DBuf<int32_t> len;
     DBuf<char> tmp;
-    ISL_CHECK_CUDA(c, len.alloc(n + 1));
-    ISL_CHECK_CUDA(c, z.rp.alloc(n + 1));
-    ISL_CHECK_CUDA(c, z.ci.alloc(z.nent));
-    ISL_CHECK_CUDA(c, z.cv.alloc((size_t)z.nc * z.nc * z.nent));
+    StreamDone done{st};
+    CZ_ALLOC(c, len, n + 1);
+    CZ_ALLOC(c, z.rp, n + 1);
+    CZ_ALLOC(c, z.ci, z.nent);
+    CZ_ALLOC(c, z.cv, (size_t)z.nc * z.nc * z.nent);
     k_pz_len<<<n / 256 + 1, 256, 0, st>>>(n, z.perm.p, ptr, len.p);
     size_t tb = 0;
     ISL_CHECK_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, tb, len.p, z.rp.p, n + 1, st));
-    ISL_CHECK_CUDA(c, tmp.alloc(std::max<size_t>(tb, 1)));
+    CZ_ALLOC(c, tmp, std::max<size_t>(tb, 1));
     ISL_CHECK_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp.p, tb, len.p, z.rp.p, n + 1, st));
     k_pz_csr_cols<<<(n + 7) / 8, 256, 0, st>>>(n, z.perm.p, z.pos.p, ptr, z.nc == 3 ? c->dbcol.p : c->dcolind.p, z.rp.p, z.ci.p);
     std::vector<int32_t> rp(n + 1);
@@ -2133,17 +2149,17 @@ int build_csr(isl_ctx* c, CzPlan& z) {
     }
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.inst.p, z.hinst.data(), (size_t)z.ninst * sizeof(CzInst), cudaMemcpyHostToDevice, st));
     if (!z.big.empty()) {
-        ISL_CHECK_CUDA(c, z.cta_big.alloc(big_cta.size()));
+        CZ_ALLOC(c, z.cta_big, big_cta.size());
         ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.cta_big.p, big_cta.data(), big_cta.size() * 4, cudaMemcpyHostToDevice, st));
         ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
     }
     z.norder = (int)order.size();
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return z.hinst[a].nrow > z.hinst[b].nrow; });
     if (z.ninst > 1 && z.norder) {
-        ISL_CHECK_CUDA(c, z.order.alloc(order.size()));
+        CZ_ALLOC(c, z.order, order.size());
         ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.order.p, order.data(), order.size() * 4, cudaMemcpyHostToDevice, st));
     }
-    ISL_CHECK_CUDA(c, z.cta.alloc(z.hcta.size()));
+    CZ_ALLOC(c, z.cta, z.hcta.size());
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.cta.p, z.hcta.data(), z.hcta.size() * 4, cudaMemcpyHostToDevice, st));
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
     c->launches += 3;
@@ -2233,6 +2249,26 @@ int coarse_plan(isl_ctx* c, int nc, int64_t nrow, int ncta) {
     return nc == 1 ? build_sell(c, z) : ISL_OK;
 }
 
+void coarse_drop(isl_ctx* c) {
+    cudaStreamSynchronize(c->stream);
+    cudaGetLastError();
+    if (c->cz_exec) cudaGraphExecDestroy(c->cz_exec);
+    c->cz_exec = nullptr;
+    c->cz_key.clear();
+    CzPlan& z = c->cz;
+    z.ok = z.sell_built = z.csr_built = false;
+    z.bnd_serial = -1;
+    for (auto* b : {&z.agg_inst, &z.order, &z.cta_big, &z.sofs, &z.perm, &z.pos, &z.soff, &z.swid, &z.col, &z.bnd, &z.rp, &z.ci, &z.cta}) b->release();
+    for (auto* b : {&z.dsub, &z.dagg, &z.scale, &z.rc, &z.a, &z.ainv, &z.panel, &z.binv, &z.val, &z.cv}) b->release();
+    z.lnode.release(); z.yrow.release(); z.inst.release(); z.res.release(); z.amax.release(); z.acc.release(); z.col16.release();
+}
+
+int coarse_results(isl_ctx* c) {
+    CZ_ALLOC(c, c->cz.res, c->ninst);
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(c->cz.res.p, 0, (size_t)c->ninst * sizeof(OlScal), c->stream));
+    return ISL_OK;
+}
+
 int coarse_numeric(isl_ctx* c, bool csr, float* dinv) {
     CzPlan& z = c->cz;
     cudaStream_t st = c->stream;
@@ -2256,7 +2292,7 @@ int coarse_numeric(isl_ctx* c, bool csr, float* dinv) {
         if (csr) A = {nullptr, nullptr, z.rp.p, z.ci.p, z.cv.p};
         else A = {z.soff.p, z.swid.p, nullptr, z.col.p, z.val.p};
     } else if (!csr && z.binv_serial != c->asm_serial) {
-        ISL_CHECK_CUDA(c, z.binv.alloc((size_t)9 * n));
+        CZ_ALLOC(c, z.binv, (size_t)9 * n);
         k_pz_binv<<<grid_for(c, n), 256, 0, st>>>(n, z.perm.p, dinv, z.binv.p);
         c->launches += 1;
         z.binv_serial = c->asm_serial;
@@ -2372,7 +2408,7 @@ int coarse_spmv_plan(isl_ctx* c) {
     CzPlan& z = c->cz;
     const int g = (int)std::min<int64_t>(z.nslice, (int64_t)SPMV_PER_SM * c->sm_count);
     if (z.bnd_serial == z.serial && z.spmv_ncta == g) return ISL_OK;
-    ISL_CHECK_CUDA(c, z.bnd.alloc((size_t)g + 1));
+    CZ_ALLOC(c, z.bnd, (size_t)g + 1);
     k_cz_bnd<<<g / 256 + 1, 256, 0, c->stream>>>(g, z.nslice, z.soff.p, z.bnd.p);
     ISL_CHECK_CUDA(c, cudaGetLastError());
     c->launches += 1;

@@ -54,6 +54,11 @@ int coarse_plan(isl_ctx* c, int nc, int64_t nrow, int ncta);
 // for the current assembly: values of the aggregate-ordered copy, inverse
 // diagonal of scalar rows (in that order), Galerkin blocks, dense inverse
 int coarse_numeric(isl_ctx* c, bool csr, float* dinv);
+// gives the plan's memory back and leaves this pattern to the one-level solve:
+// after one of the calls here returned ISL_ERR_NOMEM
+void coarse_drop(isl_ctx* c);
+// a batch's result records, cleared
+int coarse_results(isl_ctx* c);
 void coarse_args(const isl_ctx* c, CzIter& a);
 // update (or start, or restart) and coarse correction: two launches
 void launch_coarse(const isl_ctx* c, cudaStream_t st, const CzIter& a, int mode);

@@ -1495,6 +1495,7 @@ int isl_set_option(isl_ctx* c, int key, int64_t value) {
         return ISL_OK;
     }
     if (key == ISL_OPT_BARRIER_TEST) { c->barrier_test = value == 2 ? 2 : value != 0; return ISL_OK; }
+    if (key == ISL_OPT_ALLOC_TEST) { c->alloc_test = value; return ISL_OK; }
     if (key == ISL_OPT_PERSISTENT) {
         if (value < 0 || value > 2) ISL_FAIL(c, ISL_ERR_ARG, "ISL_OPT_PERSISTENT takes 0, 1 or 2");
         c->use_persist = (int)value;

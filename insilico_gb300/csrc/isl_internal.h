@@ -367,6 +367,7 @@ struct isl_ctx {
     isl::DBuf<isl::OlScal> ol_scal;
     isl::CzPlan cz;              // two-level preconditioner of the mixed solve
     bool use_coarse = true;      // ISL_OPT_TWO_LEVEL
+    int64_t alloc_test = 0;      // test hook: the allocation of the two-level plan that fails, counted down
     bool side_by_side = false;   // shares the GPU with other contexts: no launch over every SM
     cudaGraphExec_t cz_exec = nullptr;   // captured iterations of the two-level solve
     std::vector<uint64_t> cz_key;        // what the capture depends on

@@ -3132,6 +3132,10 @@ int solve_device(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t* 
             // a healthy two-level solve takes far fewer iterations than this
             const int64_t limit = std::min(max_iter, std::max<int64_t>(1000, (int64_t)c->neq / 4));
             rc = solve_two_level(c, b3 ? 3 : 1, tol, limit, &it, &rel, &ran);
+            if (rc == ISL_ERR_NOMEM) {  // no room for the coarse space: one-level
+                coarse_drop(c);
+                rc = ISL_OK;
+            }
         }
         if (rc == ISL_OK && !ran)
             rc = b3 ? solve_mixed_b3(c, tol, max_iter, &it, &rel, &nc) : solve_mixed(c, tol, max_iter, &it, &rel, &nc);
