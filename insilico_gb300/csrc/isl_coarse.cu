@@ -45,7 +45,7 @@ namespace isl {
 
 namespace {
 
-constexpr int TB = 64;            // tile of the dense inversion
+constexpr int TB = COARSE_TILE;   // tile of the dense inversion
 constexpr int NBIN = 1024;        // bins per axis of the quantile cuts
 constexpr int ROW_BITS = 29;      // lnode.w: row, and the constrained components of a padded node block above
 constexpr float REG = 1e-5f;      // added to the unit diagonal of the scaled coarse matrices
@@ -1729,16 +1729,6 @@ __global__ void __launch_bounds__(NW * 32) k_cz_nodes(const int* __restrict__ so
     }
 }
 
-// Number of aggregates for n rows: about 60 rows each, at most 150 (300 for
-// the largest systems).  More aggregates take fewer iterations; the dense
-// inversion grows with their cube.  Measured with setup (node blocks): 2,366
-// rows 3.33 ms with 24 aggregates, 2.98 with 50, 3.10 with 100; 31,744 rows
-// 5.50 with 150, 5.70 with 300; 270,400 rows 21.9 with 150, 20.0 with 300,
-// 21.3 with 400.
-int target_aggs(int64_t n) {
-    return (int)std::clamp<int64_t>(n / 60, 16, std::clamp<int64_t>(n / 900, 150, 300));
-}
-
 // Allocations of the plan.  One that fails leaves the system to the one-level
 // solve (coarse_drop); the test hook makes the n-th one fail.
 template <typename T>
@@ -1844,7 +1834,7 @@ int build_plan(isl_ctx* c, CzPlan& z) {
             b.lo[d] = z.hinst[k].nrow ? lo : 0.f;
             b.inv[d] = L[d] > 0.0 ? (float)(NBIN / L[d]) : 0.f;
         }
-        choose_boxes(D, L, std::max(1, target_aggs(z.hinst[k].nrow) / comps), b.m);
+        choose_boxes(D, L, std::max(1, coarse_target(z.hinst[k].nrow) / comps), b.m);
         b.base = (int)nbox;
         nbox += (int64_t)b.m[0] * b.m[1] * b.m[2] * comps;
     }

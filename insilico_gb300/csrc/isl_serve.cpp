@@ -117,7 +117,8 @@ namespace {
 
 // Peak device memory of a request (pattern build included), from its size:
 // element pairs (n_elem * nloc^2) bound the contributions and the nonzeros.
-void estimate(Req& r) {
+// two_level: the mixed solve also keeps a coarse space (isl_coarse.cu).
+void estimate(Req& r, bool two_level) {
     const int nloc = nverts(r.shape) * r.ncomp;
     r.pairs = r.n_elem * (int64_t)nloc * nloc;
     const int64_t nup = (int64_t)nloc * (nloc + 1) / 2;
@@ -125,7 +126,16 @@ void estimate(Req& r) {
     const int64_t nnz = std::min<int64_t>(r.pairs, neq * (int64_t)nloc * 4);
     const int64_t persistent = nnz * (4 + 4 + 8 + 4 + 4 + 4) + r.pairs * 4 + r.n_elem * nup * 8 + neq * 160 +
                                r.n_nodes * 8 * (sdim(r.shape) + r.ncomp);
-    r.footprint = persistent + r.pairs * 24;
+    int64_t coarse = 0;
+    if (two_level) {
+        const bool node = r.ncomp == 3;
+        const int64_t rows = node ? r.n_nodes : neq;
+        const int64_t ndp = isl::coarse_unknowns(rows, node ? 6 : 1 + sdim(r.shape));
+        // the Galerkin matrix in fixed point, its scaled copy and the inverse;
+        // row lists and plan scratch; the two list-order copies of the matrix
+        coarse = 16 * ndp * ndp + rows * 160 + 2 * (nnz * 4 + (node ? nnz / 9 : nnz) * 6);
+    }
+    r.footprint = persistent + coarse + r.pairs * 24;
 }
 
 int64_t free_bytes(isl_server* s) {
@@ -542,7 +552,7 @@ int isl_serve_submit(isl_server* s, const isl_serve_request* q, int64_t* ticket)
         if (r->fnode[i] < 0 || r->fnode[i] >= q->n_nodes || r->fcomp[i] < 0 || r->fcomp[i] >= q->ncomp) return ISL_ERR_ARG;
     r->load_steps = q->load_steps; r->max_newton = q->max_newton;
     r->tol = q->tolerance; r->lin_tol = q->lin_tol;
-    estimate(*r);
+    estimate(*r, s->cfg.precision != ISL_PREC_FP64 && s->cfg.max_batch == 1);
     std::lock_guard<std::mutex> lk(s->mu);
     if (s->stop) return ISL_ERR_ARG;
     r->ticket = s->next_ticket++;
