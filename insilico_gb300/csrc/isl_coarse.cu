@@ -1529,7 +1529,7 @@ __global__ void k_cz_unscale(const CzInst* __restrict__ inst, const float* __res
 // sum of two numbers does not depend on their order, so elements that share
 // an edge write the same bits), the centre of a quadrilateral
 __global__ void k_cz_points(int shape, int ngeom, int nfun, int64_t nelem, const int32_t* __restrict__ conn,
-                            const int32_t* __restrict__ edof, const double* __restrict__ X, int D, float* __restrict__ P) {
+                            const int32_t* __restrict__ edof, const double* __restrict__ X, int D, double* __restrict__ P) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= nelem) return;
     const int tetE[6][2] = {{0, 1}, {1, 2}, {2, 0}, {3, 0}, {3, 1}, {3, 2}};
@@ -1546,7 +1546,7 @@ __global__ void k_cz_points(int shape, int ngeom, int nfun, int64_t nelem, const
                 const int a = shape == ISL_QUAD ? q : tetE[q][0], b = shape == ISL_QUAD ? (q + 1) % 4 : tetE[q][1];
                 v = 0.5 * (X[(int64_t)conn[(int64_t)a * nelem + e] * D + d] + X[(int64_t)conn[(int64_t)b * nelem + e] * D + d]);
             }
-            P[o * D + d] = (float)v;
+            P[o * D + d] = v;
         }
     }
 }
@@ -1556,18 +1556,26 @@ __global__ void k_cz_eqrow(int n3, const int* __restrict__ aeq, int* __restrict_
     if (t < n3 && aeq[t] >= 0) eqrow[aeq[t]] = t / 3;
 }
 
-// point (w: the component, NC = 1, or the mask of constrained components) of every row
+// point (w: the component, NC = 1, or the mask of constrained components) of every
+// row, relative to a vertex of its instance: rounded to FP32 as they stand, the
+// points of a mesh far from the origin would coincide
 template <int NC>
 __global__ void k_cz_rowpts(int64_t ndo, int ncomp, const int32_t* __restrict__ eq, const int* __restrict__ eqrow, int D,
-                            const float* __restrict__ P, float4* __restrict__ xr) {
+                            const double* __restrict__ P, const CzInst* __restrict__ inst, int ninst,
+                            const int32_t* __restrict__ conn, const double* __restrict__ X, float4* __restrict__ xr) {
     const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (o >= ndo) return;
-    float4 v = make_float4(P[o * D], P[o * D + 1], D == 3 ? P[o * D + 2] : 0.f, 0.f);
+    auto point = [&](int row) {
+        const double* org = X + (size_t)D * conn[inst[ninst > 1 ? inst_of(inst, ninst, row) : 0].elem0];
+        return make_float4((float)(P[o * D] - org[0]), (float)(P[o * D + 1] - org[1]), D == 3 ? (float)(P[o * D + 2] - org[2]) : 0.f, 0.f);
+    };
     if (NC == 1) {
         for (int c = 0; c < ncomp; ++c) {
             const int e = eq[o * ncomp + c];
+            if (e < 0) continue;
+            float4 v = point(e);
             v.w = __int_as_float(c);
-            if (e >= 0) xr[e] = v;
+            xr[e] = v;
         }
     } else {
         int first = -1, mask = 0;
@@ -1577,8 +1585,10 @@ __global__ void k_cz_rowpts(int64_t ndo, int ncomp, const int32_t* __restrict__ 
             else if (first < 0) first = e;
         }
         if (first < 0) return;
+        const int row = eqrow ? eqrow[first] : first / 3;
+        float4 v = point(row);
         v.w = __int_as_float(mask);
-        xr[eqrow ? eqrow[first] : first / 3] = v;
+        xr[row] = v;
     }
 }
 
@@ -1789,8 +1799,9 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     for (int k = 0; k < ni; ++k) {
         z.hinst[k].row0 = ni > 1 ? (int)c->inst_eq_off[k] : 0;
         z.hinst[k].nrow = ni > 1 ? (int)(c->inst_eq_off[k + 1] - c->inst_eq_off[k]) : n;
+        z.hinst[k].elem0 = ni > 1 ? (int)c->inst_elem_off[k] : 0;
     }
-    DBuf<float> P;
+    DBuf<double> P;
     DBuf<float4> xr;
     DBuf<int32_t> eqrow, hist, key, key2, row, cnt, map;
     DBuf<unsigned> mm;
@@ -1816,7 +1827,8 @@ int build_plan(isl_ctx* c, CzPlan& z) {
         k_cz_eqrow<<<(3 * n + 255) / 256, 256, 0, st>>>(3 * n, c->dbaeq.p, eqrow.p);
         c->launches += 1;
     }
-    k_cz_rowpts<NC><<<(unsigned)((c->ndofobj + 255) / 256), 256, 0, st>>>(c->ndofobj, c->ncomp, c->deq.p, eqrow.p, D, P.p, xr.p);
+    k_cz_rowpts<NC><<<(unsigned)((c->ndofobj + 255) / 256), 256, 0, st>>>(c->ndofobj, c->ncomp, c->deq.p, eqrow.p, D, P.p, z.inst.p, ni,
+                                                                                    c->dconn.p, c->dX.p, xr.p);
     const unsigned g = grid_for(c, n);
     k_cz_bounds<<<g, 256, 0, st>>>(n, ni, z.inst.p, xr.p, mm.p);
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(hmm.data(), mm.p, hmm.size() * 4, cudaMemcpyDeviceToHost, st));

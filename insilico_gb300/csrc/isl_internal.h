@@ -129,6 +129,7 @@ struct CzInst {               // one instance (a single system: the only one)
     int row0, nrow;           // its rows (list order and natural order)
     int agg0, nagg, nd, ndp;  // its aggregates, coarse unknowns, padded to whole tiles
     int rc0;                  // first coarse vector entry (two vectors of ndp)
+    int elem0;                // its first element
     int rows, aggs, ent;      // one-launch solve: the largest share of a CTA, in rows, aggregates and stored entries
     long long a0, p0;         // first entry of its coarse matrices, of its inversion scratch
 };
