@@ -1,0 +1,42 @@
+"""High contrast between two halves of a mesh: the coarse inverse stays definite,
+so the two-level iteration itself reaches the tolerance.  (Where it breaks down
+the one-level solve runs, and the number of iterations is that solve's.)"""
+import numpy as np
+import pytest
+
+from insilico_gb300 import _abi as A
+from insilico_gb300 import workloads as W
+from insilico_gb300.system import System
+
+pytestmark = pytest.mark.gpu
+
+
+def _halves(p, contrast):
+    x = p.X[p.conn].mean(axis=1)[:, 0]
+    soft = np.where(x > 0.5, contrast, 1.0)
+    if p.kernel == "laplace":
+        p.kappa = soft
+    else:
+        p.lam, p.mu = W.lame(soft, 0.3)
+    return p
+
+
+def _iterations(config, n, contrast, persist):
+    S = W.setup_system(_halves(W.config(config, n=n), contrast))
+    S.set_option(A.OPT_PERSISTENT, persist)
+    S.assemble(A.PREC_MIXED)
+    two, rel, _ = S.solve(A.SOLVE_CG_FP32_IR, tol=1e-8)
+    S.set_option(A.OPT_TWO_LEVEL, 0)
+    one, rel1, _ = S.solve(A.SOLVE_CG_FP32_IR, tol=1e-8)
+    S.close()
+    assert rel <= 1e-8 and rel1 <= 1e-8
+    return two, one
+
+
+@pytest.mark.parametrize("persist", [1, 0])
+@pytest.mark.parametrize("config,n", [("c1", 64), ("c2", 16), ("c3", 12)], ids=["quad Q1", "hex", "tet P2"])
+def test_contrast_inside_the_aggregates(config, n, persist):
+    """1e6: aggregates across the interface give the coarse matrix a condition of
+    some 1e5, which the FP32 inversion has to survive"""
+    two, one = _iterations(config, n, 1e-6, persist)
+    assert two < one
