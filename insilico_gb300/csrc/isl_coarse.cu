@@ -50,7 +50,7 @@ constexpr int NBIN = 1024;        // bins per axis of the quantile cuts
 constexpr int ROW_BITS = 29;      // lnode.w: row, and the constrained components of a padded node block above
 constexpr float REG = 1e-5f;      // added to the unit diagonal of the scaled coarse matrices
 constexpr int CZ_KEEP = 2;        // rows of a thread that k_cz_update and k_cz_coarse hold in registers
-constexpr int FIX_BITS = 32;      // fixed point of the coarse entries: the largest diagonal entry is 2^32
+constexpr int FIX_BITS = 32;      // fixed point of the coarse entries: the bound of an entry is 2^32
 
 __device__ inline int lrow(float4 l) { return __float_as_int(l.w) & ((1 << ROW_BITS) - 1); }
 __device__ inline int lmask(float4 l) { return (int)((unsigned)__float_as_int(l.w) >> ROW_BITS); }
@@ -1042,37 +1042,47 @@ __device__ inline int inst_of(const CzInst* __restrict__ inst, int ninst, int ro
     return lo;
 }
 
-// largest diagonal entry of every instance (its bits order as integers)
-template <typename T>
-__global__ void k_cz_amax(int n, int ninst, const CzInst* __restrict__ inst, const int* __restrict__ diag, const T* __restrict__ val,
-                          int* __restrict__ out) {
-    // a warp takes 32 consecutive rows, mostly of one instance
-    const int lane = threadIdx.x & 31;
-    int cur = -1;
+// largest diagonal entry of every aggregate, and (top) of every instance (positive floats order as integers)
+template <int NC, int NW, typename T>
+__global__ void __launch_bounds__(NW * 32) k_cz_amax(const int* __restrict__ sofs, const int* __restrict__ perm,
+                                                     const int* __restrict__ aeq, const int* __restrict__ diag,
+                                                     const T* __restrict__ val, const int* __restrict__ agg_inst,
+                                                     float* __restrict__ out, float* __restrict__ top) {
+    __shared__ float sh[NW];
     float m = 0.f;
-    auto flush = [&](int k, float v) {
-        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0 && k >= 0) atomicMax(out + k, __float_as_int(v));
-    };
-    for (int base = (blockIdx.x * blockDim.x + threadIdx.x) - lane; base < n; base += gridDim.x * blockDim.x) {
-        const int i = base + lane;
-        float v = i < n ? fabsf((float)val[diag[i]]) : 0.f;
-        if (!(v < INFINITY)) v = 0.f;
-        const int first = ninst > 1 ? inst_of(inst, ninst, base) : 0, last = ninst > 1 ? inst_of(inst, ninst, min(base + 31, n - 1)) : 0;
-        if (first != cur) {
-            flush(cur, m);
-            m = 0.f;
-            cur = first;
+    for (int t = sofs[blockIdx.x * NW] + threadIdx.x; t < sofs[(blockIdx.x + 1) * NW]; t += NW * 32) {
+        const int row = perm[t];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int e = NC == 3 && aeq ? aeq[NC * row + c] : NC * row + c;
+            const float v = e >= 0 ? fabsf((float)val[diag[e]]) : 0.f;
+            if (v < INFINITY) m = fmaxf(m, v);
         }
-        if (first == last) m = fmaxf(m, v);
-        else if (i < n) atomicMax(out + inst_of(inst, ninst, i), __float_as_int(v));
     }
-    flush(cur, m);
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < NW; ++w) m = fmaxf(m, sh[w]);
+    out[blockIdx.x] = m;
+    atomicMax(reinterpret_cast<int*>(top + agg_inst[blockIdx.x]), __float_as_int(m));
 }
 
-__device__ inline float fix_scale(int amax_bits) {  // 2^(FIX_BITS - e), amax < 2^e
-    const int e = ((amax_bits >> 23) & 255) - 126;
-    return ldexpf(1.f, FIX_BITS - e);
+// Fixed point of the coarse entries between two aggregates, from their largest
+// diagonal entries: |a_ij| <= sqrt(a_ii a_jj) < 2^e, and 2^FIX_BITS stands for
+// 2^e.  (One scale for the whole matrix loses the couplings of a soft region to
+// rounding: with a contrast of 1e8 its coarse matrix was noise, and the solve
+// fell back to one-level after 160^2 Q1 iterations that now end after 52.)
+// 0: the couplings of an aggregate softer than 2^-28 of the stiffest (top) are
+// left out, which keeps the matrix definite.  With them the FP32 directions
+// hold amplitudes of both regions, and lose the stiff one's: 20^3 P2
+// tetrahedra at 1e-8 with one half softer by 1e8 160 iterations (402 one-level),
+// by 1e9 291 and by 1e10 1,057, without them 168 and 173.
+constexpr float SOFT = 1.f / (1 << 28);
+__device__ inline float fix_scale(float amax_i, float amax_j, float top) {
+    if (fminf(amax_i, amax_j) < SOFT * top) return 0.f;
+    const int e = ((__float_as_int(amax_i) >> 23) + (__float_as_int(amax_j) >> 23) - 2 * 126 + 1) >> 1;
+    return ldexpf(1.f, min(126, FIX_BITS - e));
 }
 
 // Galerkin blocks: CTA per aggregate, warp per sub-aggregate, lane per row.
@@ -1083,7 +1093,8 @@ __device__ inline float fix_scale(int amax_bits) {  // 2^(FIX_BITS - e), amax < 
 template <int NC, int M, int NW>
 __global__ void __launch_bounds__(NW * 32) k_cz_galerkin(CzMat A, const float4* __restrict__ lnode, const float4* __restrict__ yrow,
                                                          const int* __restrict__ sofs, const CzInst* __restrict__ inst,
-                                                         const int* __restrict__ agg_inst, const int* __restrict__ amax,
+                                                         const int* __restrict__ agg_inst, const float* __restrict__ amax,
+                                                         const float* __restrict__ top,
                                                          unsigned long long* __restrict__ acc, float* __restrict__ dsub,
                                                          float* __restrict__ dagg) {
     __shared__ float own[NW][M * M];
@@ -1091,7 +1102,6 @@ __global__ void __launch_bounds__(NW * 32) k_cz_galerkin(CzMat A, const float4* 
     const int I = blockIdx.x, sub = I * NW + w;
     const int ik = agg_inst[I], ndp = inst[ik].ndp, agg0 = inst[ik].agg0;
     acc += inst[ik].a0;
-    const float scale = fix_scale(amax[ik]);
     float a1[M * M], a2[M * M];
 #pragma unroll
     for (int k = 0; k < M * M; ++k) a1[k] = a2[k] = 0.f;
@@ -1120,6 +1130,7 @@ __global__ void __launch_bounds__(NW * 32) k_cz_galerkin(CzMat A, const float4* 
         int J = I;  // aggregate of the run in Tc (I: none)
         auto flush = [&]() {
             float o[M * M];
+            const float scale = fix_scale(amax[I], amax[J], top[ik]);
             outer(Tc, L, o, false);
             unsigned long long* dst = acc + (size_t)((I - agg0) * M) * ndp + (size_t)(J - agg0) * M;
 #pragma unroll
@@ -1262,7 +1273,8 @@ __global__ void k_cz_scale(int nagg, const float* __restrict__ dagg, float* __re
 // the scaled coarse matrix of every instance, padded with the identity to whole tiles
 template <int M>
 __global__ void k_cz_form(const CzInst* __restrict__ inst, const unsigned long long* __restrict__ acc, const float* __restrict__ dagg,
-                          const float* __restrict__ s, const int* __restrict__ amax, float* __restrict__ A) {
+                          const float* __restrict__ s, const float* __restrict__ amax, const float* __restrict__ top,
+                          float* __restrict__ A) {
     const CzInst in = inst[blockIdx.z];
     const int nd = in.nd, ndp = in.ndp;
     if ((int)blockIdx.x * 32 >= ndp || (int)blockIdx.y * 32 >= ndp) return;
@@ -1270,7 +1282,7 @@ __global__ void k_cz_form(const CzInst* __restrict__ inst, const unsigned long l
     A += in.a0;
     dagg += (size_t)in.agg0 * (M * M);
     s += in.agg0 * M;
-    const float inv = 1.f / fix_scale(amax[blockIdx.z]);
+    amax += in.agg0;
     const int j = blockIdx.x * 32 + (threadIdx.x & 31);
     for (int i = blockIdx.y * 32 + (threadIdx.x >> 5); i < (int)blockIdx.y * 32 + 32; i += 8) {
         float v = 0.f;
@@ -1278,7 +1290,8 @@ __global__ void k_cz_form(const CzInst* __restrict__ inst, const unsigned long l
         else if (i < nd && j < nd) {
             const int I = i / M, J = j / M;
             if (I == J) v = 0.5f * (dagg[(size_t)I * M * M + (i % M) * M + j % M] + dagg[(size_t)I * M * M + (j % M) * M + i % M]);
-            else v = (float)(long long)acc[I < J ? (size_t)i * ndp + j : (size_t)j * ndp + i] * inv;
+            else if (const float f = fix_scale(amax[I], amax[J], top[blockIdx.z]); f > 0.f)
+                v = (float)(long long)acc[I < J ? (size_t)i * ndp + j : (size_t)j * ndp + i] / f;
             v *= s[i] * s[j];
         }
         A[(size_t)i * ndp + j] = v;
@@ -1954,7 +1967,7 @@ int build_plan(isl_ctx* c, CzPlan& z) {
     CZ_ALLOC(c, z.a, (size_t)a0);
     CZ_ALLOC(c, z.ainv, (size_t)a0);
     CZ_ALLOC(c, z.panel, (size_t)p0);
-    CZ_ALLOC(c, z.amax, ni);
+    CZ_ALLOC(c, z.amax, na + ni);
     ISL_CHECK_CUDA(c, cudaMemsetAsync(z.rc.p, 0, (size_t)rc0 * 4, st));  // the padding stays zero
     c->launches += 10;
     z.hsofs = std::move(so);
@@ -2190,16 +2203,17 @@ int numeric(isl_ctx* c, CzPlan& z, const CzMat& A) {
     for (const CzInst& in : z.hinst) ndp = std::max(ndp, in.ndp);
     const int nt = ndp / TB, ni = z.ninst;
     ISL_CHECK_CUDA(c, cudaMemsetAsync(z.acc.p, 0, z.acc.n * 8, st));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.amax.p, 0, (size_t)ni * 4, st));
-    const unsigned g = grid_for(c, c->neq);
-    if (c->have64) k_cz_amax<double><<<g, 256, 0, st>>>((int)c->neq, ni, z.inst.p, c->ddiag.p, c->dval64.p, z.amax.p);
-    else k_cz_amax<float><<<g, 256, 0, st>>>((int)c->neq, ni, z.inst.p, c->ddiag.p, c->dval32.p, z.amax.p);
-    k_cz_galerkin<NC, M, NW><<<z.nagg, NW * 32, 0, st>>>(A, z.lnode.p, z.yrow.p, z.sofs.p, z.inst.p, z.agg_inst.p, z.amax.p,
+    const int* aeq = NC == 3 && c->bpad ? c->dbaeq.p : nullptr;
+    float* top = z.amax.p + z.nagg;
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(top, 0, (size_t)ni * 4, st));
+    if (c->have64) k_cz_amax<NC, NW><<<z.nagg, NW * 32, 0, st>>>(z.sofs.p, z.perm.p, aeq, c->ddiag.p, c->dval64.p, z.agg_inst.p, z.amax.p, top);
+    else k_cz_amax<NC, NW><<<z.nagg, NW * 32, 0, st>>>(z.sofs.p, z.perm.p, aeq, c->ddiag.p, c->dval32.p, z.agg_inst.p, z.amax.p, top);
+    k_cz_galerkin<NC, M, NW><<<z.nagg, NW * 32, 0, st>>>(A, z.lnode.p, z.yrow.p, z.sofs.p, z.inst.p, z.agg_inst.p, z.amax.p, top,
                                                          z.acc.p, z.dsub.p, z.dagg.p);
     k_cz_sub_inv<M><<<(z.nagg * NW + 63) / 64, 64, 0, st>>>(z.nagg * NW, z.dsub.p);
     k_cz_scale<M><<<(z.nagg + 127) / 128, 128, 0, st>>>(z.nagg, z.dagg.p, z.scale.p);
     const dim3 g32(ndp / 32, ndp / 32, ni);
-    k_cz_form<M><<<g32, 256, 0, st>>>(z.inst.p, z.acc.p, z.dagg.p, z.scale.p, z.amax.p, z.a.p);
+    k_cz_form<M><<<g32, 256, 0, st>>>(z.inst.p, z.acc.p, z.dagg.p, z.scale.p, z.amax.p, top, z.a.p);
     ISL_CHECK_CUDA(c, cudaFuncSetAttribute(k_gj_step, cudaFuncAttributeMaxDynamicSharedMemorySize, GJ_SMEM));
     k_gj_first<<<dim3(nt, ni), 256, 0, st>>>(z.inst.p, z.a.p, z.panel.p);
     for (int k = 0; k < nt; ++k) k_gj_step<<<dim3(nt * (nt + 1) / 2, ni), 256, GJ_SMEM, st>>>(z.inst.p, k, z.a.p, z.panel.p);

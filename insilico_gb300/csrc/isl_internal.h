@@ -150,7 +150,7 @@ struct CzPlan {
     int nagg = 0, nd = 0, ndp = 0;
     DBuf<float4> lnode, yrow;
     DBuf<int32_t> sofs;
-    DBuf<int> amax;
+    DBuf<float> amax;         // largest diagonal entry of every aggregate, then of every instance
     DBuf<unsigned long long> acc;
     DBuf<float> dsub, dagg, scale, rc, a, ainv, panel;
     DBuf<int32_t> perm, pos;  // list order: row of every entry, entry of every row

@@ -40,3 +40,34 @@ def test_contrast_inside_the_aggregates(config, n, persist):
     some 1e5, which the FP32 inversion has to survive"""
     two, one = _iterations(config, n, 1e-6, persist)
     assert two < one
+
+
+@pytest.mark.parametrize("persist", [1, 0])
+@pytest.mark.parametrize("config,n", [("c1", 160), ("c2", 16), ("c3", 12)], ids=["quad Q1", "hex", "tet P2"])
+@pytest.mark.parametrize("contrast", [1e-8, 1e-9])
+def test_couplings_of_the_soft_half(config, n, contrast, persist):
+    """a soft region's couplings, beside diagonal entries 1e8 and 1e9 times theirs"""
+    two, one = _iterations(config, n, contrast, persist)
+    assert two < one
+
+
+def test_couplings_of_the_soft_half_of_an_instance():
+    X, conn = W.unit_cube("quad", 160, 160)
+    kappa = W.config("c1", n=160).kappa
+    soft = np.where(X[conn].mean(axis=1)[:, 0] > 0.5, 1e-8, 1.0)
+    S = System()
+    S.upload_batch(A.QUAD, [(X, conn), (X, conn)])
+    S.create_field(1, 1)
+    S.constrain_boundary(lambda x: (np.ones((len(x), 1), dtype=bool), 0.0))
+    S.number_dofs()
+    S.register_pattern()
+    S.set_laplace(np.concatenate([soft, kappa]), 2)
+    S.set_body_force_nodal(np.tile(W.config("c1", n=160).body, (2, 1)))
+    S.assemble(A.PREC_MIXED)
+    S.solve(A.SOLVE_CG_FP32_IR, tol=1e-8)
+    two, rel = S.batch_stats()
+    S.set_option(A.OPT_TWO_LEVEL, 0)
+    S.solve(A.SOLVE_CG_FP32_IR, tol=1e-8)
+    one, _ = S.batch_stats()
+    S.close()
+    assert np.all(rel <= 1e-8) and np.all(two < one)
