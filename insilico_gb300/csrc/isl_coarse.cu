@@ -1073,12 +1073,13 @@ __global__ void __launch_bounds__(NW * 32) k_cz_amax(const int* __restrict__ sof
 // 2^e.  (One scale for the whole matrix loses the couplings of a soft region to
 // rounding: with a contrast of 1e8 its coarse matrix was noise, and the solve
 // fell back to one-level after 160^2 Q1 iterations that now end after 52.)
-// 0: the couplings of an aggregate softer than 2^-28 of the stiffest (top) are
+// 0: the couplings of an aggregate softer than 2^-30 of the stiffest (top) are
 // left out, which keeps the matrix definite.  With them the FP32 directions
 // hold amplitudes of both regions, and lose the stiff one's: 20^3 P2
-// tetrahedra at 1e-8 with one half softer by 1e8 160 iterations (402 one-level),
-// by 1e9 291 and by 1e10 1,057, without them 168 and 173.
-constexpr float SOFT = 1.f / (1 << 28);
+// tetrahedra with one half softer by 1e8 take 160 iterations (402 one-level), by
+// 1e9 291, by 1e10 1,057, without them 173 and 175; 160^2 Q1 takes 52 whatever the
+// contrast, without them 165.
+constexpr float SOFT = 1.f / (1 << 30);
 __device__ inline float fix_scale(float amax_i, float amax_j, float top) {
     if (fminf(amax_i, amax_j) < SOFT * top) return 0.f;
     const int e = ((__float_as_int(amax_i) >> 23) + (__float_as_int(amax_j) >> 23) - 2 * 126 + 1) >> 1;
