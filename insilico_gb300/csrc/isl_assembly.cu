@@ -433,8 +433,9 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
     R* sg = (R*)(sfq + (A.general ? 8 * 8 * 3 * EPB : 0));  // [8 q][8 node][3][EPB]
     R* sc = sg + 8 * 8 * 3 * EPB;                   // [8][EPB]
     R* sA = sc + 8 * EPB;                           // [8 q][81][EPB] (general StVenant)
-    R* sb = sc + 8 * EPB;                           // [8 q][8 node][3][EPB] H g (general NeoHooke), then [8 q][EPB]
-    R* sf2 = sb + 8 * 8 * 3 * EPB;                  // c (mu - lam ln J)
+    R* sb = sc + 8 * EPB;                           // [8 q][8 node][3][EPB] H g (general NeoHooke), then three of [8 q][EPB]:
+    R* sf2 = sb + 8 * 8 * 3 * EPB;                  // c (mu - lam ln J), c lam and c mu, each rounded once
+    R *scl = sf2 + 8 * EPB, *scm = scl + 8 * EPB;
     const bool neo = A.general && A.material == ISL_MAT_NEOHOOKE;
 
     const int el = threadIdx.x % EPB, role = threadIdx.x / EPB;
@@ -546,6 +547,8 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
                         P[i][J] = mu * F[i][J] - f2 * H[i][J];
                     }
                 sf2[q * EPB + el] = R(c * f2);
+                scl[q * EPB + el] = R(c * lam);
+                scm[q * EPB + el] = R(c * mu);
 #pragma unroll
                 for (int M = 0; M < 8; ++M)
 #pragma unroll
@@ -656,7 +659,7 @@ __global__ void __launch_bounds__(EPB * 8) k_hyper_hex8(const ElemArgs A, const 
                     for (int k = 0; k < 3; ++k) acc[d][i * 3 + k] += a_[i] * gN[k] + b_[k] * gN[i] + (i == k ? db : R(0));
             }
         } else if (neo) {
-            const R cl = c * R(lam), cm = c * R(mu), cf = sf2[q * EPB + el];
+            const R cl = scl[q * EPB + el], cm = scm[q * EPB + el], cf = sf2[q * EPB + el];
             R bM[3], a_[3], d_[3], e_[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -1374,7 +1377,7 @@ static int dispatch_hyper(isl_ctx* c, const ElemArgs& A) {
     auto smem_of = [&](int epb) {
         return (size_t)8 * 3 * epb * 8 * 2 + (A.general ? (size_t)8 * 8 * 3 * epb * 8 : 0) +
                (size_t)8 * 8 * 3 * epb * sizeof(R) + (size_t)8 * epb * sizeof(R) +
-               (!A.general ? 0 : A.material == ISL_MAT_NEOHOOKE ? (size_t)8 * 25 * epb * sizeof(R) : (size_t)8 * 81 * epb * sizeof(R));
+               (!A.general ? 0 : A.material == ISL_MAT_NEOHOOKE ? (size_t)8 * 27 * epb * sizeof(R) : (size_t)8 * 81 * epb * sizeof(R));
     };
     // (the limit is the process's: the same value whatever this call needs, as
     // other threads may be launching the kernel for another material)
