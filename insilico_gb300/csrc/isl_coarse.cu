@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
     float rc[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) rc[m] = 0.f;
-    float rr = 0.f, rz = 0.f;
+    typename std::conditional<MODE == CZ_UPDATE, float, double>::type rr = 0, rz = 0;  // (FP64 where it costs nothing)
     double bb = 0.0;
     // loads of a row, then (in row_step) its stores: the rows held in registers load together
     auto row_load = [&](Row<NC>& R) {
@@ -177,8 +177,8 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
             zv[c] = 0.f;
 #pragma unroll
             for (int k = 0; k < NC; ++k) zv[c] += bi[NC * c + k] * R.r[k];
-            rr += R.r[c] * R.r[c];
-            rz += R.r[c] * zv[c];
+            rr += (decltype(rr))R.r[c] * R.r[c];
+            rz += (decltype(rz))R.r[c] * zv[c];
         }
         restrict_add<NC, M>(rc, R.r, R.L);
     };
@@ -252,9 +252,9 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
         a.rc[(size_t)blockIdx.x * M + threadIdx.x] = s;
     }
     double trr, trz;
-    if (MODE == CZ_INIT) {
-        const double b1 = block_sum(bb, sh);
-        const double b2 = block_sum((double)rz, sh);
+    if constexpr (MODE != CZ_UPDATE) {
+        const double b1 = block_sum(MODE == CZ_INIT ? bb : rr, sh);
+        const double b2 = block_sum(rz, sh);
         if (threadIdx.x == 0) { a.part[2 * blockIdx.x] = b1; a.part[2 * blockIdx.x + 1] = b2; }
         if (!last_block(&S->ticket2)) return;
         reduce_parts2(a.part, gridDim.x, sh, trr, trz);
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_coarse(CzIter a) {
     S->ticket2 = 0;
     const double rzn = S->rzloc + tot;
     S->absNew = rzn;
-    if (MODE == CZ_UPDATE) S->beta = (float)rzn / (float)S->absOld;
+    if (MODE == CZ_UPDATE) S->beta = df_quotient(df_from_double(rzn), df_from_double(S->absOld));
     else if (MODE == CZ_INIT) { S->absOld = rzn; S->beta = 0.0; }
     else {
         S->beta = S->fresh ? 0.0 : rzn / S->absOld;
@@ -548,7 +548,7 @@ struct CzClu {
     CGScal* S;
     double tol, drop;
     int max_iter, exact64;
-    float2* part;            // grid form: the CTAs' sums, four slots
+    float4* part;            // grid form: the CTAs' sums, four slots
     unsigned* bar;
     int inv_smem;            // the CTA's rows of the inverse are held in shared memory
     unsigned bar_start;      // grid form: count at which the barrier starts
@@ -568,7 +568,7 @@ template <int NC, int M, int NW, int LPR, bool MS, bool GRID, int CLT>
 __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     cgrp::cluster_group cl = cgrp::this_cluster();
     extern __shared__ __align__(16) float smem[];
-    __shared__ float2 red[4][16];
+    __shared__ float4 red[4][16];
     __shared__ float bs[2][32];
     __shared__ double shd[32];
     __shared__ float sc_alpha, sc_beta;
@@ -642,8 +642,8 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
         else cl.sync();
     };
     // sums over all CTAs of u, and of v if TWO: valid in thread 0 of every CTA.
-    // FP32 inside a CTA (at most a few thousand rows), double-float across.
-    auto cl_sum = [&](auto two, float u, float v, double& ou, double& ov) {
+    // FP32 inside a warp, double-float from there.
+    auto cl_sum = [&](auto two, float u, float v, df& ou, df& ov) {
         constexpr bool TWO = decltype(two)::value;
         for (int o = 16; o > 0; o >>= 1) {
             u += __shfl_xor_sync(0xffffffffu, u, o);
@@ -652,42 +652,39 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
         if (lane == 0) { bs[0][w] = u; if (TWO) bs[1][w] = v; }
         __syncthreads();
         if (w == 0) {
-            u = lane < CLT / 32 ? bs[0][lane] : 0.f;
-            v = TWO && lane < CLT / 32 ? bs[1][lane] : 0.f;
-            for (int o = 16; o > 0; o >>= 1) {
-                u += __shfl_xor_sync(0xffffffffu, u, o);
-                if (TWO) v += __shfl_xor_sync(0xffffffffu, v, o);
-            }
+            ou = {lane < CLT / 32 ? bs[0][lane] : 0.f, 0.f};
+            ov = {TWO && lane < CLT / 32 ? bs[1][lane] : 0.f, 0.f};
+            warp_sum_df2<TWO, true, CLT / 64>(ou, ov);
+            const float4 t = make_float4(ou.hi, ou.lo, ov.hi, ov.lo);
             if constexpr (GRID) {
-                if (lane == 0) __stcg(a.part + slot * ncta + rank, make_float2(u, v));
+                if (lane == 0) __stcg(a.part + slot * ncta + rank, t);
             } else {
-                if (lane < ncta) *cl.map_shared_rank(&red[slot][rank], lane) = make_float2(u, v);
+                if (lane < ncta) *cl.map_shared_rank(&red[slot][rank], lane) = t;
             }
         }
         sync_all();
-        ou = ov = 0.0;
         if (w == 0) {
-            df du = {0.f, 0.f}, dv = {0.f, 0.f};
+            ou = ov = {0.f, 0.f};
             if constexpr (GRID) {
                 for (int base = 0; base < ncta; base += 160) {
-                    float2 r[5];
+                    float4 r[5];
 #pragma unroll
                     for (int k = 0; k < 5; ++k) {
                         const int i = base + 32 * k + lane;
-                        r[k] = i < ncta ? __ldcg(a.part + slot * ncta + i) : make_float2(0.f, 0.f);
+                        r[k] = i < ncta ? __ldcg(a.part + slot * ncta + i) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
 #pragma unroll
                     for (int k = 0; k < 5; ++k) {
-                        du = df_add_acc(du, df{r[k].x, 0.f});
-                        if (TWO) dv = df_add_acc(dv, df{r[k].y, 0.f});
+                        ou = df_add_acc(ou, df{r[k].x, r[k].y});
+                        if (TWO) ov = df_add_acc(ov, df{r[k].z, r[k].w});
                     }
                 }
             } else if (lane < ncta) {
-                du.hi = red[slot][lane].x;
-                dv.hi = red[slot][lane].y;
+                const float4 r = red[slot][lane];
+                ou = {r.x, r.y};
+                ov = {r.z, r.w};
             }
-            ou = df_value(warp_sum_df(du));
-            if (TWO) ov = df_value(warp_sum_df(dv));
+            warp_sum_df2<TWO, false, GRID ? 16 : 8>(ou, ov);  // (a cluster has 16 CTAs at most)
         }
         slot = (slot + 1) & 3;
     };
@@ -716,13 +713,15 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
         slot = (slot + 1) & 3;
     };
     // scalars, held by thread 0 of every CTA (the same values everywhere)
-    double rz = 0.0, rz_old = 0.0, rzl = 0.0, rr = 0.0, thr = 0.0, trig = 0.0, rr_true = 0.0, rr_last = 0.0, rr_best = 0.0, bn = 0.0;
+    df rz = {0.f, 0.f}, rz_old = {0.f, 0.f}, rzl = {0.f, 0.f};
+    double rr = 0.0, thr = 0.0, trig = 0.0, rr_true = 0.0, rr_last = 0.0, rr_best = 0.0, bn = 0.0;
     int iters = 0, stall = 0, careful = 0;
     enum { GO = 0, FIN1 = 1, FIN2 = 2, FIN3 = 3, STOP = 4 };
 
     // z = D0^-1 r + P_s D_s^-1 P_s^T r from rs, with rr and rz of this thread; rc written
     int par = 0;
-    auto local_part = [&](float alpha, bool update, float& frr, float& frz) {
+    // (a restart's r.z in FP64, in drz)
+    auto local_part = [&](float alpha, bool update, float& frr, float& frz, double& drz) {
         for (int u = w; u < na * NW; u += CLT / 32) {
             const int sub = ag0 * NW + u;
             const int i0 = a.sofs[sub] - t0, i1 = a.sofs[sub + 1] - t0;
@@ -746,8 +745,12 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
 #pragma unroll
                     for (int k = 0; k < NC; ++k) z += ds[(NC * c + k) * R + i] * rv[k];
                     zs[NC * i + c] = z;
-                    frr += rv[c] * rv[c];
-                    frz += rv[c] * z;
+                    if (update) {
+                        frr += rv[c] * rv[c];
+                        frz += rv[c] * z;
+                    } else {
+                        drz += (double)rv[c] * (double)z;
+                    }
                 }
                 restrict_add<NC, M>(rc, rv, ln[i]);
             }
@@ -765,7 +768,8 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
                 rz1 += rc[m] * z1[m];
             }
             if (lane == 0) {
-                frz += rz1;
+                if (update) frz += rz1;
+                else drz += (double)rz1;
 #pragma unroll
                 for (int m = 0; m < M; ++m) src[u * M + m] = rc[m];
             }
@@ -864,20 +868,26 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     constexpr int NG = CLT / LPR;
     float alpha = 0.f;
     while (ctl == GO) {
-        double s0, s1;
+        df s0 = {0.f, 0.f}, s1 = {0.f, 0.f};
         float frr = 0.f, frz = 0.f;
-        local_part(alpha, !restart, frr, frz);
-        cl_sum(std::true_type{}, frr, frz, s0, s1);
+        double drz = 0.0;
+        local_part(alpha, !restart, frr, frz, drz);
+        if (restart) {
+            cl_sum_d(drz, drz);
+            s1 = df_from_double(drz);
+        } else {
+            cl_sum(std::true_type{}, frr, frz, s0, s1);
+        }
         if (!alive) return;
         if (tid == 0) {
             int k = GO;
             rzl = s1;
             if (!restart) {
-                rr = s0;
+                rr = df_value(s0);
                 iters += 1;
                 rz_old = rz;
-                if (!(s0 == s0) || !(s1 == s1)) k = FIN3;
-                else if (s0 < thr || s0 < trig || (a.exact64 && s0 > 1e8 * rr_true) || iters >= a.max_iter) k = STOP;
+                if (!(rr == rr) || !(s1.hi == s1.hi)) k = FIN3;
+                else if (rr < thr || rr < trig || (a.exact64 && rr > 1e8 * rr_true) || iters >= a.max_iter) k = STOP;
             }
             sc_ctl = k;
         }
@@ -951,10 +961,10 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
         cl_sum(std::false_type{}, cp, 0.f, s0, s1);
         if (!alive) return;
         if (tid == 0) {
-            rz = rzl + s0;
-            const bool first = rz_old == 0.0;
-            sc_beta = (restart && (fresh || first)) ? 0.f : (float)rz / (float)rz_old;  // FP64 division: 0.3 us
-            sc_ctl = rz > 0.0 ? GO : FIN3;  // also when it is not a number
+            rz = df_add_acc(rzl, s0);
+            const bool first = rz_old.hi == 0.f;
+            sc_beta = (restart && (fresh || first)) ? 0.f : df_quotient(rz, rz_old);
+            sc_ctl = rz.hi > 0.f ? GO : FIN3;  // also when it is not a number
             fresh = false;
         }
         __syncthreads();
@@ -1007,7 +1017,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
         { float* sw = a.pa; a.pa = a.pb; a.pb = sw; }  // the buffer just written is read next time
         cl_sum(std::false_type{}, loc, 0.f, s0, s1);
         if (!alive) return;
-        if (tid == 0) sc_alpha = (float)rz / (float)s0;
+        if (tid == 0) sc_alpha = df_quotient(rz, s0);
         __syncthreads();
         alpha = sc_alpha;
     }
@@ -2404,7 +2414,7 @@ cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, float* work, const 
     a.rowptr = c->drowptr.p; a.colind = c->dcolind.p; a.val64 = c->dval64.p;
     a.S = c->dscal.p;
     a.tol = tol; a.drop = drop; a.max_iter = max_iter; a.exact64 = c->have64 ? 1 : 0;
-    a.part = reinterpret_cast<float2*>(c->dpart.p); a.bar = c->dbar.p;
+    a.part = reinterpret_cast<float4*>(c->dpart.p); a.bar = c->dbar.p;
     a.inv_smem = as ? 1 : 0;
     if (grid) {
         const cudaError_t e = grid_barrier_start(c, &a.bar_start);
