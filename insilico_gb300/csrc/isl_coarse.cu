@@ -1060,7 +1060,7 @@ __global__ void __launch_bounds__(NW * 32) k_cz_amax(const int* __restrict__ sof
                                                      float* __restrict__ out, float* __restrict__ top) {
     __shared__ float sh[NW];
     float m = 0.f;
-    for (int t = sofs[blockIdx.x * NW] + threadIdx.x; t < sofs[(blockIdx.x + 1) * NW]; t += NW * 32) {
+    for (int t = sofs[blockIdx.x * NW] + blockIdx.y * NW * 32 + threadIdx.x; t < sofs[(blockIdx.x + 1) * NW]; t += gridDim.y * NW * 32) {
         const int row = perm[t];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
@@ -1074,7 +1074,7 @@ __global__ void __launch_bounds__(NW * 32) k_cz_amax(const int* __restrict__ sof
     __syncthreads();
     if (threadIdx.x != 0) return;
     for (int w = 1; w < NW; ++w) m = fmaxf(m, sh[w]);
-    out[blockIdx.x] = m;
+    atomicMax(reinterpret_cast<int*>(out + blockIdx.x), __float_as_int(m));
     atomicMax(reinterpret_cast<int*>(top + agg_inst[blockIdx.x]), __float_as_int(m));
 }
 
@@ -2216,9 +2216,10 @@ int numeric(isl_ctx* c, CzPlan& z, const CzMat& A) {
     ISL_CHECK_CUDA(c, cudaMemsetAsync(z.acc.p, 0, z.acc.n * 8, st));
     const int* aeq = NC == 3 && c->bpad ? c->dbaeq.p : nullptr;
     float* top = z.amax.p + z.nagg;
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(top, 0, (size_t)ni * 4, st));
-    if (c->have64) k_cz_amax<NC, NW><<<z.nagg, NW * 32, 0, st>>>(z.sofs.p, z.perm.p, aeq, c->ddiag.p, c->dval64.p, z.agg_inst.p, z.amax.p, top);
-    else k_cz_amax<NC, NW><<<z.nagg, NW * 32, 0, st>>>(z.sofs.p, z.perm.p, aeq, c->ddiag.p, c->dval32.p, z.agg_inst.p, z.amax.p, top);
+    ISL_CHECK_CUDA(c, cudaMemsetAsync(z.amax.p, 0, z.amax.n * 4, st));
+    const dim3 gmax(z.nagg, 4);
+    if (c->have64) k_cz_amax<NC, NW><<<gmax, NW * 32, 0, st>>>(z.sofs.p, z.perm.p, aeq, c->ddiag.p, c->dval64.p, z.agg_inst.p, z.amax.p, top);
+    else k_cz_amax<NC, NW><<<gmax, NW * 32, 0, st>>>(z.sofs.p, z.perm.p, aeq, c->ddiag.p, c->dval32.p, z.agg_inst.p, z.amax.p, top);
     k_cz_galerkin<NC, M, NW><<<z.nagg, NW * 32, 0, st>>>(A, z.lnode.p, z.yrow.p, z.sofs.p, z.inst.p, z.agg_inst.p, z.amax.p, top,
                                                          z.acc.p, z.dsub.p, z.dagg.p);
     k_cz_sub_inv<M><<<(z.nagg * NW + 63) / 64, 64, 0, st>>>(z.nagg * NW, z.dsub.p);
