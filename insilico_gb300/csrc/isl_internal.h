@@ -367,6 +367,8 @@ struct isl_ctx {
     int spmv32_used = 0;         // FP32 product kind of the last mixed solve that chose one (ISL_OPT_SPMV32_KIND read back)
     isl::DBuf<int32_t> ol_row0;  // one-launch FP64 solves: row ranges of the CTAs, result
     isl::DBuf<isl::OlScal> ol_scal;
+    int64_t ol_half_serial = -1; // pattern that ol_half belongs to
+    int ol_half = 0;             // form of the FP64 CG beside other solves (solve_onelaunch)
     isl::CzPlan cz;              // two-level preconditioner of the mixed solve
     bool use_coarse = true;      // ISL_OPT_TWO_LEVEL
     int64_t alloc_test = 0;      // test hook: the allocation of the two-level plan that fails, counted down

@@ -17,6 +17,7 @@
 // per dependent add in the sums (1.4 us each), a division per scalar, and the
 // barriers (1-2 us each).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <vector>
 
@@ -31,6 +32,13 @@ namespace {
 // BiCGSTAB 13.7 with 512, 14.2 with 1024 (heat Q2 61 x 47)
 constexpr int OT_CG = 1024, OT_BI = 512;
 constexpr size_t OL_SMEM_MAX = 224 * 1024;
+// CG beside other such solves of this process: half the threads and at most half the
+// shared memory, so that the grids of two solves are resident at once.  The sums
+// and products of a row do not depend on the threads: the same bits.  Eight host
+// threads, Q2 90 x 90 (32k rows): @Q2@ solves a second, @Q2F@ with one grid at a time, 186
+// as graphs of kernels; Q1 100 x 100: @Q1@, @Q1F@ and 558.
+constexpr int OT_CG_HALF = 512;
+constexpr size_t OL_SMEM_HALF = 112 * 1024;
 
 struct OlArgs {
     int n;
@@ -47,7 +55,10 @@ struct OlArgs {
     int max_iter;
 };
 
-// shared-memory layout: nd vectors over the rows, nh over the columns
+// shared-memory layout: nd vectors over the rows, nh over the columns.  share: the
+// bitmap and its counts, needed while the columns are numbered only, take the room
+// of the row vectors (the layout of whole-SM launches keeps them apart: 0.7 %
+// faster, as the vectors' banks fall)
 struct OlMem {
     double *row, *hal, *vals;
     int *rps, *hc, *li;
@@ -55,22 +66,28 @@ struct OlMem {
     int* pre;
     unsigned short* cols;
 };
-__host__ __device__ inline size_t ol_bytes(int n, int R, int E, int H, int nd, int nh, bool vals) {
-    const size_t W = (n + 31) / 32;
-    return 8 * ((size_t)nd * R + (size_t)nh * H + (vals ? (size_t)E : 0)) + 4 * ((size_t)R + 1 + H + R + 2 * W) + 2 * (size_t)E + 16;
+__host__ __device__ inline size_t ol_row_words(int n, int R, int nd, bool share) {
+    const size_t W = (n + 31) / 32, v = (size_t)nd * R;  // a bitmap word and a count: 8 bytes
+    return share && W > v ? W : v;
 }
+__host__ __device__ inline size_t ol_bytes(int n, int R, int E, int H, int nd, int nh, bool vals, bool share) {
+    const size_t W = (n + 31) / 32;
+    return 8 * (ol_row_words(n, R, nd, share) + (size_t)nh * H + (vals ? (size_t)E : 0)) +
+           4 * ((size_t)R + 1 + H + R + (share ? 0 : 2 * W)) + 2 * (size_t)E + 16;
+}
+template <bool SHARE>
 __device__ inline OlMem ol_mem(const OlArgs& a, unsigned char* p, int nd, int nh) {
     OlMem m;
     const int W = (a.n + 31) / 32;
     m.row = reinterpret_cast<double*>(p);
-    m.hal = m.row + (size_t)nd * a.R;
+    m.hal = m.row + ol_row_words(a.n, a.R, nd, SHARE);
     m.vals = m.hal + (size_t)nh * a.H;
     m.rps = reinterpret_cast<int*>(m.vals + (a.vals_in ? a.E : 0));
     m.hc = m.rps + a.R + 1;
     m.li = m.hc + a.H;
-    m.bits = reinterpret_cast<unsigned*>(m.li + a.R);
+    m.bits = SHARE ? reinterpret_cast<unsigned*>(m.row) : reinterpret_cast<unsigned*>(m.li + a.R);
     m.pre = reinterpret_cast<int*>(m.bits + W);
-    m.cols = reinterpret_cast<unsigned short*>(m.pre + W);
+    m.cols = SHARE ? reinterpret_cast<unsigned short*>(m.li + a.R) : reinterpret_cast<unsigned short*>(m.pre + W);
     return m;
 }
 
@@ -208,13 +225,13 @@ __device__ inline double ol_dinv(const OlArgs& a, int row) {
 }
 
 // x0 = 0, z = D^-1 r, stop when r.r < tol^2 b.b or after max_iter iterations
-__global__ void __launch_bounds__(OT_CG, 1) k_ol_cg(OlArgs a) {
-    constexpr int OT = OT_CG;
+template <int OT>
+__global__ void __launch_bounds__(OT, OT_CG / OT) k_ol_cg(OlArgs a) {
     extern __shared__ __align__(16) unsigned char ol_smem[];
     __shared__ double s[2], sc;
     __shared__ int ctl;
     GridBarrier gb(a.bar, &a.S->fault, a.bar_start);
-    const OlMem m = ol_mem(a, ol_smem, 6, 1);
+    const OlMem m = ol_mem<OT == OT_CG_HALF>(a, ol_smem, 6, 1);
     double *xs = m.row, *rs = xs + a.R, *qs = rs + a.R, *ds = qs + a.R, *w1 = ds + a.R, *w2 = w1 + a.R, *ph = m.hal;
     const int tid = threadIdx.x;
     const int r0 = a.row0[blockIdx.x], nr = a.row0[blockIdx.x + 1] - r0, e0 = a.rp[r0], ne = a.rp[r0 + nr] - e0;
@@ -287,7 +304,7 @@ __global__ void __launch_bounds__(OT_BI, 1) k_ol_bicgstab(OlArgs a) {
     __shared__ double s[2], sc[2];
     __shared__ int ctl;
     GridBarrier gb(a.bar, &a.S->fault, a.bar_start);
-    const OlMem m = ol_mem(a, ol_smem, 7, 4);
+    const OlMem m = ol_mem<false>(a, ol_smem, 7, 4);
     double *xs = m.row, *rs = xs + a.R, *r0s = rs + a.R, *vs = r0s + a.R, *ts = vs + a.R, *w1 = ts + a.R, *w2 = w1 + a.R;
     double *ph = m.hal, *dh = ph + a.H, *rh = dh + a.H, *yh = rh + a.H;  // p, D^-1, r, and y or z at the CTA's columns
     const int tid = threadIdx.x;
@@ -411,6 +428,14 @@ __global__ void __launch_bounds__(OT_BI, 1) k_ol_bicgstab(OlArgs a) {
     }
 }
 
+// one-launch CG solves in flight, by device
+std::atomic<int> ol_running[64];
+struct OlRunning {
+    std::atomic<int>& n;
+    explicit OlRunning(int device) : n(ol_running[device & 63]) { n += 1; }
+    ~OlRunning() { n -= 1; }
+};
+
 }  // namespace
 
 // FP64 CG (bicg = false) or BiCGSTAB of a system of at most 65,536 equations in
@@ -449,33 +474,55 @@ int solve_onelaunch(isl_ctx* c, bool bicg, double tol, int64_t max_iter, int64_t
     const int nd = bicg ? 7 : 6, nh = bicg ? 4 : 1;
     bool vals = true;
     auto room = [&]() -> int64_t {
-        const size_t used = ol_bytes(n, R, E, 0, nd, nh, vals);
+        const size_t used = ol_bytes(n, R, E, 0, nd, nh, vals, false);
         return used >= OL_SMEM_MAX ? 0 : (int64_t)(OL_SMEM_MAX - used) / (8 * nh + 4);
     };
     const int64_t want = std::min<int64_t>(n, std::max<int64_t>(4 * (int64_t)R, 1024));
     if (room() < want) vals = false;
     const int64_t H = std::min<int64_t>(n, room());
     if (H < std::min<int64_t>(n, R + 64)) return ISL_OK;
+    // beside other solves: with half the shared memory, the values in it or not
+    // (how many columns a CTA touches shows in the launch: one that finds too many
+    // is done again the next way, and the pattern starts there from then on)
+    auto half_columns = [&](bool v) -> int64_t {
+        const size_t used = ol_bytes(n, R, E, 0, nd, nh, v, true);
+        return used >= OL_SMEM_HALF ? 0 : std::min<int64_t>(n, (int64_t)(OL_SMEM_HALF - used) / (8 * nh + 4));
+    };
+    const OlRunning running(c->device);
+    if (c->ol_half_serial != c->pattern_serial) {
+        c->ol_half_serial = c->pattern_serial;
+        c->ol_half = 0;
+    }
+    enum { HALF_VALS = 0, HALF = 1, WHOLE = 2 };
+    int form = bicg || running.n == 1 ? WHOLE : c->ol_half;
     if (c->ol_row0.n != row0.size()) ISL_CHECK_CUDA(c, c->ol_row0.alloc(row0.size()));
     if (!c->ol_scal.p) ISL_CHECK_CUDA(c, c->ol_scal.alloc(1));
     if (c->w64.n < (size_t)6 * n) ISL_CHECK_CUDA(c, c->w64.alloc((size_t)6 * n));
     ISL_CHECK_CUDA(c, c->dsol.alloc(n));
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(c->ol_row0.p, row0.data(), row0.size() * 4, cudaMemcpyHostToDevice, st));
-    ISL_CHECK_CUDA(c, cudaMemsetAsync(c->ol_scal.p, 0, sizeof(OlScal), st));
-    unsigned bar_start = 0;
-    ISL_CHECK_CUDA(c, grid_barrier_start(c, &bar_start));
-    const size_t smem = ol_bytes(n, R, E, (int)H, nd, nh, vals);
     OlArgs a = {n, c->drowptr.p, c->dcolind.p, c->ddiag.p, c->ol_row0.p, c->dval64.p, c->drhs.p, R, E, (int)H, vals ? 1 : 0, c->nnz <= 32 * (int64_t)n ? 2 : 4,
-                c->w64.p, c->w64.p + n, c->w64.p + 2 * (size_t)n, c->dsol.p, c->dpart.p, c->dbar.p, bar_start, c->ol_scal.p, tol,
+                c->w64.p, c->w64.p + n, c->w64.p + 2 * (size_t)n, c->dsol.p, c->dpart.p, c->dbar.p, 0u, c->ol_scal.p, tol,
                 (int)std::min<int64_t>(max_iter, INT32_MAX - 1)};
-    const void* k = bicg ? (const void*)k_ol_bicgstab : (const void*)k_ol_cg;
-    ISL_CHECK_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OL_SMEM_MAX));
-    void* args[] = {&a};
-    ISL_CHECK_CUDA(c, cudaLaunchCooperativeKernel(k, dim3(ncta), dim3(bicg ? OT_BI : OT_CG), args, smem, st));
-    c->launches += 1;
     OlScal h;
-    ISL_CHECK_CUDA(c, cudaMemcpyAsync(&h, c->ol_scal.p, sizeof(h), cudaMemcpyDeviceToHost, st));
-    ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+    for (bool done = false; !done;) {
+        const bool half = form != WHOLE;
+        a.vals_in = form == HALF_VALS || (form == WHOLE && vals);
+        a.H = (int)(half ? half_columns(a.vals_in) : H);
+        if (half && a.H < std::min<int64_t>(n, R + 64)) { c->ol_half = ++form; continue; }
+        const size_t smem = ol_bytes(n, R, E, a.H, nd, nh, a.vals_in, half);
+        const void* k = bicg ? (const void*)k_ol_bicgstab : half ? (const void*)k_ol_cg<OT_CG_HALF> : (const void*)k_ol_cg<OT_CG>;
+        ISL_CHECK_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OL_SMEM_MAX));
+        if (half) ISL_CHECK_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        ISL_CHECK_CUDA(c, grid_barrier_start(c, &a.bar_start));
+        ISL_CHECK_CUDA(c, cudaMemsetAsync(c->ol_scal.p, 0, sizeof(OlScal), st));
+        void* args[] = {&a};
+        ISL_CHECK_CUDA(c, cudaLaunchCooperativeKernel(k, dim3(ncta), dim3(bicg ? OT_BI : half ? OT_CG_HALF : OT_CG), args, smem, st));
+        c->launches += 1;
+        ISL_CHECK_CUDA(c, cudaMemcpyAsync(&h, c->ol_scal.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+        ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
+        done = !half || !h.over;
+        if (!done) c->ol_half = ++form;
+    }
     if (h.fault) ISL_FAIL(c, ISL_ERR_TIMEOUT, "one-launch FP64 solve: a grid barrier timed out");
     if (h.over || (bicg && h.fin > 2)) return ISL_OK;
     if (h.fin == 3) ISL_FAIL(c, ISL_ERR_NAN, "CG breakdown (non-finite reduction)");
