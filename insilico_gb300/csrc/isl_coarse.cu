@@ -533,6 +533,7 @@ struct CzClu {
     const float *dsub, *ainv;
     const CzInst* inst;
     const int* order;        // batch: the instance of every cluster
+    int cta_stride;          // ... and the entries of cta per instance
     int inst_id;             // the instance, where order is null
     OlScal* res;             // batch: results (null: S)
     const int *rp, *ci;      // (block) CSR in list order
@@ -578,7 +579,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     const CzInst in = a.inst[inst];
     const int ndp = in.ndp;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const int* cta = a.cta + (!GRID && a.order ? (size_t)inst * (ncta + 1) : 0);
+    const int* cta = a.cta + (!GRID && a.order ? (size_t)inst * a.cta_stride : 0);
     const int ag0 = cta[rank], ag1 = cta[rank + 1], na = ag1 - ag0;
     const int c0 = (ag0 - in.agg0) * M;                // first coarse unknown of this CTA
     const float* ainv = a.ainv + in.a0 + (size_t)c0 * ndp;
@@ -2067,16 +2068,19 @@ __global__ void k_pz_csr_values(int n, const int* __restrict__ perm, const int* 
 // shared memory of the one-launch solve; *ms, *as: the matrix and the rows of
 // the inverse fit too (in that order)
 constexpr size_t CLU_SMEM_MAX = 224 * 1024;
+constexpr int CLS_ENT = 8192;  // stored entries a CTA of a batch's cluster takes, about
 size_t cluster_need(const CzPlan& z, int rows, int aggs, int ndp, int ent, bool m, bool s) {
     return z.nc == 3 ? clu_smem<3, 6, 8>(rows, aggs, ndp, ent, m, s)
            : z.m == 4 ? clu_smem<1, 4, 8>(rows, aggs, ndp, ent, m, s) : clu_smem<1, 3, 4>(rows, aggs, ndp, ent, m, s);
 }
-size_t cluster_smem(const CzPlan& z, bool* ms, bool* as, bool big = false) {
-    const auto& need = z.smem[big];
+size_t cluster_smem(const CzClass& k, bool* ms, bool* as) {
+    const auto& need = k.smem;
     *ms = need[1][0] <= CLU_SMEM_MAX;
     *as = need[*ms][1] <= CLU_SMEM_MAX;
     return need[*ms][*as];
 }
+
+inline size_t cluster_smem_min(const CzClass& k) { return k.smem[0][0]; }
 
 // columns of the aggregate-ordered sliced-ELL copy (scalar systems), once per pattern
 int build_sell(isl_ctx* c, CzPlan& z) {
@@ -2117,7 +2121,10 @@ int build_sell(isl_ctx* c, CzPlan& z) {
 
 // (block) CSR in t-space for the one-cluster solve, once per pattern
 int build_csr(isl_ctx* c, CzPlan& z) {
-    if (z.csr_built) return ISL_OK;
+    const bool batch = c->ninst > 1 || c->force_batched;
+    if (z.csr_built && z.batch == batch) return ISL_OK;
+    z.csr_built = false;
+    z.batch = batch;
     cudaStream_t st = c->stream;
     const int n = (int)z.nrow;
     const int* ptr = z.nc == 3 ? c->dbptr.p : c->drowptr.p;
@@ -2139,12 +2146,10 @@ int build_csr(isl_ctx* c, CzPlan& z) {
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(rp.data(), z.rp.p, (size_t)(n + 1) * 4, cudaMemcpyDeviceToHost, st));
     ISL_CHECK_CUDA(c, cudaGetLastError());
     ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
-    // per instance: contiguous aggregates per CTA, balanced by stored entries; in
-    // a batch, the instances whose share of a CTA fits its shared memory
+    // per instance: contiguous aggregates per CTA, balanced by stored entries
     const int nw = z.m == 3 ? 4 : 8;
     const size_t nc1 = (size_t)z.ncta + 1;
     z.hcta.assign(nc1 * z.ninst, 0);
-    for (int k = 0; k < 8; ++k) z.smem[k >> 2][(k >> 1) & 1][k & 1] = 0;
     std::vector<int32_t> order, big_cta;
     auto split = [&](CzInst& in, int ncta, int32_t* cta) {
         in.rows = in.aggs = in.ent = 0;
@@ -2166,36 +2171,60 @@ int build_csr(isl_ctx* c, CzPlan& z) {
     };
     // an instance lays its shared memory out for itself: a launch takes what the
     // largest of its instances needs, and none is sized by the shares of two
-    auto admit = [&](const CzInst& in, int big) {
+    auto admit = [&](const CzInst& in, CzClass& cl) {
+        cl.count += 1;
         for (int k = 0; k < 4; ++k) {
-            size_t& need = z.smem[big][k >> 1][k & 1];
+            size_t& need = cl.smem[k >> 1][k & 1];
             need = std::max(need, cluster_need(z, in.rows, in.aggs, in.ndp, in.ent, k >> 1, k & 1));
         }
     };
     z.big.clear();
+    z.cls.clear();
     z.big_ncta = c->sm_count;
+    z.big_cls = {};
+    // In a batch a cluster has as few CTAs as give each at most CLS_ENT entries
+    // (and enough for them to fit), whatever the other instances: a small one
+    // waits for fewer peers, and more run at once.  600 Q1 instances to 1e-10 with 16
+    // CTAs each / so / one-level: side 4 10.4 / 0.76 / 2.1 ms, side 32 29.1 / 3.8 /
+    // 7.7 ms; with half as many entries to a CTA the latter takes 6.4 ms, and 150 P2
+    // meshes of 5^3 cells 3.6 ms instead of 2.2.  (Four of side 32 alone: 0.45 / 0.55 ms.)
+    std::vector<std::vector<int32_t>> by_size;  // by the cluster's CTAs: 1, 2, 4, ... ncta
+    for (int k = 1; k < z.ncta; k *= 2) by_size.push_back({});
+    by_size.push_back({});
     for (int i = 0; i < z.ninst; ++i) {
         CzInst& in = z.hinst[i];
-        if (!split(in, z.ncta, &z.hcta[nc1 * i]) && z.ninst > 1) {
+        int32_t* cta = &z.hcta[nc1 * i];
+        int cl = batch ? 0 : (int)by_size.size() - 1;
+        auto ctas = [&] { return std::min(1 << cl, z.ncta); };
+        while (cl + 1 < (int)by_size.size() && (int64_t)ctas() * CLS_ENT < rp[in.row0 + in.nrow] - rp[in.row0]) ++cl;
+        while (!split(in, ctas(), cta) && cl + 1 < (int)by_size.size()) ++cl;
+        if (cluster_need(z, in.rows, in.aggs, in.ndp, in.ent, false, false) > CLU_SMEM_MAX && z.ninst > 1) {
             std::vector<int32_t> cb((size_t)z.big_ncta + 1);
             if (!split(in, z.big_ncta, cb.data())) continue;  // one-level
             z.big.push_back(i);
             big_cta.insert(big_cta.end(), cb.begin(), cb.end());
-            admit(in, 1);
+            admit(in, z.big_cls);
             continue;
         }
-        order.push_back(i);
-        admit(in, 0);
+        by_size[(size_t)cl].push_back(i);
     }
+    for (int k = (int)by_size.size() - 1; k >= 0; --k) {
+        std::vector<int32_t>& v = by_size[(size_t)k];
+        if (v.empty()) continue;
+        std::stable_sort(v.begin(), v.end(), [&](int32_t a, int32_t b) { return z.hinst[a].nrow > z.hinst[b].nrow; });
+        CzClass cl = {k + 1 == (int)by_size.size() ? z.ncta : 1 << k, (int)order.size(), 0, {}};
+        for (const int32_t i : v) admit(z.hinst[i], cl);
+        order.insert(order.end(), v.begin(), v.end());
+        z.cls.push_back(cl);
+    }
+    if (batch && z.ninst == 1 && cluster_smem_min(z.cls[0]) > CLU_SMEM_MAX) z.cls.clear();
     ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.inst.p, z.hinst.data(), (size_t)z.ninst * sizeof(CzInst), cudaMemcpyHostToDevice, st));
     if (!z.big.empty()) {
         CZ_ALLOC(c, z.cta_big, big_cta.size());
         ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.cta_big.p, big_cta.data(), big_cta.size() * 4, cudaMemcpyHostToDevice, st));
         ISL_CHECK_CUDA(c, cudaStreamSynchronize(st));
     }
-    z.norder = (int)order.size();
-    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return z.hinst[a].nrow > z.hinst[b].nrow; });
-    if (z.ninst > 1 && z.norder) {
+    if (z.ninst > 1 && !order.empty()) {
         CZ_ALLOC(c, z.order, order.size());
         ISL_CHECK_CUDA(c, cudaMemcpyAsync(z.order.p, order.data(), order.size() * 4, cudaMemcpyHostToDevice, st));
     }
@@ -2351,16 +2380,14 @@ int coarse_cluster_fits(const isl_ctx* c, bool grid) {
     bool ms = false, as = false;
     int coop = 0;
     if (grid && (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !coop)) return 0;
-    if (!c->cz.ok || !c->cz.csr_built || cluster_smem(c->cz, &ms, &as) > CLU_SMEM_MAX) return 0;
+    if (!c->cz.ok || !c->cz.csr_built || c->cz.cls.empty() || cluster_smem(c->cz.cls[0], &ms, &as) > CLU_SMEM_MAX) return 0;
     return ms ? 2 : 1;
 }
 
 // (the shared-memory limit of a kernel is the process's: always the same value,
 // as other threads may be launching it too)
 template <int NC, int M, int NW, int LPR, bool MS>
-static cudaError_t launch_clu(const CzPlan& z, int grid, size_t smem, cudaStream_t st, CzClu a) {
-    const CzInst& in = z.hinst[a.inst_id];  // grid: the instance
-    const int ncl = a.order ? z.norder : 1;  // clusters
+static cudaError_t launch_clu(const CzPlan& z, const CzClass& cl, int grid, size_t smem, cudaStream_t st, CzClu a) {
     if (grid) {
         const bool wide = z.hinst[a.inst_id].rows * LPR > 1024;  // more than two rounds of 512 threads in a product
         const void* k = wide ? (const void*)k_cz_cluster<NC, M, NW, LPR, MS, true, 1024>
@@ -2374,13 +2401,13 @@ static cudaError_t launch_clu(const CzPlan& z, int grid, size_t smem, cudaStream
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(z.ncta * ncl);
+    cfg.gridDim = dim3(cl.ncta * cl.count);
     cfg.blockDim = dim3(1024);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = z.ncta;
+    at[0].val.clusterDim.x = cl.ncta;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
@@ -2392,18 +2419,20 @@ static cudaError_t launch_clu(const CzPlan& z, int grid, size_t smem, cudaStream
     return cudaLaunchKernelEx(&cfg, k, a);
 }
 
-cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, float* work, const float* dinv, double* x64, double tol, double drop,
-                                  int max_iter, int big) {
+cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, cudaStream_t st, float* work, const float* dinv, double* x64, double tol, double drop,
+                                  int max_iter, int big, int cls) {
     CzPlan& z = c->cz;
     bool ms, as;
-    const size_t smem = cluster_smem(z, &ms, &as, big >= 0);
+    const CzClass& cl = big >= 0 ? z.big_cls : z.cls[(size_t)cls];
+    const size_t smem = cluster_smem(cl, &ms, &as);
     const int grid = big >= 0 ? z.big_ncta : use_grid ? z.ncta : 0;  // CTAs of the cooperative form
     const size_t na = (size_t)z.nc * z.nrow;
     const bool batch = c->ninst > 1 || c->force_batched;
     CzClu a = {};
     a.lnode = z.lnode.p; a.sofs = z.sofs.p; a.cta = z.cta.p; a.perm = z.perm.p;
     a.dsub = z.dsub.p; a.ainv = z.ainv.p; a.inst = z.inst.p;
-    a.order = z.ninst > 1 && big < 0 ? z.order.p : nullptr;
+    a.order = z.ninst > 1 && big < 0 ? z.order.p + cl.first : nullptr;
+    a.cta_stride = z.ncta + 1;
     a.inst_id = big >= 0 ? z.big[big] : 0;
     if (big >= 0) a.cta = z.cta_big.p + (size_t)big * (z.big_ncta + 1);
     a.res = batch ? z.res.p : nullptr;
@@ -2424,11 +2453,10 @@ cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, float* work, const 
     // lanes per row: by the mean row length; in a batch by the element alone, so
     // that an instance's sums do not depend on the others
     const bool wide = batch ? !(c->dim == 2 && c->fedeg == 1) : (double)z.nent > 12.0 * (double)z.nrow;
-    cudaStream_t st = c->stream;
-    if (z.nc == 3) return ms ? launch_clu<3, 6, 8, 8, true>(z, grid, smem, st, a) : launch_clu<3, 6, 8, 8, false>(z, grid, smem, st, a);
-    if (z.m == 4) return ms ? launch_clu<1, 4, 8, 8, true>(z, grid, smem, st, a) : launch_clu<1, 4, 8, 8, false>(z, grid, smem, st, a);
-    if (wide) return ms ? launch_clu<1, 3, 4, 8, true>(z, grid, smem, st, a) : launch_clu<1, 3, 4, 8, false>(z, grid, smem, st, a);
-    return ms ? launch_clu<1, 3, 4, 4, true>(z, grid, smem, st, a) : launch_clu<1, 3, 4, 4, false>(z, grid, smem, st, a);
+    if (z.nc == 3) return ms ? launch_clu<3, 6, 8, 8, true>(z, cl, grid, smem, st, a) : launch_clu<3, 6, 8, 8, false>(z, cl, grid, smem, st, a);
+    if (z.m == 4) return ms ? launch_clu<1, 4, 8, 8, true>(z, cl, grid, smem, st, a) : launch_clu<1, 4, 8, 8, false>(z, cl, grid, smem, st, a);
+    if (wide) return ms ? launch_clu<1, 3, 4, 8, true>(z, cl, grid, smem, st, a) : launch_clu<1, 3, 4, 8, false>(z, cl, grid, smem, st, a);
+    return ms ? launch_clu<1, 3, 4, 4, true>(z, cl, grid, smem, st, a) : launch_clu<1, 3, 4, 4, false>(z, cl, grid, smem, st, a);
 }
 
 void coarse_args(const isl_ctx* c, CzIter& a) {

@@ -65,11 +65,11 @@ void launch_coarse(const isl_ctx* c, cudaStream_t st, const CzIter& a, int mode)
 // the whole solve in one launch, a thread-block cluster or a cooperative grid
 // of z.ncta CTAs (after coarse_plan with ncta > 0 and coarse_numeric): work
 // holds 3 vectors, the FP64 iterate goes to x64 and the record's fin, iters
-// and residuals to c->dscal; on a batch, every instance of z.order in a cluster
-// of its own, or the instance z.big[big] in a grid, results in z.res
+// and residuals to c->dscal; on a batch, every instance of the class z.cls[cls] in
+// a cluster of its own, or the instance z.big[big] in a grid, results in z.res
 int coarse_cluster_fits(const isl_ctx* c, bool grid);
-cudaError_t launch_coarse_cluster(isl_ctx* c, bool grid, float* work, const float* dinv, double* x64, double tol, double drop,
-                                  int max_iter, int big = -1);
+cudaError_t launch_coarse_cluster(isl_ctx* c, bool grid, cudaStream_t st, float* work, const float* dinv, double* x64, double tol, double drop,
+                                  int max_iter, int big = -1, int cls = 0);
 // scalar product (kind 102, 104, 108: 4, 8 or 12 slots in flight), and its CTAs' runs of slices (once per pattern)
 int coarse_spmv_plan(isl_ctx* c);
 void launch_coarse_spmv(const isl_ctx* c, int kind, cudaStream_t st, const CzSpmv& m);

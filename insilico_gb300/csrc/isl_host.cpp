@@ -594,6 +594,8 @@ int isl_ctx_destroy(isl_ctx* c) {
     for (auto& ev : c->mark) if (ev) cudaEventDestroy(ev);
     if (c->cz_exec) cudaGraphExecDestroy(c->cz_exec);
     for (auto& ev : c->cz_ev) if (ev) cudaEventDestroy(ev);
+    for (auto& ev : c->cz_fork) if (ev) cudaEventDestroy(ev);
+    for (auto& st : c->cz_st) if (st) cudaStreamDestroy(st);
     if (c->hscal) cudaFreeHost(c->hscal);
     cudaStream_t own = c->own_stream ? c->stream : nullptr;
     delete c;  // frees the device buffers (stream-ordered)

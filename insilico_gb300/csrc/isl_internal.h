@@ -133,13 +133,18 @@ struct CzInst {               // one instance (a single system: the only one)
     int rows, aggs, ent;      // one-launch solve: the largest share of a CTA, in rows, aggregates and stored entries
     long long a0, p0;         // first entry of its coarse matrices, of its inversion scratch
 };
+struct CzClass {              // instances (of CzPlan::order) solved in clusters of the same size
+    int ncta, first, count;
+    size_t smem[2][2];        // shared memory of the largest: [matrix on chip] [rows of the inverse too]
+};
 struct CzPlan {
     int ninst = 0;
     std::vector<CzInst> hinst;
     DBuf<CzInst> inst;
     DBuf<int32_t> agg_inst;   // instance of every aggregate
-    DBuf<int32_t> order;      // batch: instances solved in clusters, largest first
-    int norder = 0;
+    DBuf<int32_t> order;      // batch: instances solved in clusters, by class, largest first
+    std::vector<CzClass> cls; // (a single system: one class, also for its grid form)
+    CzClass big_cls = {};     // the instances of `big`
     std::vector<int32_t> big; // batch: instances too large for a cluster, one cooperative grid each
     DBuf<int32_t> cta_big;    // ... and the aggregates of its CTAs
     int big_ncta = 0;
@@ -171,8 +176,8 @@ struct CzPlan {
     // one-cluster solve: (block) CSR in list order, aggregates of every CTA
     bool csr_built = false;
     int64_t csr_serial = -1, nent = 0;
-    int ncta = 0;
-    size_t smem[2][2][2] = {}; // shared memory of the largest instance: [cluster, grid] [matrix on chip] [rows of the inverse too]
+    int ncta = 0;             // CTAs of the largest cluster, or of the grid form
+    bool batch = false;       // distributed as a batch
     DBuf<int32_t> rp, ci, cta;
     DBuf<float> cv;
     std::vector<int32_t> hcta;
@@ -376,6 +381,8 @@ struct isl_ctx {
     cudaGraphExec_t cz_exec = nullptr;   // captured iterations of the two-level solve
     std::vector<uint64_t> cz_key;        // what the capture depends on
     cudaEvent_t cz_ev[2] = {nullptr, nullptr};
+    cudaStream_t cz_st[4] = {};          // batch: the classes of the two-level solve side by side
+    cudaEvent_t cz_fork[5] = {};
     int spmv32_forced = 0;               // FP32 SpMV kind set through ISL_OPT_SPMV32_KIND (0: autotune)
 
     // timing

@@ -35,8 +35,8 @@ constexpr size_t OL_SMEM_MAX = 224 * 1024;
 // CG beside other such solves of this process: half the threads and at most half the
 // shared memory, so that the grids of two solves are resident at once.  The sums
 // and products of a row do not depend on the threads: the same bits.  Eight host
-// threads, Q2 90 x 90 (32k rows): @Q2@ solves a second, @Q2F@ with one grid at a time, 186
-// as graphs of kernels; Q1 100 x 100: @Q1@, @Q1F@ and 558.
+// threads, Q2 90 x 90 (32k rows): 241 solves a second, 150 with one grid at a time, 186
+// as graphs of kernels; Q1 100 x 100: 876, 453 and 558.
 constexpr int OT_CG_HALF = 512;
 constexpr size_t OL_SMEM_HALF = 112 * 1024;
 

@@ -2918,7 +2918,7 @@ static int solve_two_level_cluster(isl_ctx* c, int nc, bool grid, double tol, in
     int rc = coarse_numeric(c, true, d32);
     if (rc != ISL_OK) return rc;
     ISL_CHECK_CUDA(c, cudaMemsetAsync(c->dscal.p, 0, sizeof(CGScal), st));
-    ISL_CHECK_CUDA(c, launch_coarse_cluster(c, grid, V, d32, x64, tol, c->have64 ? c->ru_drop2 : 0.0,
+    ISL_CHECK_CUDA(c, launch_coarse_cluster(c, grid, st, V, d32, x64, tol, c->have64 ? c->ru_drop2 : 0.0,
                                             (int)std::min<int64_t>(max_iter, INT32_MAX - 1)));
     c->launches += 1;
     rc = read_scal(c);
