@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
         else if (trr < S->threshold) S->done = 1;
         else if (trr < S->rrtrig || (S->drop > 0.0 && trr > 1e8 * S->rr_true)) S->done = 3;  // dropped enough, or diverging
         else if (S->iters >= S->max_iter) S->done = 2;
+        else if (S->drop > 0.0 && S->iters - S->last_upd >= S->max_gap) { S->bad = 1; S->done = 1; }
     } else if (MODE == CZ_INIT) {
         S->rhsNorm2 = trr;
         S->rr_true = trr;
@@ -287,6 +288,8 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
         S->rrtrig = a.drop * trr;
         S->drop = a.drop;
         S->max_iter = a.max_iter;
+        S->max_gap = a.max_gap;
+        S->last_upd = 0;
         S->iters = 0;
         S->beta = 0.0;
         S->rst = 0;
@@ -548,7 +551,7 @@ struct CzClu {
     const double* val64;
     CGScal* S;
     double tol, drop;
-    int max_iter, exact64;
+    int max_iter, max_gap, exact64;
     float4* part;            // grid form: the CTAs' sums, four slots
     unsigned* bar;
     int inv_smem;            // the CTA's rows of the inverse are held in shared memory
@@ -716,7 +719,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
     // scalars, held by thread 0 of every CTA (the same values everywhere)
     df rz = {0.f, 0.f}, rz_old = {0.f, 0.f}, rzl = {0.f, 0.f};
     double rr = 0.0, thr = 0.0, trig = 0.0, rr_true = 0.0, rr_last = 0.0, rr_best = 0.0, bn = 0.0;
-    int iters = 0, stall = 0, careful = 0;
+    int iters = 0, last_upd = 0, stall = 0, careful = 0;
     enum { GO = 0, FIN1 = 1, FIN2 = 2, FIN3 = 3, STOP = 4 };
 
     // z = D0^-1 r + P_s D_s^-1 P_s^T r from rs, with rr and rz of this thread; rc written
@@ -889,6 +892,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
                 rz_old = rz;
                 if (!(rr == rr) || !(s1.hi == s1.hi)) k = FIN3;
                 else if (rr < thr || rr < trig || (a.exact64 && rr > 1e8 * rr_true) || iters >= a.max_iter) k = STOP;
+                else if (a.exact64 && iters - last_upd >= a.max_gap) k = FIN3;
             }
             sc_ctl = k;
         }
@@ -935,6 +939,7 @@ __global__ void __launch_bounds__(CLT, 1) k_cz_cluster(CzClu a) {
             if (!alive) return;
             if (tid == 0) {
                 int k = GO;
+                last_upd = iters;
                 if (!(t == t)) k = FIN3;
                 else {
                     const double rec = rr;
@@ -2443,7 +2448,7 @@ cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, cudaStream_t st, fl
     a.b = c->drhs.p; a.x64 = x64;
     a.rowptr = c->drowptr.p; a.colind = c->dcolind.p; a.val64 = c->dval64.p;
     a.S = c->dscal.p;
-    a.tol = tol; a.drop = drop; a.max_iter = max_iter; a.exact64 = c->have64 ? 1 : 0;
+    a.tol = tol; a.drop = drop; a.max_iter = max_iter; a.max_gap = coarse_gap(max_iter); a.exact64 = c->have64 ? 1 : 0;
     a.part = reinterpret_cast<float4*>(c->dpart.p); a.bar = c->dbar.p;
     a.inv_smem = as ? 1 : 0;
     if (grid) {

@@ -27,7 +27,7 @@ struct CzIter {
     CGScal* S;
     double* part;
     double tol, drop;     // init
-    int max_iter;
+    int max_iter, max_gap;
 };
 
 // the FP32 matrix: sliced-ELL 3x3 blocks, scalar sliced ELL, or scalar CSR
@@ -62,6 +62,12 @@ int coarse_results(isl_ctx* c);
 void coarse_args(const isl_ctx* c, CzIter& a);
 // update (or start, or restart) and coarse correction: two launches
 void launch_coarse(const isl_ctx* c, cudaStream_t st, const CzIter& a, int mode);
+// Iterations without a reliable update (a residual ten times smaller) after which
+// a solve of at most max_iter of them is given up: a healthy one takes some
+// hundred, and what FP32 directions cannot bring further ends as the one-level
+// solve does.  30^3 cells, 20 times thinner than wide, which neither solves to
+// 1e-10: 5.0 s with the limit of neq / 4 iterations alone, 4.6 s so, 4.5 s one-level.
+inline int coarse_gap(int max_iter) { return max_iter / 8 > 1000 ? max_iter / 8 : 1000; }
 // the whole solve in one launch, a thread-block cluster or a cooperative grid
 // of z.ncta CTAs (after coarse_plan with ncta > 0 and coarse_numeric): work
 // holds 3 vectors, the FP64 iterate goes to x64 and the record's fin, iters

@@ -110,6 +110,7 @@ struct CGScal {
     double rr_best;           // the smallest so far
     double drop;
     int max_iter;
+    int max_gap, last_upd;  // iterations without a reliable update that end it; the last one's
     int stall;   // reliable updates in a row without progress
     int careful; // the iterated residual has drifted from the true one
     int fin;     // 1 converged, 2 iteration limit, 3 breakdown or stagnation

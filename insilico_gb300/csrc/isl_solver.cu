@@ -2844,6 +2844,7 @@ __global__ void __launch_bounds__(BS) k_rl_residual(int n, const int* __restrict
     S->ticket1 = 0;
     if (S->bad || !(tot == tot)) { S->bad = 1; S->fin = 3; return; }
     S->rr_true = tot;
+    S->last_upd = S->iters;
     if (tot <= S->threshold) { S->fin = 1; return; }
     if (S->iters >= S->max_iter) { S->fin = 2; return; }
     // six updates in a row that did not bring the best residual down by a
@@ -3026,6 +3027,7 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
     a.S = S; a.part = c->dpart.p;
     a.tol = tol; a.drop = exact64 ? c->ru_drop2 : 0.0;
     a.max_iter = (int)std::min<int64_t>(max_iter, INT32_MAX - 1);
+    a.max_gap = coarse_gap(a.max_iter);
     ISL_CHECK_CUDA(c, cudaMemsetAsync(S, 0, 2 * sizeof(CGScal), st));
     ISL_CHECK_CUDA(c, cudaMemsetAsync(x64, 0, n * 8, st));
     launch_coarse(c, st, a, CZ_INIT);
@@ -3036,7 +3038,7 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
     // (the tolerance and the limits travel in the scalar record)
     a.b64 = r64;
     a.tol = a.drop = 0.0;
-    a.max_iter = 0;
+    a.max_iter = a.max_gap = 0;
     auto u = [](const void* p) { return (uint64_t)(uintptr_t)p; };
     std::vector<uint64_t> key = {(uint64_t)nc, (uint64_t)kind, (uint64_t)fused, (uint64_t)exact64, (uint64_t)rows, (uint64_t)n,
                                  (uint64_t)c->cz.nagg, (uint64_t)c->cz.ndp, (uint64_t)c->spmv_lpr64,

@@ -71,3 +71,26 @@ def test_couplings_of_the_soft_half_of_an_instance():
     one, _ = S.batch_stats()
     S.close()
     assert np.all(rel <= 1e-8) and np.all(two < one)
+
+
+def test_a_solve_beyond_fp32_directions_is_given_up_early():
+    """a plate 20 times thinner than wide, 16^3 cells (13,872 equations): neither
+    iteration reaches 1e-10; the two-level one gives up after 1,000 iterations
+    without a reliable update (graphs of 8 iterations, at most 32 kernels each; the
+    last update is at about iteration 200), and the solve ends as the one-level one"""
+    p = W.config("c2", n=16)
+    p.X = p.X * np.array([1.0, 1.0, 0.05])
+    S = W.setup_system(p)
+    S.set_option(A.OPT_PERSISTENT, 0)
+    S.assemble(A.PREC_MIXED)
+    out = {}
+    for two_level in (0, 1):
+        S.set_option(A.OPT_TWO_LEVEL, two_level)
+        S.solve(A.SOLVE_CG_FP32_IR, tol=1e-10, check=False)
+        l0 = S.launch_count()
+        it, rel, st = S.solve(A.SOLVE_CG_FP32_IR, tol=1e-10, check=False)
+        out[two_level] = S.launch_count() - l0, it, rel, st, S.solution()
+    S.close()
+    assert out[0][3] == out[1][3] == A.ISL_ERR_NOT_CONVERGED
+    assert out[0][1:3] == out[1][1:3] and np.array_equal(out[0][4], out[1][4])
+    assert out[1][0] - out[0][0] <= (1500 / 8 + 2) * 32 + 100
