@@ -410,10 +410,10 @@ enum { ISL_OPT_BLOCK_SOLVER = 0, ISL_OPT_BLOCKED = 1, ISL_OPT_NBLOCKS = 2, ISL_O
  * variants the autotune prefers. */
 /* ISL_OPT_TUNE_RUNS (read-only): autotunes of this context that timed their
  * candidates; the others took their choice from the tuning cache.
- * ISL_OPT_ELEM_VARIANT (read-only): the launch shape the element kernel
- * autotune chose (threads per block of the one-thread-per-element kernels,
- * elements per block of the eight-threads-per-element hexahedron kernel);
- * 0 before the first assembly. */
+ * ISL_OPT_ELEM_VARIANT (read-only): the launch shape of the element kernel:
+ * the threads per block that the autotune of the one-thread-per-element kernels
+ * chose, or the elements per block of the eight-threads-per-element hexahedron
+ * kernel, which follow from their number; 0 before the first assembly. */
 /* ISL_OPT_DIRECT_BLOCKS (read-only): 1 when the last assembly formed the
  * matrix blocks directly: ISL_PREC_MIXED small-strain HyperElastic<StVenant>
  * (u = 0, no body force or time-integration terms) on trilinear

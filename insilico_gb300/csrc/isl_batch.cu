@@ -822,11 +822,11 @@ int solve_batched(isl_ctx* c, int method, double tol, int64_t max_iter, int64_t*
     }
     double* W = c->w64.p;
     float* V = c->w32.p;
-    // Two-level solve of every instance in a cluster of its own, as many
-    // clusters at once as the GPU holds (isl_coarse.cu), and of the instances
-    // too large for a cluster one after the other over the whole GPU.  What
+    // Two-level solve of every instance in a cluster of its own, as large as the
+    // instance needs and as many at once as the GPU holds (isl_coarse.cu), and of
+    // the instances too large for one after the other over the whole GPU.  What
     // does not converge there follows in the shared one-level iteration below.
-    // 24 Q2 instances of side 8-96: 49.8 -> 5.1 ms (at most 100 iterations
+    // 24 Q2 instances of side 8-96: 49.8 -> 3.9 ms (at most 100 iterations
     // instead of 804, 61 us each for all).
     std::vector<OlScal> res((size_t)ni);
     int left = ni;

@@ -1,4 +1,5 @@
-// Two-level preconditioner of the mixed CG (single systems).
+// Two-level preconditioner of the mixed CG (single systems and the instances of a
+// batch).
 //
 //   M^-1 = D0^-1 + sum_s P_s D_s^-1 P_s^T + P A_c^-1 P^T
 //
@@ -27,9 +28,9 @@
 // sub-aggregate solve stay inside a warp; one more launch multiplies by the
 // dense inverse (its rows for one aggregate per CTA) and prolongs into z.
 //
-// Determinism: rows of an aggregate are listed in ascending order and summed
-// in that order; the coarse entries between aggregates, which several threads
-// add to, are summed in 64-bit fixed point.
+// Determinism: the rows of a sub-aggregate are listed in a fixed order (ascending,
+// scalar rows by their length first) and summed in it; the coarse entries between
+// aggregates, which several threads add to, are summed in 64-bit fixed point.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -2401,6 +2402,10 @@ static cudaError_t launch_clu(const CzPlan& z, const CzClass& cl, int grid, size
         void* args[] = {&a};
         return e == cudaSuccess ? cudaLaunchCooperativeKernel(k, dim3(grid), dim3(wide ? 1024 : 512), args, smem, st) : e;
     }
+    // (node blocks whose matrix does not fit on chip take a grid)
+    if constexpr (NC == 3 && !MS) {
+        return cudaErrorInvalidConfiguration;
+    } else {
     auto k = k_cz_cluster<NC, M, NW, LPR, MS, false, 1024>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLU_SMEM_MAX);
@@ -2422,6 +2427,7 @@ static cudaError_t launch_clu(const CzPlan& z, const CzClass& cl, int grid, size
     if (e != cudaSuccess) return e;
     if (n < 1) return cudaErrorInvalidConfiguration;
     return cudaLaunchKernelEx(&cfg, k, a);
+    }
 }
 
 cudaError_t launch_coarse_cluster(isl_ctx* c, bool use_grid, cudaStream_t st, float* work, const float* dinv, double* x64, double tol, double drop,
