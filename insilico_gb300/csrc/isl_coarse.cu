@@ -86,10 +86,9 @@ __device__ __forceinline__ void prolong(const float (&c)[M], const float4& y, fl
 // Sums of the (hi, lo) pairs part[i].xy and .zw, i < n, by warp 0 (at most a
 // few hundred partials, one per aggregate): ten loads in flight per lane, one
 // round trip for 320 blocks, and no block barrier.  Valid in warp 0.
-__device__ __forceinline__ void reduce_parts2_df_warp(const float4* part, int n, double& o0, double& o1) {
-    o0 = o1 = 0.0;
+__device__ __forceinline__ void reduce_parts2_df_warp(const float4* part, int n, df& s0, df& s1) {
+    s0 = s1 = {0.f, 0.f};
     if (threadIdx.x >= 32) return;
-    df s0 = {0.f, 0.f}, s1 = {0.f, 0.f};
     for (int base = 0; base < n; base += 320) {
         float4 v[10];
 #pragma unroll
@@ -103,8 +102,8 @@ __device__ __forceinline__ void reduce_parts2_df_warp(const float4* part, int n,
             s1 = df_add_acc(s1, df{v[u].z, v[u].w});
         }
     }
-    o0 = df_value(warp_sum_df(s0));
-    o1 = df_value(warp_sum_df(s1));
+    s0 = warp_sum_df(s0);
+    s1 = warp_sum_df(s1);
 }
 
 // ---------------------------------------------------------------------------
@@ -252,28 +251,34 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_update(CzIter a) {
         for (int k = 0; k < NW * WPS; ++k) s += src[k][threadIdx.x];
         a.rc[(size_t)blockIdx.x * M + threadIdx.x] = s;
     }
-    double trr, trz;
+    double trr;
+    df trz;
     if constexpr (MODE != CZ_UPDATE) {
         const double b1 = block_sum(MODE == CZ_INIT ? bb : rr, sh);
         const double b2 = block_sum(rz, sh);
         if (threadIdx.x == 0) { a.part[2 * blockIdx.x] = b1; a.part[2 * blockIdx.x + 1] = b2; }
         if (!last_block(&S->ticket2)) return;
-        reduce_parts2(a.part, gridDim.x, sh, trr, trz);
+        double t;
+        reduce_parts2(a.part, gridDim.x, sh, trr, t);
+        trz = df_from_double(t);
     } else {
         df b1, b2;
         block_sum_df2(rr, rz, reinterpret_cast<float*>(sh), b1, b2);
         if (threadIdx.x == 0) reinterpret_cast<float4*>(a.part)[blockIdx.x] = make_float4(b1.hi, b1.lo, b2.hi, b2.lo);
         if (!last_block(&S->ticket2)) return;
-        reduce_parts2_df_warp(reinterpret_cast<const float4*>(a.part), gridDim.x, trr, trz);
+        df t;
+        reduce_parts2_df_warp(reinterpret_cast<const float4*>(a.part), gridDim.x, t, trz);
+        trr = df_value(t);
     }
     if (threadIdx.x != 0) return;
     S->rr = trr;
-    S->rzloc = trz;
+    S->rzloc = make_float2(trz.hi, trz.lo);
     S->ticket2 = 0;
     if (MODE == CZ_UPDATE) {
         S->iters += 1;
         S->absOld = S->absNew;
-        if (!(trr == trr) || !(trz == trz)) { S->bad = 1; S->done = 1; }
+        S->rz_old = S->rz_new;
+        if (!(trr == trr) || !(trz.hi == trz.hi)) { S->bad = 1; S->done = 1; }
         else if (trr < S->threshold) S->done = 1;
         else if (trr < S->rrtrig || (S->drop > 0.0 && trr > 1e8 * S->rr_true)) S->done = 3;  // dropped enough, or diverging
         else if (S->iters >= S->max_iter) S->done = 2;
@@ -376,20 +381,22 @@ __global__ void __launch_bounds__(NW * WPS * 32) k_cz_coarse(CzIter a) {
     }
     if (threadIdx.x == 0) reinterpret_cast<float2*>(a.part)[blockIdx.x] = make_float2(rz, 0.f);
     if (!last_block(&S->ticket2)) return;
-    const double tot = reduce_parts_df(reinterpret_cast<const float2*>(a.part), gridDim.x);
+    const df tot = reduce_parts_df_sum(reinterpret_cast<const float2*>(a.part), gridDim.x);
     if (threadIdx.x != 0) return;
     S->ticket2 = 0;
-    const double rzn = S->rzloc + tot;
+    const df rz_new = df_add_acc(df{S->rzloc.x, S->rzloc.y}, tot), rz_old = {S->rz_old.x, S->rz_old.y};
+    const double rzn = df_value(rz_new);
     S->absNew = rzn;
-    if (MODE == CZ_UPDATE) S->beta = df_quotient(df_from_double(rzn), df_from_double(S->absOld));
-    else if (MODE == CZ_INIT) { S->absOld = rzn; S->beta = 0.0; }
+    S->rz_new = make_float2(rz_new.hi, rz_new.lo);
+    if (MODE == CZ_UPDATE) S->beta = df_quotient(rz_new, rz_old);  // (through FP64 the tail takes 0.6 us more)
+    else if (MODE == CZ_INIT) { S->absOld = rzn; S->rz_old = S->rz_new; S->beta = 0.0; }
     else {
         S->beta = S->fresh ? 0.0 : rzn / S->absOld;
         S->done = 0;
         S->rst = 0;
     }
     // not positive: the matrix or the inverse is not definite; the host solves one-level
-    if (!(rzn > 0.0)) { S->bad = 1; S->done = 1; }
+    if (!(rz_new.hi > 0.f)) { S->bad = 1; S->done = 1; }
 }
 
 // q = A p and p.q for scalar rows: sliced ELL in aggregate order.
@@ -1100,7 +1107,7 @@ constexpr float SOFT = 1.f / (1 << 30);
 __device__ inline float fix_scale(float amax_i, float amax_j, float top) {
     if (fminf(amax_i, amax_j) < SOFT * top) return 0.f;
     const int e = ((__float_as_int(amax_i) >> 23) + (__float_as_int(amax_j) >> 23) - 2 * 126 + 1) >> 1;
-    return ldexpf(1.f, min(126, FIX_BITS - e));
+    return __int_as_float((min(126, FIX_BITS - e) + 127) << 23);
 }
 
 // Galerkin blocks: CTA per aggregate, warp per sub-aggregate, lane per row.

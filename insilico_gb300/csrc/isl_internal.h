@@ -105,7 +105,7 @@ struct CGScal {
     int fault;   // persistent CG: a grid barrier timed out
     unsigned int ticket1, ticket2;
     // two-level solve: its reliable updates are decided on the device
-    double rzloc;             // r.z without the coarse term
+    float2 rzloc, rz_new, rz_old;  // r.z without the coarse term, and whole (absNew, absOld), in double-float
     double rr_true, rr_last;  // FP64 residuals of the last two reliable updates
     double rr_best;           // the smallest so far
     double drop;
