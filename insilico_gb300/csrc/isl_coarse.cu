@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(256) k_cz_dir(int n, const float* z, float* p,
 // storing its pair into every peer before the barrier, so that no CTA reads
 // remotely after it.  The FP64 reliable updates run in the same launch.
 // One iteration takes about a third of the three launches of the graph path,
-// whose latency does not shrink with the system, and uses 16 SMs, so that
+// whose latency does not shrink with the system, and uses at most 16 SMs, so that
 // concurrent solves run side by side.
 namespace cgrp = cooperative_groups;
 

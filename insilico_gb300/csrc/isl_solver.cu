@@ -2954,9 +2954,12 @@ static int solve_two_level(isl_ctx* c, int nc, double tol, int64_t max_iter, int
     // cooperative grid with one CTA per SM above (its shared memory holds
     // matrices of up to about 30 MB), up to the sizes where the one-level solve
     // leaves its one-launch kernels.  us per iteration, cluster / grid / three
-    // graph launches: 35k entries 9.5 / 11.3 / 28.7, 150k 9.7 / 12.4 / -,
-    // 190k 15.1 / 12.7 / 33, 1.9M - / 13.3 / 22.5, 6.9M - / 26.3 / 29.3.  A context that shares the GPU
-    // with others (side_by_side) takes the cluster, 16 SMs, or the graph.
+    // graph launches, reliable updates included: 35k entries 9.5 / 11.3 / 28.7, 150k
+    // 9.7 / 12.4 / -, 190k 15.1 / 12.7 / 33, 1.9M - / 13.3 / 22.5, 6.9M - / 26.3 /
+    // 29.3 (the double-float sums since then: 0.2 to 0.7 more in one launch); in FP32
+    // alone 35k 6.8 / - / 18.1, 146k 10.1 / - / 19.6, 187k - / 9.5 / 18.7, 1.9M - /
+    // 11.7 / 20.9, 6.6M - / 24.7 / 25.9.  A context that shares the GPU with others
+    // (side_by_side) takes the cluster, 16 SMs, or the graph.
     const int64_t ent = nc == 3 ? 9 * c->nblk : c->nnz;
     const bool one = c->use_persist == 1;
     if ((one || c->side_by_side) && rows <= (nc == 3 ? PERSIST_MAX_NBR : CLUSTER_MAX_N)) {
