@@ -364,7 +364,8 @@ enum { ISL_OPT_BLOCK_SOLVER = 0, ISL_OPT_BLOCKED = 1, ISL_OPT_NBLOCKS = 2, ISL_O
        ISL_OPT_BARRIER_TEST = 5, ISL_OPT_SPMV32_KIND = 6, ISL_OPT_SCALAR_SLOTS = 7, ISL_OPT_HOST_SETUP = 8,
        ISL_OPT_BICGSTAB_KIND = 9, ISL_OPT_BATCHED_SOLVE = 10, ISL_OPT_DIRECT_BLOCKS = 11, ISL_OPT_TUNE_RUNS = 12,
        ISL_OPT_ELEM_VARIANT = 13, ISL_OPT_FOLD_DIRECTION = 14, ISL_OPT_BLOCK_UPDATE = 15,
-       ISL_OPT_SHORT_COLUMNS = 16, ISL_OPT_RELIABLE_DROP = 17, ISL_OPT_SHARED_GEOMETRY = 18, ISL_OPT_TWO_LEVEL = 19, ISL_OPT_ALLOC_TEST = 20 };
+       ISL_OPT_SHORT_COLUMNS = 16, ISL_OPT_RELIABLE_DROP = 17, ISL_OPT_SHARED_GEOMETRY = 18, ISL_OPT_TWO_LEVEL = 19,
+       ISL_OPT_ALLOC_TEST = 20 };
 /* ISL_OPT_TWO_LEVEL (default 1): the mixed CG of one system (at least 64 node
  * blocks, or 1,280 with ISL_OPT_PERSISTENT 0; at least 2,048 equations where it
  * is not node-blocked) is preconditioned by (block) Jacobi plus a coarse space
